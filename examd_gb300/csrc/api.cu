@@ -120,6 +120,85 @@ int round_block_length(double want, double* out, int* q_out, int* k_out) {
   return EXAMD_OK;
 }
 
+// r at which |F(r)| = 24 eps (2 s^12 - s^6) / r, s = sigma / r, falls to fmax
+// (it falls monotonically from r -> 0 to its zero at 2^(1/6) sigma), squared
+// and widened by 1e-4, which covers the rounding of a pair's r^2 and force.
+double r2_of_force(double eps, double sigma, double fmax) {
+  auto fmag = [&](double rr) {
+    const double s6 = std::pow(sigma / rr, 6.0);
+    return 24.0 * eps * (2.0 * s6 * s6 - s6) / rr;
+  };
+  double lo = 1e-3 * sigma, hi = std::pow(2.0, 1.0 / 6.0) * sigma;
+  if (!(fmag(lo) > fmax)) {
+    hi = lo;
+  } else {
+    for (int it = 0; it < 200; ++it) {
+      const double mid = 0.5 * (lo + hi);
+      (fmag(mid) > fmax ? lo : hi) = mid;
+    }
+  }
+  return hi * hi * (1.0 + 1e-4);
+}
+
+// x >= 0 in units of 2^ue, modulo 2^64; exact for an x of at least 2^(ue + 52).
+long long fixed_of(double x, int ue) {
+  int e = 0;
+  const unsigned long long m = (unsigned long long)std::ldexp(std::frexp(x, &e), 53);
+  const int sh = e - 53 - ue;
+  return (long long)(sh < 0 || sh > 63 ? 0ull : m << sh);
+}
+
+// The tables of the FP64 form's fixed-point pass (pair.cu, force_batch_fix), or
+// false where the parameters do not suit it and the FP64 body computes every
+// tile: type pairs whose force scales eps / sigma differ by more than 16 (the
+// sums have one unit, and the weakest pair's forces keep 2^-45 of its scale), a
+// cutoff inside the range of the forces too large for the sums, or lengths and
+// energies whose powers leave FP64's range.
+bool build_fix(const LJTable& lj, const examd_params& p, FixTable& fx) {
+  const int n2 = lj.nt * lj.nt;
+  double rmax = 0.0, f0max = 0.0, f0min = INFINITY;
+  for (int k = 0; k < n2; ++k) {
+    rmax = std::max(rmax, p.rc[k]);
+    f0max = std::max(f0max, p.eps[k] / p.sigma[k]);
+    f0min = std::min(f0min, p.eps[k] / p.sigma[k]);
+  }
+  if (!(f0min * 16.0 >= f0max) || !std::isnormal(f0max)) return false;
+  int f0 = std::ilogb(f0max);  // F0 = 2^f0
+  if (std::ldexp(1.0, f0) < f0max) ++f0;
+  fx.ue = std::ilogb(rmax) + 1 - 62;  // every separation within the cutoff is below 2^62 units
+  fx.sf = kFixSumBits - f0;
+  const double fbig = std::ldexp(1.0, kFixTermBits + f0);
+  const int w = 2 * fx.ue + 64;  // r^2 = D 2^w
+  double r2big[EXAMD_MAX_TYPES * EXAMD_MAX_TYPES], gmax = 0.0;
+  for (int k = 0; k < n2; ++k) {
+    r2big[k] = std::max(r2_of_force(p.eps[k], p.sigma[k], fbig), 1.001e-12);  // coincident atoms (kR2Min64) as well
+    gmax = std::max(gmax, fbig / std::sqrt(r2big[k]));
+  }
+  if (!std::isnormal(gmax)) return false;
+  const int sg = 61 - std::ilogb(gmax);  // |dg| 2^sg < 2^62
+  const int K = sg - fx.ue - fx.sf;
+  if (K < 33 || K > 63) return false;
+  fx.ka = 64 - K;
+  fx.kb = K - 32;
+  for (int k = 0; k < n2; ++k) {
+    FixPair& q = fx.p[k];
+    const long double s2 = (long double)lj.p64[k].sig2, s6 = s2 * s2 * s2, e = (long double)p.eps[k];
+    q.c6 = (double)std::ldexp(24.0L * e * s6, sg - 4 * w);
+    q.c12 = (double)std::ldexp(48.0L * e * s6 * s6, sg - 7 * w);
+    q.s6 = (double)std::ldexp(s6, -3 * w);
+    q.e4 = lj.p64[k].eps4;
+    q.eshift = lj.p64[k].eshift;
+    const double lim = std::ldexp(lj.p64[k].rcut2, -w), big = std::ldexp(r2big[k], -w);
+    if (!std::isnormal(q.c6) || !std::isnormal(q.c12) || !std::isnormal(q.s6) || !(big >= 0x1p36) ||
+        !(lim >= 0x1p44) || !(lim < 0x1p61) || !(big < lim))
+      return false;
+    q.limh = (int)((long long)lim >> 32);
+    q.bigh = (int)((long long)big >> 32) + 1;
+    q.pre = lj.p32[k].rc2 * 1.0001f;
+  }
+  return true;
+}
+
 // Split of one box axis of nb cells into tiles of at most tile_len cells (an
 // even split: tile_len or tile_len - 1 cells), so that the largest staged
 // tile, which sizes shared memory, stays (tile_len + 2)^3 cells; every tile
@@ -160,9 +239,10 @@ struct examd_ctx {
   int NC = 0, ntiles = 0, ne_max = 0, ext_max = 0;
   double bl = 0.0;
   LJTable lj{};
+  FixTable fx{};
   PairConfig pc;
   int cap = 0, smem = 0, smem_limit = 0;
-  int cap_redo = 0;     // mixed form: staged-atom capacity of the redo pass
+  int cap_redo = 0;     // staged-atom capacity of the redo pass
   int pair_tables = 0;  // examd_params.pair_tables
   int dev = 0;
   cudaStream_t st = nullptr;
@@ -192,7 +272,7 @@ struct examd_ctx {
   double* tileE = nullptr;
   double* tileW = nullptr;
   long long* tileC = nullptr;
-  int* redo = nullptr;  // mixed form: tiles for the redo pass (large pair-force terms)
+  int* redo = nullptr;  // tiles for the redo pass (large pair-force terms)
   int* redo_n = nullptr;  // [0] count, [1] done counter of the redo pass
   double* boxE = nullptr;  // per box (graph chunk: [chunk][nboxes])
   double* boxW = nullptr;
@@ -521,26 +601,7 @@ int examd_gpu_create(const examd_params* params, int nboxes, const examd_box* bo
     lj.p32[k].rcut2 = p.potential == EXAMD_POT_WCA ? (float)rcut2 : INFINITY;
     lj.p32[k].eshift = (float)eshift;
     lj.p32[k].rl2 = (float)((r + skin) * (r + skin));
-    {
-      // |F(r)| = 24 eps (2 s^12 - s^6) / r, s = sigma / r, falls monotonically
-      // from r -> 0 to its zero at 2^(1/6) sigma: bisect for |F| = kFixMaxForce,
-      // then widen by 1e-4 (the FP32 d2 of a pair and the FP32 force differ
-      // from the exact ones by far less)
-      auto fmag = [&](double rr) {
-        const double s6 = std::pow(s / rr, 6.0);
-        return 24.0 * e * (2.0 * s6 * s6 - s6) / rr;
-      };
-      double lo = 1e-3 * s, hi = std::pow(2.0, 1.0 / 6.0) * s;
-      if (!(fmag(lo) > kFixMaxForce)) {
-        hi = lo;
-      } else {
-        for (int it = 0; it < 200; ++it) {
-          const double mid = 0.5 * (lo + hi);
-          (fmag(mid) > kFixMaxForce ? lo : hi) = mid;
-        }
-      }
-      lj.p32[k].r2big = (float)(hi * hi * (1.0 + 1e-4));
-    }
+    lj.p32[k].r2big = (float)r2_of_force(e, s, kFixMaxForce);
     rc2max = std::max(rc2max, lj.p32[k].rc2);
   }
   lj.rc2max = rc2max;
@@ -554,6 +615,8 @@ int examd_gpu_create(const examd_params* params, int nboxes, const examd_box* bo
     lj.mass[a] = m;
     lj.minv[a] = 1.0 / m;
   }
+
+  ctx->pc.fix = ctx->pc.fp64 && build_fix(lj, p, ctx->fx);
 
   // Tiles of a batch: the tile edge T is the densest box's.  A box with fewer
   // atoms per cell gets tiles up to 2 cells longer per axis, as long as its
@@ -600,6 +663,14 @@ int examd_gpu_create(const examd_params* params, int nboxes, const examd_box* bo
       }
       B.nb[a] = (int)q;
     }
+    if (ctx->pc.fix)
+      for (int a = 0; a < 3; ++a) {
+        const int e = std::ilogb(B.L[a]);
+        B.Lq[a] = fixed_of(B.L[a], ctx->fx.ue);
+        B.qbit[a] = e - 52 - ctx->fx.ue;  // >= 10: L is more than twice the cutoff
+        const double over = std::ldexp(B.L[a] - std::ldexp(1.0, e), -ctx->fx.ue);
+        B.qthr[a] = over < 0x1p62 ? (long long)over : (1ll << 62);
+      }
     B.bl = bl;
     B.bli = 1.0 / bl;
     B.blq = blq;
@@ -768,9 +839,9 @@ int examd_gpu_create(const examd_params* params, int nboxes, const examd_box* bo
     ctx->Fown = f;
     ALLOC(f, 7 * N);
     ctx->P = f;
-    ALLOC(ctx->redo, std::max(1, ctx->ntiles));
-    ALLOC(ctx->redo_n, 2);
   }
+  ALLOC(ctx->redo, std::max(1, ctx->ntiles));
+  ALLOC(ctx->redo_n, 2);
   ALLOC(ctx->tileE, ctx->ntiles);
   ALLOC(ctx->tileW, ctx->ntiles);
   ALLOC(ctx->tileC, 3 * (size_t)ctx->ntiles);
@@ -924,9 +995,10 @@ int check_status(examd_ctx* ctx) {
 }
 
 // Staged-atom capacities of a tile from the current binning: +25% + 64
-// headroom for the FP64 form and for the mixed form's redo pass; +6% + 32 for
-// the mixed form's first pass (a tile that outgrows it before the next update
-// is computed in full by the redo pass, at the redo capacity).
+// headroom for the redo pass and for the FP64 form without one (no fixed-point
+// pass); +6% + 32 for a first pass with a redo pass behind it (a tile that
+// outgrows it before the next update is computed in full by the redo pass, at
+// the redo capacity).
 int update_capacity(examd_ctx* ctx, bool* grew = nullptr) {
   if (grew) *grew = false;
   CK(cudaMemsetAsync(ctx->d_occ, 0, 2 * sizeof(int), ctx->st));
@@ -936,7 +1008,7 @@ int update_capacity(examd_ctx* ctx, bool* grew = nullptr) {
   CK(cudaMemcpyAsync(&occ, ctx->d_occ, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaStreamSynchronize(ctx->st));
   int want_r = std::max(((occ + occ / 4 + 64) + 7) & ~7, ctx->cap_redo);
-  int want = ctx->pc.fp64 ? want_r : ((occ + occ / 16 + 32) + 7) & ~7;
+  int want = ctx->pc.fp64 && !ctx->pc.fix ? want_r : ((occ + occ / 16 + 32) + 7) & ~7;
   if (want <= ctx->cap) return EXAMD_OK;
   // mixed form with pair_tables = 0: the compact per-warp tables where they
   // fit more CTAs on an SM at this capacity (or where only they fit at all)
@@ -968,13 +1040,15 @@ int update_capacity(examd_ctx* ctx, bool* grew = nullptr) {
   ctx->cap_redo = want_r;
   ctx->smem = bytes;
   if (grew) *grew = true;
-  // all variants used by this context
+  // all variants used by this context (the attribute is the kernel's, shared
+  // with every other context of the process: the device's limit, so that none
+  // takes away what another needs)
   PairConfig c = ctx->pc;
   for (int e = 0; e < 2; ++e)
     for (int n = 0; n < 2; ++n) {
       c.energy = e;
       c.count = n;
-      CK(pair_prepare(c, bytes));
+      CK(pair_prepare(c, ctx->smem_limit));
     }
   return EXAMD_OK;
 }
@@ -1001,6 +1075,7 @@ PairArgs pair_args(examd_ctx* ctx) {
   a.ne_max = ctx->ne_max;
   a.ext_max = ctx->ext_max;
   a.lj = ctx->lj;
+  a.fx = ctx->fx;
   a.redo = ctx->redo;
   a.redo_n = ctx->redo_n;
   a.redo_done = (unsigned*)(ctx->redo_n + 1);

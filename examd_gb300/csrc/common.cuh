@@ -94,6 +94,11 @@ struct BoxDev {
   int cell0;       // first global cell id of the box
   int tile0;       // first tile of the box
   int nt[3];       // tiles per axis
+  // FP64 form's fixed-point pass, in units of 2^FixTable::ue: L modulo 2^64; the
+  // lowest bit of a double of L's exponent; the separation across the periodic
+  // face beyond which L less it has the next lower exponent
+  long long Lq[3], qthr[3];
+  int qbit[3];
 };
 
 // LJ parameters per ordered type pair, FP32 (mixed) and FP64.
@@ -113,9 +118,32 @@ struct LJ32 {
 // component of a kept term is below 2^28 in fixed point, so a component's
 // int32 sum needs more than 8 near-maximal terms of one sign to overflow.
 constexpr float kFixMaxForce = 2048.f;
+// FP64 form's fixed-point pass: the force sums' unit is 2^-49 of the power of
+// two F0 at or above the largest eps / sigma, the largest kept term 2^11 F0, so
+// that a sum overflows 64 bits only by more than 8 near-maximal terms of one sign
+// (as above; 2^-49 F0 is about 1e-17 of a liquid's rms force)
+constexpr int kFixSumBits = 49, kFixTermBits = 11;
 struct LJ64 {
   double sig2, eps24, eps4, rc2;   // as user_func.f90:58-59 computes them
   double rcut2, eshift;
+};
+
+// FP64 form, fixed-point first pass: one ordered type pair.  D is the squared
+// distance in units of 2^(2 ue + 64) (an int64), y = 1 / D; the pair's force
+// per unit distance, scaled to an integer, is y^4 (c6 - c12 y^3).
+struct FixPair {
+  double c6, c12;
+  double e4, s6;    // energy: 4 eps, and sigma^6 in units of D^3
+  double eshift;
+  int limh, bigh;   // high words of D at the range (rc or the potential's own) and at the largest kept force
+  float pre;        // FP32 prefilter of the candidates: rc^2 widened
+};
+
+struct FixTable {
+  int ue;           // the positions' unit is 2^ue
+  int ka, kb;       // a force term's 128-bit product is taken at bit 64 - ka = 32 + kb
+  int sf;           // the force sums' unit is 2^-sf
+  FixPair p[EXAMD_MAX_TYPES * EXAMD_MAX_TYPES];
 };
 
 struct LJTable {
@@ -266,6 +294,18 @@ __device__ __forceinline__ int cell_offset(double x, const BoxDev& B, int a, flo
   }
   u = d2f_rn_nonneg(x - mul_pow2((unsigned)(c * B.blq), B.blk));
   return c;
+}
+
+// A coordinate x >= 0 in units of 2^ue, rounded to the nearest integer, modulo
+// 2^64 (differences of nearby coordinates are then exact in 64 bits).
+__device__ __forceinline__ unsigned long long to_fixed(double x, int ue) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const int e = (int)(b >> 52) & 0x7ff;
+  if (e == 0) return 0ull;  // zero (either sign) and subnormals
+  const unsigned long long m = (b & 0xfffffffffffffull) | 0x10000000000000ull;
+  const int sh = e - 1075 - ue;
+  if (sh >= 0) return sh < 64 ? m << sh : 0ull;
+  return sh > -55 ? ((m >> (-sh - 1)) + 1ull) >> 1 : 0ull;
 }
 
 // Global cell of a position inside its box (the offsets are not needed).

@@ -56,13 +56,15 @@ struct PairArgs {
   double* tileW;     // per tile virial
   long long* tileC;  // per tile (candidates, accepted)
   int* status;
-  int cap;     // staged-atom capacity of a tile (mixed form: of the first pass)
-  int cap_redo;  // mixed form: capacity of the redo pass
+  int cap;     // staged-atom capacity of a tile in the first pass
+  int cap_redo;  // capacity of the redo pass (the FP64 form without the fixed-point pass has none)
   int ne_max;  // largest ext-cell count of a tile
   int ext_max;  // largest ext extent of a tile on one axis
   LJTable lj;
-  // mixed form: tiles whose pair-force terms exceeded the fixed-point range,
-  // for the redo pass (ntiles entries; count and done counter zero between launches)
+  FixTable fx;   // FP64 form's fixed-point pass
+  // tiles whose pair-force terms exceeded the fixed-point range or that outgrew
+  // the first pass's capacity, for the redo pass (ntiles entries; count and
+  // done counter zero between launches)
   int* redo;
   int* redo_n;
   unsigned* redo_done;
@@ -95,6 +97,7 @@ struct PairArgs {
 
 struct PairConfig {
   bool fp64 = false;
+  bool fix = false;     // FP64 form: fixed-point first pass (the FP64 pass then only redoes listed tiles)
   bool multi = false;   // more than one atom type
   bool pack = false;    // mixed form: compact per-warp tables (more CTAs per SM)
   bool energy = false;  // potential energy and virial

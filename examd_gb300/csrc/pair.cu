@@ -88,7 +88,9 @@ constexpr int kRedoBlocks = 152;       // grid of the redo pass (1 per SM)
 // mode: the list build (the first pass's enumeration at the list cutoff,
 // writing the tile's pairs instead of their forces), the forces from the
 // list, and the redo of a listed tile's large terms.
-constexpr int kMain = 0, kRedoBig = 1, kRedoFull = 2, kListBuild = 3, kList = 4, kListBig = 5;
+// kFixed: the FP64 form's first pass in fixed point (enumerated as the mixed
+// form's first pass; its listed tiles are redone by the FP64 form's own body).
+constexpr int kMain = 0, kRedoBig = 1, kRedoFull = 2, kListBuild = 3, kList = 4, kListBig = 5, kFixed = 6;
 constexpr int kFullBit = 1 << 30;      // redo-list entry: tile | kFullBit for an overflowed tile
 constexpr int kSeg = 4;                // lanes per segment of the i-side force sums
 constexpr int kMaxListK = 1024;        // pair-list mode: most list entries of one atom
@@ -138,21 +140,22 @@ __host__ __device__ inline Layout make_layout(bool fp64, int cap, int ne_max, in
   L.oz = o;     o = align16(o + 4 * (ext_max + 1));
   L.dyt = o;    o = align16(o + 8 * ext_max * kDT);  // float2 (row origin offset, near face) per (l, d)
   L.dzt = o;    o = align16(o + 8 * ext_max * kDT);
-  L.img = o;    o = align16(o + (fp64 ? 3 * 32 : 0));  // periodic image per ext coordinate (FP64 form)
+  const bool fix = mode == kFixed;
+  L.img = o;    o = align16(o + (fp64 || fix ? 3 * 32 : 0));  // periodic image per ext coordinate (FP64 form)
   L.cw = o;     o = align16(o + 16);  // unit counter, large-term flag, staged-atom total
   L.r2l = o;    o = align16(o + (fp64 ? 64 * nw : 0));  // rank -> lane tables (FP64 form)
   L.lut = o;    o = align16(o + (from_list ? 0 : (int)sizeof(OwnLut)));
   // the LJ table per ordered type pair (several types): per-lane type indices
   // would serialise on the kernel-parameter bank, shared memory serves them at once
-  L.ljt = o;    o = align16(o + (int)sizeof(LJ64) * EXAMD_MAX_TYPES * EXAMD_MAX_TYPES);
+  L.ljt = o;    o = align16(o + (fix ? (int)sizeof(FixPair) : (int)sizeof(LJ64)) * EXAMD_MAX_TYPES * EXAMD_MAX_TYPES);
   const int tab = pack ? kWarpTabCompact : kWarpTabWide;
   const int qbytes = (fp64 ? 4 * kQueue + kWarpTabFp64
-                           : (from_list ? 64 : (mode == kListBuild ? 0 : 16) * kQueue + tab)) * nw;
+                           : (from_list ? 64 : (mode == kListBuild ? 0 : fix ? 4 : 16) * kQueue + tab)) * nw;
   L.queue = o;  o = align16(o + qbytes);
   L.pf = o;     o = align16(o + 16 * (from_list ? cap + 1 : cap));  // list passes: + the padding atom
-  if (fp64) {
-    L.fa = o;   o = align16(o + 3 * 8 * cap);  // FP64 force sums
-    L.px = o;   o = align16(o + 3 * 8 * cap);  // FP64 positions
+  if (fp64 || fix) {
+    L.fa = o;   o = align16(o + 3 * 8 * cap);  // FP64 force sums (kFixed: low words, then high words)
+    L.px = o;   o = align16(o + 3 * 8 * cap);  // FP64 (kFixed: fixed-point) positions
   } else {
     L.fa = o;   o = align16(o + (mode == kListBuild ? 1 : 3) * 4 * cap);  // fixed-point force sums (build: counts)
     L.px = o;
@@ -178,6 +181,7 @@ __host__ __device__ inline Layout make_layout(bool fp64, int cap, int ne_max, in
 }
 
 static int redo_smem_bytes(const PairConfig& cfg, int cap_redo, int ne_max, int ext_max) {
+  if (cfg.fix) return make_layout(true, cap_redo, ne_max, ext_max, cfg.warps, kRedoFull, false).bytes;
   const int b = std::max(make_layout(false, cap_redo, ne_max, ext_max, cfg.warps, kRedoBig, cfg.pack).bytes,
                          make_layout(false, cap_redo, ne_max, ext_max, cfg.warps, kRedoFull, cfg.pack).bytes);
   return cfg.list ? std::max(b, make_layout(false, cap_redo, ne_max, ext_max, cfg.warps, kListBig, cfg.pack).bytes)
@@ -188,6 +192,7 @@ static int redo_smem_bytes(const PairConfig& cfg, int cap_redo, int ne_max, int 
 // counters, which the enumeration gives) the list pass's.
 static int main_smem_bytes(const PairConfig& cfg, int cap, int ne_max, int ext_max) {
   const int mode = (cfg.list && !cfg.count && !cfg.fp64) ? kList : kMain;
+  if (cfg.fix) return make_layout(false, cap, ne_max, ext_max, cfg.warps, kFixed, true).bytes;
   return make_layout(cfg.fp64, cap, ne_max, ext_max, cfg.warps, mode, cfg.pack).bytes;
 }
 
@@ -196,6 +201,7 @@ static int build_smem_bytes(const PairConfig& cfg, int cap, int ne_max, int ext_
 }
 
 int pair_smem_bytes(const PairConfig& cfg, int cap, int cap_redo, int ne_max, int ext_max) {
+  if (cfg.fix) return std::max(main_smem_bytes(cfg, cap, ne_max, ext_max), redo_smem_bytes(cfg, cap_redo, ne_max, ext_max));
   int b = make_layout(cfg.fp64, cap, ne_max, ext_max, cfg.warps, kMain, cfg.pack).bytes;
   if (cfg.fp64) return b;
   b = std::max(b, redo_smem_bytes(cfg, cap_redo, ne_max, ext_max));
@@ -379,6 +385,149 @@ __device__ __forceinline__ void force_batch64(int cnt, const QK& qk, const PD& p
   }
 }
 
+// FP64 form, fixed-point first pass: the forces of cnt queued pairs that
+// passed the FP32 prefilter, one per lane (key as in force_batch).
+//
+// GB300 runs FP64 arithmetic at 1/64 of the FP32 rate (1.6-2.0 per clock per
+// SM), a correctly rounded FP64 reciprocal at the price of about six
+// operations, and FP64 shared-memory atomics as compare-and-swap loops that
+// add on the same pipe.  With the reference's operations and six such atomics
+// a pair cost 35 FP64 operations and more, and the pass was bound by that
+// pipe (79 % busy, issue 17 %).  Here the pair keeps eight:
+// - positions are integers in units of 2^ue (L < 2^62 of them modulo 2^64,
+//   rc < 2^62), so the separation is exact, and D = r^2 / 2^64 to one unit in
+//   2^57 or better by 32-bit multiplies (the lowest product, below one unit
+//   of D, is left out);
+// - D becomes a double (one rounding), y = 1/D from an FP32 estimate (relative
+//   error e of 2^-22) by one step of Householder's third-order iteration,
+//   y (1 + e + e^2), error e^3: three operations;
+// - the LJ force per unit distance is y^4 (c6 - c12 y^3), five operations;
+//   as an integer it multiplies the separation in 32-bit pieces, rounded at
+//   bit 2^-sf of the sum's unit;
+// - the sums are 64-bit integers in shared memory (low word with carry into
+//   the high word): exact, in any order, with native 32-bit atomics.
+// Every step keeps at least FP64's bits, and the forces do not depend on the
+// order.  Where the reference itself rounds coarsely, its rounding is kept: a
+// pair across the periodic face is first subtracted at box scale (x_j - x_i,
+// rounded to 53 bits of about L, then L added exactly), which moves its
+// separation by up to ulp(L) / 2; `face` gives that rounded separation.
+// A pair within a unit of D's high word (a few 1e-9) of its range is decided on
+// the FP64 body's own r^2 (in64), so that both accept the same pairs; a pair
+// whose force is too large for the sums' range flags the tile, and the FP64
+// body redoes it.
+template <bool MULTI, bool ENERGY, bool COUNT, class QK, class PX, class FA, class FACE, class IN64>
+__device__ __forceinline__ void force_batch_fix(int cnt, int qh, const QK& qk, const PX& px, FA& fa, int cap,
+                                                const PairArgs& A, const FixPair* ljx, double& s12, double& s6s,
+                                                double& shift, int& nacc, int* big_flag, bool edge, const FACE& face,
+                                                const IN64& in64) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  int i = -1, m = 0;
+  long long fx = 0, fy = 0, fz = 0;  // the force on i, in units of 2^-sf
+  bool app = false;
+  if (lane < cnt) {
+    const unsigned key = (unsigned)qk[(qh + lane) & (kQueue - 1)];
+    i = key & 0x3fff;
+    m = (key >> 14) & 0x3fff;
+    const int ti = MULTI ? (key >> 28) & 3 : 0, tj = MULTI ? key >> 30 : 0;
+    const FixPair P = MULTI ? ljx[ti * A.lj.nt + tj] : A.fx.p[0];
+    long long dx = (long long)(px[m] - px[i]);
+    long long dy = (long long)(px[cap + m] - px[cap + i]);
+    long long dz = (long long)(px[2 * cap + m] - px[2 * cap + i]);
+    if (edge) face(i, m, dx, dy, dz);  // the tile holds periodic copies
+    // d = h 2^32 + l with signed l: r^2 / 2^64 = sum h^2 + 2^-31 sum h l + (sum l^2 / 2^64, below one)
+    const int hx = (int)((dx + 0x80000000ll) >> 32), lx = (int)dx;
+    const int hy = (int)((dy + 0x80000000ll) >> 32), ly = (int)dy;
+    const int hz = (int)((dz + 0x80000000ll) >> 32), lz = (int)dz;
+    const long long D = (long long)hx * hx + (long long)hy * hy + (long long)hz * hz +
+                        (((long long)hx * lx + (long long)hy * ly + (long long)hz * lz) >> 31);
+    const int Dh = (int)(D >> 32);
+    app = Dh < P.limh;
+    if (abs(Dh - P.limh) <= 1) app = in64(i, m, ti, tj);
+    if (app && Dh < P.bigh) {
+      *big_flag = 1;
+      app = false;
+    }
+    if (app) {
+      // D as a double: normalised so that its first bit is bit 62, 53 bits kept
+      const int s = __clz(Dh) - 1;
+      const unsigned long long N = ((unsigned long long)D << s) + 512ull;  // (a carry moves into the exponent)
+      const double Dd = __longlong_as_double((long long)((N >> 10) + ((unsigned long long)(1084 - s) << 52)));
+      // 1/D: the reciprocal of the mantissa in FP32, its exponent put back
+      const float mf = __uint_as_float(((unsigned)(N >> 32) >> 7) + 0x3f000000u);
+      const unsigned rb = __float_as_uint(rcp_approx(mf));
+      const double y0 = __hiloint2double((int)((rb >> 3) + ((unsigned)(834 + s) << 20)), (int)(rb << 29));
+      double e = fma(-Dd, y0, 1.0);
+      e = fma(e, e, e);
+      const double y = fma(y0, e, y0);
+      const double y2 = y * y;
+      const double y3 = y2 * y;
+      const double g = (y2 * y2) * fma(-P.c12, y3, P.c6);
+      if (ENERGY) {
+        const double q6 = P.s6 * y3, e6 = P.e4 * q6;
+        s12 = fma(e6, q6, s12);
+        s6s += e6;
+        if (A.lj.pot != EXAMD_POT_LJ) shift += P.eshift;
+      }
+      if (COUNT) ++nacc;
+      // g as a 63-bit integer (|g| < 2^62), then G d / 2^(64 - ka), rounded
+      const int gb = __double2hiint(g);
+      const unsigned long long gm =
+          ((((unsigned long long)(unsigned)((gb & 0xfffff) | 0x100000)) << 32) | (unsigned)__double2loint(g)) << 10;
+      const int gs = min(1085 - ((gb >> 20) & 0x7ff), 63);
+      long long G = (long long)(gm >> gs);
+      if (gb < 0) G = -G;
+      const int gh = (int)((G + 0x80000000ll) >> 32), gl = (int)G;
+      const int ka = A.fx.ka, kb = A.fx.kb;
+      const int half = 1 << (kb - 1);
+      auto term = [&](int h, int l) {
+        const long long hi = (long long)gh * h;
+        const long long mid = (long long)gh * l + ((long long)gl * h + ((long long)__mulhi(gl, l) + half));
+        const unsigned h0 = (unsigned)hi, h1 = (unsigned)((unsigned long long)hi >> 32);
+        const unsigned m0 = (unsigned)mid, m1 = (unsigned)((unsigned long long)mid >> 32);
+        const unsigned long long a = ((unsigned long long)__funnelshift_l(h0, h1, ka) << 32) | (h0 << ka);
+        const unsigned long long b =
+            ((unsigned long long)(unsigned)((int)m1 >> kb) << 32) | __funnelshift_r(m0, m1, kb);
+        return (long long)(a + b);
+      };
+      fx = term(hx, lx);
+      fy = term(hy, ly);
+      fz = term(hz, lz);
+    }
+  }
+  // v to the 64-bit sum of component c of atom t: low word, carry, high word
+  auto add = [&](int t, int c, long long v) {
+    const unsigned lo = (unsigned)v;
+    const unsigned old = atomicAdd((unsigned*)&fa[c * cap + t], lo);
+    atomicAdd(&fa[(3 + c) * cap + t], (int)(v >> 32) + (old + lo < lo ? 1 : 0));
+  };
+  if (app) {
+    add(m, 0, -fx);
+    add(m, 1, -fy);
+    add(m, 2, -fz);
+  }
+  // i side: runs of equal i in segments of kSeg lanes, as in pair_force32
+  const int ip = __shfl_up_sync(FULL, i, 1);
+  const unsigned hb = __ballot_sync(FULL, lane == 0 || ip != i);
+  const int dist = (lane - (31 - __clz(hb & (FULL >> (31 - lane))))) & (kSeg - 1);
+#pragma unroll
+  for (int o = 1; o < kSeg; o <<= 1) {
+    const long long yx = __shfl_up_sync(FULL, fx, o), yy = __shfl_up_sync(FULL, fy, o),
+                    yz = __shfl_up_sync(FULL, fz, o);
+    if (o <= dist) {
+      fx += yx;
+      fy += yy;
+      fz += yz;
+    }
+  }
+  const bool tail = lane == 31 || dist == kSeg - 1 || ((hb >> (lane + 1)) & 1u);
+  if (i >= 0 && tail && (fx | fy | fz) != 0) {
+    add(i, 0, fx);
+    add(i, 1, fy);
+    add(i, 2, fz);
+  }
+}
+
 // One tile.  MODE (mixed form; the FP64 form has only kMain):
 // - kMain: the first pass, at capacity A.cap; a tile with more staged atoms
 //   is listed for a full redo, one with a large term for a large-term redo;
@@ -410,7 +559,8 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   const int NE = EX * EY * EZ;
   constexpr bool kFromList = MODE == kList || MODE == kListBig;
   if (kFromList && MODE == kList && A.lcount[tile] < 0) return;  // a fallback tile: the redo pass computes it
-  const int cap = (MODE == kMain || MODE == kListBuild || MODE == kList) ? A.cap : A.cap_redo;
+  constexpr bool FIX = MODE == kFixed;
+  const int cap = (MODE == kMain || MODE == kListBuild || MODE == kList || FIX) ? A.cap : A.cap_redo;
   const Layout L = make_layout(FP64, cap, A.ne_max, A.ext_max, nw, MODE, PACK);
   // shared-memory arrays (index-checked in the checked build)
   int* const st = A.status;  // the index checks' status word (checked build)
@@ -422,13 +572,14 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   auto oz = EXAMD_ARR(float, smem + L.oz, A.ext_max + 1, st);
   auto dyt = EXAMD_ARR(float2, smem + L.dyt, A.ext_max * kDT, st);
   auto dzt = EXAMD_ARR(float2, smem + L.dzt, A.ext_max * kDT, st);
-  auto img = EXAMD_ARR(signed char, smem + L.img, FP64 ? 96 : 1, st);
+  auto img = EXAMD_ARR(signed char, smem + L.img, FP64 || FIX ? 96 : 1, st);
   double* red = (double*)(smem + L.queue);  // scan and reduction scratch, before and after the queues' use
   int* cw = (int*)(smem + L.cw);
   OwnLut* sown = (OwnLut*)(smem + L.lut);
   const signed char* srows = &sown->rows[0][0];
   LJ32* ljs32 = (LJ32*)(smem + L.ljt);
   LJ64* ljs64 = (LJ64*)(smem + L.ljt);
+  FixPair* ljx = (FixPair*)(smem + L.ljt);
   auto pf = EXAMD_ARR(float4, smem + L.pf, kFromList ? cap + 1 : cap, st);
   auto code = EXAMD_ARR(unsigned short, smem + L.code, cap, st);
   auto U = EXAMD_ARR(const float4, A.U, A.N, st);
@@ -455,7 +606,9 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
       for (int k = tid; k < (int)(sizeof(OwnLut) / 16); k += blockDim.x) dst[k] = src[k];
     if (MULTI)
       for (int k = tid; k < A.lj.nt * A.lj.nt; k += blockDim.x) {
-        if (FP64)
+        if (FIX)
+          ljx[k] = A.fx.p[k];
+        else if (FP64)
           ljs64[k] = A.lj.p64[k];
         else
           ljs32[k] = A.lj.p32[k];
@@ -485,7 +638,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         const int n = nimg(l);
         (a == 0 ? ox : (a == 1 ? oy : oz))[l] = fmaf((float)(2 * (l - 1) - t), 0.5f * blf, (float)n * rf);
         if (l < E) {
-          if (FP64) img[32 * a + l] = (signed char)n;
+          if (FP64 || FIX) img[32 * a + l] = (signed char)n;
           if (a > 0) {
             auto dt = a == 1 ? dyt : dzt;
 #pragma unroll
@@ -548,7 +701,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
     }
     return;
   }
-  if (!FP64 && MODE == kMain && total > cap) {  // the redo pass computes it at its capacity
+  if ((FIX || (!FP64 && MODE == kMain)) && total > cap) {  // the redo pass computes it at its capacity
     if (tid == 0) A.redo[atomicAdd(A.redo_n, 1)] = tile | kFullBit;
     return;
   }
@@ -568,10 +721,11 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
     return;
   }
   // (3) stage atoms, one thread per ext cell
-  auto fa = EXAMD_ARR(int, smem + L.fa, (MODE == kListBuild ? 1 : 3) * cap, st);
+  auto fa = EXAMD_ARR(int, smem + L.fa, (MODE == kListBuild ? 1 : FIX ? 6 : 3) * cap, st);
   auto fr = EXAMD_ARR(float, smem + L.fr, 3 * cap, st);  // redo pass: FP32 sums of the large terms
   auto fd = EXAMD_ARR(double, smem + L.fa, 3 * cap, st);
   auto pd = EXAMD_ARR(double, smem + L.px, 3 * cap, st);
+  auto px = EXAMD_ARR(unsigned long long, smem + L.px, 3 * cap, st);  // kFixed: fixed-point positions, images applied
   for (int e = tid; e < NE; e += blockDim.x) {
     const int lx = e % EX, rr = e / EX, ly = rr % EY, lz = rr / EY;
     const int a0 = lstart[e], a1 = lstart[e + 1], g0 = gfirst[e];
@@ -591,6 +745,14 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         // reads both atoms' rows from them)
         pf[t] = make_float4(ox[lx] + u.x, u.y, u.z,
                             kFromList ? __int_as_float((__float_as_int(u.w) & 3) | ((int)cc << 2)) : u.w);
+        if (FIX) {
+          const int64_t gg = EXAMD_IDX(g, A.N, st);
+          px[t] = to_fixed(A.X0[gg], A.fx.ue) + (unsigned long long)(img[lx] * B.Lq[0]);
+          px[cap + t] = to_fixed(A.X1[gg], A.fx.ue) + (unsigned long long)(img[32 + ly] * B.Lq[1]);
+          px[2 * cap + t] = to_fixed(A.X2[gg], A.fx.ue) + (unsigned long long)(img[64 + lz] * B.Lq[2]);
+#pragma unroll
+          for (int c = 0; c < 6; ++c) fa[c * cap + t] = 0;
+        }
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           if (MODE == kRedoBig || MODE == kRedoFull || MODE == kListBig) fr[c * cap + t] = 0.f;
@@ -614,13 +776,14 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
 
   const LJ32 q32 = A.lj.p32[0];
   const float rcpre = A.lj.rc2max * 1.0001f + 1e-4f;  // FP32 prefilter of the FP64 form
-  double esum = 0.0, wsum = 0.0;  // FP64 form
+  double esum = 0.0, wsum = 0.0;  // FP64 form (kFixed: the sums of 4 eps s^12 and 4 eps s^6)
+  double shsum = 0.0;             // kFixed: the sum of the energy shifts
   FixSum ek, wk;                  // mixed form: exact fixed-point sums of FP32 terms
   int ncand = 0, neval = 0, nacc = 0;
   // per-warp queue of accepted pairs (mixed form: the separation and the key
   // in one 16-byte entry, r^2 recomputed from it; FP64 form: the key only)
   // bytes per queue entry (the list build writes its pairs to the lists directly)
-  constexpr int kQe = FP64 ? 4 : (MODE == kListBuild ? 0 : 16);
+  constexpr int kQe = FP64 || FIX ? 4 : (MODE == kListBuild ? 0 : 16);
   auto qd = EXAMD_ARR(float4, (float4*)(smem + L.queue) + warp * kQueue, kQueue, st);
   auto qk = EXAMD_ARR(int, (int*)(smem + L.queue) + warp * kQueue, kQueue, st);
   // per-warp tables (kWarpTab*): one step's items (ptA, ptB) and, mixed
@@ -651,30 +814,6 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
     if (k < A.lk)
       A.lraw[EXAMD_IDX((ltile + i) * A.lk + k, (size_t)A.ntiles * A.lslots * A.lk, st)] = (unsigned short)m;
   };
-  auto enqueue = [&](bool acc, const float4& dq, int key) {
-    const unsigned bal = __ballot_sync(FULL, acc);
-    if (acc) {
-      const int p = (qh + qn + __popc(bal & lt)) & (kQueue - 1);
-      if (FP64)
-        qk[p] = key;
-      else
-        qd[p] = make_float4(dq.x, dq.y, dq.z, __int_as_float(key));
-    }
-    qn += __popc(bal);
-    if (qn >= 32) {  // a batch only moves the ring's head
-      __syncwarp();
-      if (FP64)
-        force_batch64<MULTI, ENERGY, COUNT>(32, qk, pd, code, img, B.L, fd, cap, A.lj, ljs64, esum, wsum, A.status,
-                                            nacc, qh);
-      else
-        force_batch<MULTI, ENERGY, COUNT, MODE == kRedoFull>(32, qh, qd, fa, fr, cap, A, ljs32, ek, wk, nacc,
-                                                             big_flag);
-      __syncwarp();
-      qh = (qh + 32) & (kQueue - 1);
-      qn -= 32;
-    }
-  };
-
   // ---- mixed form: the FP64 cutoff test of a pair of staged atoms (a, b)
   // at the border, r^2 from the FP64 positions as the FP64 form and the
   // reference form it: the difference, then the periodic image (the pair is
@@ -694,7 +833,56 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
       d = __dsub_rn(d, __dmul_rn(rint(__dmul_rn(d, B.Li[ax])), B.L[ax]));
       d2 = ax == 0 ? __dmul_rn(d, d) : __dadd_rn(d2, __dmul_rn(d, d));
     }
-    return d2 <= A.lj.p64[ta * A.lj.nt + tb].rc2;
+    const LJ64& Q = A.lj.p64[ta * A.lj.nt + tb];
+    return d2 <= (FIX ? Q.rcut2 : Q.rc2);  // (kFixed: the potential's own range, as pair_fn64 decides it)
+  };
+
+  // kFixed: the separation of a pair whose copies lie in different periodic
+  // images, d = t + n L with t = x_j - x_i: t rounded to 53 bits, ties to even,
+  // as the FP64 subtraction rounds it (|t| = L - |d| has L's exponent, or the
+  // next lower one where |d| is above qthr; L is a multiple of that bit)
+  const bool edge = FIX && (X0 == 0 || Y0 == 0 || Z0 == 0 || X0 + tx >= B.nb[0] || Y0 + ty >= B.nb[1] ||
+                            Z0 + tz >= B.nb[2]);
+  auto face = [&](int i, int m, long long& dx, long long& dy, long long& dz) {
+    const int ci = code[i], cm = code[m];
+    auto round_axis = [&](int a, int li, int lm, long long& d) {
+      const int n = img[32 * a + lm] - img[32 * a + li];
+      if (n == 0) return;
+      const long long nl = n > 0 ? B.Lq[a] : -B.Lq[a];
+      const unsigned long long t = (unsigned long long)(d - nl);
+      const int q = B.qbit[a] - ((d < 0 ? -d : d) > B.qthr[a] ? 1 : 0);
+      const unsigned long long r = t + (1ull << (q - 1)) - 1ull + ((t >> q) & 1ull);
+      d = (long long)((r >> q) << q) + nl;
+    };
+    round_axis(0, ci & 31, cm & 31, dx);
+    round_axis(1, (ci >> 5) & 31, (cm >> 5) & 31, dy);
+    round_axis(2, ci >> 10, cm >> 10, dz);
+  };
+  auto enqueue = [&](bool acc, const float4& dq, int key) {
+    const unsigned bal = __ballot_sync(FULL, acc);
+    if (acc) {
+      const int p = (qh + qn + __popc(bal & lt)) & (kQueue - 1);
+      if (FP64 || FIX)
+        qk[p] = key;
+      else
+        qd[p] = make_float4(dq.x, dq.y, dq.z, __int_as_float(key));
+    }
+    qn += __popc(bal);
+    if (qn >= 32) {  // a batch only moves the ring's head
+      __syncwarp();
+      if (FP64)
+        force_batch64<MULTI, ENERGY, COUNT>(32, qk, pd, code, img, B.L, fd, cap, A.lj, ljs64, esum, wsum, A.status,
+                                            nacc, qh);
+      else if (FIX)
+        force_batch_fix<MULTI, ENERGY, COUNT>(32, qh, qk, px, fa, cap, A, ljx, esum, wsum, shsum, nacc, big_flag,
+                                              edge, face, inside64);
+      else
+        force_batch<MULTI, ENERGY, COUNT, MODE == kRedoFull>(32, qh, qd, fa, fr, cap, A, ljs32, ek, wk, nacc,
+                                                             big_flag);
+      __syncwarp();
+      qh = (qh + 32) & (kQueue - 1);
+      qn -= 32;
+    }
   };
 
   // ---- redo pass: the force of each accepted pair at once; only the large
@@ -783,7 +971,8 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
       const int tj = __float_as_int(pj.w);
       const int kb = __float_as_int(a.w);
       if (COUNT && valid) ++neval;
-      const float thr = MODE == kListBuild ? (MULTI ? ljs32[((kb >> 28) & 3) * A.lj.nt + tj].rl2 : q32.rl2)
+      const float thr = FIX ? (MULTI ? ljx[((kb >> 28) & 3) * A.lj.nt + tj].pre : A.fx.p[0].pre)
+                        : MODE == kListBuild ? (MULTI ? ljs32[((kb >> 28) & 3) * A.lj.nt + tj].rl2 : q32.rl2)
                                            : (MULTI ? ljs32[((kb >> 28) & 3) * A.lj.nt + tj].rc2 : q32.rc2);
       // disjoint bit fields: the sum is the OR, in one instruction
       const int key = (int)((unsigned)kb + ((unsigned)m << 14) + (MULTI ? (unsigned)tj << 30 : 0u));
@@ -1240,13 +1429,18 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
     if (FP64)
       force_batch64<MULTI, ENERGY, COUNT>(qn, qk, pd, code, img, B.L, fd, cap, A.lj, ljs64, esum, wsum, A.status,
                                           nacc, qh);
+    else if (FIX)
+      force_batch_fix<MULTI, ENERGY, COUNT>(qn, qh, qk, px, fa, cap, A, ljx, esum, wsum, shsum, nacc, big_flag,
+                                            edge, face, inside64);
     else
       force_batch<MULTI, ENERGY, COUNT, MODE == kRedoFull>(qn, qh, qd, fa, fr, cap, A, ljs32, ek, wk, nacc,
                                                            big_flag);
   }
   __syncthreads();
   // a large term was left out: list the tile for the redo pass
-  if (!FP64 && (MODE == kMain || MODE == kList) && tid == 0 && *big_flag) A.redo[atomicAdd(A.redo_n, 1)] = tile;
+  // (kFixed: the FP64 body computes it in full)
+  if (!FP64 && (MODE == kMain || MODE == kList || FIX) && tid == 0 && *big_flag)
+    A.redo[atomicAdd(A.redo_n, 1)] = FIX ? tile | kFullBit : tile;
   if (MODE == kListBuild) {
     // The atoms in the order of their entry counts, most first (a counting
     // sort), and the entries moved from the scratch into that order; a tile
@@ -1344,10 +1538,20 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
                      ((lz == 0 || lz == EZ - 1) ? 4 : 0);
     const int e = lx + EX * (ly + EY * lz);
     const int64_t g = gfirst[e] + (t - lstart[e]);
-    if (FP64) {
+    if (FP64 || FIX) {
       double* F = slot == 0 ? (double*)A.Fown : (double*)A.P + (size_t)(slot - 1) * 3 * A.N;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) F[EXAMD_IDX(c * A.N + g, 3 * A.N, st)] = fd[c * cap + t];
+      for (int c = 0; c < 3; ++c) {
+        double f;
+        if (FIX) {  // the integer sum, times 2^-sf
+          const long long v = ((long long)fa[(3 + c) * cap + t] << 32) | (unsigned)fa[c * cap + t];
+          const double d = __ll2double_rn(v);
+          f = v ? __hiloint2double(__double2hiint(d) - (A.fx.sf << 20), __double2loint(d)) : 0.0;
+        } else {
+          f = fd[c * cap + t];
+        }
+        F[EXAMD_IDX(c * A.N + g, 3 * A.N, st)] = f;
+      }
     } else {
       float4* F = slot == 0 ? (float4*)A.Fown : (float4*)A.P + (size_t)(slot - 1) * A.N;
       if (MODE == kRedoBig || MODE == kListBig) {
@@ -1380,7 +1584,10 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
     double e = 0.0, w = 0.0;
     long long ev = 0, wv = 0;
     if (ENERGY) {
-      if (FP64) {
+      if (FIX) {
+        e = esum - wsum - shsum;
+        w = 12.0 * esum - 6.0 * wsum;
+      } else if (FP64) {
         e = esum;
         w = wsum;
       } else {
@@ -1438,6 +1645,13 @@ __global__ void __launch_bounds__(256, FP64 ? 3 : 4) k_pair(const PairArgs A) {
   pair_tile<FP64, MULTI, ENERGY, COUNT, kMain, PACK>(A, A.order[blockIdx.x]);
 }
 
+// FP64 form: the first pass in fixed point, and the FP64 body for the tiles that
+// it listed (normally none).
+template <bool MULTI, bool ENERGY, bool COUNT>
+__global__ void __launch_bounds__(256, 3) k_pair_fix(const PairArgs A) {
+  pair_tile<false, MULTI, ENERGY, COUNT, kFixed, true>(A, A.order[blockIdx.x]);
+}
+
 // Pair-list mode: the forces of every tile from its list (fallback tiles
 // return at once: the redo pass enumerates them).
 template <bool MULTI, bool ENERGY, bool CUT>
@@ -1482,6 +1696,22 @@ __global__ void __launch_bounds__(256, 3) k_pair_redo(const PairArgs A) {
   }
 }
 
+template <bool MULTI, bool ENERGY, bool COUNT>
+__global__ void __launch_bounds__(256, 3) k_pair_redo64(const PairArgs A) {
+  const int n = *(volatile const int*)A.redo_n;
+  for (int j = blockIdx.x; j < n; j += gridDim.x) {
+    pair_tile<true, MULTI, ENERGY, COUNT, kRedoFull, false>(A, A.redo[j] & ~kFullBit);
+    __syncthreads();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (atomicAdd(A.redo_done, 1u) == gridDim.x - 1) {
+      *A.redo_n = 0;
+      *A.redo_done = 0;
+    }
+  }
+}
+
 template <bool FP64, bool MULTI, bool ENERGY, bool COUNT, bool PACK>
 static void* kfn() {
   return (void*)&k_pair<FP64, MULTI, ENERGY, COUNT, PACK>;
@@ -1511,7 +1741,20 @@ static void* pick_enum(const PairConfig& c) {
 // enumeration counts) the list pass.
 static bool uses_list(const PairConfig& c) { return c.list && !c.fp64 && !c.count; }
 
+template <bool MULTI>
+static void* pick_fix(const PairConfig& c) {
+  if (c.energy) return c.count ? (void*)&k_pair_fix<MULTI, true, true> : (void*)&k_pair_fix<MULTI, true, false>;
+  return c.count ? (void*)&k_pair_fix<MULTI, false, true> : (void*)&k_pair_fix<MULTI, false, false>;
+}
+
+template <bool MULTI>
+static void* pick_redo64(const PairConfig& c) {
+  if (c.energy) return c.count ? (void*)&k_pair_redo64<MULTI, true, true> : (void*)&k_pair_redo64<MULTI, true, false>;
+  return c.count ? (void*)&k_pair_redo64<MULTI, false, true> : (void*)&k_pair_redo64<MULTI, false, false>;
+}
+
 static void* pick(const PairConfig& c) {
+  if (c.fix) return c.multi ? pick_fix<true>(c) : pick_fix<false>(c);
   if (uses_list(c)) {
     if (c.cut) {
       if (c.multi) return c.energy ? (void*)&k_pair_list<true, true, true> : (void*)&k_pair_list<true, false, true>;
@@ -1542,11 +1785,14 @@ static void* pick_redo_l(const PairConfig& c) {
   return c.multi ? pick_redo_ec<true, false, LIST>(c) : pick_redo_ec<false, false, LIST>(c);
 }
 
-static void* pick_redo(const PairConfig& c) { return uses_list(c) ? pick_redo_l<true>(c) : pick_redo_l<false>(c); }
+static void* pick_redo(const PairConfig& c) {
+  if (c.fix) return c.multi ? pick_redo64<true>(c) : pick_redo64<false>(c);
+  return uses_list(c) ? pick_redo_l<true>(c) : pick_redo_l<false>(c);
+}
 
 cudaError_t pair_prepare(const PairConfig& cfg, int smem_bytes) {
   cudaError_t e = cudaFuncSetAttribute(pick(cfg), cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-  if (e != cudaSuccess || cfg.fp64) return e;
+  if (e != cudaSuccess || (cfg.fp64 && !cfg.fix)) return e;
   e = cudaFuncSetAttribute(pick_redo(cfg), cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
   if (e != cudaSuccess || !uses_list(cfg)) return e;
   return cudaFuncSetAttribute(pick_build(cfg), cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
@@ -1572,7 +1818,7 @@ cudaError_t launch_pair(const PairConfig& cfg, const PairArgs& a, int ntiles, in
   const int main_smem = main_smem_bytes(cfg, a.cap, a.ne_max, a.ext_max);
   if (main_smem > smem_bytes) return cudaErrorInvalidValue;
   cudaError_t e = cudaLaunchKernel(fn, dim3(ntiles), dim3(32 * cfg.warps), args, (size_t)main_smem, st);
-  if (e != cudaSuccess || cfg.fp64) return e;
+  if (e != cudaSuccess || (cfg.fp64 && !cfg.fix)) return e;
   // the redo pass: a few blocks per SM at most; nothing to do in a thermal system
   const int redo_smem = redo_smem_bytes(cfg, a.cap_redo, a.ne_max, a.ext_max);
   if (redo_smem > smem_bytes) return cudaErrorInvalidValue;
