@@ -129,7 +129,7 @@ __host__ __device__ inline int align16(int x) { return (x + 15) & ~15; }
 // reduction scratch; kListBig's fr after everything).
 // ne_max, ext_max: the largest tile's ext cells and ext extent on one axis.
 __host__ __device__ inline Layout make_layout(bool fp64, int cap, int ne_max, int ext_max, int nw, int mode,
-                                              bool pack) {
+                                              bool pack, bool multi) {
   const bool from_list = mode == kList || mode == kListBig;
   Layout L;
   int o = 0;
@@ -147,7 +147,7 @@ __host__ __device__ inline Layout make_layout(bool fp64, int cap, int ne_max, in
   L.lut = o;    o = align16(o + (from_list ? 0 : (int)sizeof(OwnLut)));
   // the LJ table per ordered type pair (several types): per-lane type indices
   // would serialise on the kernel-parameter bank, shared memory serves them at once
-  L.ljt = o;    o = align16(o + (fix ? (int)sizeof(FixPair) : (int)sizeof(LJ64)) * EXAMD_MAX_TYPES * EXAMD_MAX_TYPES);
+  L.ljt = o;    o = align16(o + (multi ? (fix ? (int)sizeof(FixPair) : (int)sizeof(LJ64)) * EXAMD_MAX_TYPES * EXAMD_MAX_TYPES : 0));
   const int tab = pack ? kWarpTabCompact : kWarpTabWide;
   const int qbytes = (fp64 ? 4 * kQueue + kWarpTabFp64
                            : (from_list ? 64 : (mode == kListBuild ? 0 : fix ? 4 : 16) * kQueue + tab)) * nw;
@@ -181,10 +181,10 @@ __host__ __device__ inline Layout make_layout(bool fp64, int cap, int ne_max, in
 }
 
 static int redo_smem_bytes(const PairConfig& cfg, int cap_redo, int ne_max, int ext_max) {
-  if (cfg.fix) return make_layout(true, cap_redo, ne_max, ext_max, cfg.warps, kRedoFull, false).bytes;
-  const int b = std::max(make_layout(false, cap_redo, ne_max, ext_max, cfg.warps, kRedoBig, cfg.pack).bytes,
-                         make_layout(false, cap_redo, ne_max, ext_max, cfg.warps, kRedoFull, cfg.pack).bytes);
-  return cfg.list ? std::max(b, make_layout(false, cap_redo, ne_max, ext_max, cfg.warps, kListBig, cfg.pack).bytes)
+  if (cfg.fix) return make_layout(true, cap_redo, ne_max, ext_max, cfg.warps, kRedoFull, false, cfg.multi).bytes;
+  const int b = std::max(make_layout(false, cap_redo, ne_max, ext_max, cfg.warps, kRedoBig, cfg.pack, cfg.multi).bytes,
+                         make_layout(false, cap_redo, ne_max, ext_max, cfg.warps, kRedoFull, cfg.pack, cfg.multi).bytes);
+  return cfg.list ? std::max(b, make_layout(false, cap_redo, ne_max, ext_max, cfg.warps, kListBig, cfg.pack, cfg.multi).bytes)
                   : b;
 }
 
@@ -192,17 +192,17 @@ static int redo_smem_bytes(const PairConfig& cfg, int cap_redo, int ne_max, int 
 // counters, which the enumeration gives) the list pass's.
 static int main_smem_bytes(const PairConfig& cfg, int cap, int ne_max, int ext_max) {
   const int mode = (cfg.list && !cfg.count && !cfg.fp64) ? kList : kMain;
-  if (cfg.fix) return make_layout(false, cap, ne_max, ext_max, cfg.warps, kFixed, true).bytes;
-  return make_layout(cfg.fp64, cap, ne_max, ext_max, cfg.warps, mode, cfg.pack).bytes;
+  if (cfg.fix) return make_layout(false, cap, ne_max, ext_max, cfg.warps, kFixed, true, cfg.multi).bytes;
+  return make_layout(cfg.fp64, cap, ne_max, ext_max, cfg.warps, mode, cfg.pack, cfg.multi).bytes;
 }
 
 static int build_smem_bytes(const PairConfig& cfg, int cap, int ne_max, int ext_max) {
-  return make_layout(false, cap, ne_max, ext_max, kBuildWarps, kListBuild, cfg.pack).bytes;
+  return make_layout(false, cap, ne_max, ext_max, kBuildWarps, kListBuild, cfg.pack, cfg.multi).bytes;
 }
 
 int pair_smem_bytes(const PairConfig& cfg, int cap, int cap_redo, int ne_max, int ext_max) {
   if (cfg.fix) return std::max(main_smem_bytes(cfg, cap, ne_max, ext_max), redo_smem_bytes(cfg, cap_redo, ne_max, ext_max));
-  int b = make_layout(cfg.fp64, cap, ne_max, ext_max, cfg.warps, kMain, cfg.pack).bytes;
+  int b = make_layout(cfg.fp64, cap, ne_max, ext_max, cfg.warps, kMain, cfg.pack, cfg.multi).bytes;
   if (cfg.fp64) return b;
   b = std::max(b, redo_smem_bytes(cfg, cap_redo, ne_max, ext_max));
   if (cfg.list) b = std::max(b, std::max(main_smem_bytes(cfg, cap, ne_max, ext_max),
@@ -561,7 +561,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   if (kFromList && MODE == kList && A.lcount[tile] < 0) return;  // a fallback tile: the redo pass computes it
   constexpr bool FIX = MODE == kFixed;
   const int cap = (MODE == kMain || MODE == kListBuild || MODE == kList || FIX) ? A.cap : A.cap_redo;
-  const Layout L = make_layout(FP64, cap, A.ne_max, A.ext_max, nw, MODE, PACK);
+  const Layout L = make_layout(FP64, cap, A.ne_max, A.ext_max, nw, MODE, PACK, MULTI);
   // shared-memory arrays (index-checked in the checked build)
   int* const st = A.status;  // the index checks' status word (checked build)
   (void)st;
@@ -677,6 +677,10 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
     for (int k = b; k < e; ++k) {
       int c = lstart[k];
       lstart[k] = run;
+      // the cell of each staged atom, for the staging and the write-back
+      const int lx = k % EX, rr = k / EX, ly = rr % EY, lz = rr / EY;
+      const unsigned short cc = (unsigned short)(lx | (ly << 5) | (lz << 10));
+      for (int t = run, t1 = min(run + c, cap); t < t1; ++t) code[t] = cc;
       run += c;
     }
     if (tid == blockDim.x - 1) {
@@ -720,36 +724,58 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
     }
     return;
   }
-  // (3) stage atoms, one thread per ext cell
+  // (3) stage atoms, one thread per atom, kStage atoms' reads in flight at a
+  // time.  (One thread per ext cell, the cell's atoms one after the other, waited
+  // for a read per atom: a third of the lanes idle and 188 us of the FP64 form's
+  // 950 us on a 1M-atom liquid went into staging and write-back.)
   auto fa = EXAMD_ARR(int, smem + L.fa, (MODE == kListBuild ? 1 : FIX ? 6 : 3) * cap, st);
   auto fr = EXAMD_ARR(float, smem + L.fr, 3 * cap, st);  // redo pass: FP32 sums of the large terms
   auto fd = EXAMD_ARR(double, smem + L.fa, 3 * cap, st);
   auto pd = EXAMD_ARR(double, smem + L.px, 3 * cap, st);
   auto px = EXAMD_ARR(unsigned long long, smem + L.px, 3 * cap, st);  // kFixed: fixed-point positions, images applied
-  for (int e = tid; e < NE; e += blockDim.x) {
-    const int lx = e % EX, rr = e / EX, ly = rr % EY, lz = rr / EY;
-    const int a0 = lstart[e], a1 = lstart[e + 1], g0 = gfirst[e];
-    const unsigned short cc = (unsigned short)(lx | (ly << 5) | (lz << 10));
-    for (int t = a0; t < a1; ++t) {
-      const int g = g0 + (t - a0);
-      const float4 u = U[g];
+  constexpr int kStage = FP64 || FIX ? 2 : 4;
+  for (int t0 = tid; t0 < total; t0 += kStage * blockDim.x) {
+    float4 uu[kStage];
+    double xx[kStage][3];
+#pragma unroll
+    for (int k = 0; k < kStage; ++k) {
+      const int t = t0 + k * blockDim.x;
+      if (t < total) {
+        const int cc = code[t];
+        const int e = (cc & 31) + EX * (((cc >> 5) & 31) + EY * (cc >> 10));
+        const int g = gfirst[e] + (t - (int)lstart[e]);
+        uu[k] = U[g];
+        if (FP64 || FIX) {
+          const int64_t gg = EXAMD_IDX(g, A.N, st);
+          xx[k][0] = A.X0[gg];
+          xx[k][1] = A.X1[gg];
+          xx[k][2] = A.X2[gg];
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kStage; ++k) {
+      const int t = t0 + k * blockDim.x;
+      if (t >= total) break;
+      const int cc = code[t];
+      const int lx = cc & 31, ly = (cc >> 5) & 31, lz = cc >> 10;
+      const float4 u = uu[k];
       if (FP64) {
         pf[t] = make_float4(ox[lx] + u.x, oy[ly] + u.y, oz[lz] + u.z, u.w);
-        pd[t] = A.X0[EXAMD_IDX(g, A.N, st)];
-        pd[cap + t] = A.X1[EXAMD_IDX(g, A.N, st)];
-        pd[2 * cap + t] = A.X2[EXAMD_IDX(g, A.N, st)];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) fd[c * cap + t] = 0.0;
+        for (int c = 0; c < 3; ++c) {
+          pd[c * cap + t] = xx[k][c];
+          fd[c * cap + t] = 0.0;
+        }
       } else {
         // from a list: the type and the ext-cell code in w (the list pass
         // reads both atoms' rows from them)
         pf[t] = make_float4(ox[lx] + u.x, u.y, u.z,
-                            kFromList ? __int_as_float((__float_as_int(u.w) & 3) | ((int)cc << 2)) : u.w);
+                            kFromList ? __int_as_float((__float_as_int(u.w) & 3) | (cc << 2)) : u.w);
         if (FIX) {
-          const int64_t gg = EXAMD_IDX(g, A.N, st);
-          px[t] = to_fixed(A.X0[gg], A.fx.ue) + (unsigned long long)(img[lx] * B.Lq[0]);
-          px[cap + t] = to_fixed(A.X1[gg], A.fx.ue) + (unsigned long long)(img[32 + ly] * B.Lq[1]);
-          px[2 * cap + t] = to_fixed(A.X2[gg], A.fx.ue) + (unsigned long long)(img[64 + lz] * B.Lq[2]);
+          px[t] = to_fixed(xx[k][0], A.fx.ue) + (unsigned long long)(img[lx] * B.Lq[0]);
+          px[cap + t] = to_fixed(xx[k][1], A.fx.ue) + (unsigned long long)(img[32 + ly] * B.Lq[1]);
+          px[2 * cap + t] = to_fixed(xx[k][2], A.fx.ue) + (unsigned long long)(img[64 + lz] * B.Lq[2]);
 #pragma unroll
           for (int c = 0; c < 6; ++c) fa[c * cap + t] = 0;
         }
@@ -761,7 +787,6 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
             fa[c * cap + t] = 0;
         }
       }
-      code[t] = cc;
     }
   }
   int* big_flag = cw + 1;  // mixed form: a term was too large for the fixed-point sums
@@ -1648,7 +1673,7 @@ __global__ void __launch_bounds__(256, FP64 ? 3 : 4) k_pair(const PairArgs A) {
 // FP64 form: the first pass in fixed point, and the FP64 body for the tiles that
 // it listed (normally none).
 template <bool MULTI, bool ENERGY, bool COUNT>
-__global__ void __launch_bounds__(256, 3) k_pair_fix(const PairArgs A) {
+__global__ void __launch_bounds__(256, 4) k_pair_fix(const PairArgs A) {
   pair_tile<false, MULTI, ENERGY, COUNT, kFixed, true>(A, A.order[blockIdx.x]);
 }
 
@@ -1803,7 +1828,7 @@ cudaError_t pair_prepare(const PairConfig& cfg, int smem_bytes) {
 int pair_blocks_per_sm(const PairConfig& cfg, int cap, int ne_max, int ext_max) {
   PairConfig c = cfg;
   c.list = false;
-  const int smem = make_layout(c.fp64, cap, ne_max, ext_max, c.warps, kMain, c.pack).bytes;
+  const int smem = make_layout(c.fp64, cap, ne_max, ext_max, c.warps, kMain, c.pack, c.multi).bytes;
   int n = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pick_enum(c), 32 * c.warps, (size_t)smem) != cudaSuccess)
     return 0;
