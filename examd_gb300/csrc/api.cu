@@ -226,6 +226,7 @@ int examd_tile_split(int nb, double last_width, int tile_len, int tile_balance, 
 }
 
 constexpr int kIoChunks = 4;            // host <-> device transfers of the force call, in chunks
+constexpr int kEagerSlots = 32;         // energies of eager steps kept on the device before one copy
 constexpr int64_t kIoMinChunk = 1 << 16;  // atoms; smaller calls use fewer chunks
 
 struct examd_ctx {
@@ -286,7 +287,7 @@ struct examd_ctx {
   int64_t* d_atom0 = nullptr;
   double* keAtom = nullptr;
   double* partial = nullptr;  // chunk partial sums of the per-box reductions
-  int* h_status = nullptr;    // pinned host copy of the status word
+  int* h_status = nullptr;    // pinned host copies of the status word and, behind it, of d_occ
   // caller-order I/O in chunks, copies on a second stream
   int* inv = nullptr;         // caller index -> sorted slot
   bool inv_valid = false;     // inv matches the current sorted order
@@ -295,6 +296,12 @@ struct examd_ctx {
   cudaEvent_t ev_io[3 * kIoChunks + 1] = {};
   int maxc_atoms = 1, maxc_tiles = 1;
   int ebuf_steps = 0;
+  double* h_e = nullptr;      // pinned copies of boxKE and boxE (ebuf_steps + 1 steps each), for the runs with energies
+  // a step's energy sums run on the second stream: the events that order them
+  // (kick done, pair pass done; kinetic sums done, potential sums done), and
+  // whether the last two are to be waited for
+  cudaEvent_t ev_side[4] = {};
+  bool side_ke = false, side_pe = false;
 
   bool atoms_set = false;
   bool forces_valid = false;  // Fown/P hold F(X[cur])
@@ -382,6 +389,9 @@ void free_all(examd_ctx* ctx) {
   }
   if (ctx->h_status) cudaFreeHost(ctx->h_status);
   if (ctx->h_lw) cudaFreeHost(ctx->h_lw);
+  if (ctx->h_e) cudaFreeHost(ctx->h_e);
+  for (cudaEvent_t e : ctx->ev_side)
+    if (e) cudaEventDestroy(e);
   if (ctx->inv) cudaFree(ctx->inv);
   for (cudaEvent_t e : ctx->ev_io)
     if (e) cudaEventDestroy(e);
@@ -791,7 +801,7 @@ int examd_gpu_create(const examd_params* params, int nboxes, const examd_box* bo
     delete ctx;
     return EXAMD_ERR_CUDA;
   }
-  if (cudaHostAlloc((void**)&ctx->h_status, sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
+  if (cudaHostAlloc((void**)&ctx->h_status, 2 * sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
     ctx->h_status = nullptr;
     free_all(ctx);
     delete ctx;
@@ -800,6 +810,7 @@ int examd_gpu_create(const examd_params* params, int nboxes, const examd_box* bo
   *ctx->h_status = 0;
   bool io_ok = cudaStreamCreateWithFlags(&ctx->st2, cudaStreamNonBlocking) == cudaSuccess &&
                cudaStreamCreateWithFlags(&ctx->stc, cudaStreamNonBlocking) == cudaSuccess;
+  for (cudaEvent_t& e : ctx->ev_side) io_ok = io_ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
   for (cudaEvent_t& e : ctx->ev_io) io_ok = io_ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
   if (!io_ok) {
     free_all(ctx);
@@ -998,15 +1009,19 @@ int check_status(examd_ctx* ctx) {
 // headroom for the redo pass and for the FP64 form without one (no fixed-point
 // pass); +6% + 32 for a first pass with a redo pass behind it (a tile that
 // outgrows it before the next update is computed in full by the redo pass, at
-// the redo capacity).
-int update_capacity(examd_ctx* ctx, bool* grew = nullptr) {
-  if (grew) *grew = false;
+// the redo capacity).  In two parts, so that a run waits once per chunk: the
+// occupancy queued to its pinned word, and the capacities from it.
+int queue_occupancy(examd_ctx* ctx) {
   CK(cudaMemsetAsync(ctx->d_occ, 0, 2 * sizeof(int), ctx->st));
   k_tile_occupancy<<<ctx->ntiles, 128, 0, ctx->st>>>(ctx->d_tiles, ctx->d_boxes, ctx->cstart, ctx->d_occ);
   CK(cudaGetLastError());
-  int occ = 0;
-  CK(cudaMemcpyAsync(&occ, ctx->d_occ, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
-  CK(cudaStreamSynchronize(ctx->st));
+  CK(cudaMemcpyAsync(ctx->h_status + 1, ctx->d_occ, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
+  return EXAMD_OK;
+}
+
+int apply_capacity(examd_ctx* ctx, bool* grew = nullptr) {
+  if (grew) *grew = false;
+  const int occ = ctx->h_status[1];
   int want_r = std::max(((occ + occ / 4 + 64) + 7) & ~7, ctx->cap_redo);
   int want = ctx->pc.fp64 && !ctx->pc.fix ? want_r : ((occ + occ / 16 + 32) + 7) & ~7;
   if (want <= ctx->cap) return EXAMD_OK;
@@ -1051,6 +1066,13 @@ int update_capacity(examd_ctx* ctx, bool* grew = nullptr) {
       CK(pair_prepare(c, ctx->smem_limit));
     }
   return EXAMD_OK;
+}
+
+int update_capacity(examd_ctx* ctx) {
+  const int rc = queue_occupancy(ctx);
+  if (rc) return rc;
+  CK(cudaStreamSynchronize(ctx->st));
+  return apply_capacity(ctx);
 }
 
 PairArgs pair_args(examd_ctx* ctx) {
@@ -1201,9 +1223,15 @@ int set_list_capacity(examd_ctx* ctx, int want) {
 
 // Pair-list mode: the list words, read after the stream's work; the longest
 // list since the last read is reset.
-int read_list_words(examd_ctx* ctx) {
+int queue_list_words(examd_ctx* ctx) {
   CK(cudaMemcpyAsync(ctx->h_lw, ctx->lw, LW_WORDS * sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaMemsetAsync(ctx->lw + LW_LMAX, 0, sizeof(int), ctx->st));
+  return EXAMD_OK;
+}
+
+int read_list_words(examd_ctx* ctx) {
+  const int rc = queue_list_words(ctx);
+  if (rc) return rc;
   CK(cudaStreamSynchronize(ctx->st));
   return EXAMD_OK;
 }
@@ -1256,9 +1284,9 @@ int run_pair(examd_ctx* ctx, bool energy, bool count, double* boxE = nullptr, do
 // a fresh sort (a build needs every atom inside its cell), and the forces
 // again in the new order.  A staged-atom capacity that grew within the slots
 // makes the next step rebuild, so that the tiles over the old one get lists.
+// (h_lw holds the list words.)
 int update_lists(examd_ctx* ctx, bool cap_grew) {
-  int rc = read_list_words(ctx);
-  if (rc) return rc;
+  int rc;
   const int longest = ctx->h_lw[LW_LMAX];
   const bool fixed = ctx->p.pair_list_capacity > 0;
   const int want = fixed ? ctx->lk : std::max(ctx->lk, list_capacity_for(longest));
@@ -1279,11 +1307,30 @@ int run_pair(examd_ctx* ctx, bool energy, bool count, double* boxE, double* boxW
   PairConfig c = ctx->pc;
   c.energy = energy;
   c.count = count;
+  if (ctx->side_pe) {  // the last step's sums read the tile energies that this pass writes
+    CK(cudaStreamWaitEvent(ctx->st, ctx->ev_side[3], 0));
+    ctx->side_pe = false;
+  }
   CK(launch_pair(c, pair_args(ctx), ctx->ntiles, ctx->smem, ctx->st));
-  if (energy)
+  if (energy && !boxE)
     CK(launch_reduce_tiles(ctx->nboxes, ctx->d_tile0, ctx->maxc_tiles, ctx->tileE, ctx->tileW, ctx->partial,
-                           boxE ? boxE : ctx->boxE,
-                           boxW ? boxW : ctx->boxW, ctx->st));
+                           ctx->boxE, ctx->boxW, ctx->st));
+  if (energy && boxE) {  // a step's sums: on the second stream
+    CK(cudaEventRecord(ctx->ev_side[1], ctx->st));
+    CK(cudaStreamWaitEvent(ctx->st2, ctx->ev_side[1], 0));
+    CK(launch_reduce_tiles(ctx->nboxes, ctx->d_tile0, ctx->maxc_tiles, ctx->tileE, ctx->tileW, ctx->partial, boxE,
+                           boxW, ctx->st2));
+    CK(cudaEventRecord(ctx->ev_side[3], ctx->st2));
+    ctx->side_pe = true;
+  }
+  return EXAMD_OK;
+}
+
+// The first stream waits for the energy sums queued on the second one.
+int join_side(examd_ctx* ctx) {
+  if (ctx->side_ke) CK(cudaStreamWaitEvent(ctx->st, ctx->ev_side[2], 0));
+  if (ctx->side_pe) CK(cudaStreamWaitEvent(ctx->st, ctx->ev_side[3], 0));
+  ctx->side_ke = ctx->side_pe = false;
   return EXAMD_OK;
 }
 
@@ -1528,7 +1575,7 @@ int examd_gpu_forces_at(examd_ctx* ctx, const double* pos, double* forces, doubl
 
 namespace {
 
-KickArgs kick_args(examd_ctx* ctx, double ckick, double dt, bool drift, double hk, double* boxKE) {
+KickArgs kick_args(examd_ctx* ctx, double ckick, double dt, bool drift, double hk) {
   KickArgs k{};
   k.s = step_args(ctx);
   const int c = ctx->cur;
@@ -1545,12 +1592,7 @@ KickArgs kick_args(examd_ctx* ctx, double ckick, double dt, bool drift, double h
     k.ckm[t] = ckick * ctx->lj.minv[t];
     k.hkm[t] = hk * ctx->lj.minv[t];
   }
-  k.boxKE = boxKE;
   k.keAtom = ctx->keAtom;
-  k.partial = ctx->partial;
-  k.maxc = ctx->maxc_atoms;
-  k.atom0 = ctx->d_atom0;
-  k.nboxes = ctx->nboxes;
   k.lj = ctx->lj;
   k.cellOld = ctx->cellOld;
   k.slot = ctx->slot;
@@ -1566,16 +1608,42 @@ KickArgs kick_args(examd_ctx* ctx, double ckick, double dt, bool drift, double h
 // One step after the first: kick(ck) + drift + bin, pair.  keSlot receives the
 // kinetic energy at the start of this step, eSlot the potential energy after.
 // Pair-list mode: the binning and the lists only on the steps that the
-// device decides to rebuild.
+// device decides to rebuild.  The energy sums (four small kernels, a fifth of a
+// 32,000-atom step when they stood between its kernels) run on the second
+// stream beside the binning and the next kick.
+int kick(examd_ctx* ctx, double ck, double dt, bool drift, double* keSlot) {
+  if (ctx->side_ke) {  // the last step's sums read the per-atom energies that this kick writes
+    CK(cudaStreamWaitEvent(ctx->st, ctx->ev_side[2], 0));
+    ctx->side_ke = false;
+  }
+  CK(launch_kick(kick_args(ctx, ck, dt, drift, keSlot ? 0.5 * dt : 0.0), ctx->st));
+  if (!keSlot) return EXAMD_OK;
+  CK(cudaEventRecord(ctx->ev_side[0], ctx->st));
+  CK(cudaStreamWaitEvent(ctx->st2, ctx->ev_side[0], 0));
+  CK(launch_box_sums(ctx->nboxes, ctx->d_atom0, ctx->maxc_atoms, ctx->keAtom, ctx->partial, keSlot, ctx->st2));
+  CK(cudaEventRecord(ctx->ev_side[2], ctx->st2));
+  ctx->side_ke = true;
+  return EXAMD_OK;
+}
+
 int step_once(examd_ctx* ctx, double ck, double dt, double* keSlot, double* eSlot, double* wSlot) {
-  const double h = 0.5 * dt;
-  CK(launch_kick(kick_args(ctx, ck, dt, true, keSlot ? h : 0.0, keSlot), ctx->st));
-  int rc = ctx->list ? maybe_rebuild(ctx) : finish_binning(ctx, false);
+  int rc = kick(ctx, ck, dt, true, keSlot);
+  if (rc) return rc;
+  rc = ctx->list ? maybe_rebuild(ctx) : finish_binning(ctx, false);
   if (rc) return rc;
   return run_pair(ctx, eSlot != nullptr, false, eSlot, wSlot);
 }
 
-int ensure_ebuf(examd_ctx* ctx, int steps) {
+int ensure_ebuf(examd_ctx* ctx, int steps, bool host) {
+  if (steps <= ctx->ebuf_steps && (!host || ctx->h_e)) return EXAMD_OK;
+  steps = std::max(steps, ctx->ebuf_steps);
+  if (ctx->h_e) cudaFreeHost(ctx->h_e);
+  ctx->h_e = nullptr;
+  if (host && cudaHostAlloc((void**)&ctx->h_e, 2 * (size_t)(steps + 1) * ctx->nboxes * sizeof(double),
+                            cudaHostAllocDefault) != cudaSuccess) {
+    ctx->h_e = nullptr;
+    return EXAMD_ERR_NOMEM;
+  }
   if (steps <= ctx->ebuf_steps) return EXAMD_OK;
   if (ctx->boxE) cudaFree(ctx->boxE);
   if (ctx->boxW) cudaFree(ctx->boxW);
@@ -1612,6 +1680,7 @@ int ensure_chunk_graph(examd_ctx* ctx, int chunk, double dt, bool wantE, int par
   ctx->gexec = nullptr;
   const int nb = ctx->nboxes;
   const int saved = ctx->cur;
+  if (const int rc = join_side(ctx)) return rc;  // (the graph's own first step waits for nothing outside it)
   ctx->cur = parity;
   cudaGraph_t g;
   CK(cudaStreamBeginCapture(ctx->st, cudaStreamCaptureModeThreadLocal));
@@ -1619,7 +1688,9 @@ int ensure_chunk_graph(examd_ctx* ctx, int chunk, double dt, bool wantE, int par
   for (int j = 0; j < chunk && src == EXAMD_OK; ++j)
     src = step_once(ctx, dt, dt, wantE ? ctx->boxKE + (size_t)j * nb : nullptr,
                     wantE ? ctx->boxE + (size_t)j * nb : nullptr, wantE ? ctx->boxW + (size_t)j * nb : nullptr);
+  if (src == EXAMD_OK) src = join_side(ctx);
   cudaError_t ce = cudaStreamEndCapture(ctx->st, &g);
+  ctx->side_ke = ctx->side_pe = false;
   // capture advanced the host-side parity; the graph leaves it unchanged (chunk
   // even; pair-list mode: no step swaps the buffers)
   ctx->cur = saved;
@@ -1652,7 +1723,9 @@ int examd_gpu_run(examd_ctx* ctx, int nsteps, double dt, int graph_chunk, double
   const int nb = ctx->nboxes;
   const bool wantE = energies != nullptr;
   int chunk = graph_chunk > 0 ? (graph_chunk + 1) / 2 * 2 : 0;
-  int rc = ensure_ebuf(ctx, std::max(chunk, 1) + 1);
+  // eager steps' energies wait on the device too, up to kEagerSlots of them
+  const int slots = std::max(chunk, wantE ? kEagerSlots : 1) + 1;
+  int rc = ensure_ebuf(ctx, slots, wantE);
   if (rc) return rc;
   if (!ctx->forces_valid) {
     rc = run_pair(ctx, false, false);
@@ -1661,69 +1734,88 @@ int examd_gpu_run(examd_ctx* ctx, int nsteps, double dt, int graph_chunk, double
   }
   if (nsteps == 0) return EXAMD_OK;
   const double h = 0.5 * dt;
+  // Energies: slot j of boxE holds the potential energy after step first + j
+  // (0-based), slot j of boxKE the kinetic energy before it, i.e. after step
+  // first + j - 1; `held` slots are filled.  fetch() brings them to the caller
+  // in one copy each (a copy per box and step took 0.36 of the 0.40 s that 41
+  // steps of a 512-box ensemble took).
+  int first = 0, held = 0;
+  auto queue_energies = [&](int extra_ke) -> int {
+    const size_t n = (size_t)held * nb, nk = (size_t)(held + extra_ke) * nb;
+    double* he = ctx->h_e + (size_t)(ctx->ebuf_steps + 1) * nb;
+    if (const int jrc = join_side(ctx)) return jrc;
+    if (nk) CK(cudaMemcpyAsync(ctx->h_e, ctx->boxKE, nk * sizeof(double), cudaMemcpyDeviceToHost, st));
+    if (n) CK(cudaMemcpyAsync(he, ctx->boxE, n * sizeof(double), cudaMemcpyDeviceToHost, st));
+    return EXAMD_OK;
+  };
+  auto store_energies = [&](int extra_ke) {  // after the stream's work
+    const double* he = ctx->h_e + (size_t)(ctx->ebuf_steps + 1) * nb;
+    for (int j = 0; j < held + extra_ke; ++j)
+      for (int b = 0; b < nb; ++b) {
+        const size_t g = (size_t)(first + j);
+        if (g > 0) energies[2 * ((g - 1) * nb + b)] = ctx->h_e[(size_t)j * nb + b];
+        if (j < held) energies[2 * (g * nb + b) + 1] = he[(size_t)j * nb + b];
+      }
+    first += held;
+    held = 0;
+  };
+  auto fetch = [&]() -> int {
+    if (!wantE || held == 0) return EXAMD_OK;
+    if (const int qrc = queue_energies(0)) return qrc;
+    CK(cudaStreamSynchronize(st));
+    store_energies(0);
+    return EXAMD_OK;
+  };
+  auto slot = [&](double* p) { return wantE ? p + (size_t)held * nb : nullptr; };
   CK(cudaEventRecord(ctx->e0, st));
   // step 1: half kick + drift, then forces
-  rc = step_once(ctx, h, dt, nullptr, wantE ? ctx->boxE : nullptr, wantE ? ctx->boxW : nullptr);
+  rc = step_once(ctx, h, dt, nullptr, slot(ctx->boxE), slot(ctx->boxW));
   if (rc) return rc;
-  if (wantE) {
-    // energies[0] epot now; ekin later
-    for (int b = 0; b < nb; ++b)
-      CK(cudaMemcpyAsync(&energies[2 * b + 1], ctx->boxE + b, sizeof(double), cudaMemcpyDeviceToHost, st));
-  }
+  held = 1;
   int done = 1;
   // steady state: merged kicks v += dt F/m
   while (done < nsteps) {
     const int left = nsteps - done;
     if (chunk > 0 && left >= chunk) {
+      if ((rc = fetch())) return rc;  // the graph writes the slots from the first
+      first = done;
       rc = ensure_chunk_graph(ctx, chunk, dt, wantE, ctx->cur);
       if (rc) return rc;
       CK(cudaGraphLaunch(ctx->gexec, st));
-      if (wantE) {
-        // slot j: ekin at the start of local step j (= after global step done + j), epot after it
-        for (int j = 0; j < chunk; ++j)
-          for (int b = 0; b < nb; ++b) {
-            const size_t gs = (size_t)(done + j);  // global 0-based step index of epot
-            CK(cudaMemcpyAsync(&energies[2 * ((gs - 1) * nb + b)], ctx->boxKE + (size_t)j * nb + b,
-                               sizeof(double), cudaMemcpyDeviceToHost, st));
-            CK(cudaMemcpyAsync(&energies[2 * (gs * nb + b) + 1], ctx->boxE + (size_t)j * nb + b, sizeof(double),
-                               cudaMemcpyDeviceToHost, st));
-          }
-        CK(cudaStreamSynchronize(st));  // buffers are reused by the next replay
-      }
+      held = chunk;
       done += chunk;
-      // the capacities may need to grow as the density fluctuates
+      // the capacities may need to grow as the density fluctuates: the status
+      // word, the occupancy, the list words and the energies in one wait
+      CK(queue_status(ctx));
+      if ((rc = queue_occupancy(ctx))) return rc;
+      if (ctx->list && (rc = queue_list_words(ctx))) return rc;
+      if (wantE && (rc = queue_energies(0))) return rc;
       CK(cudaStreamSynchronize(st));
-      rc = check_status(ctx);
+      if (wantE) store_energies(0);
+      rc = take_status(ctx);
       if (rc) return rc;
       bool grew = false;
-      rc = update_capacity(ctx, &grew);
+      rc = apply_capacity(ctx, &grew);
       if (rc) return rc;
       if (ctx->list && (rc = update_lists(ctx, grew))) return rc;
     } else {
-      double* ke = nullptr;
-      if (wantE) ke = ctx->boxKE;
-      rc = step_once(ctx, dt, dt, ke, wantE ? ctx->boxE : nullptr, wantE ? ctx->boxW : nullptr);
+      if (wantE && held == kEagerSlots && (rc = fetch())) return rc;
+      if (held == 0) first = done;
+      rc = step_once(ctx, dt, dt, slot(ctx->boxKE), slot(ctx->boxE), slot(ctx->boxW));
       if (rc) return rc;
-      if (wantE)
-        for (int b = 0; b < nb; ++b) {
-          CK(cudaMemcpyAsync(&energies[2 * ((size_t)(done - 1) * nb + b)], ctx->boxKE + b, sizeof(double),
-                             cudaMemcpyDeviceToHost, st));
-          CK(cudaMemcpyAsync(&energies[2 * ((size_t)done * nb + b) + 1], ctx->boxE + b, sizeof(double),
-                             cudaMemcpyDeviceToHost, st));
-        }
-      if (wantE) CK(cudaStreamSynchronize(st));
+      held += 1;
       done += 1;
     }
   }
   // closing half kick: v(t_n) = v(t_n - h) + h F/m
-  CK(launch_kick(kick_args(ctx, h, dt, false, wantE ? h : 0.0, ctx->boxKE), st));
-  if (wantE)
-    for (int b = 0; b < nb; ++b)
-      CK(cudaMemcpyAsync(&energies[2 * ((size_t)(nsteps - 1) * nb + b)], ctx->boxKE + b, sizeof(double),
-                         cudaMemcpyDeviceToHost, st));
+  if (held == 0) first = nsteps;
+  if ((rc = kick(ctx, h, dt, false, slot(ctx->boxKE)))) return rc;
+  if (wantE && (rc = queue_energies(1))) return rc;
   CK(cudaEventRecord(ctx->e1, st));
+  CK(queue_status(ctx));
   CK(cudaStreamSynchronize(st));
-  rc = check_status(ctx);
+  if (wantE) store_energies(1);
+  rc = take_status(ctx);
   if (rc) return rc;
   ctx->forces_valid = true;
   if (stats) {
@@ -1747,7 +1839,7 @@ int examd_gpu_prepare_run(examd_ctx* ctx, double dt, int graph_chunk, int energi
   if (!ctx->atoms_set) return EXAMD_ERR_STATE;
   cudaSetDevice(ctx->dev);
   const int chunk = graph_chunk > 0 ? (graph_chunk + 1) / 2 * 2 : 0;
-  int rc = ensure_ebuf(ctx, std::max(chunk, 1) + 1);
+  int rc = ensure_ebuf(ctx, std::max(chunk, energies ? kEagerSlots : 1) + 1, energies != 0);
   if (rc) return rc;
   if (!ctx->forces_valid) {
     rc = run_pair(ctx, false, false);
@@ -1780,7 +1872,7 @@ int examd_gpu_time_phases(examd_ctx* ctx, int nsteps, double dt, double* ms) {
   for (int k = 0; k < nsteps; ++k) {
     // one steady-state step (merged kick), as the captured loop runs it
     CK(cudaEventRecord(ctx->e0, st));
-    CK(launch_kick(kick_args(ctx, dt, dt, true, 0.0, nullptr), st));
+    CK(launch_kick(kick_args(ctx, dt, dt, true, 0.0), st));
     CK(cudaEventRecord(ctx->e1, st));
     rc = ctx->list ? maybe_rebuild(ctx) : finish_binning(ctx, false);
     if (rc) return rc;

@@ -151,15 +151,10 @@ struct KickArgs {
   double ckick;  // dt or dt/2
   double dt;
   bool drift;
-  double hk;        // > 0: also the kinetic energy at v + hk F / m, per box
+  double hk;        // > 0: also the kinetic energy at v + hk F / m, per atom
   double ckm[4];    // ckick / m per type
   double hkm[4];    // hk / m per type
-  double* keAtom;   // per-atom kinetic energy scratch (N)
-  double* boxKE;    // per-box kinetic energy (fixed-order reduction of keAtom)
-  double* partial;  // chunk partial sums of that reduction
-  int maxc;         // chunks per box
-  const int64_t* atom0;  // nboxes + 1 atom offsets (sorted order is grouped by box)
-  int nboxes;
+  double* keAtom;   // per-atom kinetic energy (N), summed per box by launch_box_sums
   LJTable lj;
   // binning outputs (drift only)
   int* cellOld;

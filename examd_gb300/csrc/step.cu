@@ -361,7 +361,6 @@ cudaError_t launch_gather_pos_list(int64_t i0, int64_t i1, const double* aos, co
 
 cudaError_t launch_kick(const KickArgs& k, cudaStream_t st) {
   if (k.s.N > 0) k_kick<<<(unsigned)((k.s.N + 255) / 256), 256, 0, st>>>(k);
-  if (k.hk > 0.0) return launch_box_sums(k.nboxes, k.atom0, k.maxc, k.keAtom, k.partial, k.boxKE, st);
   return cudaGetLastError();
 }
 
