@@ -611,7 +611,8 @@ int examd_gpu_create(const examd_params* params, int nboxes, const examd_box* bo
     lj.p32[k].rcut2 = p.potential == EXAMD_POT_WCA ? (float)rcut2 : INFINITY;
     lj.p32[k].eshift = (float)eshift;
     lj.p32[k].rl2 = (float)((r + skin) * (r + skin));
-    lj.p32[k].r2big = (float)r2_of_force(e, s, kFixMaxForce);
+    // (not below kR2Min32, so that a pair-function error is found among the large terms)
+    lj.p32[k].r2big = std::max((float)r2_of_force(e, s, kFixMaxForce), 1e-12f);
     rc2max = std::max(rc2max, lj.p32[k].rc2);
   }
   lj.rc2max = rc2max;

@@ -70,8 +70,10 @@ struct PairArgs {
   unsigned* redo_done;
   // pair-list mode, per tile (lslots staged-atom slots, a multiple of 32, of
   // up to lk entries each, lk a multiple of 8 and at most 1024): the staged
-  // atoms in the order of their entry counts, most first (lperm), and their
-  // counts in that order (lcnt); the entries, the staged indices m of the
+  // atoms in the order of their entry counts, most first (lperm, with several
+  // types the atom's type above 14 bits), and their
+  // counts in that order (lcnt); the entries, the staged indices m (with several
+  // types m's type above 14 bits) of the
   // pairs (i, m) that the tile owns within the list cutoff, in that order by
   // groups of 32 atoms, entries k..k+3 of the group's 32 atoms side by side
   // (list[tile][p / 32][k / 4][p % 32][k % 4] for the atom at position p),

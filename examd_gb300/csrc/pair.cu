@@ -45,6 +45,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 // The list build returns before the write-back that the other passes of the
@@ -157,7 +158,7 @@ __host__ __device__ inline Layout make_layout(bool fp64, int cap, int ne_max, in
     L.fa = o;   o = align16(o + 3 * 8 * cap);  // FP64 force sums (kFixed: low words, then high words)
     L.px = o;   o = align16(o + 3 * 8 * cap);  // FP64 (kFixed: fixed-point) positions
   } else {
-    L.fa = o;   o = align16(o + (mode == kListBuild ? 1 : 3) * 4 * cap);  // fixed-point force sums (build: counts)
+    L.fa = o;   o = align16(o + (mode == kListBuild ? 1 : 3) * 4 * cap);  // fixed-point force sums, x y z per atom (build: counts)
     L.px = o;
   }
   L.code = o;   o = align16(o + 2 * cap);
@@ -263,9 +264,9 @@ __device__ __forceinline__ void pair_force32(bool act, int i, int m, float4 d, c
     ix = __float2int_rn(fx);
     iy = __float2int_rn(fy);
     iz = __float2int_rn(fz);
-    atomicAdd(&fa[m], -ix);
-    atomicAdd(&fa[cap + m], -iy);
-    atomicAdd(&fa[2 * cap + m], -iz);
+    atomicAdd(&fa[3 * m], -ix);
+    atomicAdd(&fa[3 * m + 1], -iy);
+    atomicAdd(&fa[3 * m + 2], -iz);
   }
   if (big) {
     if (SIDE) {
@@ -297,9 +298,9 @@ __device__ __forceinline__ void pair_force32(bool act, int i, int m, float4 d, c
   }
   const bool tail = lane == 31 || dist == kSeg - 1 || ((hb >> (lane + 1)) & 1u);
   if (i >= 0 && tail && (ix | iy | iz) != 0) {
-    atomicAdd(&fa[i], ix);
-    atomicAdd(&fa[cap + i], iy);
-    atomicAdd(&fa[2 * cap + i], iz);
+    atomicAdd(&fa[3 * i], ix);
+    atomicAdd(&fa[3 * i + 1], iy);
+    atomicAdd(&fa[3 * i + 2], iz);
   }
 }
 
@@ -612,6 +613,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
           ljs64[k] = A.lj.p64[k];
         else
           ljs32[k] = A.lj.p32[k];
+        if (MODE == kList) ljs32[k].m24eps *= kFix;  // (a power of two: the same bits)
       }
   }
   // Per-axis tables.  Ext coordinate l (cell X0 + l - 1, l = 0..E; l = E is
@@ -768,10 +770,12 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
           fd[c * cap + t] = 0.0;
         }
       } else {
-        // from a list: the type and the ext-cell code in w (the list pass
-        // reads both atoms' rows from them)
+        // from a list: the atom's row (ly, lz) as two bf16 numbers in w (the list
+        // pass subtracts both rows' at once; small integers, exact)
         pf[t] = make_float4(ox[lx] + u.x, u.y, u.z,
-                            kFromList ? __int_as_float((__float_as_int(u.w) & 3) | (cc << 2)) : u.w);
+                            kFromList ? __uint_as_float((__float_as_uint((float)ly) >> 16) |
+                                                        __float_as_uint((float)lz))
+                                      : u.w);
         if (FIX) {
           px[t] = to_fixed(xx[k][0], A.fx.ue) + (unsigned long long)(img[lx] * B.Lq[0]);
           px[cap + t] = to_fixed(xx[k][1], A.fx.ue) + (unsigned long long)(img[32 + ly] * B.Lq[1]);
@@ -784,7 +788,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
           if (MODE == kRedoBig || MODE == kRedoFull || MODE == kListBig) fr[c * cap + t] = 0.f;
           // (list build: fa holds the atoms' entry counts, one word each)
           if (MODE == kMain || MODE == kRedoFull || MODE == kList || (MODE == kListBuild && c == 0))
-            fa[c * cap + t] = 0;
+            fa[MODE == kListBuild ? t : 3 * t + c] = 0;
         }
       }
     }
@@ -832,9 +836,9 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   // entries beyond lk are counted, not written (the tile then goes to the
   // fallback list)
   const size_t ltile = (size_t)tile * A.lslots;
-  auto list_add = [&](bool acc, int key) {
+  auto list_add = [&](bool acc, int key, int tj) {
     if (!acc) return;
-    const int i = key & 0x3fff, m = (key >> 14) & 0x3fff;
+    const int i = key & 0x3fff, m = ((key >> 14) & 0x3fff) | (MULTI ? tj << 14 : 0);
     const int k = atomicAdd(&fa[i], 1);
     if (k < A.lk)
       A.lraw[EXAMD_IDX((ltile + i) * A.lk + k, (size_t)A.ntiles * A.lslots * A.lk, st)] = (unsigned short)m;
@@ -1007,7 +1011,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
       if (MODE == kRedoBig)
         redo_pair(acc, dq, key);
       else if (MODE == kListBuild)
-        list_add(acc, key);
+        list_add(acc, key, tj);
       else
         enqueue(acc, dq, key);
     }
@@ -1114,8 +1118,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
     const bool taby = B.remf[1] != 0.f && (Y0 == 0 || Y0 + ty >= B.nb[1]);
     const bool tabz = B.remf[2] != 0.f && (Z0 == 0 || Z0 + tz >= B.nb[2]);
     const float blf = B.blf;
-    // d as a float, exactly, without a conversion instruction (|d| < 2^22)
-    auto dfloat = [](int d) { return __fsub_rn(__int_as_float(0x4B400000 + d), 12582912.f); };
+    const float band0 = kBorder * q32.rc2, m24k0 = kFix * q32.m24eps;
     while (true) {
       int g = 0;
       if (lane == 0) g = atomicAdd(ucnt, 1);
@@ -1123,13 +1126,14 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
       if (g >= ng) break;
       const int r = g * 32 + lane;
       const bool vi = r < total;
-      const int i = vi ? perm[r] : 0;
+      const int ip = vi ? perm[r] : 0;
+      const int i = MULTI ? ip & 0x3fff : ip, ti = MULTI ? ip >> 14 : 0;
       const int cnt = vi ? cnts[r] : 0;
       const int gm = __shfl_sync(FULL, cnt, 0);  // the order puts the group's longest first
       const float4 pi = pf[i];
-      const int wi = __float_as_int(pi.w);
-      const int ti = wi & 3;
-      const int lyi = (wi >> 7) & 31, lzi = (wi >> 12) & 31;
+      const unsigned wi = __float_as_uint(pi.w);
+      const int ci = code[i];
+      const int lrow = ti * A.lj.nt;
       // entries k..k+3 of this lane: 8 bytes at brick k / 4 of the group
       const uint2* col = reinterpret_cast<const uint2*>(lst + (size_t)g * 32 * lk) + lane;
       // (every lane's bricks hold entries up to the group's longest, the
@@ -1147,30 +1151,33 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         const unsigned wv[2] = {cur.x, cur.y};
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const int m = (int)((wv[q >> 1] >> (16 * (q & 1))) & 0xffffu);
+          const unsigned en = (q & 1) ? wv[q >> 1] >> 16 : wv[q >> 1] & 0xffffu;
+          const int m = MULTI ? en & 0x3fff : en;  // the entry: the staged atom, and its type above 14 bits
           const float4 pj = pf[m];
-          const int wj = __float_as_int(pj.w);
-          const int lyj = (wj >> 7) & 31, lzj = (wj >> 12) & 31;
-          // (the table entry of rows l, l + d: l kDT + d + 2)
-          float cy, cz;
-          if constexpr (TAB) {
-            cy = dyt[lyi * (kDT - 1) + 2 + lyj].x;
-            cz = dzt[lzi * (kDT - 1) + 2 + lzj].x;
-          } else {
-            cy = __fmul_rn(dfloat(lyj - lyi), blf);
-            cz = __fmul_rn(dfloat(lzj - lzi), blf);
+          // y, z of atom i in the frame of atom j's row: (the row origins'
+          // offset) - pi, rounded once
+          float yi, zi;
+          if constexpr (TAB) {  // (the table entry of rows l, l + d: l kDT + d + 2)
+            const int cm = code[EXAMD_IDX(min(m, total - 1), cap, st)];
+            yi = dyt[((ci >> 5) & 31) * (kDT - 1) + 2 + ((cm >> 5) & 31)].x - pi.y;
+            zi = dzt[(ci >> 10) * (kDT - 1) + 2 + (cm >> 10)].x - pi.z;
+          } else {  // d bl, exact: both rows' differences d in one bf16x2 subtraction
+            const unsigned wj = __float_as_uint(pj.w);
+            const __nv_bfloat162 dr = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&wj),
+                                              *reinterpret_cast<const __nv_bfloat162*>(&wi));
+            const unsigned du = *reinterpret_cast<const unsigned*>(&dr);
+            yi = fmaf(__uint_as_float(du << 16), blf, -pi.y);
+            zi = fmaf(__uint_as_float(du & 0xffff0000u), blf, -pi.z);
           }
           float4 dq;
-          dq.x = pj.x + (-pi.x);
-          dq.y = pj.y + (cy - pi.y);
-          dq.z = pj.z + (cz - pi.z);
+          dq.x = pj.x - pi.x;
+          dq.y = pj.y + yi;
+          dq.z = pj.z + zi;
           dq.w = fmaf(dq.x, dq.x, fmaf(dq.y, dq.y, dq.z * dq.z));
-          const int tj = wj & 3;
-          const LJ32 P = MULTI ? ljs32[ti * A.lj.nt + tj] : q32;
-          bool acc = dq.w <= P.rc2;
-          if (MODE == kList && fabsf(dq.w - P.rc2) <= kBorder * P.rc2)
-            acc = inside64(i, m, ti, tj);  // at the border: the FP64 test
+          const int tj = MULTI ? en >> 14 : 0;
+          const LJ32 P = MULTI ? ljs32[lrow + tj] : q32;
           if (MODE == kListBig) {
+            bool acc = dq.w <= P.rc2;
             redo_pair(acc, dq, i | (m << 14) | (ti << 28) | (tj << 30));
           } else {
             // The LJ family's expression of pair_fn32 (the potential was
@@ -1178,31 +1185,42 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
             // entry applies: some lane of the warp takes nearly every entry,
             // so a branch would only add reconvergence, and without it the
             // four entries' arithmetic interleaves.  The same expressions:
-            // the same bits as pair_fn32 where it applies.
+            // the same bits as pair_fn32 where it applies.  The scale kFix is
+            // in m24 (a power of two).
+            const float m24 = MULTI ? P.m24eps : m24k0;
+            const float band = MULTI ? kBorder * P.rc2 : band0;
             const float ri = rcp_approx(dq.w);
             const float s2 = P.sig2 * ri;
             const float s6 = s2 * s2 * s2;
-            const float dg = P.m24eps * s6 * fmaf(2.f, s6, -1.f) * ri;
-            perr |= acc && !(dq.w >= kR2Min32);  // pair_fn32's error return
-            const bool app = acc && dq.w >= kR2Min32 && !(CUT && dq.w > P.rcut2);
+            const float dgs = m24 * s6 * fmaf(2.f, s6, -1.f) * ri;
+            // an entry applies within rc (and the potential's own range) unless its
+            // term is too large; the rest is rare: an r^2 at the border (the
+            // FP64 test), a large term (left to the redo pass), a pair-function
+            // error (r^2 < kR2Min32 <= r2big)
+            bool fix = dq.w <= P.rc2 && dq.w >= P.r2big && !(CUT && dq.w > P.rcut2);
+            bool app = fix;
+            if (fabsf(dq.w - P.rc2) <= band || dq.w < P.r2big) {
+              const bool acc = fabsf(dq.w - P.rc2) <= band ? inside64(i, m, ti, tj) : dq.w <= P.rc2;
+              perr |= acc && !(dq.w >= kR2Min32);
+              app = acc && dq.w >= kR2Min32 && !(CUT && dq.w > P.rcut2);
+              bigl |= app && dq.w < P.r2big;
+              fix = app && !(dq.w < P.r2big);
+            }
             if (ENERGY && app) {
               ek.add(P.c4eps * s6 * (s6 - 1.f) - P.eshift);
-              wk.add(-dg * dq.w);
+              wk.add(-(dgs * kFixInv) * dq.w);
             }
-            const bool big = app && dq.w < P.r2big;  // left to the redo pass
-            bigl |= big;
-            const bool fix = app && !big;
-            const float dgs = fix ? kFix * dg : 0.f;
-            const int ix = __float2int_rn(dgs * dq.x), iy = __float2int_rn(dgs * dq.y),
-                      iz = __float2int_rn(dgs * dq.z);
+            // atom m's terms; atom i's are the same with the other sign
+            const int jx = __float2int_rn(-(dgs * dq.x)), jy = __float2int_rn(-(dgs * dq.y)),
+                      jz = __float2int_rn(-(dgs * dq.z));
             if (fix) {
-              atomicAdd(&fa[m], -ix);
-              atomicAdd(&fa[cap + m], -iy);
-              atomicAdd(&fa[2 * cap + m], -iz);
+              atomicAdd(&fa[3 * m], jx);
+              atomicAdd(&fa[3 * m + 1], jy);
+              atomicAdd(&fa[3 * m + 2], jz);
+              sx -= jx;
+              sy -= jy;
+              sz -= jz;
             }
-            sx += ix;
-            sy += iy;
-            sz += iz;
           }
         }
       }
@@ -1212,9 +1230,9 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
       else
         walk(std::false_type{});
       if (MODE == kList && (sx | sy | sz) != 0) {
-        atomicAdd(&fa[i], sx);
-        atomicAdd(&fa[cap + i], sy);
-        atomicAdd(&fa[2 * cap + i], sz);
+        atomicAdd(&fa[3 * i], sx);
+        atomicAdd(&fa[3 * i + 1], sy);
+        atomicAdd(&fa[3 * i + 2], sz);
       }
     }
     if (bigl) *big_flag = 1;
@@ -1500,45 +1518,81 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
       }
     }
     __syncthreads();
-    for (int t = tid; t < total; t += blockDim.x) perm[atomicAdd(&hist[min((int)fa[t], lk)], 1)] = (unsigned short)t;
+    for (int t = tid; t < total; t += blockDim.x)
+      perm[atomicAdd(&hist[min((int)fa[t], lk)], 1)] = (unsigned short)(t | (MULTI ? __float_as_int(pf[t].w) << 14 : 0));
     __syncthreads();
-    // a lane moves its atom's entries eight at a time (16 bytes from the
-    // atom's scratch row, two 8-byte bricks that the warp's lanes store side
-    // by side); every lane fills the group's bricks up to the group's longest
-    // count, the entries past its own count naming the padding atom `total`
-    // (staged by the list passes beyond every cutoff), so that the list pass
-    // tests no per-lane count
+    // A lane moves its atom's entries from the scratch row into the group's
+    // bricks (4 entries of 32 lanes side by side); every lane fills the group's
+    // bricks up to the group's longest count, the entries past its own count
+    // naming the padding atom `total` (staged by the list passes beyond every
+    // cutoff), so that the list pass tests no per-lane count.
+    //
+    // On the way every 32 entries are put in an order that spreads the list
+    // pass's shared-memory reads: at step k its lane reads the 16-byte position
+    // of entry k, eight lanes a wavefront, and adds to three words of the same
+    // atom.  Entry k is therefore taken, where there is one, among those with
+    // m = lane + k modulo 8: eight neighbouring lanes then read eight different
+    // bank groups, and of the four lanes of one residue few meet in a bank.
+    // (Unordered, bank conflicts were 55 % of the list pass's shared wavefronts
+    // and those 68 % of its cycles.)  The entry of rank r in residue class c goes
+    // to step (c - lane) % 8 + 8 r, or, if that is past the atom's entries or
+    // taken, to the last free step.  The sums are exact integers, so the order
+    // changes no bit.
+    constexpr int kRowBytes = 72, kOrd = 32;  // a lane's row of kOrd entries; 18 words: 8-byte reads without conflicts
+    const int row0 = align16(L.perm < L.pf ? L.hist + 4 * (kMaxListK + 1) : L.queue);  // up to the counts at L.fa: free now
+    const int nrow = min(nw, (L.fa - row0) / (32 * kRowBytes));  // warps that have room for their rows
     const size_t nbrick = (size_t)A.ntiles * A.lslots * lk / 4;
     const unsigned short* raw = A.lraw + ltile * lk;
     (void)nbrick;
-    for (int g = warp; g * 32 < total; g += nw) {
+    for (int g = warp < nrow ? warp : total; g * 32 < total; g += nrow) {
       const int p = g * 32 + lane;
-      const int t = p < total ? perm[p] : 0;
+      const int pv = p < total ? perm[p] : 0;
+      const int t = MULTI ? pv & 0x3fff : pv;
       const int c = p < total ? min((int)fa[t], lk) : 0;
-      A.lperm[EXAMD_IDX(ltile + p, (size_t)A.lslots * A.ntiles, st)] = (unsigned short)t;
+      A.lperm[EXAMD_IDX(ltile + p, (size_t)A.lslots * A.ntiles, st)] = (unsigned short)pv;
       A.lcnt[EXAMD_IDX(ltile + p, (size_t)A.lslots * A.ntiles, st)] = (unsigned short)c;
       const int gm = __shfl_sync(FULL, c, 0);
-      const uint4* src = reinterpret_cast<const uint4*>(raw + (size_t)t * lk);
+      const unsigned short* own = raw + (size_t)t * lk;
+      unsigned short* row = (unsigned short*)(smem + row0 + (32 * warp + lane) * kRowBytes);
       const size_t b0 = (ltile + (size_t)g * 32) * lk / 4 + lane;  // brick k / 4 of this lane: b0 + (k / 4) * 32
       uint2* dst = reinterpret_cast<uint2*>(A.list);
-      // 32 entries a round: the four 16-byte reads issued before the stores
       const unsigned dd = (unsigned)total * 0x10001u;  // two padding entries
-      // word w of a 16-byte piece holds entries 2w, 2w + 1; n of the piece are the atom's
-      auto pad = [&](unsigned w, int n) { return n >= 2 ? w : (n == 1 ? (w & 0xffffu) | (dd & 0xffff0000u) : dd); };
-      for (int k0 = 0; k0 < gm; k0 += 32) {
-        uint4 v[4];
+      // word w holds two entries, left of them the atom's
+      auto pad = [&](unsigned w, int left) {
+        return left >= 2 ? w : (left == 1 ? (w & 0xffffu) | (dd & 0xffff0000u) : dd);
+      };
+      for (int k0 = 0; k0 < gm; k0 += kOrd) {
+        const int n = min(c - k0, kOrd);  // this lane's entries of the round
+        uint4 v[4];                       // the four 16-byte reads issued first
 #pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = k0 + 8 * u < c ? src[(k0 >> 3) + u] : make_uint4(dd, dd, dd, dd);
+        for (int u = 0; u < 4; ++u)
+          v[u] = 8 * u < n ? reinterpret_cast<const uint4*>(own + k0)[u] : make_uint4(0, 0, 0, 0);
+        unsigned cl = 0, ch = 0;  // entries so far of classes 0-3 and 4-7, 8 bits each
+        unsigned free = n >= 32 ? FULL : n > 0 ? (1u << n) - 1u : 0u;  // steps not taken
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const int k = k0 + 8 * u;
-          if (k < gm) {
-            const int n = c - k;
-            if (n < 8) v[u] = make_uint4(pad(v[u].x, n), pad(v[u].y, n - 2), pad(v[u].z, n - 4), pad(v[u].w, n - 6));
-            dst[EXAMD_IDX(b0 + (size_t)(k >> 2) * 32, nbrick, st)] = make_uint2(v[u].x, v[u].y);
-            if (k + 4 < gm)
-              dst[EXAMD_IDX(b0 + (size_t)((k >> 2) + 1) * 32, nbrick, st)] = make_uint2(v[u].z, v[u].w);
+          const unsigned w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+          if (k0 + 8 * u >= gm) break;
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const unsigned en = (q & 1) ? w[q >> 1] >> 16 : w[q >> 1] & 0xffffu;
+            const int sh = 8 * (en & 3);
+            const unsigned cc = (en & 4) ? ch : cl, ci = cc + (1u << sh);
+            int k = ((en - lane) & 7) + 8 * ((cc >> sh) & 255);
+            if (8 * u + q < n) {
+              cl = (en & 4) ? cl : ci;
+              ch = (en & 4) ? ci : ch;
+              if (k > 31 || !((free >> (k & 31)) & 1u)) k = 31 - __clz(free);
+              free ^= 1u << k;
+              row[k] = (unsigned short)en;
+            }
           }
+        }
+#pragma unroll
+        for (int k = 0; k < kOrd; k += 4) {
+          if (k0 + k >= gm) break;
+          const uint2 w = *reinterpret_cast<const uint2*>(row + k);
+          dst[EXAMD_IDX(b0 + (size_t)((k0 + k) >> 2) * 32, nbrick, st)] = make_uint2(pad(w.x, n - k), pad(w.y, n - k - 2));
         }
       }
     }
@@ -1595,8 +1649,8 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         float f[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c)
-          f[c] = MODE == kRedoFull ? fmaf((float)fa[c * cap + t], kFixInv, fr[c * cap + t])
-                                   : (float)fa[c * cap + t] * kFixInv;
+          f[c] = MODE == kRedoFull ? fmaf((float)fa[3 * t + c], kFixInv, fr[c * cap + t])
+                                   : (float)fa[3 * t + c] * kFixInv;
         F[EXAMD_IDX(g, A.N, st)] = make_float4(f[0], f[1], f[2], 0.f);
       }
     }
