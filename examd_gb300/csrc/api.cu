@@ -55,7 +55,7 @@ bool class_ok(int cls, int h) {  // home offset h keeps the home cell inside the
 
 // Derive the row structure and the per-class ownership masks from the table.
 // Returns false if the table does not have the expected shape.
-bool build_own_lut(OwnLut& L) {
+bool build_own_lut(OwnLut& L, signed char (*rowsOut)[2] = nullptr, unsigned char (*byRow)[kRows] = nullptr) {
   std::memset(&L, 0, sizeof(L));
   std::vector<std::pair<int, int>> rows;
   std::map<std::pair<int, int>, std::map<int, std::array<int, 3>>> byrow;
@@ -72,8 +72,10 @@ bool build_own_lut(OwnLut& L) {
   if (rows.size() != 12 || byrow.size() != 13) return false;
   rows.push_back({0, 0});
   for (int r = 0; r < kRows; ++r) {
-    L.rows[r][0] = (signed char)rows[r].first;
-    L.rows[r][1] = (signed char)rows[r].second;
+    if (rowsOut) {
+      rowsOut[r][0] = (signed char)rows[r].first;
+      rowsOut[r][1] = (signed char)rows[r].second;
+    }
     const auto& m = byrow[rows[r]];
     if (r < 12) {
       if (m.size() != 5) return false;
@@ -92,10 +94,10 @@ bool build_own_lut(OwnLut& L) {
             if (class_ok(cx, h[0]) && class_ok(cy, h[1]) && class_ok(cz, h[2])) mask |= 1u << (kv.first + 2);
           }
           if (r == kRows - 1 && class_ok(cx, 0) && class_ok(cy, 0) && class_ok(cz, 0)) mask |= 1u << 2;
-          if (mask) {
-            L.lut[cls][L.nrow[cls]] = (unsigned char)mask;  // by position in the class's row list
-            L.rlist[cls][L.nrow[cls]++] = (unsigned char)r;
-          }
+          if (byRow) byRow[cls][r] = (unsigned char)mask;
+          if (mask)
+            L.ent[cls][L.nrow[cls]++] =
+                (unsigned short)(mask | ((unsigned)(rows[r].first + 2) << 5) | ((unsigned)(rows[r].second + 2) << 8));
         }
       }
   return true;
@@ -244,7 +246,6 @@ struct examd_ctx {
   PairConfig pc;
   int cap = 0, smem = 0, smem_limit = 0;
   int cap_redo = 0;     // staged-atom capacity of the redo pass
-  int pair_tables = 0;  // examd_params.pair_tables
   int dev = 0;
   cudaStream_t st = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr, e3 = nullptr;
@@ -337,7 +338,6 @@ struct examd_ctx {
     cudaGraphExec_t exec = nullptr;
     const void *pos = nullptr, *forces = nullptr, *epot = nullptr, *virial = nullptr;
     int accumulate = -1, cap = 0, cap_redo = 0, list_gen = 0;
-    bool pack = false;
   } io_graph[2];
 
   int cuda_fail(cudaError_t e, const char* what) {
@@ -483,12 +483,7 @@ const char* examd_gpu_last_error(examd_ctx* ctx) { return ctx ? ctx->lasterr.c_s
 int examd_own_table(signed char* rows, unsigned char* lut) {
   if (!rows || !lut) return EXAMD_ERR_ARG;
   OwnLut L;
-  if (!build_own_lut(L)) return EXAMD_ERR_ARG;
-  std::memcpy(rows, L.rows, sizeof(L.rows));
-  std::memset(lut, 0, sizeof(L.lut));  // by row, as the header documents it
-  for (int c = 0; c < kClasses; ++c)
-    for (int n = 0; n < L.nrow[c]; ++n) lut[c * kRows + L.rlist[c][n]] = L.lut[c][n];
-  return EXAMD_OK;
+  return build_own_lut(L, (signed char(*)[2])rows, (unsigned char(*)[kRows])lut) ? EXAMD_OK : EXAMD_ERR_ARG;
 }
 
 int examd_host_alloc(void** ptr, int64_t bytes) {
@@ -548,8 +543,6 @@ int examd_gpu_create(const examd_params* params, int nboxes, const examd_box* bo
   ctx->pc.fp64 = p.precision == EXAMD_FP64;
   ctx->pc.multi = nt > 1;
   ctx->pc.cut = p.potential == EXAMD_POT_WCA;
-  ctx->pc.pack = p.pair_tables == 2;
-  ctx->pair_tables = p.pair_tables;
   if (p.pair_tables < 0 || p.pair_tables > 2 || p.tile_balance < 0 || p.tile_balance > 1) {
     delete ctx;
     return EXAMD_ERR_ARG;
@@ -618,16 +611,19 @@ int examd_gpu_create(const examd_params* params, int nboxes, const examd_box* bo
   lj.rc2max = rc2max;
   // pair-list mode: atoms may be up to skin/2 outside the cells they were
   // sorted into, so an enumeration between builds prunes at rc + skin/2
-  const double reach_now = rcmax + 0.5 * skin + 1e-4;
+  // The margin covers the rounding of the FP32 coordinates, at most 18 cell
+  // edges from the tile's centre: 1e-4, or 2e-5 of the edge where lengths are large
+  const double margin = std::max(1e-4, 2e-5 * bl), reach_now = rcmax + 0.5 * skin + margin;
   lj.prune2 = (float)(reach_now * reach_now);
-  lj.prune2_list = (float)((reach + 1e-4) * (reach + 1e-4));
+  lj.prune2_list = (float)((reach + margin) * (reach + margin));
   for (int a = 0; a < EXAMD_MAX_TYPES; ++a) {
     double m = (a < nt && p.mass[a] > 0) ? p.mass[a] : 1.0;
     lj.mass[a] = m;
     lj.minv[a] = 1.0 / m;
   }
 
-  ctx->pc.fix = ctx->pc.fp64 && build_fix(lj, p, ctx->fx);
+  // (the prefilter's margin covers the FP32 coordinates for edges up to 8 rc)
+  ctx->pc.fix = ctx->pc.fp64 && bl <= 8.0 * rcmax && build_fix(lj, p, ctx->fx);
 
   // Tiles of a batch: the tile edge T is the densest box's.  A box with fewer
   // atoms per cell gets tiles up to 2 cells longer per axis, as long as its
@@ -1026,32 +1022,13 @@ int apply_capacity(examd_ctx* ctx, bool* grew = nullptr) {
   int want_r = std::max(((occ + occ / 4 + 64) + 7) & ~7, ctx->cap_redo);
   int want = ctx->pc.fp64 && !ctx->pc.fix ? want_r : ((occ + occ / 16 + 32) + 7) & ~7;
   if (want <= ctx->cap) return EXAMD_OK;
-  // mixed form with pair_tables = 0: the compact per-warp tables where they
-  // fit more CTAs on an SM at this capacity (or where only they fit at all)
-  auto choose = [&](int cap) {
-    PairConfig c = ctx->pc;
-    if (c.fp64 || ctx->pair_tables != 0) return c;
-    PairConfig w = c, k = c;
-    w.pack = false;
-    k.pack = true;
-    for (int e = 0; e < 2; ++e) {  // the occupancy query needs the opt-in limit set
-      PairConfig q = e ? k : w;
-      if (pair_prepare(q, ctx->smem_limit) != cudaSuccess) return c;
-    }
-    c.pack = pair_smem_bytes(w, cap, want_r, ctx->ne_max, ctx->ext_max) > ctx->smem_limit ||
-             pair_blocks_per_sm(k, cap, ctx->ne_max, ctx->ext_max) > pair_blocks_per_sm(w, cap, ctx->ne_max, ctx->ext_max);
-    return c;
-  };
-  PairConfig pc = choose(want);
-  int bytes = pair_smem_bytes(pc, want, want_r, ctx->ne_max, ctx->ext_max);
+  int bytes = pair_smem_bytes(ctx->pc, want, want_r, ctx->ne_max, ctx->ext_max);
   if (bytes > ctx->smem_limit) {
     // fall back to the exact need if the headroom does not fit
     want = want_r = (occ + 7) & ~7;
-    pc = choose(want);
-    bytes = pair_smem_bytes(pc, want, want_r, ctx->ne_max, ctx->ext_max);
+    bytes = pair_smem_bytes(ctx->pc, want, want_r, ctx->ne_max, ctx->ext_max);
     if (bytes > ctx->smem_limit) return EXAMD_ERR_CELL_OVERFLOW;
   }
-  ctx->pc.pack = pc.pack;
   ctx->cap = want;
   ctx->cap_redo = want_r;
   ctx->smem = bytes;
@@ -1538,7 +1515,7 @@ int examd_gpu_forces_at(examd_ctx* ctx, const double* pos, double* forces, doubl
   auto& g = ctx->io_graph[ctx->cur];
   const bool hit = g.exec && g.pos == pos && g.forces == forces && g.epot == epot && g.virial == virial &&
                    g.accumulate == accumulate && g.cap == ctx->cap && g.cap_redo == ctx->cap_redo &&
-                   g.pack == ctx->pc.pack && g.list_gen == ctx->list_gen;
+                   g.list_gen == ctx->list_gen;
   if (!hit) {
     if (g.exec) cudaGraphExecDestroy(g.exec);
     g = examd_ctx::IoGraph{};
@@ -1563,7 +1540,6 @@ int examd_gpu_forces_at(examd_ctx* ctx, const double* pos, double* forces, doubl
     g.accumulate = accumulate;
     g.cap = ctx->cap;
     g.cap_redo = ctx->cap_redo;
-    g.pack = ctx->pc.pack;
     g.list_gen = ctx->list_gen;
   }
   CK(cudaGraphLaunch(g.exec, ctx->st));

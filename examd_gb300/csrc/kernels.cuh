@@ -101,7 +101,6 @@ struct PairConfig {
   bool fp64 = false;
   bool fix = false;     // FP64 form: fixed-point first pass (the FP64 pass then only redoes listed tiles)
   bool multi = false;   // more than one atom type
-  bool pack = false;    // mixed form: compact per-warp tables (more CTAs per SM)
   bool energy = false;  // potential energy and virial
   bool count = false;   // candidate / accepted counters
   bool list = false;    // mixed form: pair-list mode (forces from the per-tile lists)
@@ -113,8 +112,6 @@ struct PairConfig {
 // pass's need at cap and, mixed form, the redo pass's at cap_redo.
 int pair_smem_bytes(const PairConfig& cfg, int cap, int cap_redo, int ne_max, int ext_max);
 cudaError_t pair_prepare(const PairConfig& cfg, int smem_bytes);  // opt-in smem attribute
-// Resident CTAs per SM of the pair kernel at this capacity (occupancy calculator).
-int pair_blocks_per_sm(const PairConfig& cfg, int cap, int ne_max, int ext_max);
 cudaError_t launch_pair(const PairConfig& cfg, const PairArgs& a, int ntiles, int smem_bytes, cudaStream_t st);
 // Pair-list mode: build the per-tile lists (gated by a.gate).
 cudaError_t launch_pair_build(const PairConfig& cfg, const PairArgs& a, int ntiles, int smem_bytes, cudaStream_t st);

@@ -109,15 +109,10 @@ struct Layout {
   int bytes;
 };
 
-// Per-warp tables after the accepted-pair queues.  Mixed form: one step's
-// items by rank (ptA float4 + ptB) and the work unit's atoms by rank (btA
-// float4 + btB); wide: ptB int4, btB float4 of full values; compact: ptB
-// int2 with two 16-bit offsets, the atom's squared x-gaps as FP16 rounded
-// toward zero (so the pruning stays conservative) and btB int2.  The host
-// takes the compact tables where they fit more CTAs on an SM.  FP64 form: one
-// step's items by lane (float4).
-constexpr int kWarpTabWide = 32 * 16 + 32 * 16 + 32 * 16 + 32 * 16;
-constexpr int kWarpTabCompact = 32 * 16 + 32 * 8 + 32 * 16 + 32 * 8;
+// Per-warp tables after the accepted-pair queues.  Mixed form and kFixed: one
+// step's items by rank (pt, float4) and the work unit's atoms by rank (bt, two
+// float4).  FP64 form: one step's items by lane (float4).
+constexpr int kWarpTab = 32 * 16 + 32 * 32;
 constexpr int kWarpTabFp64 = 32 * 16;
 
 __host__ __device__ inline int align16(int x) { return (x + 15) & ~15; }
@@ -130,7 +125,7 @@ __host__ __device__ inline int align16(int x) { return (x + 15) & ~15; }
 // reduction scratch; kListBig's fr after everything).
 // ne_max, ext_max: the largest tile's ext cells and ext extent on one axis.
 __host__ __device__ inline Layout make_layout(bool fp64, int cap, int ne_max, int ext_max, int nw, int mode,
-                                              bool pack, bool multi) {
+                                              bool multi) {
   const bool from_list = mode == kList || mode == kListBig;
   Layout L;
   int o = 0;
@@ -139,7 +134,7 @@ __host__ __device__ inline Layout make_layout(bool fp64, int cap, int ne_max, in
   L.ox = o;     o = align16(o + 4 * (ext_max + 1));
   L.oy = o;     o = align16(o + 4 * (ext_max + 1));
   L.oz = o;     o = align16(o + 4 * (ext_max + 1));
-  L.dyt = o;    o = align16(o + 8 * ext_max * kDT);  // float2 (row origin offset, near face) per (l, d)
+  L.dyt = o;    o = align16(o + 8 * ext_max * kDT);  // float2 (row origin offset, near face, both from row l) per (l, d)
   L.dzt = o;    o = align16(o + 8 * ext_max * kDT);
   const bool fix = mode == kFixed;
   L.img = o;    o = align16(o + (fp64 || fix ? 3 * 32 : 0));  // periodic image per ext coordinate (FP64 form)
@@ -149,9 +144,8 @@ __host__ __device__ inline Layout make_layout(bool fp64, int cap, int ne_max, in
   // the LJ table per ordered type pair (several types): per-lane type indices
   // would serialise on the kernel-parameter bank, shared memory serves them at once
   L.ljt = o;    o = align16(o + (multi ? (fix ? (int)sizeof(FixPair) : (int)sizeof(LJ64)) * EXAMD_MAX_TYPES * EXAMD_MAX_TYPES : 0));
-  const int tab = pack ? kWarpTabCompact : kWarpTabWide;
   const int qbytes = (fp64 ? 4 * kQueue + kWarpTabFp64
-                           : (from_list ? 64 : (mode == kListBuild ? 0 : fix ? 4 : 16) * kQueue + tab)) * nw;
+                           : (from_list ? 64 : (mode == kListBuild ? 0 : fix ? 4 : 16) * kQueue + kWarpTab)) * nw;
   L.queue = o;  o = align16(o + qbytes);
   L.pf = o;     o = align16(o + 16 * (from_list ? cap + 1 : cap));  // list passes: + the padding atom
   if (fp64 || fix) {
@@ -182,10 +176,10 @@ __host__ __device__ inline Layout make_layout(bool fp64, int cap, int ne_max, in
 }
 
 static int redo_smem_bytes(const PairConfig& cfg, int cap_redo, int ne_max, int ext_max) {
-  if (cfg.fix) return make_layout(true, cap_redo, ne_max, ext_max, cfg.warps, kRedoFull, false, cfg.multi).bytes;
-  const int b = std::max(make_layout(false, cap_redo, ne_max, ext_max, cfg.warps, kRedoBig, cfg.pack, cfg.multi).bytes,
-                         make_layout(false, cap_redo, ne_max, ext_max, cfg.warps, kRedoFull, cfg.pack, cfg.multi).bytes);
-  return cfg.list ? std::max(b, make_layout(false, cap_redo, ne_max, ext_max, cfg.warps, kListBig, cfg.pack, cfg.multi).bytes)
+  if (cfg.fix) return make_layout(true, cap_redo, ne_max, ext_max, cfg.warps, kRedoFull, cfg.multi).bytes;
+  const int b = std::max(make_layout(false, cap_redo, ne_max, ext_max, cfg.warps, kRedoBig, cfg.multi).bytes,
+                         make_layout(false, cap_redo, ne_max, ext_max, cfg.warps, kRedoFull, cfg.multi).bytes);
+  return cfg.list ? std::max(b, make_layout(false, cap_redo, ne_max, ext_max, cfg.warps, kListBig, cfg.multi).bytes)
                   : b;
 }
 
@@ -193,17 +187,17 @@ static int redo_smem_bytes(const PairConfig& cfg, int cap_redo, int ne_max, int 
 // counters, which the enumeration gives) the list pass's.
 static int main_smem_bytes(const PairConfig& cfg, int cap, int ne_max, int ext_max) {
   const int mode = (cfg.list && !cfg.count && !cfg.fp64) ? kList : kMain;
-  if (cfg.fix) return make_layout(false, cap, ne_max, ext_max, cfg.warps, kFixed, true, cfg.multi).bytes;
-  return make_layout(cfg.fp64, cap, ne_max, ext_max, cfg.warps, mode, cfg.pack, cfg.multi).bytes;
+  if (cfg.fix) return make_layout(false, cap, ne_max, ext_max, cfg.warps, kFixed, cfg.multi).bytes;
+  return make_layout(cfg.fp64, cap, ne_max, ext_max, cfg.warps, mode, cfg.multi).bytes;
 }
 
 static int build_smem_bytes(const PairConfig& cfg, int cap, int ne_max, int ext_max) {
-  return make_layout(false, cap, ne_max, ext_max, kBuildWarps, kListBuild, cfg.pack, cfg.multi).bytes;
+  return make_layout(false, cap, ne_max, ext_max, kBuildWarps, kListBuild, cfg.multi).bytes;
 }
 
 int pair_smem_bytes(const PairConfig& cfg, int cap, int cap_redo, int ne_max, int ext_max) {
   if (cfg.fix) return std::max(main_smem_bytes(cfg, cap, ne_max, ext_max), redo_smem_bytes(cfg, cap_redo, ne_max, ext_max));
-  int b = make_layout(cfg.fp64, cap, ne_max, ext_max, cfg.warps, kMain, cfg.pack, cfg.multi).bytes;
+  int b = make_layout(cfg.fp64, cap, ne_max, ext_max, cfg.warps, kMain, cfg.multi).bytes;
   if (cfg.fp64) return b;
   b = std::max(b, redo_smem_bytes(cfg, cap_redo, ne_max, ext_max));
   if (cfg.list) b = std::max(b, std::max(main_smem_bytes(cfg, cap, ne_max, ext_max),
@@ -305,7 +299,7 @@ __device__ __forceinline__ void pair_force32(bool act, int i, int m, float4 d, c
 }
 
 // Forces of cnt queued accepted pairs, one per lane: entry = (d = x_j - x_i,
-// key) with key = i | j << 14 | type_i << 28 | type_j << 30; r^2 is recomputed
+// key) with key = i | type_i << 14 | j << 16 | type_j << 30; r^2 is recomputed
 // with the distance test's expression, so it has the same bits.  user_func.f90:58-69
 // in FP32: dg = -24 eps (2 s^12 - s^6) / r^2, f_i += dg d, f_j -= dg d.
 // The queue keeps an atom's accepted pairs next to each other, so the i-side
@@ -332,8 +326,8 @@ __device__ __forceinline__ void force_batch(int cnt, int qh, const QD& qd, FA& f
     const unsigned key = __float_as_uint(d.w);
     d.w = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));  // r^2 exactly as the distance test computed it
     i = key & 0x3fff;
-    m = (key >> 14) & 0x3fff;
-    if (MULTI) P = ljs[((key >> 28) & 3) * A.lj.nt + (key >> 30)];
+    m = (key >> 16) & 0x3fff;
+    if (MULTI) P = ljs[((key >> 14) & 3) * A.lj.nt + (key >> 30)];
   }
   pair_force32<ENERGY, COUNT, SIDE>(act, i, m, d, P, fa, fr, cap, A, ek, wk, nacc, big_flag);
 }
@@ -351,7 +345,7 @@ __device__ __forceinline__ void force_batch64(int cnt, const QK& qk, const PD& p
   const int lane = threadIdx.x & 31;
   if (lane >= cnt) return;
   const unsigned key = (unsigned)qk[(qh + lane) & (kQueue - 1)];
-  const int i = key & 0x3fff, m = (key >> 14) & 0x3fff;
+  const int i = key & 0x3fff, m = (key >> 16) & 0x3fff;
   const int ci = code[i], cm = code[m];
   // difference of the copies' periodic images per axis: -1, 0 or +1 box
   const int nx = img[cm & 31] - img[ci & 31];
@@ -365,7 +359,7 @@ __device__ __forceinline__ void force_batch64(int cnt, const QK& qk, const PD& p
   if (nz) dz = __dadd_rn(dz, nz > 0 ? Lbox[2] : -Lbox[2]);
   const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
   LJ64 P = lj.p64[0];
-  if (MULTI) P = ljs[((key >> 28) & 3) * lj.nt + (key >> 30)];
+  if (MULTI) P = ljs[((key >> 14) & 3) * lj.nt + (key >> 30)];
   double dg = 0.0, e = 0.0;
   const int rv = pair_fn64<ENERGY>(lj.pot, d2, P, dg, e);
   if (rv == 0) {
@@ -429,8 +423,8 @@ __device__ __forceinline__ void force_batch_fix(int cnt, int qh, const QK& qk, c
   if (lane < cnt) {
     const unsigned key = (unsigned)qk[(qh + lane) & (kQueue - 1)];
     i = key & 0x3fff;
-    m = (key >> 14) & 0x3fff;
-    const int ti = MULTI ? (key >> 28) & 3 : 0, tj = MULTI ? key >> 30 : 0;
+    m = (key >> 16) & 0x3fff;
+    const int ti = MULTI ? (key >> 14) & 3 : 0, tj = MULTI ? key >> 30 : 0;
     const FixPair P = MULTI ? ljx[ti * A.lj.nt + tj] : A.fx.p[0];
     long long dx = (long long)(px[m] - px[i]);
     long long dy = (long long)(px[cap + m] - px[cap + i]);
@@ -547,7 +541,7 @@ __device__ __forceinline__ void force_batch_fix(int cnt, int qh, const QK& qk, c
 //   the list was built), outputs, energy and the large-term flag as there;
 // - kListBig: kRedoBig from the list.
 // CUT (list pass): the potential's own range rcut2 is tested (WCA; infinite otherwise).
-template <bool FP64, bool MULTI, bool ENERGY, bool COUNT, int MODE, bool PACK, bool CUT = true>
+template <bool FP64, bool MULTI, bool ENERGY, bool COUNT, int MODE, bool CUT = true>
 __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   extern __shared__ __align__(16) unsigned char smem[];
   const unsigned FULL = 0xffffffffu;
@@ -562,7 +556,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   if (kFromList && MODE == kList && A.lcount[tile] < 0) return;  // a fallback tile: the redo pass computes it
   constexpr bool FIX = MODE == kFixed;
   const int cap = (MODE == kMain || MODE == kListBuild || MODE == kList || FIX) ? A.cap : A.cap_redo;
-  const Layout L = make_layout(FP64, cap, A.ne_max, A.ext_max, nw, MODE, PACK, MULTI);
+  const Layout L = make_layout(FP64, cap, A.ne_max, A.ext_max, nw, MODE, MULTI);
   // shared-memory arrays (index-checked in the checked build)
   int* const st = A.status;  // the index checks' status word (checked build)
   (void)st;
@@ -577,7 +571,6 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   double* red = (double*)(smem + L.queue);  // scan and reduction scratch, before and after the queues' use
   int* cw = (int*)(smem + L.cw);
   OwnLut* sown = (OwnLut*)(smem + L.lut);
-  const signed char* srows = &sown->rows[0][0];
   LJ32* ljs32 = (LJ32*)(smem + L.ljt);
   LJ64* ljs64 = (LJ64*)(smem + L.ljt);
   FixPair* ljx = (FixPair*)(smem + L.ljt);
@@ -622,8 +615,8 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   // box's last cell.  o*[l]: origin relative to the tile centre, FP32 (the
   // multiple of bl is exact, so the value is rounded once).  d*t[l*6 + d + 2]
   // (y, z): the origin difference between ext rows l and l + d (d = -2..3),
-  // rounded once, and o*[l + d + (d < 0)], the near face of row l + d seen
-  // from row l (the same value as the o* entry).  img[32a + l] (FP64 form): n.
+  // rounded once, and the same for l + d + (d < 0), the near face of row l + d
+  // seen from row l.  img[32a + l] (FP64 form): n.
   {
     const int a = tid >> 5, l = tid & 31;
     if (a < 3) {
@@ -648,7 +641,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
               const int l2 = l + d, ln = l + d + (d < 0);
               const float off = (l2 >= 0 && l2 <= E) ? fmaf((float)(nimg(l2) - n), rf, (float)d * blf) : 0.f;
               const float near =
-                  (ln >= 0 && ln <= E) ? fmaf((float)(2 * (ln - 1) - t), 0.5f * blf, (float)nimg(ln) * rf) : 0.f;
+                  (ln >= 0 && ln <= E) ? fmaf((float)(nimg(ln) - n), rf, (float)(d + (d < 0)) * blf) : 0.f;
               dt[l * kDT + d + 2] = make_float2(off, near);
             }
           }
@@ -815,16 +808,12 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   constexpr int kQe = FP64 || FIX ? 4 : (MODE == kListBuild ? 0 : 16);
   auto qd = EXAMD_ARR(float4, (float4*)(smem + L.queue) + warp * kQueue, kQueue, st);
   auto qk = EXAMD_ARR(int, (int*)(smem + L.queue) + warp * kQueue, kQueue, st);
-  // per-warp tables (kWarpTab*): one step's items (ptA, ptB) and, mixed
-  // form, the work unit's atoms (bt)
-  unsigned char* wtab =
-      smem + L.queue + kQe * kQueue * nw + warp * (FP64 ? kWarpTabFp64 : (PACK ? kWarpTabCompact : kWarpTabWide));
-  auto ptA = EXAMD_ARR(float4, wtab, 32, st);
-  auto ptB2 = EXAMD_ARR(int2, wtab + 32 * 16, 32, st);  // the compact layout's view
-  auto ptB4 = EXAMD_ARR(int4, wtab + 32 * 16, 32, st);  // the wide layout's view
-  auto btA = EXAMD_ARR(float4, wtab + (PACK ? 32 * 24 : 32 * 32), 32, st);
-  auto btB2 = EXAMD_ARR(int2, wtab + (PACK ? 32 * 40 : 32 * 48), 32, st);
-  auto btB4 = EXAMD_ARR(float4, wtab + (PACK ? 32 * 40 : 32 * 48), 32, st);
+  // per-warp tables: one step's items (pt) and, but for the FP64 form, the
+  // work unit's atoms (bt)
+  unsigned char* wtab = smem + L.queue + kQe * kQueue * nw + warp * (FP64 ? kWarpTabFp64 : kWarpTab);
+  auto pt = EXAMD_ARR(float4, wtab, 32, st);
+  auto btA = EXAMD_ARR(float4, wtab + 32 * 16, 32, st);
+  auto btB = EXAMD_ARR(float4, wtab + 32 * 32, 32, st);
   int qn = 0, qh = 0;  // queued pairs and the ring's head
   const unsigned lt = (1u << lane) - 1u;
   const unsigned le = FULL >> (31 - lane);
@@ -836,9 +825,9 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   // entries beyond lk are counted, not written (the tile then goes to the
   // fallback list)
   const size_t ltile = (size_t)tile * A.lslots;
-  auto list_add = [&](bool acc, int key, int tj) {
+  auto list_add = [&](bool acc, int key) {
     if (!acc) return;
-    const int i = key & 0x3fff, m = ((key >> 14) & 0x3fff) | (MULTI ? tj << 14 : 0);
+    const int i = key & 0x3fff, m = (int)((unsigned)key >> 16);  // with several types: m and its type above 14 bits
     const int k = atomicAdd(&fa[i], 1);
     if (k < A.lk)
       A.lraw[EXAMD_IDX((ltile + i) * A.lk + k, (size_t)A.ntiles * A.lslots * A.lk, st)] = (unsigned short)m;
@@ -918,9 +907,9 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   // terms, decided exactly as force_batch decides them, are summed (both atoms)
   auto redo_pair = [&](bool acc, const float4& dq, int key) {
     if (!acc) return;
-    const int i = key & 0x3fff, m = (key >> 14) & 0x3fff;
+    const int i = key & 0x3fff, m = (key >> 16) & 0x3fff;
     LJ32 P = A.lj.p32[0];
-    if (MULTI) P = ljs32[((key >> 28) & 3) * A.lj.nt + ((unsigned)key >> 30)];
+    if (MULTI) P = ljs32[((key >> 14) & 3) * A.lj.nt + ((unsigned)key >> 30)];
     float dg = 0.f, e = 0.f;
     if (pair_fn32<false>(A.lj.pot, dq.w, P, dg, e) != 0) return;
     const float dgs = kFix * dg;
@@ -934,38 +923,33 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
     atomicAdd(&fr[2 * cap + m], -fz * kFixInv);
   };
 
-  // ---- mixed form: consume one step's (atom, row) items, at most one per
-  // lane (nt = 0: none).  The items' candidate pairs are laid end to end and
-  // the warp walks them 32 at a time, one pair per lane, so no lane idles
-  // while another finishes a long j-range.  A lane finds its item from the
-  // bitmask of the items that start in the current 32 candidates, and reads
-  // the item's data from the per-warp tables by its rank.
-  auto consume = [&](int i, float cy, float cz, int lo1, int n1, int lo2, int n2) {
-    const int nt = n1 + n2;
-    const unsigned hb = __ballot_sync(FULL, nt > 0);
+  // ---- consume one step's (atom, row) items, at most one per lane (n <= 0:
+  // none): the atom at (x, y, z) (tile-frame x; y, z from its row's origin)
+  // against the staged atoms [lo, lo + n), whose row's origin is offset by
+  // (cy, cz).  The items' candidate pairs are laid end to end and the warp
+  // walks them 32 at a time, one pair per lane, so no lane idles while another
+  // finishes a long j-range.  A lane finds its item from the bitmask of the
+  // items that start in the current 32 candidates, and reads it from the
+  // per-warp table by its rank: one 16-byte word, the atom's position moved into
+  // the j-cells' frame and id + ((lo - s0) << 16), to which candidate k adds
+  // k << 16: the sum is the pair's key (the j-range's upper half wraps).
+  // (Shared-memory wavefronts bound this walk: 83 % of the cycles on a mixture.
+  // An item of two words, with room for the rare second run, cost 2 of 13 per
+  // window; a second run is now an item of a second call.)
+  auto consume = [&](int id, float x, float y, float z, float cy, float cz, int lo, int n) {
+    const unsigned hb = __ballot_sync(FULL, n > 0);
     if (hb == 0u) return;
+    const int nt = max(n, 0);
     // exclusive scan of the items' candidate counts
     int incl = nt;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(FULL, incl, o);
-      if (lane >= o) incl += y;
+      const int y2 = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += y2;
     }
     const int s0 = incl - nt;
     const int T = __shfl_sync(FULL, incl, 31);
-    if (nt > 0) {
-      // the atom's position moved into the j-cells' frame: d = x_j + C
-      // (y, z relative to the cell origin; cy, cz: the j-row's origin offset)
-      const float4 pi = pf[i];
-      // by rank: the item's key base and frame shift, and the offsets that map
-      // candidate k to its staged atom: m = k + (k < e1 ? o1 : o2)
-      const int rk = __popc(hb & lt);
-      ptA[rk] = make_float4(-pi.x, cy - pi.y, cz - pi.z, __int_as_float(MULTI ? i | (__float_as_int(pi.w) << 28) : i));
-      if (PACK)
-        ptB2[rk] = make_int2(((lo1 - s0) & 0xffff) | ((lo2 - n1 - s0) << 16), s0 + n1);
-      else
-        ptB4[rk] = make_int4(lo1 - s0, s0 + n1, lo2 - n1 - s0, 0);
-    }
+    if (nt > 0) pt[__popc(hb & lt)] = make_float4(-x, cy - y, cz - z, __int_as_float(id + ((lo - s0) << 16)));
     __syncwarp();
     // distance tests; accepted pairs go to the queue
     int qb = 0;  // items that start before K
@@ -975,43 +959,30 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
       const unsigned M = __reduce_or_sync(FULL, sw == kw ? sbit : 0u);
       const int qr = qb + __popc(M & le) - 1;  // >= 0: the first item starts at 0
       qb += __popc(M);
-      const float4 a = ptA[qr];
-      int o1, e1, o2;
-      if (PACK) {
-        const int2 b = ptB2[qr];
-        o1 = (int)(short)(b.x & 0xffff);
-        o2 = b.x >> 16;
-        e1 = b.y;
-      } else {
-        const int4 b = ptB4[qr];
-        o1 = b.x;
-        e1 = b.y;
-        o2 = b.z;
-      }
+      const float4 a = pt[qr];
       const int k = K + lane;
       const bool valid = k < T;
-      const int m = (k < e1 ? o1 : o2) + k;
+      const unsigned kb = (unsigned)__float_as_int(a.w) + ((unsigned)k << 16);
+      const int m = (int)(kb >> 16);
       const float4 pj = pf[valid ? m : 0];
       float4 dq;
       dq.x = pj.x + a.x;
       dq.y = pj.y + a.y;
       dq.z = pj.z + a.z;
       dq.w = fmaf(dq.x, dq.x, fmaf(dq.y, dq.y, dq.z * dq.z));
-      const int tj = __float_as_int(pj.w);
-      const int kb = __float_as_int(a.w);
+      const int tj = __float_as_int(pj.w), ti = MULTI ? (kb >> 14) & 3 : 0;
       if (COUNT && valid) ++neval;
-      const float thr = FIX ? (MULTI ? ljx[((kb >> 28) & 3) * A.lj.nt + tj].pre : A.fx.p[0].pre)
-                        : MODE == kListBuild ? (MULTI ? ljs32[((kb >> 28) & 3) * A.lj.nt + tj].rl2 : q32.rl2)
-                                           : (MULTI ? ljs32[((kb >> 28) & 3) * A.lj.nt + tj].rc2 : q32.rc2);
-      // disjoint bit fields: the sum is the OR, in one instruction
-      const int key = (int)((unsigned)kb + ((unsigned)m << 14) + (MULTI ? (unsigned)tj << 30 : 0u));
+      const float thr = FIX ? (MULTI ? ljx[ti * A.lj.nt + tj].pre : A.fx.p[0].pre)
+                        : MODE == kListBuild ? (MULTI ? ljs32[ti * A.lj.nt + tj].rl2 : q32.rl2)
+                                             : (MULTI ? ljs32[ti * A.lj.nt + tj].rc2 : q32.rc2);
+      const int key = (int)(kb + (MULTI ? (unsigned)tj << 30 : 0u));
       bool acc = valid && dq.w <= thr;
       if ((MODE == kMain || MODE == kRedoFull) && valid && fabsf(dq.w - thr) <= kBorder * thr)
-        acc = inside64(kb & 0x3fff, m, MULTI ? (kb >> 28) & 3 : 0, MULTI ? tj : 0);  // at the border: FP64
+        acc = inside64(kb & 0x3fff, m, ti, MULTI ? tj : 0);  // at the border: FP64
       if (MODE == kRedoBig)
         redo_pair(acc, dq, key);
       else if (MODE == kListBuild)
-        list_add(acc, key, tj);
+        list_add(acc, key);
       else
         enqueue(acc, dq, key);
     }
@@ -1044,7 +1015,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
     const int T = __shfl_sync(FULL, incl, 31);
     const int pa = i0 | (ni << 16), p1 = lo1 | (n1 << 16), l2 = lo2 - n1, pn = nj | (self ? 1 << 16 : 0);
     if (nt > 0) {
-      ptA[lane] = make_float4(0.f, 0.f, 1.0f / (float)nj, __int_as_float(s0));
+      pt[lane] = make_float4(0.f, 0.f, 1.0f / (float)nj, __int_as_float(s0));
       r2l[32 + __popc(hb & lt)] = (unsigned char)lane;
     }
     __syncwarp();
@@ -1058,7 +1029,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
       const int ql = r2l[32 + qr];
       const int bpa = __shfl_sync(FULL, pa, ql), bp1 = __shfl_sync(FULL, p1, ql);
       const int bl2 = __shfl_sync(FULL, l2, ql), bpn = __shfl_sync(FULL, pn, ql);
-      const float4 a = ptA[ql];
+      const float4 a = pt[ql];
       const int k = K + lane;
       const int kl = k - __float_as_int(a.w);
       const int bnj = bpn & 0xffff;
@@ -1085,7 +1056,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         ++ncand;
         ++neval;
       }
-      enqueue(valid && dq.w <= rcpre, dq, i | (m << 14) | (ti << 28) | (tj << 30));
+      enqueue(valid && dq.w <= rcpre, dq, i | (ti << 14) | (m << 16) | (tj << 30));
     }
     __syncwarp();
   };
@@ -1178,7 +1149,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
           const LJ32 P = MULTI ? ljs32[lrow + tj] : q32;
           if (MODE == kListBig) {
             bool acc = dq.w <= P.rc2;
-            redo_pair(acc, dq, i | (m << 14) | (ti << 28) | (tj << 30));
+            redo_pair(acc, dq, i | (ti << 14) | (m << 16) | (tj << 30));
           } else {
             // The LJ family's expression of pair_fn32 (the potential was
             // checked per tile) for every entry, its result kept where the
@@ -1264,8 +1235,6 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
       const int acls = pos_class(ax - 1, tx) * 25 + pos_class(ay - 1, ty) * 5 + pos_class(az - 1, tz);
       const int aw = va ? (sown->nrow[acls] + kParts - 1 - part) / kParts : 0;
       const float4 pa = pf[va ? ia : 0];
-      const float apy = FP64 ? pa.y : oy[ay] + pa.y;  // tile-frame y, z
-      const float apz = FP64 ? pa.z : oz[az] + pa.z;
       // squared x-gaps to the cells dx = -2, -1, +1, +2 (ox has EX + 1 entries)
       const float gm2 = fmaxf(pa.x - ox[max(ax - 1, 0)], 0.f), gm1 = fmaxf(pa.x - ox[ax], 0.f);
       const float gp1 = fmaxf(ox[min(ax + 1, EX)] - pa.x, 0.f), gp2 = fmaxf(ox[min(ax + 2, EX)] - pa.x, 0.f);
@@ -1280,16 +1249,12 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
       const unsigned wb = __ballot_sync(FULL, aw > 0);
       if (aw > 0) {  // the working atoms' data by rank (as0 < 512, ia < 2^14, acls < 128)
         const int rk = __popc(wb & lt);
-        const int wa = as0 | (ia << 9), wc = cia | (acls << 15);
-        if (PACK) {
-          const __half2 hm = __halves2half2(__float2half_rz(am2), __float2half_rz(am1));
-          const __half2 hp = __halves2half2(__float2half_rz(ap1), __float2half_rz(ap2));
-          btA[rk] = make_float4(apy, apz, *reinterpret_cast<const float*>(&hm), *reinterpret_cast<const float*>(&hp));
-          btB2[rk] = make_int2(wa, wc);
-        } else {
-          btA[rk] = make_float4(apy, apz, am2, am1);
-          btB4[rk] = make_float4(ap1, ap2, __int_as_float(wa), __int_as_float(wc));
-        }
+        const int wa = as0 | (ia << 9), wc = cia | (acls << 15) | (MULTI ? __float_as_int(pa.w) << 22 : 0);
+        // the gaps as FP16 rounded toward zero: they prune no more than they may
+        const __half2 hm = __halves2half2(__float2half_rz(am2), __float2half_rz(am1));
+        const __half2 hp = __halves2half2(__float2half_rz(ap1), __float2half_rz(ap2));
+        btA[rk] = make_float4(pa.x, pa.y, pa.z, *reinterpret_cast<const float*>(&hm));
+        btB[rk] = make_float4(*reinterpret_cast<const float*>(&hp), __int_as_float(wa), __int_as_float(wc), 0.f);
       }
       __syncwarp();
       int qb = 0;  // working atoms that start before K
@@ -1301,61 +1266,41 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         qb += __popc(M);
         const int k = K + lane;
         const bool valid = k < W;
-        const float4 b0v = btA[qr];
-        const float py = b0v.x, pz = b0v.y;
-        float xm2, xm1, xp1, xp2;
-        int sq, cc;
-        if (PACK) {
-          const float2 gm = __half22float2(*reinterpret_cast<const __half2*>(&b0v.z));
-          const float2 gp = __half22float2(*reinterpret_cast<const __half2*>(&b0v.w));
-          const int2 b1v = btB2[qr];
-          xm2 = gm.x;
-          xm1 = gm.y;
-          xp1 = gp.x;
-          xp2 = gp.y;
-          sq = b1v.x;
-          cc = b1v.y;
-        } else {
-          const float4 b1v = btB4[qr];
-          xm2 = b0v.z;
-          xm1 = b0v.w;
-          xp1 = b1v.x;
-          xp2 = b1v.y;
-          sq = __float_as_int(b1v.z);
-          cc = __float_as_int(b1v.w);
-        }
+        const float4 b0v = btA[qr], b1v = btB[qr];
+        const float2 gm = __half22float2(*reinterpret_cast<const __half2*>(&b0v.w));
+        const float2 gp = __half22float2(*reinterpret_cast<const __half2*>(&b1v.x));
+        const int sq = __float_as_int(b1v.y), cc = __float_as_int(b1v.z);
         const int s_q = sq & 511, i = sq >> 9;
-        const int ci = cc & 0x7fff, cls = cc >> 15;
-        const int lx = ci & 31, ly = (ci >> 5) & 31, lz = ci >> 10;
-        int r = 0, mask = 0;
-        if (valid) {
-          r = sown->rlist[cls][kParts * (k - s_q) + part];
-          mask = sown->lut[cls][kParts * (k - s_q) + part];
-        }
+        const int cls = (cc >> 15) & 127;
+        const int lx = cc & 31, ly = (cc >> 5) & 31, lz = (cc >> 10) & 31;
+        const unsigned ent = valid ? sown->ent[cls][kParts * (k - s_q) + part] : 0u;
+        int mask = ent & 31;
         int lo1 = 0, n1 = 0, lo2 = 0, n2 = 0;
         float cy = 0.f, cz = 0.f;
         if (mask) {
-          const int dy = srows[2 * r], dz = srows[2 * r + 1];
+          const int yc = (ent >> 5) & 7, zc = ent >> 8;  // dy + 2, dz + 2
+          const int dy = yc - 2, dz = zc - 2;
+          const bool selfrow = (dy | dz) == 0;
           const int rowbase = ((ly + dy) + EY * (lz + dz)) * EX + lx - 2;  // + bit b -> ext cell of dx = b - 2
-          const float2 ry = dyt[ly * kDT + dy + 2], rz = dzt[lz * kDT + dz + 2];
+          const float2 ry = dyt[ly * kDT + yc], rz = dzt[lz * kDT + zc];
           cy = ry.x;
           cz = rz.x;
           if (COUNT) {  // every atom of the owned cells, as the reference visits them
             for (int b = 0; b < 5; ++b)
               if ((mask >> b) & 1) {
                 const int e = rowbase + b;
-                ncand += (r == kRows - 1 && b == 2) ? lstart[e + 1] - i - 1 : lstart[e + 1] - lstart[e];
+                ncand += (selfrow && b == 2) ? lstart[e + 1] - i - 1 : lstart[e + 1] - lstart[e];
               }
           }
           // distance from the atom to the row's cell boxes
           // (the row's near face comes with its origin offset)
-          const float ty = ry.y - py, tz = rz.y - pz;
+          const float ty = ry.y - b0v.y, tz = rz.y - b0v.z;
           const float gy = dy == 0 ? 0.f : fmaxf(dy > 0 ? ty : -ty, 0.f);
           const float gz = dz == 0 ? 0.f : fmaxf(dz > 0 ? tz : -tz, 0.f);
           const float g2 = gy * gy + gz * gz;
           const float tr = prune2 - g2;
           if (tr < 0.f) mask = 0;
-          mask &= ~((xm2 > tr ? 1 : 0) | (xm1 > tr ? 2 : 0) | (xp1 > tr ? 8 : 0) | (xp2 > tr ? 16 : 0));
+          mask &= ~((gm.x > tr ? 1 : 0) | (gm.y > tr ? 2 : 0) | (gp.x > tr ? 8 : 0) | (gp.y > tr ? 16 : 0));
           if (mask) {
             const int b0 = __ffs(mask) - 1, b1 = 31 - __clz(mask);
             const int mm = mask >> b0;
@@ -1369,19 +1314,20 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
               hi1 = lstart[rowbase + e1];
             }
             n1 = hi1 - lo1;
-            if (r == kRows - 1 && b0 == 2) {  // pairs inside the cell: a2 > a1
+            if (selfrow && b0 == 2) {  // pairs inside the cell: a2 > a1
               n1 -= i + 1 - lo1;
               lo1 = i + 1;
             }
-            if (n1 <= 0) {
-              lo1 = lo2;
-              n1 = n2;
-              lo2 = 0;
-              n2 = 0;
-            }
           }
         }
-        consume(i, cy, cz, lo1, n1, lo2, n2);
+        const int id = i | (MULTI ? (cc >> 22) << 14 : 0);
+        while (true) {
+          consume(id, b0v.x, b0v.y, b0v.z, cy, cz, lo1, n1);
+          if (!__any_sync(FULL, n2 > 0)) break;  // a second run: 0.6 % of the items, most steps have none
+          lo1 = lo2;
+          n1 = n2;
+          n2 = 0;
+        }
       }
       __syncwarp();
     }
@@ -1432,15 +1378,12 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         const int geo = __shfl_sync(FULL, ageo, ql);
         const int qpa = __shfl_sync(FULL, apa, ql);
         const int lx = geo & 31, ly = (geo >> 5) & 31, lz = (geo >> 10) & 31, cls = geo >> 15;
-        int r = 0, mask = 0;
-        if (valid) {
-          r = sown->rlist[cls][kCellParts * (k - s_q) + part];
-          mask = sown->lut[cls][kCellParts * (k - s_q) + part];
-        }
+        const unsigned ent = valid ? sown->ent[cls][kCellParts * (k - s_q) + part] : 0u;
+        const int mask = ent & 31;
         int lo1 = 0, n1 = 0, lo2 = 0, n2 = 0;
         bool self = false;
         if (mask) {
-          const int dy = srows[2 * r], dz = srows[2 * r + 1];
+          const int dy = (int)((ent >> 5) & 7) - 2, dz = (int)(ent >> 8) - 2;
           const int rowbase = ((ly + dy) + EY * (lz + dz)) * EX + lx - 2;  // + bit b -> ext cell of dx = b - 2
           const int b0 = __ffs(mask) - 1, b1 = 31 - __clz(mask);
           const int mm = mask >> b0;
@@ -1454,7 +1397,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
             hi1 = lstart[rowbase + e1];
           }
           n1 = hi1 - lo1;
-          self = r == kRows - 1 && b0 == 2;  // the first run starts at the cell itself
+          self = (dy | dz) == 0 && b0 == 2;  // the first run starts at the cell itself
           if (n1 <= 0 && !self) {
             lo1 = lo2;
             n1 = n2;
@@ -1719,30 +1662,30 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   }
 }
 
-template <bool FP64, bool MULTI, bool ENERGY, bool COUNT, bool PACK>
+template <bool FP64, bool MULTI, bool ENERGY, bool COUNT>
 __global__ void __launch_bounds__(256, FP64 ? 3 : 4) k_pair(const PairArgs A) {
-  pair_tile<FP64, MULTI, ENERGY, COUNT, kMain, PACK>(A, A.order[blockIdx.x]);
+  pair_tile<FP64, MULTI, ENERGY, COUNT, kMain>(A, A.order[blockIdx.x]);
 }
 
 // FP64 form: the first pass in fixed point, and the FP64 body for the tiles that
 // it listed (normally none).
 template <bool MULTI, bool ENERGY, bool COUNT>
-__global__ void __launch_bounds__(256, 4) k_pair_fix(const PairArgs A) {
-  pair_tile<false, MULTI, ENERGY, COUNT, kFixed, true>(A, A.order[blockIdx.x]);
+__global__ void __launch_bounds__(256, MULTI ? 3 : 4) k_pair_fix(const PairArgs A) {
+  pair_tile<false, MULTI, ENERGY, COUNT, kFixed>(A, A.order[blockIdx.x]);
 }
 
 // Pair-list mode: the forces of every tile from its list (fallback tiles
 // return at once: the redo pass enumerates them).
 template <bool MULTI, bool ENERGY, bool CUT>
 __global__ void __launch_bounds__(256, 4) k_pair_list(const PairArgs A) {
-  pair_tile<false, MULTI, ENERGY, false, kList, false, CUT>(A, A.order[blockIdx.x]);
+  pair_tile<false, MULTI, ENERGY, false, kList, CUT>(A, A.order[blockIdx.x]);
 }
 
 // Pair-list mode: the lists of every tile, on the steps whose gate is set.
-template <bool MULTI, bool PACK>
+template <bool MULTI>
 __global__ void __launch_bounds__(32 * kBuildWarps, 3) k_pair_build(const PairArgs A) {
   if (A.gate && !*A.gate) return;
-  pair_tile<false, MULTI, false, false, kListBuild, PACK>(A, A.order[blockIdx.x]);
+  pair_tile<false, MULTI, false, false, kListBuild>(A, A.order[blockIdx.x]);
 }
 
 // Mixed form: the redo pass over the tiles that k_pair listed (normally none,
@@ -1752,18 +1695,18 @@ __global__ void __launch_bounds__(32 * kBuildWarps, 3) k_pair_build(const PairAr
 // mode): the listed tiles' large terms are redone from their lists, and the
 // fallback tiles (over capacity or with lists that did not fit when they were
 // built) are computed in full by enumeration, every step until the next build.
-template <bool MULTI, bool PACK, bool ENERGY, bool COUNT, bool LIST>
+template <bool MULTI, bool ENERGY, bool COUNT, bool LIST>
 __global__ void __launch_bounds__(256, 3) k_pair_redo(const PairArgs A) {
   const int n = *(volatile const int*)A.redo_n;
   const int nfb = LIST ? *(volatile const int*)&A.lw[LW_FBN] : 0;
   for (int j = blockIdx.x; j < n + nfb; j += gridDim.x) {
     const int w = j < n ? A.redo[j] : (A.fb[j - n] | kFullBit);
     if (w & kFullBit)
-      pair_tile<false, MULTI, ENERGY, COUNT, kRedoFull, PACK>(A, w & ~kFullBit);
+      pair_tile<false, MULTI, ENERGY, COUNT, kRedoFull>(A, w & ~kFullBit);
     else if (LIST)
-      pair_tile<false, MULTI, false, false, kListBig, PACK>(A, w);
+      pair_tile<false, MULTI, false, false, kListBig>(A, w);
     else
-      pair_tile<false, MULTI, false, false, kRedoBig, PACK>(A, w);
+      pair_tile<false, MULTI, false, false, kRedoBig>(A, w);
     __syncthreads();
   }
   __syncthreads();
@@ -1779,7 +1722,7 @@ template <bool MULTI, bool ENERGY, bool COUNT>
 __global__ void __launch_bounds__(256, 3) k_pair_redo64(const PairArgs A) {
   const int n = *(volatile const int*)A.redo_n;
   for (int j = blockIdx.x; j < n; j += gridDim.x) {
-    pair_tile<true, MULTI, ENERGY, COUNT, kRedoFull, false>(A, A.redo[j] & ~kFullBit);
+    pair_tile<true, MULTI, ENERGY, COUNT, kRedoFull>(A, A.redo[j] & ~kFullBit);
     __syncthreads();
   }
   __syncthreads();
@@ -1791,29 +1734,16 @@ __global__ void __launch_bounds__(256, 3) k_pair_redo64(const PairArgs A) {
   }
 }
 
-template <bool FP64, bool MULTI, bool ENERGY, bool COUNT, bool PACK>
-static void* kfn() {
-  return (void*)&k_pair<FP64, MULTI, ENERGY, COUNT, PACK>;
+template <bool FP64, bool MULTI>
+static void* pick_enum_ec(const PairConfig& c) {
+  if (c.energy) return c.count ? (void*)&k_pair<FP64, MULTI, true, true> : (void*)&k_pair<FP64, MULTI, true, false>;
+  return c.count ? (void*)&k_pair<FP64, MULTI, false, true> : (void*)&k_pair<FP64, MULTI, false, false>;
 }
 
-// The enumeration's first pass.  The FP64 form has one table layout (PACK = false).
+// The enumeration's first pass.
 static void* pick_enum(const PairConfig& c) {
-#define EXAMD_PICK(F, M, P)                                            \
-  if (c.energy && c.count) return kfn<F, M, true, true, P>();         \
-  if (c.energy) return kfn<F, M, true, false, P>();                   \
-  if (c.count) return kfn<F, M, false, true, P>();                    \
-  return kfn<F, M, false, false, P>();
-  if (c.fp64) {
-    if (c.multi) { EXAMD_PICK(true, true, false) }
-    EXAMD_PICK(true, false, false)
-  }
-  if (c.pack) {
-    if (c.multi) { EXAMD_PICK(false, true, true) }
-    EXAMD_PICK(false, false, true)
-  }
-  if (c.multi) { EXAMD_PICK(false, true, false) }
-  EXAMD_PICK(false, false, false)
-#undef EXAMD_PICK
+  if (c.fp64) return c.multi ? pick_enum_ec<true, true>(c) : pick_enum_ec<true, false>(c);
+  return c.multi ? pick_enum_ec<false, true>(c) : pick_enum_ec<false, false>(c);
 }
 
 // The first pass: in pair-list mode (the counters excepted, which the
@@ -1846,27 +1776,20 @@ static void* pick(const PairConfig& c) {
 }
 
 static void* pick_build(const PairConfig& c) {
-  if (c.pack) return c.multi ? (void*)&k_pair_build<true, true> : (void*)&k_pair_build<false, true>;
-  return c.multi ? (void*)&k_pair_build<true, false> : (void*)&k_pair_build<false, false>;
+  return c.multi ? (void*)&k_pair_build<true> : (void*)&k_pair_build<false>;
 }
 
-template <bool MULTI, bool PACK, bool LIST>
+template <bool MULTI, bool LIST>
 static void* pick_redo_ec(const PairConfig& c) {
-  if (c.energy && c.count) return (void*)&k_pair_redo<MULTI, PACK, true, true, LIST>;
-  if (c.energy) return (void*)&k_pair_redo<MULTI, PACK, true, false, LIST>;
-  if (c.count) return (void*)&k_pair_redo<MULTI, PACK, false, true, LIST>;
-  return (void*)&k_pair_redo<MULTI, PACK, false, false, LIST>;
-}
-
-template <bool LIST>
-static void* pick_redo_l(const PairConfig& c) {
-  if (c.pack) return c.multi ? pick_redo_ec<true, true, LIST>(c) : pick_redo_ec<false, true, LIST>(c);
-  return c.multi ? pick_redo_ec<true, false, LIST>(c) : pick_redo_ec<false, false, LIST>(c);
+  if (c.energy)
+    return c.count ? (void*)&k_pair_redo<MULTI, true, true, LIST> : (void*)&k_pair_redo<MULTI, true, false, LIST>;
+  return c.count ? (void*)&k_pair_redo<MULTI, false, true, LIST> : (void*)&k_pair_redo<MULTI, false, false, LIST>;
 }
 
 static void* pick_redo(const PairConfig& c) {
   if (c.fix) return c.multi ? pick_redo64<true>(c) : pick_redo64<false>(c);
-  return uses_list(c) ? pick_redo_l<true>(c) : pick_redo_l<false>(c);
+  if (uses_list(c)) return c.multi ? pick_redo_ec<true, true>(c) : pick_redo_ec<false, true>(c);
+  return c.multi ? pick_redo_ec<true, false>(c) : pick_redo_ec<false, false>(c);
 }
 
 cudaError_t pair_prepare(const PairConfig& cfg, int smem_bytes) {
@@ -1875,18 +1798,6 @@ cudaError_t pair_prepare(const PairConfig& cfg, int smem_bytes) {
   e = cudaFuncSetAttribute(pick_redo(cfg), cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
   if (e != cudaSuccess || !uses_list(cfg)) return e;
   return cudaFuncSetAttribute(pick_build(cfg), cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-}
-
-// Occupancy of the enumeration's first pass (the pair-list mode's build uses
-// the same tables).
-int pair_blocks_per_sm(const PairConfig& cfg, int cap, int ne_max, int ext_max) {
-  PairConfig c = cfg;
-  c.list = false;
-  const int smem = make_layout(c.fp64, cap, ne_max, ext_max, c.warps, kMain, c.pack, c.multi).bytes;
-  int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pick_enum(c), 32 * c.warps, (size_t)smem) != cudaSuccess)
-    return 0;
-  return n;
 }
 
 cudaError_t launch_pair(const PairConfig& cfg, const PairArgs& a, int ntiles, int smem_bytes, cudaStream_t st) {
