@@ -217,6 +217,27 @@ int split_axis(int nb, double last_width, int tile_len, int balance, int* starts
   return nt;
 }
 
+// Home cells per tile and axis where the caller leaves it to the library: 4.
+// The FP64 form, whose tiles take longer and whose results do not depend on
+// them, takes smaller ones where 4^3 would leave SMs idle: 3 below four tiles an
+// SM, 2 where even 3^3 gives less than one.  (Pair pass at 4 / 3 / 2, us: 1,000
+// atoms in 27 / 64 / 125 tiles 24.7 / 19.9 / 16.5; 8,788 in 125 / 216 / 729
+// 47 / 33 / 33; 32,000 in 343 / 729 / 2197 59.5 / 52.8 / 64; 87,808 in 1000 / 2197
+// 97 / 108.)  The mixed form keeps 4: its FP32 x coordinates are the tile's.
+int default_tile(const examd_params& p, int nboxes, const examd_box* boxes, double bl, int sms) {
+  if (p.precision != EXAMD_FP64) return 4;
+  auto tiles = [&](int t) {
+    double n = 0.0;
+    for (int b = 0; b < nboxes; ++b) {
+      double v = 1.0;
+      for (int a = 0; a < 3; ++a) v *= std::ceil(std::floor(boxes[b].L[a] / bl) / t);
+      n += v;
+    }
+    return n;
+  };
+  return tiles(4) >= 4.0 * sms ? 4 : tiles(3) >= sms ? 3 : 2;
+}
+
 }  // namespace
 
 int examd_tile_split(int nb, double last_width, int tile_len, int tile_balance, int* starts, int* nt) {
@@ -229,6 +250,13 @@ int examd_tile_split(int nb, double last_width, int tile_len, int tile_balance, 
 
 constexpr int kIoChunks = 4;            // host <-> device transfers of the force call, in chunks
 constexpr int kEagerSlots = 32;         // energies of eager steps kept on the device before one copy
+// Force calls at new positions of at most this many atoms go through the
+// context's own page-locked arrays (two host copies of up to 393 KB) from the
+// third call on, so that they replay one captured graph whatever the caller's
+// arrays are: 1,000 atoms cost 104 us as some twenty separate calls, the GPU
+// idle between them.
+constexpr int64_t kSmallIo = 1 << 14;
+constexpr int64_t kHostTypes = 1 << 14;  // atoms whose types are checked by the host
 constexpr int64_t kIoMinChunk = 1 << 16;  // atoms; smaller calls use fewer chunks
 
 struct examd_ctx {
@@ -338,7 +366,9 @@ struct examd_ctx {
     cudaGraphExec_t exec = nullptr;
     const void *pos = nullptr, *forces = nullptr, *epot = nullptr, *virial = nullptr;
     int accumulate = -1, cap = 0, cap_redo = 0, list_gen = 0;
-  } io_graph[2];
+  } io_graph[2], small_graph[2][4];  // small calls: by parity, then energies | accumulate << 1
+  int small_calls = 0;      // small calls so far, up to 2
+  double* h_io = nullptr;   // small calls: positions, forces, energies, virials (pinned)
 
   int cuda_fail(cudaError_t e, const char* what) {
     lasterr = std::string(what) + ": " + cudaGetErrorString(e);
@@ -366,11 +396,22 @@ int dalloc(examd_ctx* ctx, T** p, size_t count) {
   return EXAMD_OK;
 }
 
+// The captured force calls, dropped (the buffers they name change).
+void drop_io_graphs(examd_ctx* ctx) {
+  auto drop = [](examd_ctx::IoGraph& g) {
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+    g = examd_ctx::IoGraph{};
+  };
+  for (int b = 0; b < 2; ++b) {
+    drop(ctx->io_graph[b]);
+    for (auto& g : ctx->small_graph[b]) drop(g);
+  }
+}
+
 void free_all(examd_ctx* ctx) {
   if (ctx->gexec) cudaGraphExecDestroy(ctx->gexec);
   ctx->gexec = nullptr;
-  for (auto& g : ctx->io_graph)
-    if (g.exec) cudaGraphExecDestroy(g.exec);
+  drop_io_graphs(ctx);
   void* ptrs[] = {ctx->d_boxes, ctx->d_tiles, ctx->d_order, ctx->d_tile0, ctx->d_bmask, ctx->U, ctx->cellS,
                   ctx->cellOld, ctx->slot, ctx->count, ctx->cstart, ctx->bsum,
                   ctx->Fown, ctx->P, ctx->tileE, ctx->tileW, ctx->tileC, ctx->boxE, ctx->boxW, ctx->boxKE,
@@ -390,6 +431,7 @@ void free_all(examd_ctx* ctx) {
   if (ctx->h_status) cudaFreeHost(ctx->h_status);
   if (ctx->h_lw) cudaFreeHost(ctx->h_lw);
   if (ctx->h_e) cudaFreeHost(ctx->h_e);
+  if (ctx->h_io) cudaFreeHost(ctx->h_io);
   for (cudaEvent_t e : ctx->ev_side)
     if (e) cudaEventDestroy(e);
   if (ctx->inv) cudaFree(ctx->inv);
@@ -405,6 +447,7 @@ void free_all(examd_ctx* ctx) {
 }
 
 int status_to_code(int st) {
+  if (st & ST_TYPE) return EXAMD_ERR_ARG;
   if (st & ST_PAIRFN) return EXAMD_ERR_PAIRFN;
   if (st & ST_NONFINITE) return EXAMD_ERR_NONFINITE;
   if (st & ST_OUTSIDE) return EXAMD_ERR_OUTSIDE;
@@ -557,8 +600,8 @@ int examd_gpu_create(const examd_params* params, int nboxes, const examd_box* bo
     delete ctx;
     return EXAMD_ERR_ARG;
   }
-  const int deftile = 4;
   int T[3];
+  const int deftile = default_tile(p, nboxes, boxes, bl, prop.multiProcessorCount);
   for (int a = 0; a < 3; ++a) {
     T[a] = p.tile[a] > 0 ? p.tile[a] : deftile;
     if (T[a] < 2 || T[a] > 14) {
@@ -943,7 +986,7 @@ int finish_binning(examd_ctx* ctx, bool want_inv, const int* gate = nullptr) {
   const int s = ctx->cur, d = 1 - ctx->cur;
   const bool list = ctx->list;
   if (list) want_inv = true;
-  k_scan_reduce<<<nsb, 256, 0, st>>>(nc, ctx->count, ctx->bsum, gate);
+  if (nsb > 1) k_scan_reduce<<<nsb, 256, 0, st>>>(nc, ctx->count, ctx->bsum, gate);  // (one block has none before it)
   k_scan_final<<<nsb, 256, 0, st>>>(nc, ctx->count, ctx->bsum, ctx->cstart, gate);
   if (ctx->N > 0) {
     k_finalize<<<nblk(ctx->N), 256, 0, st>>>(ctx->N, ctx->cellOld, ctx->slot, ctx->cstart, ctx->d_boxes,
@@ -1044,13 +1087,6 @@ int apply_capacity(examd_ctx* ctx, bool* grew = nullptr) {
       CK(pair_prepare(c, ctx->smem_limit));
     }
   return EXAMD_OK;
-}
-
-int update_capacity(examd_ctx* ctx) {
-  const int rc = queue_occupancy(ctx);
-  if (rc) return rc;
-  CK(cudaStreamSynchronize(ctx->st));
-  return apply_capacity(ctx);
 }
 
 PairArgs pair_args(examd_ctx* ctx) {
@@ -1192,10 +1228,7 @@ int set_list_capacity(examd_ctx* ctx, int want) {
     cudaGraphExecDestroy(ctx->gexec);
     ctx->gexec = nullptr;
   }
-  for (auto& g : ctx->io_graph) {
-    if (g.exec) cudaGraphExecDestroy(g.exec);
-    g = examd_ctx::IoGraph{};
-  }
+  drop_io_graphs(ctx);
   return EXAMD_OK;
 }
 
@@ -1404,19 +1437,27 @@ int examd_gpu_set_atoms(examd_ctx* ctx, int64_t n, const double* pos, const int*
   if (!ctx || (n > 0 && !pos) || n != ctx->N) return EXAMD_ERR_ARG;
   cudaSetDevice(ctx->dev);
   cudaStream_t st = ctx->st;
-  std::vector<int> meta((size_t)n);
-  for (int b = 0; b < ctx->nboxes; ++b)
-    for (int64_t i = ctx->atom0[b]; i < ctx->atom0[b + 1]; ++i) {
-      int t = type ? type[i] : 0;
-      if (t < 0 || t >= ctx->p.ntypes) return EXAMD_ERR_ARG;
-      meta[(size_t)i] = (b << 8) | t;
-    }
+  // The types: up to kHostTypes atoms are checked here, more of them by the
+  // kernel that makes the meta words (which then costs a wait; a host loop and a
+  // host array of 16.8M words took 40 of the call's 65 ms).
+  const bool host_check = n <= kHostTypes;
+  if (type && host_check)
+    for (int64_t i = 0; i < n; ++i)
+      if (type[i] < 0 || type[i] >= ctx->p.ntypes) return EXAMD_ERR_ARG;
+  CK(cudaMemsetAsync(ctx->status, 0, sizeof(int), st));
   if (n > 0) {
     CK(cudaMemcpyAsync(ctx->stage, pos, 3 * n * sizeof(double), cudaMemcpyHostToDevice, st));
     if (vel) CK(cudaMemcpyAsync(ctx->stage2, vel, 3 * n * sizeof(double), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(ctx->d_meta_in, meta.data(), n * sizeof(int), cudaMemcpyHostToDevice, st));
+    if (type) CK(cudaMemcpyAsync(ctx->d_meta_in, type, n * sizeof(int), cudaMemcpyHostToDevice, st));
+    k_make_meta<<<nblk(n), 256, 0, st>>>(n, ctx->nboxes, ctx->d_atom0, type != nullptr, ctx->p.ntypes, ctx->d_meta_in,
+                                         ctx->status);
+    CK(cudaGetLastError());
+    if (type && !host_check) {  // nothing of the context's atoms has been touched yet
+      CK(queue_status(ctx));
+      CK(cudaStreamSynchronize(st));
+      if (const int trc = take_status(ctx)) return trc;
+    }
   }
-  CK(cudaMemsetAsync(ctx->status, 0, sizeof(int), st));
   const int s = ctx->cur;
   if (n > 0) {
     k_load_bin<<<nblk(n), 256, 0, st>>>(n, ctx->stage, vel ? ctx->stage2 : nullptr, ctx->d_meta_in, ctx->d_boxes,
@@ -1427,10 +1468,12 @@ int examd_gpu_set_atoms(examd_ctx* ctx, int64_t n, const double* pos, const int*
   }
   int rc = finish_binning(ctx, true);
   if (rc) return rc;
+  CK(queue_status(ctx));
+  if ((rc = queue_occupancy(ctx))) return rc;
   CK(cudaStreamSynchronize(st));
-  rc = check_status(ctx);
+  rc = take_status(ctx);
   if (rc) return rc;
-  rc = update_capacity(ctx);
+  rc = apply_capacity(ctx);
   if (rc) return rc;
   if (ctx->list) {
     CK(cudaMemsetAsync(ctx->lw, 0, LW_WORDS * sizeof(int), st));
@@ -1499,20 +1542,10 @@ int finish_forces_at_eager(examd_ctx* ctx, const double* pos, double* forces, do
   return rc ? rc : finish_forces(ctx);
 }
 
-}  // namespace
-
-extern "C" {
-
-int examd_gpu_forces_at(examd_ctx* ctx, const double* pos, double* forces, double* epot, double* virial,
-                        int accumulate) {
-  if (!ctx || (ctx->N > 0 && !pos)) return EXAMD_ERR_ARG;
-  if (!ctx->atoms_set) return EXAMD_ERR_STATE;
-  cudaSetDevice(ctx->dev);
-  CK(ensure_inv(ctx));  // outside any captured sequence
-  if (ctx->N < kIoMinChunk || !pinned(pos) || !pinned(forces) || !pinned(epot) || !pinned(virial))
-    return finish_forces_at_eager(ctx, pos, forces, epot, virial, accumulate);
-  // same pinned buffers as last time at this parity: replay the captured call
-  auto& g = ctx->io_graph[ctx->cur];
+// The force call at new positions with pinned buffers, as a captured graph kept
+// in g (of the current parity) while its buffers and capacities stay.
+int forces_at_graph(examd_ctx* ctx, examd_ctx::IoGraph& g, const double* pos, double* forces, double* epot,
+                    double* virial, int accumulate) {
   const bool hit = g.exec && g.pos == pos && g.forces == forces && g.epot == epot && g.virial == virial &&
                    g.accumulate == accumulate && g.cap == ctx->cap && g.cap_redo == ctx->cap_redo &&
                    g.list_gen == ctx->list_gen;
@@ -1546,6 +1579,49 @@ int examd_gpu_forces_at(examd_ctx* ctx, const double* pos, double* forces, doubl
   if (!ctx->list) ctx->cur = 1 - ctx->cur;  // the host-side effects of the captured call
   ctx->inv_valid = true;
   return finish_forces(ctx);
+}
+
+// The same for at most kSmallIo atoms in any host arrays.
+int forces_at_small(examd_ctx* ctx, const double* pos, double* forces, double* epot, double* virial, int accumulate) {
+  const size_t n3 = 3 * (size_t)ctx->N, nb = (size_t)ctx->nboxes;
+  if (!ctx->h_io && cudaHostAlloc((void**)&ctx->h_io, (2 * n3 + 2 * nb) * sizeof(double), cudaHostAllocDefault) !=
+                        cudaSuccess) {
+    ctx->h_io = nullptr;
+    cudaGetLastError();
+    return finish_forces_at_eager(ctx, pos, forces, epot, virial, accumulate);
+  }
+  double *hp = ctx->h_io, *hf = hp + n3, *he = hf + n3, *hv = he + nb;
+  const bool energy = epot || virial;
+  accumulate = accumulate && forces ? 1 : 0;
+  std::memcpy(hp, pos, n3 * sizeof(double));
+  if (accumulate) std::memcpy(hf, forces, n3 * sizeof(double));
+  const int rc = forces_at_graph(ctx, ctx->small_graph[ctx->cur][(energy ? 1 : 0) | (accumulate << 1)], hp,
+                                 forces ? hf : nullptr, energy ? he : nullptr, energy ? hv : nullptr, accumulate);
+  if (rc == EXAMD_ERR_CUDA) return rc;
+  if (forces) std::memcpy(forces, hf, n3 * sizeof(double));  // (with a bad status too, as an eager call)
+  if (epot) std::memcpy(epot, he, nb * sizeof(double));
+  if (virial) std::memcpy(virial, hv, nb * sizeof(double));
+  return rc;
+}
+
+}  // namespace
+
+extern "C" {
+
+int examd_gpu_forces_at(examd_ctx* ctx, const double* pos, double* forces, double* epot, double* virial,
+                        int accumulate) {
+  if (!ctx || (ctx->N > 0 && !pos)) return EXAMD_ERR_ARG;
+  if (!ctx->atoms_set) return EXAMD_ERR_STATE;
+  cudaSetDevice(ctx->dev);
+  CK(ensure_inv(ctx));  // outside any captured sequence
+  if (ctx->N > 0 && ctx->N <= kSmallIo) {
+    if (ctx->small_calls == 2) return forces_at_small(ctx, pos, forces, epot, virial, accumulate);
+    ++ctx->small_calls;  // a context used for a call or two is not worth a capture
+  }
+  if (ctx->N < kIoMinChunk || !pinned(pos) || !pinned(forces) || !pinned(epot) || !pinned(virial))
+    return finish_forces_at_eager(ctx, pos, forces, epot, virial, accumulate);
+  // same pinned buffers as last time at this parity: replay the captured call
+  return forces_at_graph(ctx, ctx->io_graph[ctx->cur], pos, forces, epot, virial, accumulate);
 }
 
 }  // extern "C"
@@ -1638,10 +1714,7 @@ int ensure_ebuf(examd_ctx* ctx, int steps, bool host) {
     cudaGraphExecDestroy(ctx->gexec);
     ctx->gexec = nullptr;
   }
-  for (auto& g : ctx->io_graph) {
-    if (g.exec) cudaGraphExecDestroy(g.exec);
-    g = examd_ctx::IoGraph{};
-  }
+  drop_io_graphs(ctx);
   return EXAMD_OK;
 }
 

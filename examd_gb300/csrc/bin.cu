@@ -28,6 +28,25 @@ __device__ __forceinline__ void bin_one(int s, double x, double y, double z, int
   slot[s] = atomicAdd(&count[EXAMD_IDX(gc, B.cell0 + B.nb[0] * B.nb[1] * B.nb[2], status)], 1);
 }
 
+// meta[i] = box << 8 | type of the caller's atom i, over the types in place
+// (typed; else all type 0): the box by bisection of the boxes' atom offsets.
+__global__ void k_make_meta(int64_t n, int nboxes, const int64_t* __restrict__ atom0, bool typed, int ntypes,
+                            int* __restrict__ meta, int* __restrict__ status) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int t = typed ? meta[i] : 0;
+  if (t < 0 || t >= ntypes) atomicOr(status, ST_TYPE);
+  int lo = 0, hi = nboxes;  // atom0[lo] <= i < atom0[hi]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (atom0[mid] <= i)
+      lo = mid;
+    else
+      hi = mid;
+  }
+  meta[i] = (lo << 8) | (t & 0xff);
+}
+
 // Load caller-order AoS positions (and velocities) into the SoA master arrays,
 // wrapping (or, in strict mode, rejecting) positions outside [0, L), and bin.
 __global__ void k_load_bin(int64_t n, const double* __restrict__ aos, const double* __restrict__ vaos,

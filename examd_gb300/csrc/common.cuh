@@ -33,6 +33,7 @@ enum StatusBits : int {
   ST_OUTSIDE = 4,    // position outside [0,L) in strict mode
   ST_TIMEOUT = 8,    // a bounded wait gave up
   ST_PAIRFN = 16,    // the pair function returned an error
+  ST_TYPE = 64,      // an atom's type is outside [0, ntypes)
   ST_BOUNDS = 32,    // checked build: an index check failed (the access went to index 0)
 };
 

@@ -6,6 +6,8 @@
 namespace examd {
 
 // ---- bin.cu -----------------------------------------------------------------
+__global__ void k_make_meta(int64_t n, int nboxes, const int64_t* atom0, bool typed, int ntypes, int* meta,
+                            int* status);
 __global__ void k_load_bin(int64_t n, const double* aos, const double* vaos, const int* meta_in,
                            const BoxDev* boxes, int strict, double* X0, double* X1, double* X2, double* V0,
                            double* V1, double* V2, int* meta, int* id, int* cellOld, int* slot,

@@ -169,7 +169,8 @@ constexpr int kRedChunk = 4096;
 
 template <typename Off, int NV>
 __global__ void k_chunk_sums(const Off* __restrict__ off, const double* __restrict__ v0,
-                             const double* __restrict__ v1, int maxc, double* __restrict__ partial) {
+                             const double* __restrict__ v1, int maxc, double* __restrict__ p0,
+                             double* __restrict__ p1) {
   __shared__ double sh[NV][256];
   const int c = blockIdx.x, b = blockIdx.y;
   const int64_t a0 = (int64_t)off[b] + (int64_t)c * kRedChunk;
@@ -190,8 +191,8 @@ __global__ void k_chunk_sums(const Off* __restrict__ off, const double* __restri
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    partial[(size_t)b * maxc + c] = sh[0][0];
-    if (NV > 1) partial[((size_t)gridDim.y + b) * maxc + c] = sh[NV - 1][0];
+    p0[(size_t)b * maxc + c] = sh[0][0];
+    if (NV > 1) p1[(size_t)b * maxc + c] = sh[NV - 1][0];
   }
 }
 
@@ -225,15 +226,17 @@ int red_chunks(int64_t max_per_box) { return (int)std::max<int64_t>(1, (max_per_
 
 cudaError_t launch_box_sums(int nboxes, const int64_t* atom0, int maxc, const double* v, double* partial,
                             double* out, cudaStream_t st) {
-  k_chunk_sums<int64_t, 1><<<dim3(maxc, nboxes), 256, 0, st>>>(atom0, v, nullptr, maxc, partial);
-  k_box_sums<1><<<nboxes, 256, 0, st>>>(partial, maxc, nboxes, out, nullptr);
+  // one chunk a box: its sum is the box's
+  k_chunk_sums<int64_t, 1><<<dim3(maxc, nboxes), 256, 0, st>>>(atom0, v, nullptr, maxc, maxc > 1 ? partial : out, nullptr);
+  if (maxc > 1) k_box_sums<1><<<nboxes, 256, 0, st>>>(partial, maxc, nboxes, out, nullptr);
   return cudaGetLastError();
 }
 
 cudaError_t launch_reduce_tiles(int nboxes, const int* tile0, int maxc, const double* tileE, const double* tileW,
                                 double* partial, double* boxE, double* boxW, cudaStream_t st) {
-  k_chunk_sums<int, 2><<<dim3(maxc, nboxes), 256, 0, st>>>(tile0, tileE, tileW, maxc, partial);
-  k_box_sums<2><<<nboxes, 256, 0, st>>>(partial, maxc, nboxes, boxE, boxW);
+  k_chunk_sums<int, 2><<<dim3(maxc, nboxes), 256, 0, st>>>(tile0, tileE, tileW, maxc, maxc > 1 ? partial : boxE,
+                                                           maxc > 1 ? partial + (size_t)nboxes * maxc : boxW);
+  if (maxc > 1) k_box_sums<2><<<nboxes, 256, 0, st>>>(partial, maxc, nboxes, boxE, boxW);
   return cudaGetLastError();
 }
 
