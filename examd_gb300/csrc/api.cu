@@ -97,7 +97,8 @@ bool build_own_lut(OwnLut& L, signed char (*rowsOut)[2] = nullptr, unsigned char
           if (byRow) byRow[cls][r] = (unsigned char)mask;
           if (mask)
             L.ent[cls][L.nrow[cls]++] =
-                (unsigned short)(mask | ((unsigned)(rows[r].first + 2) << 5) | ((unsigned)(rows[r].second + 2) << 8));
+                (unsigned short)(mask | ((unsigned)(rows[r].first + 2) << 5) | ((unsigned)(rows[r].second + 2) << 8) |
+                                 (r == kRows - 1 ? 1u << 11 : 0u));
         }
       }
   return true;

@@ -163,7 +163,7 @@ struct LJTable {
 
 // Ownership of the midpoint table, filled once per process: per position class,
 // its owned rows in ascending order, each as mask | (dy + 2) << 5 |
-// (dz + 2) << 8, with the 5-bit mask over dx = -2..2 of the cell pairs (A, A + d)
+// (dz + 2) << 8 | (dy = dz = 0) << 11, with the 5-bit mask over dx = -2..2 of the cell pairs (A, A + d)
 // of row (dy, dz) that the tile owns when A's class is the entry's.  The row
 // (0, 0) uses bit 2 for the pairs inside A (a1 < a2) and bits 3, 4 for dx = +1, +2.
 // 16-byte aligned so that a CTA copies it to shared memory as uint4 words.

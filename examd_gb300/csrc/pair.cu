@@ -58,9 +58,11 @@
 
 namespace examd {
 
-__constant__ OwnLut c_own;
+// In global memory: a CTA's threads read different words of it, which the
+// constant bank would serve one after the other.
+__device__ OwnLut g_own;
 
-cudaError_t upload_own_lut(const OwnLut& lut) { return cudaMemcpyToSymbol(c_own, &lut, sizeof(OwnLut)); }
+cudaError_t upload_own_lut(const OwnLut& lut) { return cudaMemcpyToSymbol(g_own, &lut, sizeof(OwnLut)); }
 
 constexpr int kDT = 6;        // origin differences for d = -2..3
 constexpr int kQueue = 64;    // per-warp queue of accepted pairs
@@ -100,6 +102,7 @@ constexpr int kMaxListK = 1024;        // pair-list mode: most list entries of o
 // as the FP64 form decides it, so that no pair straddling the cutoff enters
 // one form's sums and not the other's (about 1e-4 of an atom's pairs)
 constexpr float kBorder = 4e-6f;
+constexpr float kWiden = 1.f + 2.f * kBorder;  // of rc^2: the pairs that the batch of forces looks at
 
 // Shared-memory carve-up, identical on host and device.
 struct Layout {
@@ -312,22 +315,26 @@ __device__ __forceinline__ void pair_force32(bool act, int i, int m, float4 d, c
 // thermal configurations do not reach) is left out here and raises the
 // tile's flag (*big_flag); the redo pass adds it.  SIDE (the full redo pass):
 // such terms go to the FP32 side sums fr instead.
-template <bool MULTI, bool ENERGY, bool COUNT, bool SIDE, class QD, class FA, class FR>
-__device__ __forceinline__ void force_batch(int cnt, int qh, const QD& qd, FA& fa, FR& fr, int cap, const PairArgs& A,
-                                            const LJ32* ljs, FixSum& ek, FixSum& wk, int& nacc, int* big_flag) {
+template <bool MULTI, bool ENERGY, bool COUNT, bool SIDE, class QD, class FA, class FR, class IN64>
+__device__ __forceinline__ void force_batch(int cnt, int q0, const QD& qd, FA& fa, FR& fr, int cap, const PairArgs& A,
+                                            const LJ32* ljs, FixSum& ek, FixSum& wk, int& nacc, int* big_flag,
+                                            const IN64& in64) {
   const int lane = threadIdx.x & 31;
-  const bool act = lane < cnt;
+  bool act = lane < cnt;
   int i = -1, m = 0;
   float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
   LJ32 P = A.lj.p32[0];
   if (act) {
-    const int slot = (qh + lane) & (kQueue - 1);
-    d = qd[slot];
+    d = qd[q0 + lane];
     const unsigned key = __float_as_uint(d.w);
     d.w = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));  // r^2 exactly as the distance test computed it
     i = key & 0x3fff;
     m = (key >> 16) & 0x3fff;
-    if (MULTI) P = ljs[((key >> 14) & 3) * A.lj.nt + (key >> 30)];
+    const int ti = MULTI ? (key >> 14) & 3 : 0, tj = MULTI ? key >> 30 : 0;
+    if (MULTI) P = ljs[ti * A.lj.nt + tj];
+    // the queue also holds the pairs just beyond the cutoff: at the border (kBorder) the FP64 test decides
+    act = d.w <= P.rc2;
+    if (fabsf(d.w - P.rc2) <= kBorder * P.rc2) act = in64(i, m, ti, tj);
   }
   pair_force32<ENERGY, COUNT, SIDE>(act, i, m, d, P, fa, fr, cap, A, ek, wk, nacc, big_flag);
 }
@@ -341,10 +348,10 @@ template <bool MULTI, bool ENERGY, bool COUNT, class QK, class PD, class CODE, c
 __device__ __forceinline__ void force_batch64(int cnt, const QK& qk, const PD& pd, const CODE& code, const IMG& img,
                                               const double* Lbox, FD& fd, int cap, const LJTable& lj,
                                               const LJ64* ljs, double& esum, double& wsum, int* status, int& nacc,
-                                              int qh) {
+                                              int q0) {
   const int lane = threadIdx.x & 31;
   if (lane >= cnt) return;
-  const unsigned key = (unsigned)qk[(qh + lane) & (kQueue - 1)];
+  const unsigned key = (unsigned)qk[q0 + lane];
   const int i = key & 0x3fff, m = (key >> 16) & 0x3fff;
   const int ci = code[i], cm = code[m];
   // difference of the copies' periodic images per axis: -1, 0 or +1 box
@@ -411,7 +418,7 @@ __device__ __forceinline__ void force_batch64(int cnt, const QK& qk, const PD& p
 // whose force is too large for the sums' range flags the tile, and the FP64
 // body redoes it.
 template <bool MULTI, bool ENERGY, bool COUNT, class QK, class PX, class FA, class FACE, class IN64>
-__device__ __forceinline__ void force_batch_fix(int cnt, int qh, const QK& qk, const PX& px, FA& fa, int cap,
+__device__ __forceinline__ void force_batch_fix(int cnt, int q0, const QK& qk, const PX& px, FA& fa, int cap,
                                                 const PairArgs& A, const FixPair* ljx, double& s12, double& s6s,
                                                 double& shift, int& nacc, int* big_flag, bool edge, const FACE& face,
                                                 const IN64& in64) {
@@ -421,7 +428,7 @@ __device__ __forceinline__ void force_batch_fix(int cnt, int qh, const QK& qk, c
   long long fx = 0, fy = 0, fz = 0;  // the force on i, in units of 2^-sf
   bool app = false;
   if (lane < cnt) {
-    const unsigned key = (unsigned)qk[(qh + lane) & (kQueue - 1)];
+    const unsigned key = (unsigned)qk[q0 + lane];
     i = key & 0x3fff;
     m = (key >> 16) & 0x3fff;
     const int ti = MULTI ? (key >> 14) & 3 : 0, tj = MULTI ? key >> 30 : 0;
@@ -579,8 +586,10 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   auto U = EXAMD_ARR(const float4, A.U, A.N, st);
 
   // (1) ext cells: global cell, count, first atom; ownership tables to smem
+  int cc0 = 0;  // the code of cell tid
   for (int e = tid; e < NE; e += blockDim.x) {
     int lx = e % EX, rr = e / EX, ly = rr % EY, lz = rr / EY;
+    if (e == tid) cc0 = lx | (ly << 5) | (lz << 10);
     int gx = X0 + lx - 1, gy = Y0 + ly - 1, gz = Z0 + lz - 1;
     gx += (gx < 0) ? B.nb[0] : 0;
     gx -= (gx >= B.nb[0]) ? B.nb[0] : 0;
@@ -594,7 +603,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
     lstart[e] = (unsigned short)min(A.cstart[gc + 1] - s0, 0xffff);  // a larger count overflows any capacity
   }
   {
-    const uint4* src = reinterpret_cast<const uint4*>(&c_own);
+    const uint4* src = reinterpret_cast<const uint4*>(&g_own);
     uint4* dst = reinterpret_cast<uint4*>(sown);
     if (!kFromList)
       for (int k = tid; k < (int)(sizeof(OwnLut) / 16); k += blockDim.x) dst[k] = src[k];
@@ -640,8 +649,9 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
             for (int d = -2; d <= 3; ++d) {
               const int l2 = l + d, ln = l + d + (d < 0);
               const float off = (l2 >= 0 && l2 <= E) ? fmaf((float)(nimg(l2) - n), rf, (float)d * blf) : 0.f;
-              const float near =
-                  (ln >= 0 && ln <= E) ? fmaf((float)(nimg(ln) - n), rf, (float)(d + (d < 0)) * blf) : 0.f;
+              const float near = d == 0 ? -1e30f  // the atom's own row: no gap
+                                 : (ln >= 0 && ln <= E) ? fmaf((float)(nimg(ln) - n), rf, (float)(d + (d < 0)) * blf)
+                                                        : 0.f;
               dt[l * kDT + d + 2] = make_float2(off, near);
             }
           }
@@ -673,8 +683,12 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
       int c = lstart[k];
       lstart[k] = run;
       // the cell of each staged atom, for the staging and the write-back
-      const int lx = k % EX, rr = k / EX, ly = rr % EY, lz = rr / EY;
-      const unsigned short cc = (unsigned short)(lx | (ly << 5) | (lz << 10));
+      int ck = cc0;
+      if (k != tid) {
+        const int lx = k % EX, rr = k / EX, ly = rr % EY, lz = rr / EY;
+        ck = lx | (ly << 5) | (lz << 10);
+      }
+      const unsigned short cc = (unsigned short)ck;
       for (int t = run, t1 = min(run + c, cap); t < t1; ++t) code[t] = cc;
       run += c;
     }
@@ -814,7 +828,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   auto pt = EXAMD_ARR(float4, wtab, 32, st);
   auto btA = EXAMD_ARR(float4, wtab + 32 * 16, 32, st);
   auto btB = EXAMD_ARR(float4, wtab + 32 * 32, 32, st);
-  int qn = 0, qh = 0;  // queued pairs and the ring's head
+  int qn = 0;  // queued pairs
   const unsigned lt = (1u << lane) - 1u;
   const unsigned le = FULL >> (31 - lane);
   auto r2l = EXAMD_ARR(unsigned char, smem + L.r2l + 64 * warp, FP64 ? 64 : 1, st);  // FP64 form: two rank -> lane tables of 32
@@ -879,27 +893,26 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   auto enqueue = [&](bool acc, const float4& dq, int key) {
     const unsigned bal = __ballot_sync(FULL, acc);
     if (acc) {
-      const int p = (qh + qn + __popc(bal & lt)) & (kQueue - 1);
+      const int p = qn + __popc(bal & lt);
       if (FP64 || FIX)
         qk[p] = key;
       else
         qd[p] = make_float4(dq.x, dq.y, dq.z, __int_as_float(key));
     }
     qn += __popc(bal);
-    if (qn >= 32) {  // a batch only moves the ring's head
+    if (qn >= 32) {  // a batch: the last 32, so that what is left stays where it is
+      qn -= 32;
       __syncwarp();
       if (FP64)
         force_batch64<MULTI, ENERGY, COUNT>(32, qk, pd, code, img, B.L, fd, cap, A.lj, ljs64, esum, wsum, A.status,
-                                            nacc, qh);
+                                            nacc, qn);
       else if (FIX)
-        force_batch_fix<MULTI, ENERGY, COUNT>(32, qh, qk, px, fa, cap, A, ljx, esum, wsum, shsum, nacc, big_flag,
+        force_batch_fix<MULTI, ENERGY, COUNT>(32, qn, qk, px, fa, cap, A, ljx, esum, wsum, shsum, nacc, big_flag,
                                               edge, face, inside64);
       else
-        force_batch<MULTI, ENERGY, COUNT, MODE == kRedoFull>(32, qh, qd, fa, fr, cap, A, ljs32, ek, wk, nacc,
-                                                             big_flag);
+        force_batch<MULTI, ENERGY, COUNT, MODE == kRedoFull>(32, qn, qd, fa, fr, cap, A, ljs32, ek, wk, nacc,
+                                                             big_flag, inside64);
       __syncwarp();
-      qh = (qh + 32) & (kQueue - 1);
-      qn -= 32;
     }
   };
 
@@ -974,11 +987,10 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
       if (COUNT && valid) ++neval;
       const float thr = FIX ? (MULTI ? ljx[ti * A.lj.nt + tj].pre : A.fx.p[0].pre)
                         : MODE == kListBuild ? (MULTI ? ljs32[ti * A.lj.nt + tj].rl2 : q32.rl2)
-                                             : (MULTI ? ljs32[ti * A.lj.nt + tj].rc2 : q32.rc2);
+                        : MODE == kRedoBig   ? (MULTI ? ljs32[ti * A.lj.nt + tj].rc2 : q32.rc2)
+                                             : (MULTI ? ljs32[ti * A.lj.nt + tj].rc2 * kWiden : q32.rc2 * kWiden);
       const int key = (int)(kb + (MULTI ? (unsigned)tj << 30 : 0u));
-      bool acc = valid && dq.w <= thr;
-      if ((MODE == kMain || MODE == kRedoFull) && valid && fabsf(dq.w - thr) <= kBorder * thr)
-        acc = inside64(kb & 0x3fff, m, ti, MULTI ? tj : 0);  // at the border: FP64
+      const bool acc = valid && dq.w <= thr;
       if (MODE == kRedoBig)
         redo_pair(acc, dq, key);
       else if (MODE == kListBuild)
@@ -1267,8 +1279,6 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         const int k = K + lane;
         const bool valid = k < W;
         const float4 b0v = btA[qr], b1v = btB[qr];
-        const float2 gm = __half22float2(*reinterpret_cast<const __half2*>(&b0v.w));
-        const float2 gp = __half22float2(*reinterpret_cast<const __half2*>(&b1v.x));
         const int sq = __float_as_int(b1v.y), cc = __float_as_int(b1v.z);
         const int s_q = sq & 511, i = sq >> 9;
         const int cls = (cc >> 15) & 127;
@@ -1278,9 +1288,9 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         int lo1 = 0, n1 = 0, lo2 = 0, n2 = 0;
         float cy = 0.f, cz = 0.f;
         if (mask) {
-          const int yc = (ent >> 5) & 7, zc = ent >> 8;  // dy + 2, dz + 2
+          const int yc = (ent >> 5) & 7, zc = (ent >> 8) & 7;  // dy + 2, dz + 2
           const int dy = yc - 2, dz = zc - 2;
-          const bool selfrow = (dy | dz) == 0;
+          const bool selfrow = ent >> 11;
           const int rowbase = ((ly + dy) + EY * (lz + dz)) * EX + lx - 2;  // + bit b -> ext cell of dx = b - 2
           const float2 ry = dyt[ly * kDT + yc], rz = dzt[lz * kDT + zc];
           cy = ry.x;
@@ -1295,12 +1305,15 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
           // distance from the atom to the row's cell boxes
           // (the row's near face comes with its origin offset)
           const float ty = ry.y - b0v.y, tz = rz.y - b0v.z;
-          const float gy = dy == 0 ? 0.f : fmaxf(dy > 0 ? ty : -ty, 0.f);
-          const float gz = dz == 0 ? 0.f : fmaxf(dz > 0 ? tz : -tz, 0.f);
-          const float g2 = gy * gy + gz * gz;
-          const float tr = prune2 - g2;
+          const float gy = fmaxf(__int_as_float(__float_as_int(ty) ^ (dy & 0x80000000)), 0.f);
+          const float gz = fmaxf(__int_as_float(__float_as_int(tz) ^ (dz & 0x80000000)), 0.f);
+          const float tr = prune2 - (gy * gy + gz * gz);
           if (tr < 0.f) mask = 0;
-          mask &= ~((gm.x > tr ? 1 : 0) | (gm.y > tr ? 2 : 0) | (gp.x > tr ? 8 : 0) | (gp.y > tr ? 16 : 0));
+          // the x-gaps beyond tr, compared as FP16 (tr rounded up, so that no cell is pruned wrongly)
+          const __half2 tr2 = __half2half2(__float2half_ru(tr));
+          const unsigned pm = (__hgt2_mask(*reinterpret_cast<const __half2*>(&b0v.w), tr2) & 0x00020001u) |
+                              (__hgt2_mask(*reinterpret_cast<const __half2*>(&b1v.x), tr2) & 0x00100008u);
+          mask &= ~(pm | (pm >> 16));
           if (mask) {
             const int b0 = __ffs(mask) - 1, b1 = 31 - __clz(mask);
             const int mm = mask >> b0;
@@ -1383,7 +1396,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         int lo1 = 0, n1 = 0, lo2 = 0, n2 = 0;
         bool self = false;
         if (mask) {
-          const int dy = (int)((ent >> 5) & 7) - 2, dz = (int)(ent >> 8) - 2;
+          const int dy = (int)((ent >> 5) & 7) - 2, dz = (int)((ent >> 8) & 7) - 2;
           const int rowbase = ((ly + dy) + EY * (lz + dz)) * EX + lx - 2;  // + bit b -> ext cell of dx = b - 2
           const int b0 = __ffs(mask) - 1, b1 = 31 - __clz(mask);
           const int mm = mask >> b0;
@@ -1414,13 +1427,13 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
     __syncwarp();
     if (FP64)
       force_batch64<MULTI, ENERGY, COUNT>(qn, qk, pd, code, img, B.L, fd, cap, A.lj, ljs64, esum, wsum, A.status,
-                                          nacc, qh);
+                                          nacc, 0);
     else if (FIX)
-      force_batch_fix<MULTI, ENERGY, COUNT>(qn, qh, qk, px, fa, cap, A, ljx, esum, wsum, shsum, nacc, big_flag,
+      force_batch_fix<MULTI, ENERGY, COUNT>(qn, 0, qk, px, fa, cap, A, ljx, esum, wsum, shsum, nacc, big_flag,
                                             edge, face, inside64);
     else
-      force_batch<MULTI, ENERGY, COUNT, MODE == kRedoFull>(qn, qh, qd, fa, fr, cap, A, ljs32, ek, wk, nacc,
-                                                           big_flag);
+      force_batch<MULTI, ENERGY, COUNT, MODE == kRedoFull>(qn, 0, qd, fa, fr, cap, A, ljs32, ek, wk, nacc,
+                                                           big_flag, inside64);
   }
   __syncthreads();
   // a large term was left out: list the tile for the redo pass
