@@ -218,21 +218,30 @@ struct KSum {
 // with integer operations, and spend FP64 instructions only on the arithmetic
 // that needs them.
 
+// The bits of x, opaque to the compiler: it turns the integer tests below back
+// into FP64 comparisons where it sees that the bits are a double's (measured as
+// FP64 operations executed: three of k_bin_count's three, ten of k_kick's 19).
+__device__ __forceinline__ long long dbits(double x) {
+  long long b;
+  asm("mov.b64 %0, %1;" : "=l"(b) : "d"(x));
+  return b;
+}
+
 // 0 <= x < L (either zero), for L > 0: non-negative doubles are ordered as
 // their bit patterns, and every negative one has the sign bit set.
 __device__ __forceinline__ bool in_range_bits(double x, double L) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  return b < (unsigned long long)__double_as_longlong(L) || b == 0x8000000000000000ull;
+  const unsigned long long b = (unsigned long long)dbits(x);
+  return b < (unsigned long long)dbits(L) || b == 0x8000000000000000ull;
 }
 
 __device__ __forceinline__ bool finite_bits(double x) {
-  return ((__double_as_longlong(x) >> 52) & 0x7ff) != 0x7ff;
+  return ((dbits(x) >> 52) & 0x7ff) != 0x7ff;
 }
 
 // A float within one FP32 ulp of x (mantissa truncated), for estimates only;
 // 0 for |x| < 2^-126.  x must be below 2^128 in magnitude.
 __device__ __forceinline__ float d2f_trunc(double x) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const unsigned long long b = (unsigned long long)dbits(x);
   const int e = (int)((b >> 52) & 0x7ff);
   if (e < 1023 - 126) return 0.f;
   return __uint_as_float((unsigned)(b >> 32 & 0x80000000u) | ((unsigned)(e - 1023 + 127) << 23) |
@@ -243,7 +252,7 @@ __device__ __forceinline__ float d2f_trunc(double x) {
 // below 2^-126 become 0 (no subnormals).  Same result as (float)x in the
 // normal range.
 __device__ __forceinline__ float d2f_rn_nonneg(double x) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+  const unsigned long long b = (unsigned long long)dbits(x) & 0x7fffffffffffffffull;
   const int e = (int)(b >> 52);
   if (e < 1023 - 126) return 0.f;
   const unsigned mf = (unsigned)((b >> 29) & 0x7fffff);
@@ -282,11 +291,11 @@ __device__ __forceinline__ int cell_offset(double x, const BoxDev& B, int a, flo
   const int nb = B.nb[a];
   int c = (int)(d2f_trunc(x) * B.blif);
   c = min(max(c, 0), nb - 1);
-  long long bx = __double_as_longlong(x);
+  long long bx = dbits(x);
   if (bx == (long long)0x8000000000000000ull) bx = 0;  // -0
-  if (bx < __double_as_longlong(mul_pow2((unsigned)(c * B.blq), B.blk))) {
+  if (bx < dbits(mul_pow2((unsigned)(c * B.blq), B.blk))) {
     c = max(c - 1, 0);  // the estimate was one too high
-  } else if (c < nb - 1 && bx >= __double_as_longlong(mul_pow2((unsigned)((c + 1) * B.blq), B.blk))) {
+  } else if (c < nb - 1 && bx >= dbits(mul_pow2((unsigned)((c + 1) * B.blq), B.blk))) {
     ++c;  // one too low
   }
   u = d2f_rn_nonneg(x - mul_pow2((unsigned)(c * B.blq), B.blk));
@@ -296,7 +305,7 @@ __device__ __forceinline__ int cell_offset(double x, const BoxDev& B, int a, flo
 // A coordinate x >= 0 in units of 2^ue, rounded to the nearest integer, modulo
 // 2^64 (differences of nearby coordinates are then exact in 64 bits).
 __device__ __forceinline__ unsigned long long to_fixed(double x, int ue) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const unsigned long long b = (unsigned long long)dbits(x);
   const int e = (int)(b >> 52) & 0x7ff;
   if (e == 0) return 0ull;  // zero (either sign) and subnormals
   const unsigned long long m = (b & 0xfffffffffffffull) | 0x10000000000000ull;

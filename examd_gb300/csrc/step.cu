@@ -8,6 +8,7 @@
 // are HBM-bound; FP64 is used only where positions, velocities and the
 // reductions need it.
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.cuh"
@@ -29,7 +30,7 @@ __device__ __forceinline__ void bin_store(int s, double x, double y, double z, c
 
 // x rounded to the nearest float, either sign, on the integer pipe.
 __device__ __forceinline__ float d2f_rn_signed(double x) {
-  const long long b = __double_as_longlong(x);
+  const long long b = dbits(x);
   const float m = d2f_rn_nonneg(__longlong_as_double(b & 0x7fffffffffffffffll));
   return b < 0 ? -m : m;
 }
@@ -45,7 +46,7 @@ static __device__ __noinline__ double offset_wrapped(double u, double L) { retur
 // image nearest the cell (it moved less than half the skin).
 __device__ __forceinline__ float list_offset(double x, int c, const BoxDev& B, int a) {
   double u = x - mul_pow2((unsigned)(c * B.blq), B.blk);
-  const long long b = __double_as_longlong(u) & 0x7fffffffffffffffll;
+  const long long b = dbits(u) & 0x7fffffffffffffffll;
   if (d2f_trunc(__longlong_as_double(b)) > 0.5f * B.Lf[a]) u = offset_wrapped(u, B.L[a]);
   return d2f_rn_signed(u);
 }
@@ -89,10 +90,11 @@ __device__ __forceinline__ void disp_max(float d2, int* lw) {
 
 // Sum of an atom's force partials: the owning tile's, then the halo slots in
 // increasing order (fixed order: deterministic).  Mixed form: Kahan in FP32.
+template <bool FP64>
 __device__ __forceinline__ void gather_force(const StepArgs& a, int64_t s, double f[3]) {
   s = EXAMD_IDX(s, a.N, a.status);
   const int m = a.bmask[EXAMD_IDX(a.cellS[s], a.nc, a.status)];
-  if (a.fp64) {
+  if (FP64) {
     const double* Fo = (const double*)a.Fown;
     const double* P = (const double*)a.P;
     double fx = Fo[s], fy = Fo[a.N + s], fz = Fo[2 * a.N + s];
@@ -135,12 +137,13 @@ __device__ __forceinline__ void gather_force(const StepArgs& a, int64_t s, doubl
 
 // Forces of the caller's atoms [i0, i1) in caller order (AoS): the atom's
 // partials gathered at its sorted slot inv[i]; written or added (acc).
+template <bool FP64>
 __global__ void k_forces_out(const StepArgs a, int64_t i0, int64_t i1, const int* __restrict__ inv,
                              double* __restrict__ out, int acc) {
   const int64_t i = i0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= i1) return;
   double f[3];
-  gather_force(a, inv[i], f);
+  gather_force<FP64>(a, inv[i], f);
   if (acc) {
     out[3 * i] += f[0];
     out[3 * i + 1] += f[1];
@@ -155,7 +158,11 @@ __global__ void k_forces_out(const StepArgs a, int64_t i0, int64_t i1, const int
 cudaError_t launch_forces_out(const StepArgs& s, int64_t i0, int64_t i1, const int* inv, double* out, int accumulate,
                               cudaStream_t st) {
   if (i1 <= i0) return cudaSuccess;
-  k_forces_out<<<(unsigned)((i1 - i0 + 255) / 256), 256, 0, st>>>(s, i0, i1, inv, out, accumulate);
+  const unsigned g = (unsigned)((i1 - i0 + 255) / 256);
+  if (s.fp64)
+    k_forces_out<true><<<g, 256, 0, st>>>(s, i0, i1, inv, out, accumulate);
+  else
+    k_forces_out<false><<<g, 256, 0, st>>>(s, i0, i1, inv, out, accumulate);
   return cudaGetLastError();
 }
 
@@ -264,23 +271,26 @@ cudaError_t launch_reduce_atoms(int nboxes, const int64_t* atom0, const double* 
   return cudaGetLastError();
 }
 
-// v += ckick F/m; optional kinetic energy at v + hk F/m; optional drift
-// x += dt v with periodic wrap followed by the binning count of the next step
-// (pair-list mode: by the offsets from the build cells and the displacement
-// since the build instead).
-__global__ void k_kick(const KickArgs k) {
+// v += ckick F/m; KE: also the kinetic energy at v + hk F/m; DRIFT: x += dt v
+// with periodic wrap followed by the binning count of the next step (LIST: by
+// the offsets from the build cells and the displacement since the build
+// instead).  Bound by HBM and the FP64 pipe: 9 FP64 operations an atom (three
+// kicks, three drifts, three offsets); the range and finiteness tests go by the
+// bits (dbits).
+template <bool FP64, bool KE, bool LIST, bool DRIFT>
+__global__ void __launch_bounds__(256) k_kick(const KickArgs k) {
   int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const bool in = s < k.s.N;
   const int64_t ss = in ? s : 0;
   double f[3];
-  gather_force(k.s, ss, f);
+  gather_force<FP64>(k.s, ss, f);
   const int mt = k.meta[ss];
   const int type = mt & 0xff, box = mt >> 8;
   const double ck = k.ckm[type];
   double v[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) v[a] = k.V[a][ss];
-  if (k.hk > 0.0) {
+  if (KE) {
     const double hm = k.hkm[type];
     double ke = 0.0;
 #pragma unroll
@@ -298,7 +308,7 @@ __global__ void k_kick(const KickArgs k) {
       v[a] = v[a] + ck * f[a];
       k.V[a][s] = v[a];
     }
-    if (k.drift) {
+    if (DRIFT) {
       const BoxDev& B = k.s.boxes[box];
       double x[3];
 #pragma unroll
@@ -310,13 +320,13 @@ __global__ void k_kick(const KickArgs k) {
         atomicOr(k.status, ST_NONFINITE);
         x[0] = x[1] = x[2] = 0.0;
       }
-      if (k.list)
+      if (LIST)
         d2 = list_update(s, x, k.s.cellS[s], type, B, k.U, k.Ub);
       else
         bin_store((int)s, x[0], x[1], x[2], B, k.cellOld, k.slot, k.count, k.s.nc, k.status);
     }
   }
-  if (k.list && k.drift) disp_max(d2, k.lw);
+  if (LIST && DRIFT) disp_max(d2, k.lw);
 }
 
 // Pair-list mode: new positions for the caller's atoms [i0, i1) (AoS, caller
@@ -363,7 +373,21 @@ cudaError_t launch_gather_pos_list(int64_t i0, int64_t i1, const double* aos, co
 }
 
 cudaError_t launch_kick(const KickArgs& k, cudaStream_t st) {
-  if (k.s.N > 0) k_kick<<<(unsigned)((k.s.N + 255) / 256), 256, 0, st>>>(k);
+  if (k.s.N <= 0) return cudaSuccess;
+  const unsigned g = (unsigned)((k.s.N + 255) / 256);
+  auto go = [&](auto fp64, auto ke) {
+    constexpr bool F = decltype(fp64)::value, E = decltype(ke)::value;
+    if (!k.drift)
+      k_kick<F, E, false, false><<<g, 256, 0, st>>>(k);
+    else if (k.list)
+      k_kick<F, E, true, true><<<g, 256, 0, st>>>(k);
+    else
+      k_kick<F, E, false, true><<<g, 256, 0, st>>>(k);
+  };
+  if (k.s.fp64)
+    k.hk > 0.0 ? go(std::true_type{}, std::true_type{}) : go(std::true_type{}, std::false_type{});
+  else
+    k.hk > 0.0 ? go(std::false_type{}, std::true_type{}) : go(std::false_type{}, std::false_type{});
   return cudaGetLastError();
 }
 
