@@ -72,6 +72,7 @@ constexpr int kParts = 2;     // work units per 32 staged atoms (1, 3 and 4 meas
 // room 12 warps fit 3 CTAs on an SM at the tiles of a dense liquid (36 warps
 // against 24 with 8), to hide its shared-memory latency.
 constexpr int kBuildWarps = 12;
+constexpr int kWideWarps = 12;
 // Fixed-point scale 2^17: each term is rounded to 2^-18 in absolute value.
 // With the pairs at the cutoff decided in FP64, the mixed form's error on an
 // equilibrated 1M-atom liquid was 2.38e-6 RMS of F_rms at 2^16, about 1.6e-6
@@ -186,11 +187,14 @@ static int redo_smem_bytes(const PairConfig& cfg, int cap_redo, int ne_max, int 
                   : b;
 }
 
+static bool uses_wide(const PairConfig& c) { return c.wide && !c.fp64 && !c.list && !c.count; }
+
 // The first pass's layout: the enumeration's, or in pair-list mode (without
 // counters, which the enumeration gives) the list pass's.
 static int main_smem_bytes(const PairConfig& cfg, int cap, int ne_max, int ext_max) {
   const int mode = (cfg.list && !cfg.count && !cfg.fp64) ? kList : kMain;
   if (cfg.fix) return make_layout(false, cap, ne_max, ext_max, cfg.warps, kFixed, cfg.multi).bytes;
+  if (uses_wide(cfg)) return make_layout(false, cap, ne_max, ext_max, kWideWarps, kMain, cfg.multi).bytes;
   return make_layout(cfg.fp64, cap, ne_max, ext_max, cfg.warps, mode, cfg.multi).bytes;
 }
 
@@ -200,7 +204,7 @@ static int build_smem_bytes(const PairConfig& cfg, int cap, int ne_max, int ext_
 
 int pair_smem_bytes(const PairConfig& cfg, int cap, int cap_redo, int ne_max, int ext_max) {
   if (cfg.fix) return std::max(main_smem_bytes(cfg, cap, ne_max, ext_max), redo_smem_bytes(cfg, cap_redo, ne_max, ext_max));
-  int b = make_layout(cfg.fp64, cap, ne_max, ext_max, cfg.warps, kMain, cfg.multi).bytes;
+  int b = make_layout(cfg.fp64, cap, ne_max, ext_max, cfg.wide ? kWideWarps : cfg.warps, kMain, cfg.multi).bytes;
   if (cfg.fp64) return b;
   b = std::max(b, redo_smem_bytes(cfg, cap_redo, ne_max, ext_max));
   if (cfg.list) b = std::max(b, std::max(main_smem_bytes(cfg, cap, ne_max, ext_max),
@@ -1680,6 +1684,14 @@ __global__ void __launch_bounds__(256, FP64 ? 3 : 4) k_pair(const PairArgs A) {
   pair_tile<FP64, MULTI, ENERGY, COUNT, kMain>(A, A.order[blockIdx.x]);
 }
 
+// The mixed form's enumeration with kWideWarps warps per CTA, for grids that one
+// wave of 3 CTAs per SM holds: an SM then has 2 or 3 CTAs however few warps they
+// are, and 12 warps instead of 8 shorten each.
+template <bool MULTI, bool ENERGY>
+__global__ void __launch_bounds__(32 * kWideWarps, 3) k_pair_wide(const PairArgs A) {
+  pair_tile<false, MULTI, ENERGY, false, kMain>(A, A.order[blockIdx.x]);
+}
+
 // FP64 form: the first pass in fixed point, and the FP64 body for the tiles that
 // it listed (normally none).
 template <bool MULTI, bool ENERGY, bool COUNT>
@@ -1776,6 +1788,10 @@ static void* pick_redo64(const PairConfig& c) {
 }
 
 static void* pick(const PairConfig& c) {
+  if (uses_wide(c)) {
+    if (c.multi) return c.energy ? (void*)&k_pair_wide<true, true> : (void*)&k_pair_wide<true, false>;
+    return c.energy ? (void*)&k_pair_wide<false, true> : (void*)&k_pair_wide<false, false>;
+  }
   if (c.fix) return c.multi ? pick_fix<true>(c) : pick_fix<false>(c);
   if (uses_list(c)) {
     if (c.cut) {
@@ -1820,7 +1836,8 @@ cudaError_t launch_pair(const PairConfig& cfg, const PairArgs& a, int ntiles, in
   // smem_bytes (the larger of the passes' needs) bounds every launch
   const int main_smem = main_smem_bytes(cfg, a.cap, a.ne_max, a.ext_max);
   if (main_smem > smem_bytes) return cudaErrorInvalidValue;
-  cudaError_t e = cudaLaunchKernel(fn, dim3(ntiles), dim3(32 * cfg.warps), args, (size_t)main_smem, st);
+  const int warps = uses_wide(cfg) ? kWideWarps : cfg.warps;
+  cudaError_t e = cudaLaunchKernel(fn, dim3(ntiles), dim3(32 * warps), args, (size_t)main_smem, st);
   if (e != cudaSuccess || (cfg.fp64 && !cfg.fix)) return e;
   // the redo pass: a few blocks per SM at most; nothing to do in a thermal system
   const int redo_smem = redo_smem_bytes(cfg, a.cap_redo, a.ne_max, a.ext_max);
