@@ -333,6 +333,7 @@ struct examd_ctx {
   cudaEvent_t ev_side[4] = {};
   bool side_ke = false, side_pe = false;
 
+  bool in_call = false;  // the work of a force call is being queued
   bool atoms_set = false;
   bool forces_valid = false;  // Fown/P hold F(X[cur])
   bool energy_valid = false;
@@ -973,6 +974,13 @@ void examd_gpu_destroy(examd_ctx* ctx) {
 // --------------------------------------------------------------------------
 namespace {
 
+struct InCall {  // marks the queueing of a force call (its launches are chained)
+  examd_ctx* ctx;
+  bool was;
+  explicit InCall(examd_ctx* c) : ctx(c), was(c->in_call) { c->in_call = true; }
+  ~InCall() { ctx->in_call = was; }
+};
+
 inline unsigned nblk(int64_t n, int t = 256) { return (unsigned)std::max<int64_t>(1, (n + t - 1) / t); }
 
 // Scan and final ordering after a counting pass; swaps the buffers.
@@ -989,16 +997,16 @@ int finish_binning(examd_ctx* ctx, bool want_inv, const int* gate = nullptr) {
   const int s = ctx->cur, d = 1 - ctx->cur;
   const bool list = ctx->list;
   if (list) want_inv = true;
-  if (nsb > 1) k_scan_reduce<<<nsb, 256, 0, st>>>(nc, ctx->count, ctx->bsum, gate);  // (one block has none before it)
-  k_scan_final<<<nsb, 256, 0, st>>>(nc, ctx->count, ctx->bsum, ctx->cstart, gate);
+  const bool chain = ctx->in_call && !list;  // (in pair-list mode these may be the body of a conditional node)
+  if (nsb > 1)  // (one block has none before it)
+    CK(launch_chained(chain, k_scan_reduce, nsb, 256, st, nc, ctx->count, ctx->bsum, gate));
+  CK(launch_chained(chain, k_scan_final, nsb, 256, st, nc, ctx->count, ctx->bsum, ctx->cstart, gate));
   if (ctx->N > 0) {
-    k_finalize<<<nblk(ctx->N), 256, 0, st>>>(ctx->N, ctx->cellOld, ctx->slot, ctx->cstart, ctx->d_boxes,
-                                              ctx->X[s][0], ctx->X[s][1], ctx->X[s][2], ctx->V[s][0],
-                                              ctx->V[s][1], ctx->V[s][2], ctx->meta[s], ctx->id[s],
-                                              ctx->X[d][0], ctx->X[d][1], ctx->X[d][2], ctx->V[d][0],
-                                              ctx->V[d][1], ctx->V[d][2], ctx->meta[d], ctx->id[d], ctx->U,
-                                              list ? ctx->Ub : nullptr, ctx->cellS, want_inv ? ctx->inv : nullptr,
-                                              ctx->NC, ctx->status, gate);
+    CK(launch_chained(chain, k_finalize, nblk(ctx->N), 256, st, ctx->N, ctx->cellOld, ctx->slot, ctx->cstart,
+                      ctx->d_boxes, ctx->X[s][0], ctx->X[s][1], ctx->X[s][2], ctx->V[s][0], ctx->V[s][1],
+                      ctx->V[s][2], ctx->meta[s], ctx->id[s], ctx->X[d][0], ctx->X[d][1], ctx->X[d][2], ctx->V[d][0],
+                      ctx->V[d][1], ctx->V[d][2], ctx->meta[d], ctx->id[d], ctx->U, list ? ctx->Ub : nullptr,
+                      ctx->cellS, want_inv ? ctx->inv : nullptr, ctx->NC, ctx->status, gate));
     if (list)
       k_copy_back<<<nblk(ctx->N), 256, 0, st>>>(ctx->N, ctx->X[d][0], ctx->X[d][1], ctx->X[d][2], ctx->V[d][0],
                                                  ctx->V[d][1], ctx->V[d][2], ctx->meta[d], ctx->id[d], ctx->X[s][0],
@@ -1321,6 +1329,7 @@ int run_pair(examd_ctx* ctx, bool energy, bool count, double* boxE, double* boxW
   PairConfig c = ctx->pc;
   c.energy = energy;
   c.count = count;
+  c.chain = ctx->in_call || !(c.wide || boxE);
   if (ctx->side_pe) {  // the last step's sums read the tile energies that this pass writes
     CK(cudaStreamWaitEvent(ctx->st, ctx->ev_side[3], 0));
     ctx->side_pe = false;
@@ -1369,6 +1378,7 @@ StepArgs step_args(examd_ctx* ctx) {
 // The work of the force call, queued on the context's streams; the second
 // stream rejoins the first at the end (so the sequence can be captured).
 int enqueue_forces(examd_ctx* ctx, double* forces, double* epot, double* virial, int accumulate) {
+  const InCall in_call(ctx);
   cudaStream_t st = ctx->st, st2 = ctx->st2;
   const bool energy = epot || virial;
   const int64_t N = ctx->N;
@@ -1504,6 +1514,7 @@ namespace {
 // The force call at new positions, queued (see examd_gpu_forces_at).
 int enqueue_forces_at(examd_ctx* ctx, const double* pos, double* forces, double* epot, double* virial,
                       int accumulate) {
+  const InCall in_call(ctx);
   cudaStream_t st = ctx->st, st2 = ctx->st2;
   const int s = ctx->cur;
   const int64_t N = ctx->N;
@@ -1526,11 +1537,9 @@ int enqueue_forces_at(examd_ctx* ctx, const double* pos, double* forces, double*
                                   ctx->X[s][1], ctx->X[s][2], ctx->meta[s], ctx->inv, ctx->cellS, ctx->U, ctx->Ub,
                                   ctx->lw, ctx->status, st));
       } else {
-        k_gather_pos_bin_range<<<nblk(i1 - i0), 256, 0, st>>>(i0, i1, ctx->stage2, ctx->d_boxes,
-                                                              ctx->p.strict_box, ctx->X[s][0], ctx->X[s][1],
-                                                              ctx->X[s][2], ctx->meta[s], ctx->inv, ctx->cellOld,
-                                                              ctx->slot, ctx->count, ctx->status);
-        CK(cudaGetLastError());
+        CK(launch_chained(true, k_gather_pos_bin_range, nblk(i1 - i0), 256, st, i0, i1, ctx->stage2, ctx->d_boxes,
+                          ctx->p.strict_box, ctx->X[s][0], ctx->X[s][1], ctx->X[s][2], ctx->meta[s], ctx->inv,
+                          ctx->cellOld, ctx->slot, ctx->count, ctx->status));
       }
     }
   }

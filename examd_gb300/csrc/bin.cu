@@ -89,6 +89,8 @@ __global__ void k_gather_pos_bin_range(int64_t i0, int64_t i1, const double* __r
                                        const int* __restrict__ meta, const int* __restrict__ inv,
                                        int* __restrict__ cellOld, int* __restrict__ slot, int* __restrict__ count,
                                        int* __restrict__ status) {
+  grid_trigger();
+  grid_wait();
   const int64_t i = i0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= i1) return;
   const int s = inv[i];
@@ -141,6 +143,8 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* sh, int& total) 
 __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(int nc, const int* __restrict__ count,
                                                               int* __restrict__ bsum, const int* gate) {
   __shared__ int sh[kScanThreads / 32];
+  grid_trigger();
+  grid_wait();
   if (gate && !*gate) return;
   int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
   int s = 0;
@@ -159,6 +163,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_final(int nc, int* __rest
                                                              const int* __restrict__ bsum,
                                                              int* __restrict__ cstart, const int* gate) {
   __shared__ int sh[kScanThreads / 32];
+  grid_trigger();
+  grid_wait();
   if (gate && !*gate) return;
   int pre = 0;
   for (int k = threadIdx.x; k < (int)blockIdx.x; k += blockDim.x) pre += bsum[k];
@@ -201,6 +207,8 @@ __global__ void k_finalize(int64_t n, const int* __restrict__ cellOld, const int
                            int* __restrict__ id2, float4* __restrict__ U, float4* __restrict__ Ub,
                            int* __restrict__ cellS, int* __restrict__ inv, int nc, int* __restrict__ status,
                            const int* gate) {
+  grid_trigger();
+  grid_wait();
   if (gate && !*gate) return;
   const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (s >= n) return;

@@ -178,6 +178,14 @@ __host__ __device__ inline int pos_class(int l, int t) {
 
 // Tile descriptor: int4 {box, x0, y0, z0}, int4 {tx, ty, tz, 0}.
 
+// Chained kernels (launch_chained, kernels.cuh): a kernel lets the next one of
+// its stream be launched once all its blocks run (grid_trigger), and touches
+// nothing that earlier kernels write or read before they are complete
+// (grid_wait, on every path: the next kernel's wait then covers them too).  Both
+// do nothing in a kernel launched plainly.
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ float rcp_approx(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

@@ -1,9 +1,47 @@
 // kernels.cuh -- host-side launchers of the device kernels (one per .cu file).
 #pragma once
 
+#include <tuple>
+
 #include "common.cuh"
 
 namespace examd {
+
+// Launches of a force call's kernels, each of which waits for the one before it
+// on the device (grid_wait, common.cuh): with programmatic stream serialization
+// the next kernel's blocks are placed while the last ones of this kernel run.
+// chain = false: a plain launch.  A force call chains its binning, pair pass, redo
+// pass and gather (276k atoms 368 -> 349 us, 104k in FP64 286 -> 270 us).  A step
+// loop chains the pair and redo pass only (116 -> 112 us a step at 88k atoms,
+// FP64), and not where the pair pass is one wave of wide CTAs or the energy sums
+// run beside it: chained kicks and binning took 77 us a step against 69 (32k
+// crystal, FP64; pair and redo alone 67, with energies 77 against 75), and the
+// wide pass 59 against 56.
+inline cudaError_t launch_chained_ptr(bool chain, const void* fn, dim3 grid, dim3 block, void** args, size_t smem,
+                                      cudaStream_t st) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = chain ? 1 : 0;
+  return cudaLaunchKernelExC(&c, fn, args);
+}
+
+template <class... P, class... A>
+cudaError_t launch_chained(bool chain, void (*fn)(P...), unsigned grid, unsigned block, cudaStream_t st, A... a) {
+  std::tuple<P...> v{static_cast<P>(a)...};
+  return std::apply(
+      [&](auto&... x) {
+        void* args[] = {(void*)&x...};
+        return launch_chained_ptr(chain, (const void*)fn, dim3(grid), dim3(block), args, 0, st);
+      },
+      v);
+}
 
 // ---- bin.cu -----------------------------------------------------------------
 __global__ void k_make_meta(int64_t n, int nboxes, const int64_t* atom0, bool typed, int ntypes, int* meta,
@@ -107,6 +145,7 @@ struct PairConfig {
   bool count = false;   // candidate / accepted counters
   bool list = false;    // mixed form: pair-list mode (forces from the per-tile lists)
   bool cut = true;      // list pass: the potential's own range is finite (WCA) and tested
+  bool chain = false;   // the pair and redo passes as chained launches
   bool wide = false;    // mixed form without lists: the enumeration with 12 warps per CTA
   int warps = 8;
 };

@@ -556,6 +556,7 @@ template <bool FP64, bool MULTI, bool ENERGY, bool COUNT, int MODE, bool CUT = t
 __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   extern __shared__ __align__(16) unsigned char smem[];
   const unsigned FULL = 0xffffffffu;
+  // ownership table, type table and axis tables come first: they are fixed for the context
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   const int4 t0 = A.tiles[2 * tile], t1 = A.tiles[2 * tile + 1];
   const BoxDev& B = A.boxes[t0.x];
@@ -564,6 +565,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   const int EX = tx + 2, EY = ty + 2, EZ = tz + 2;
   const int NE = EX * EY * EZ;
   constexpr bool kFromList = MODE == kList || MODE == kListBig;
+  if (MODE == kMain || MODE == kFixed) grid_trigger();
   if (kFromList && MODE == kList && A.lcount[tile] < 0) return;  // a fallback tile: the redo pass computes it
   constexpr bool FIX = MODE == kFixed;
   const int cap = (MODE == kMain || MODE == kListBuild || MODE == kList || FIX) ? A.cap : A.cap_redo;
@@ -589,23 +591,6 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   auto code = EXAMD_ARR(unsigned short, smem + L.code, cap, st);
   auto U = EXAMD_ARR(const float4, A.U, A.N, st);
 
-  // (1) ext cells: global cell, count, first atom; ownership tables to smem
-  int cc0 = 0;  // the code of cell tid
-  for (int e = tid; e < NE; e += blockDim.x) {
-    int lx = e % EX, rr = e / EX, ly = rr % EY, lz = rr / EY;
-    if (e == tid) cc0 = lx | (ly << 5) | (lz << 10);
-    int gx = X0 + lx - 1, gy = Y0 + ly - 1, gz = Z0 + lz - 1;
-    gx += (gx < 0) ? B.nb[0] : 0;
-    gx -= (gx >= B.nb[0]) ? B.nb[0] : 0;
-    gy += (gy < 0) ? B.nb[1] : 0;
-    gy -= (gy >= B.nb[1]) ? B.nb[1] : 0;
-    gz += (gz < 0) ? B.nb[2] : 0;
-    gz -= (gz >= B.nb[2]) ? B.nb[2] : 0;
-    int gc = B.cell0 + gx + B.nb[0] * (gy + B.nb[1] * gz);
-    int s0 = A.cstart[gc];
-    gfirst[e] = s0;
-    lstart[e] = (unsigned short)min(A.cstart[gc + 1] - s0, 0xffff);  // a larger count overflows any capacity
-  }
   {
     const uint4* src = reinterpret_cast<const uint4*>(&g_own);
     uint4* dst = reinterpret_cast<uint4*>(sown);
@@ -662,6 +647,24 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         }
       }
     }
+  }
+  // (1) ext cells: global cell, count, first atom
+  grid_wait();  // what came before this line depends on no earlier kernel
+  int cc0 = 0;  // the code of cell tid
+  for (int e = tid; e < NE; e += blockDim.x) {
+    int lx = e % EX, rr = e / EX, ly = rr % EY, lz = rr / EY;
+    if (e == tid) cc0 = lx | (ly << 5) | (lz << 10);
+    int gx = X0 + lx - 1, gy = Y0 + ly - 1, gz = Z0 + lz - 1;
+    gx += (gx < 0) ? B.nb[0] : 0;
+    gx -= (gx >= B.nb[0]) ? B.nb[0] : 0;
+    gy += (gy < 0) ? B.nb[1] : 0;
+    gy -= (gy >= B.nb[1]) ? B.nb[1] : 0;
+    gz += (gz < 0) ? B.nb[2] : 0;
+    gz -= (gz >= B.nb[2]) ? B.nb[2] : 0;
+    int gc = B.cell0 + gx + B.nb[0] * (gy + B.nb[1] * gz);
+    int s0 = A.cstart[gc];
+    gfirst[e] = s0;
+    lstart[e] = (unsigned short)min(A.cstart[gc + 1] - s0, 0xffff);  // a larger count overflows any capacity
   }
   __syncthreads();
 
@@ -1722,6 +1725,8 @@ __global__ void __launch_bounds__(32 * kBuildWarps, 3) k_pair_build(const PairAr
 // built) are computed in full by enumeration, every step until the next build.
 template <bool MULTI, bool ENERGY, bool COUNT, bool LIST>
 __global__ void __launch_bounds__(256, 3) k_pair_redo(const PairArgs A) {
+  grid_trigger();
+  grid_wait();
   const int n = *(volatile const int*)A.redo_n;
   const int nfb = LIST ? *(volatile const int*)&A.lw[LW_FBN] : 0;
   for (int j = blockIdx.x; j < n + nfb; j += gridDim.x) {
@@ -1745,6 +1750,8 @@ __global__ void __launch_bounds__(256, 3) k_pair_redo(const PairArgs A) {
 
 template <bool MULTI, bool ENERGY, bool COUNT>
 __global__ void __launch_bounds__(256, 3) k_pair_redo64(const PairArgs A) {
+  grid_trigger();
+  grid_wait();
   const int n = *(volatile const int*)A.redo_n;
   for (int j = blockIdx.x; j < n; j += gridDim.x) {
     pair_tile<true, MULTI, ENERGY, COUNT, kRedoFull>(A, A.redo[j] & ~kFullBit);
@@ -1837,13 +1844,15 @@ cudaError_t launch_pair(const PairConfig& cfg, const PairArgs& a, int ntiles, in
   const int main_smem = main_smem_bytes(cfg, a.cap, a.ne_max, a.ext_max);
   if (main_smem > smem_bytes) return cudaErrorInvalidValue;
   const int warps = uses_wide(cfg) ? kWideWarps : cfg.warps;
-  cudaError_t e = cudaLaunchKernel(fn, dim3(ntiles), dim3(32 * warps), args, (size_t)main_smem, st);
+  // (the list pass follows a conditional graph node or the list build: launched plainly)
+  const bool chain = cfg.chain && !uses_list(cfg);
+  cudaError_t e = launch_chained_ptr(chain, fn, dim3(ntiles), dim3(32 * warps), args, (size_t)main_smem, st);
   if (e != cudaSuccess || (cfg.fp64 && !cfg.fix)) return e;
   // the redo pass: a few blocks per SM at most; nothing to do in a thermal system
   const int redo_smem = redo_smem_bytes(cfg, a.cap_redo, a.ne_max, a.ext_max);
   if (redo_smem > smem_bytes) return cudaErrorInvalidValue;
-  return cudaLaunchKernel(pick_redo(cfg), dim3(std::min(ntiles, kRedoBlocks)), dim3(32 * cfg.warps), args,
-                          (size_t)redo_smem, st);
+  return launch_chained_ptr(chain, pick_redo(cfg), dim3(std::min(ntiles, kRedoBlocks)), dim3(32 * cfg.warps), args,
+                            (size_t)redo_smem, st);
 }
 
 cudaError_t launch_pair_build(const PairConfig& cfg, const PairArgs& a, int ntiles, int smem_bytes, cudaStream_t st) {

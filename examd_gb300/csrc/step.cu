@@ -140,6 +140,8 @@ __device__ __forceinline__ void gather_force(const StepArgs& a, int64_t s, doubl
 template <bool FP64>
 __global__ void k_forces_out(const StepArgs a, int64_t i0, int64_t i1, const int* __restrict__ inv,
                              double* __restrict__ out, int acc) {
+  grid_trigger();
+  grid_wait();
   const int64_t i = i0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= i1) return;
   double f[3];
@@ -160,10 +162,8 @@ cudaError_t launch_forces_out(const StepArgs& s, int64_t i0, int64_t i1, const i
   if (i1 <= i0) return cudaSuccess;
   const unsigned g = (unsigned)((i1 - i0 + 255) / 256);
   if (s.fp64)
-    k_forces_out<true><<<g, 256, 0, st>>>(s, i0, i1, inv, out, accumulate);
-  else
-    k_forces_out<false><<<g, 256, 0, st>>>(s, i0, i1, inv, out, accumulate);
-  return cudaGetLastError();
+    return launch_chained(true, k_forces_out<true>, g, 256, st, s, i0, i1, inv, out, accumulate);
+  return launch_chained(true, k_forces_out<false>, g, 256, st, s, i0, i1, inv, out, accumulate);
 }
 
 // Per-box FP64 sums of per-tile partials: one block per box, fixed-order tree.
