@@ -785,6 +785,7 @@ int examd_gpu_create(const examd_params* params, int nboxes, const examd_box* bo
   ctx->N = a0;
   ctx->NC = cell0;
   ctx->ntiles = (int)tiles.size() / 2;
+  ctx->pc.fine = ctx->ntiles <= 16 * prop.multiProcessorCount;  // about four waves
   // where the caller leaves the warps to the library and three CTAs an SM hold every tile
   ctx->pc.wide = p.warps <= 0 && !ctx->pc.fp64 && !ctx->list && ctx->ntiles <= 3 * prop.multiProcessorCount;
   if (ctx->N >= (int64_t)1 << 31 || (int64_t)cell0 >= ((int64_t)1 << 31) - 1 ||

@@ -145,6 +145,7 @@ struct PairConfig {
   bool count = false;   // candidate / accepted counters
   bool list = false;    // mixed form: pair-list mode (forces from the per-tile lists)
   bool cut = true;      // list pass: the potential's own range is finite (WCA) and tested
+  bool fine = false;    // FP64 form: finer work units (grids of few waves)
   bool chain = false;   // the pair and redo passes as chained launches
   bool wide = false;    // mixed form without lists: the enumeration with 12 warps per CTA
   int warps = 8;

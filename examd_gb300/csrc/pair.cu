@@ -66,7 +66,11 @@ cudaError_t upload_own_lut(const OwnLut& lut) { return cudaMemcpyToSymbol(g_own,
 
 constexpr int kDT = 6;        // origin differences for d = -2..3
 constexpr int kQueue = 64;    // per-warp queue of accepted pairs
-constexpr int kParts = 2;     // work units per 32 staged atoms (1, 3 and 4 measured slower)
+// Work units per 32 staged atoms.  Finer units end a CTA more evenly and set up
+// more: 2 in a grid of many waves (1, 3 and 4 measured slower), 4 where the CTAs'
+// own time shows (few waves: pair pass of 104k atoms in FP64 129 -> 124 us, 32k
+// 46 -> 44, 2,048 18.6 -> 15.1; but 1M 867 -> 873).
+constexpr int kUnitParts = 2, kFineParts = 4;
 // Warps per CTA of the list build, whatever the other passes use: the build
 // needs one count word per atom where they keep three force sums, and in the
 // room 12 warps fit 3 CTAs on an SM at the tiles of a dense liquid (36 warps
@@ -552,7 +556,7 @@ __device__ __forceinline__ void force_batch_fix(int cnt, int q0, const QK& qk, c
 //   the list was built), outputs, energy and the large-term flag as there;
 // - kListBig: kRedoBig from the list.
 // CUT (list pass): the potential's own range rcut2 is tested (WCA; infinite otherwise).
-template <bool FP64, bool MULTI, bool ENERGY, bool COUNT, int MODE, bool CUT = true>
+template <bool FP64, bool MULTI, bool ENERGY, bool COUNT, int MODE, bool CUT = true, int kParts = kUnitParts>
 __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   extern __shared__ __align__(16) unsigned char smem[];
   const unsigned FULL = 0xffffffffu;
@@ -1692,14 +1696,14 @@ __global__ void __launch_bounds__(256, FP64 ? 3 : 4) k_pair(const PairArgs A) {
 // are, and 12 warps instead of 8 shorten each.
 template <bool MULTI, bool ENERGY>
 __global__ void __launch_bounds__(32 * kWideWarps, 3) k_pair_wide(const PairArgs A) {
-  pair_tile<false, MULTI, ENERGY, false, kMain>(A, A.order[blockIdx.x]);
+  pair_tile<false, MULTI, ENERGY, false, kMain, true, kFineParts>(A, A.order[blockIdx.x]);
 }
 
 // FP64 form: the first pass in fixed point, and the FP64 body for the tiles that
 // it listed (normally none).
-template <bool MULTI, bool ENERGY, bool COUNT>
+template <bool MULTI, bool ENERGY, bool COUNT, int PARTS>
 __global__ void __launch_bounds__(256, MULTI ? 3 : 4) k_pair_fix(const PairArgs A) {
-  pair_tile<false, MULTI, ENERGY, COUNT, kFixed>(A, A.order[blockIdx.x]);
+  pair_tile<false, MULTI, ENERGY, COUNT, kFixed, true, PARTS>(A, A.order[blockIdx.x]);
 }
 
 // Pair-list mode: the forces of every tile from its list (fallback tiles
@@ -1784,8 +1788,10 @@ static bool uses_list(const PairConfig& c) { return c.list && !c.fp64 && !c.coun
 
 template <bool MULTI>
 static void* pick_fix(const PairConfig& c) {
-  if (c.energy) return c.count ? (void*)&k_pair_fix<MULTI, true, true> : (void*)&k_pair_fix<MULTI, true, false>;
-  return c.count ? (void*)&k_pair_fix<MULTI, false, true> : (void*)&k_pair_fix<MULTI, false, false>;
+  constexpr int P = kUnitParts, F = kFineParts;
+  if (c.count) return c.energy ? (void*)&k_pair_fix<MULTI, true, true, P> : (void*)&k_pair_fix<MULTI, false, true, P>;
+  if (c.fine) return c.energy ? (void*)&k_pair_fix<MULTI, true, false, F> : (void*)&k_pair_fix<MULTI, false, false, F>;
+  return c.energy ? (void*)&k_pair_fix<MULTI, true, false, P> : (void*)&k_pair_fix<MULTI, false, false, P>;
 }
 
 template <bool MULTI>
