@@ -1372,8 +1372,24 @@ StepArgs step_args(examd_ctx* ctx) {
   return s;
 }
 
-// The pair path at the resident positions, then the forces to the caller in
-// chunks of its own order: the device->host copy of chunk c (second stream)
+// The device's address of a page-locked host array, or nullptr for any other.
+const void* device_view(const void* p) {
+  if (!p) return nullptr;
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();  // clear the sticky-free error of an unknown pointer
+    return nullptr;
+  }
+  return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
+}
+
+bool pinned(const void* p) { return !p || device_view(p); }
+
+// The pair path at the resident positions, then the forces to the caller.  A
+// page-locked array of the caller is read and written across the link by the
+// kernels themselves (at the copy engines' rate, 0.2 TB/s each way): no staging
+// copy, no chunks, and their events between two kernels.  Other arrays in
+// chunks of the caller's order: the device->host copy of chunk c (second stream)
 // overlaps the gather of chunk c + 1.  With accumulate, the caller's forces
 // come in on the second stream while the pair kernel runs.
 // The work of the force call, queued on the context's streams; the second
@@ -1385,7 +1401,8 @@ int enqueue_forces(examd_ctx* ctx, double* forces, double* epot, double* virial,
   const int64_t N = ctx->N;
   const int nch = io_chunks(N);
   cudaEvent_t* ev_acc = ctx->ev_io + 2 * kIoChunks;
-  if (forces && accumulate && N > 0) {
+  double* const df = (double*)device_view(forces);  // the caller's array, written in place
+  if (forces && accumulate && N > 0 && !df) {
     CK(cudaEventRecord(ctx->ev_io[3 * kIoChunks], st));  // stage is free once earlier work is done
     CK(cudaStreamWaitEvent(st2, ctx->ev_io[3 * kIoChunks], 0));
     for (int c = 0; c < nch; ++c) {
@@ -1398,7 +1415,10 @@ int enqueue_forces(examd_ctx* ctx, double* forces, double* epot, double* virial,
   }
   int rc = run_pair(ctx, energy, false);
   if (rc) return rc;
-  if (forces && N > 0) {
+  if (df && N > 0) {
+    CK(ensure_inv(ctx));
+    CK(launch_forces_out(step_args(ctx), 0, N, ctx->inv, df, accumulate, st));
+  } else if (forces && N > 0) {
     CK(ensure_inv(ctx));
     for (int c = 0; c < nch; ++c) {
       int64_t i0, i1;
@@ -1413,8 +1433,10 @@ int enqueue_forces(examd_ctx* ctx, double* forces, double* epot, double* virial,
   }
   if (epot) CK(cudaMemcpyAsync(epot, ctx->boxE, ctx->nboxes * sizeof(double), cudaMemcpyDeviceToHost, st));
   if (virial) CK(cudaMemcpyAsync(virial, ctx->boxW, ctx->nboxes * sizeof(double), cudaMemcpyDeviceToHost, st));
-  CK(cudaEventRecord(ctx->ev_io[3 * kIoChunks], st2));
-  CK(cudaStreamWaitEvent(st, ctx->ev_io[3 * kIoChunks], 0));
+  if (forces && N > 0 && !df) {
+    CK(cudaEventRecord(ctx->ev_io[3 * kIoChunks], st2));
+    CK(cudaStreamWaitEvent(st, ctx->ev_io[3 * kIoChunks], 0));
+  }
   return EXAMD_OK;
 }
 
@@ -1431,16 +1453,6 @@ int finish_forces(examd_ctx* ctx) {
 int forces_common(examd_ctx* ctx, double* forces, double* epot, double* virial, int accumulate) {
   const int rc = enqueue_forces(ctx, forces, epot, virial, accumulate);
   return rc ? rc : finish_forces(ctx);
-}
-
-bool pinned(const void* p) {
-  if (!p) return true;
-  cudaPointerAttributes a{};
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-    cudaGetLastError();  // clear the sticky-free error of an unknown pointer
-    return false;
-  }
-  return a.type == cudaMemoryTypeHost;
 }
 
 }  // namespace
@@ -1520,27 +1532,34 @@ int enqueue_forces_at(examd_ctx* ctx, const double* pos, double* forces, double*
   const int s = ctx->cur;
   const int64_t N = ctx->N;
   if (N > 0) {
-    // positions in chunks of the caller's order: the host->device copy of
-    // chunk c + 1 (second stream) overlaps the gather and binning count of chunk c
+    // positions read in place, or in chunks of the caller's order: the
+    // host->device copy of chunk c + 1 (second stream) overlaps the gather and
+    // binning count of chunk c
     CK(ensure_inv(ctx));
-    CK(cudaEventRecord(ctx->ev_io[3 * kIoChunks], st));
-    CK(cudaStreamWaitEvent(st2, ctx->ev_io[3 * kIoChunks], 0));
-    const int nch = io_chunks(N);
-    for (int c = 0; c < nch; ++c) {
-      int64_t i0, i1;
-      io_range(N, nch, c, i0, i1);
-      CK(cudaMemcpyAsync(ctx->stage2 + 3 * i0, pos + 3 * i0, 3 * (i1 - i0) * sizeof(double),
-                         cudaMemcpyHostToDevice, st2));
-      CK(cudaEventRecord(ctx->ev_io[c], st2));
-      CK(cudaStreamWaitEvent(st, ctx->ev_io[c], 0));
-      if (ctx->list) {
-        CK(launch_gather_pos_list(i0, i1, ctx->stage2, ctx->d_boxes, ctx->p.strict_box, ctx->X[s][0],
-                                  ctx->X[s][1], ctx->X[s][2], ctx->meta[s], ctx->inv, ctx->cellS, ctx->U, ctx->Ub,
-                                  ctx->lw, ctx->status, st));
-      } else {
-        CK(launch_chained(true, k_gather_pos_bin_range, nblk(i1 - i0), 256, st, i0, i1, ctx->stage2, ctx->d_boxes,
-                          ctx->p.strict_box, ctx->X[s][0], ctx->X[s][1], ctx->X[s][2], ctx->meta[s], ctx->inv,
-                          ctx->cellOld, ctx->slot, ctx->count, ctx->status));
+    const double* const dp = (const double*)device_view(pos);
+    auto gather = [&](const double* src, int64_t i0, int64_t i1) {
+      if (ctx->list)
+        return launch_gather_pos_list(i0, i1, src, ctx->d_boxes, ctx->p.strict_box, ctx->X[s][0], ctx->X[s][1],
+                                      ctx->X[s][2], ctx->meta[s], ctx->inv, ctx->cellS, ctx->U, ctx->Ub, ctx->lw,
+                                      ctx->status, st);
+      return launch_chained(true, k_gather_pos_bin_range, nblk(i1 - i0, kIoThreads), kIoThreads, st, i0, i1, src,
+                            ctx->d_boxes, ctx->p.strict_box, ctx->X[s][0], ctx->X[s][1], ctx->X[s][2], ctx->meta[s],
+                            ctx->inv, ctx->cellOld, ctx->slot, ctx->count, ctx->status);
+    };
+    if (dp) {
+      CK(gather(dp, 0, N));
+    } else {
+      CK(cudaEventRecord(ctx->ev_io[3 * kIoChunks], st));
+      CK(cudaStreamWaitEvent(st2, ctx->ev_io[3 * kIoChunks], 0));
+      const int nch = io_chunks(N);
+      for (int c = 0; c < nch; ++c) {
+        int64_t i0, i1;
+        io_range(N, nch, c, i0, i1);
+        CK(cudaMemcpyAsync(ctx->stage2 + 3 * i0, pos + 3 * i0, 3 * (i1 - i0) * sizeof(double),
+                           cudaMemcpyHostToDevice, st2));
+        CK(cudaEventRecord(ctx->ev_io[c], st2));
+        CK(cudaStreamWaitEvent(st, ctx->ev_io[c], 0));
+        CK(gather(ctx->stage2, i0, i1));
       }
     }
   }

@@ -81,17 +81,20 @@ __global__ void k_load_bin(int64_t n, const double* __restrict__ aos, const doub
   bin_one((int)s, p[0], p[1], p[2], mt, boxes, cellOld, slot, count, status);
 }
 
-// New positions for the caller's atoms [i0, i1) (AoS, caller order, as they
-// arrive in chunks): wrap, store at the atom's sorted slot inv[i], bin.
+// New positions for the caller's atoms [i0, i1) (AoS, caller order; the caller's
+// own page-locked array, or a copy of it as it arrives in chunks): wrap, store at
+// the atom's sorted slot inv[i], bin.
 __global__ void k_gather_pos_bin_range(int64_t i0, int64_t i1, const double* __restrict__ aos,
                                        const BoxDev* __restrict__ boxes, int strict, double* __restrict__ X0,
                                        double* __restrict__ X1, double* __restrict__ X2,
                                        const int* __restrict__ meta, const int* __restrict__ inv,
                                        int* __restrict__ cellOld, int* __restrict__ slot, int* __restrict__ count,
                                        int* __restrict__ status) {
+  __shared__ double sh[3 * kIoThreads];
   grid_trigger();
   grid_wait();
-  const int64_t i = i0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t b0 = i0 + blockIdx.x * (int64_t)kIoThreads, i = b0 + threadIdx.x;
+  aos_in(aos + 3 * b0, (int)min((int64_t)kIoThreads, i1 - b0), sh);
   if (i >= i1) return;
   const int s = inv[i];
   const int mt = meta[s];
@@ -99,7 +102,7 @@ __global__ void k_gather_pos_bin_range(int64_t i0, int64_t i1, const double* __r
   double p[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    double x = aos[3 * i + a];
+    double x = sh[3 * threadIdx.x + a];
     if (strict && !in_range_bits(x, B.L[a])) atomicOr(status, ST_OUTSIDE);
     p[a] = finite_bits(x) ? wrap_coord(x, B.L[a], B.Li[a]) : x;
   }

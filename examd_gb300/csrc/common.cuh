@@ -186,6 +186,20 @@ __host__ __device__ inline int pos_class(int l, int t) {
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// The caller's atoms in (x, y, z) order, kIoThreads of them per block (of as many
+// threads), through shared memory: 8-byte accesses side by side, whether the
+// array is device memory or the caller's page-locked host memory read or written
+// across the link.  Every thread of the block calls it.
+constexpr int kIoThreads = 256;
+__device__ __forceinline__ void aos_in(const double* __restrict__ src, int n, double* sh) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int e = k * kIoThreads + (int)threadIdx.x;
+    if (e < 3 * n) sh[e] = src[e];
+  }
+  __syncthreads();
+}
+
 __device__ __forceinline__ float rcp_approx(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

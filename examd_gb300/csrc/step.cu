@@ -138,32 +138,42 @@ __device__ __forceinline__ void gather_force(const StepArgs& a, int64_t s, doubl
 // Forces of the caller's atoms [i0, i1) in caller order (AoS): the atom's
 // partials gathered at its sorted slot inv[i]; written or added (acc).
 template <bool FP64>
-__global__ void k_forces_out(const StepArgs a, int64_t i0, int64_t i1, const int* __restrict__ inv,
-                             double* __restrict__ out, int acc) {
+__global__ void __launch_bounds__(kIoThreads) k_forces_out(const StepArgs a, int64_t i0, int64_t i1,
+                                                           const int* __restrict__ inv, double* __restrict__ out,
+                                                           int acc) {
+  __shared__ double sh[3 * kIoThreads];
   grid_trigger();
   grid_wait();
-  const int64_t i = i0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= i1) return;
-  double f[3];
-  gather_force<FP64>(a, inv[i], f);
-  if (acc) {
-    out[3 * i] += f[0];
-    out[3 * i + 1] += f[1];
-    out[3 * i + 2] += f[2];
-  } else {
-    out[3 * i] = f[0];
-    out[3 * i + 1] = f[1];
-    out[3 * i + 2] = f[2];
+  const int64_t b0 = i0 + blockIdx.x * (int64_t)kIoThreads, i = b0 + threadIdx.x;
+  const int n = (int)min((int64_t)kIoThreads, i1 - b0);
+  out += 3 * b0;
+  double old[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {  // the caller's forces, on their way while the partials are gathered
+    const int e = k * kIoThreads + (int)threadIdx.x;
+    old[k] = acc && e < 3 * n ? out[e] : 0.0;
+  }
+  if (i < i1) {
+    double f[3];
+    gather_force<FP64>(a, inv[i], f);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) sh[3 * threadIdx.x + k] = f[k];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int e = k * kIoThreads + (int)threadIdx.x;
+    if (e < 3 * n) out[e] = acc ? old[k] + sh[e] : sh[e];
   }
 }
 
 cudaError_t launch_forces_out(const StepArgs& s, int64_t i0, int64_t i1, const int* inv, double* out, int accumulate,
                               cudaStream_t st) {
   if (i1 <= i0) return cudaSuccess;
-  const unsigned g = (unsigned)((i1 - i0 + 255) / 256);
+  const unsigned g = (unsigned)((i1 - i0 + kIoThreads - 1) / kIoThreads);
   if (s.fp64)
-    return launch_chained(true, k_forces_out<true>, g, 256, st, s, i0, i1, inv, out, accumulate);
-  return launch_chained(true, k_forces_out<false>, g, 256, st, s, i0, i1, inv, out, accumulate);
+    return launch_chained(true, k_forces_out<true>, g, kIoThreads, st, s, i0, i1, inv, out, accumulate);
+  return launch_chained(true, k_forces_out<false>, g, kIoThreads, st, s, i0, i1, inv, out, accumulate);
 }
 
 // Per-box FP64 sums of per-tile partials: one block per box, fixed-order tree.
@@ -337,7 +347,9 @@ __global__ void k_gather_pos_list(int64_t i0, int64_t i1, const double* __restri
                                   double* __restrict__ X1, double* __restrict__ X2, const int* __restrict__ meta,
                                   const int* __restrict__ inv, const int* __restrict__ cellS, float4* __restrict__ U,
                                   const float4* __restrict__ Ub, int* __restrict__ lw, int* __restrict__ status) {
-  const int64_t i = i0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  __shared__ double sh[3 * kIoThreads];
+  const int64_t b0 = i0 + blockIdx.x * (int64_t)kIoThreads, i = b0 + threadIdx.x;
+  aos_in(aos + 3 * b0, (int)min((int64_t)kIoThreads, i1 - b0), sh);
   float d2 = 0.f;
   if (i < i1) {
     const int s = inv[i];
@@ -346,7 +358,7 @@ __global__ void k_gather_pos_list(int64_t i0, int64_t i1, const double* __restri
     double p[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      double x = aos[3 * i + a];
+      double x = sh[3 * threadIdx.x + a];
       if (strict && !in_range_bits(x, B.L[a])) atomicOr(status, ST_OUTSIDE);
       p[a] = finite_bits(x) ? wrap_coord(x, B.L[a], B.Li[a]) : x;
     }
@@ -367,7 +379,7 @@ cudaError_t launch_gather_pos_list(int64_t i0, int64_t i1, const double* aos, co
                                    const int* cellS, float4* U, const float4* Ub, int* lw, int* status,
                                    cudaStream_t st) {
   if (i1 <= i0) return cudaSuccess;
-  k_gather_pos_list<<<(unsigned)((i1 - i0 + 255) / 256), 256, 0, st>>>(i0, i1, aos, boxes, strict, X0, X1, X2, meta,
+  k_gather_pos_list<<<(unsigned)((i1 - i0 + kIoThreads - 1) / kIoThreads), kIoThreads, 0, st>>>(i0, i1, aos, boxes, strict, X0, X1, X2, meta,
                                                                        inv, cellS, U, Ub, lw, status);
   return cudaGetLastError();
 }
