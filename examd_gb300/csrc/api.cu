@@ -1298,7 +1298,8 @@ int init_lists(examd_ctx* ctx) {
   return EXAMD_OK;  // any tile still over its list is computed by enumeration
 }
 
-int run_pair(examd_ctx* ctx, bool energy, bool count, double* boxE = nullptr, double* boxW = nullptr);
+int run_pair(examd_ctx* ctx, bool energy, bool count, double* boxE = nullptr, double* boxW = nullptr,
+             bool side = false);
 
 // Pair-list mode, between runs of steps: a tile with an atom whose list
 // outgrew its capacity since the last check, or with more staged atoms than
@@ -1326,25 +1327,28 @@ int update_lists(examd_ctx* ctx, bool cap_grew) {
   return EXAMD_OK;
 }
 
-int run_pair(examd_ctx* ctx, bool energy, bool count, double* boxE, double* boxW) {
+// The pair pass; with energy the per-box sums to boxE, boxW (nullptr: the
+// context's), on the second stream for a step of a loop (side).
+int run_pair(examd_ctx* ctx, bool energy, bool count, double* boxE, double* boxW, bool side) {
   PairConfig c = ctx->pc;
   c.energy = energy;
   c.count = count;
-  c.chain = ctx->in_call || !(c.wide || boxE);
+  c.chain = ctx->in_call || !(c.wide || side);
   if (ctx->side_pe) {  // the last step's sums read the tile energies that this pass writes
     CK(cudaStreamWaitEvent(ctx->st, ctx->ev_side[3], 0));
     ctx->side_pe = false;
   }
   CK(launch_pair(c, pair_args(ctx), ctx->ntiles, ctx->smem, ctx->st));
-  if (energy && !boxE)
-    CK(launch_reduce_tiles(ctx->nboxes, ctx->d_tile0, ctx->maxc_tiles, ctx->tileE, ctx->tileW, ctx->partial,
-                           ctx->boxE, ctx->boxW, ctx->st));
-  if (energy && boxE) {  // a step's sums: on the second stream
+  if (!energy) return EXAMD_OK;
+  cudaStream_t sums = side ? ctx->st2 : ctx->st;
+  if (side) {
     CK(cudaEventRecord(ctx->ev_side[1], ctx->st));
-    CK(cudaStreamWaitEvent(ctx->st2, ctx->ev_side[1], 0));
-    CK(launch_reduce_tiles(ctx->nboxes, ctx->d_tile0, ctx->maxc_tiles, ctx->tileE, ctx->tileW, ctx->partial, boxE,
-                           boxW, ctx->st2));
-    CK(cudaEventRecord(ctx->ev_side[3], ctx->st2));
+    CK(cudaStreamWaitEvent(sums, ctx->ev_side[1], 0));
+  }
+  CK(launch_reduce_tiles(ctx->nboxes, ctx->d_tile0, ctx->maxc_tiles, ctx->tileE, ctx->tileW, ctx->partial,
+                         boxE ? boxE : ctx->boxE, boxW ? boxW : ctx->boxW, sums));
+  if (side) {
+    CK(cudaEventRecord(ctx->ev_side[3], sums));
     ctx->side_pe = true;
   }
   return EXAMD_OK;
@@ -1413,7 +1417,9 @@ int enqueue_forces(examd_ctx* ctx, double* forces, double* epot, double* virial,
       CK(cudaEventRecord(ev_acc[c], st2));
     }
   }
-  int rc = run_pair(ctx, energy, false);
+  // (the energies too, where the arrays allow)
+  double *const de = (double*)device_view(epot), *const dw = (double*)device_view(virial);
+  int rc = run_pair(ctx, energy, false, de, dw);
   if (rc) return rc;
   if (df && N > 0) {
     CK(ensure_inv(ctx));
@@ -1431,18 +1437,18 @@ int enqueue_forces(examd_ctx* ctx, double* forces, double* epot, double* virial,
                          cudaMemcpyDeviceToHost, st2));
     }
   }
-  if (epot) CK(cudaMemcpyAsync(epot, ctx->boxE, ctx->nboxes * sizeof(double), cudaMemcpyDeviceToHost, st));
-  if (virial) CK(cudaMemcpyAsync(virial, ctx->boxW, ctx->nboxes * sizeof(double), cudaMemcpyDeviceToHost, st));
+  if (epot && !de) CK(cudaMemcpyAsync(epot, ctx->boxE, ctx->nboxes * sizeof(double), cudaMemcpyDeviceToHost, st));
+  if (virial && !dw) CK(cudaMemcpyAsync(virial, ctx->boxW, ctx->nboxes * sizeof(double), cudaMemcpyDeviceToHost, st));
   if (forces && N > 0 && !df) {
     CK(cudaEventRecord(ctx->ev_io[3 * kIoChunks], st2));
     CK(cudaStreamWaitEvent(st, ctx->ev_io[3 * kIoChunks], 0));
   }
+  CK(queue_status(ctx));
   return EXAMD_OK;
 }
 
-// Waits for the force call and reads its status word.
+// Waits for the force call and takes its status word.
 int finish_forces(examd_ctx* ctx) {
-  CK(queue_status(ctx));
   CK(cudaStreamSynchronize(ctx->st));
   const int rc = take_status(ctx);
   if (rc) return rc;
@@ -1716,7 +1722,7 @@ int step_once(examd_ctx* ctx, double ck, double dt, double* keSlot, double* eSlo
   if (rc) return rc;
   rc = ctx->list ? maybe_rebuild(ctx) : finish_binning(ctx, false);
   if (rc) return rc;
-  return run_pair(ctx, eSlot != nullptr, false, eSlot, wSlot);
+  return run_pair(ctx, eSlot != nullptr, false, eSlot, wSlot, eSlot != nullptr);
 }
 
 int ensure_ebuf(examd_ctx* ctx, int steps, bool host) {
