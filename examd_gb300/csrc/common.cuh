@@ -223,6 +223,17 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
+// The warp's sum of a on lanes 0-15, of b on lanes 16-31.
+template <class T>
+__device__ __forceinline__ T warp_sum2(T a, T b) {
+  const bool up = threadIdx.x & 16;
+  T v = up ? b : a;
+  v += __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 // Kahan-compensated FP32 accumulator.
 struct KSum {
   float s = 0.f, c = 0.f;

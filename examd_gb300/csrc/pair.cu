@@ -219,11 +219,20 @@ int pair_smem_bytes(const PairConfig& cfg, int cap, int cap_redo, int ne_max, in
 // Exact sum of FP32 terms in 64-bit fixed point (2^-32 resolution): the total
 // does not depend on the order of the terms.  A term of magnitude >= 30000
 // (a pair closer than ~0.46 sigma) goes to an FP32 side sum.
+// Below 8192 the term is split at 2^-9 and rounded at 2^-32 by adding constants
+// whose ulp is that bit and taking the difference of the sums' bits (the same
+// value as the conversions', which run at an eighth of the FP32 rate and were
+// six of a pair's nine).
 struct FixSum {
   long long v = 0;
   float side = 0.f;
   __device__ __forceinline__ void add(float x) {
-    if (fabsf(x) < 30000.f) {
+    if (fabsf(x) < 8192.f) {
+      constexpr float kHi = 24576.f, kLo = 1.5f / 512.f;  // 1.5 2^14 (ulp 2^-9), 1.5 2^-9 (ulp 2^-32)
+      const float hi = __fadd_rn(x, kHi);
+      const float lo = __fadd_rn(__fsub_rn(x, __fsub_rn(hi, kHi)), kLo);  // (inner differences exact, at most 2^-10)
+      v += (long long)(__float_as_int(hi) - 0x46c00000) * (1 << 23) + (__float_as_int(lo) - 0x3b400000);
+    } else if (fabsf(x) < 30000.f) {
       const float hs = x * 65536.f;  // exact power-of-two scaling
       const int h = __float2int_rz(hs);
       const int l = __float2int_rn((hs - (float)h) * 65536.f);  // hs - h is exact
@@ -1625,10 +1634,12 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
 
   // (5) per-tile energy / virial / counters
   if (ENERGY || COUNT) {
-    // mixed form: exact integer sums (the same bits whatever the order);
-    // FP64 form: FP64 sums
+    // mixed form: exact integer sums (the same bits whatever the order) and the
+    // rare large terms' FP32 ones; FP64 form: FP64 sums.  Two sums share a warp's
+    // exchange, and warp 0 adds up the warps' (one thread's loop over all of them
+    // and unneeded sums were 6 % of a small-box ensemble's instructions).
+    long long* redl = (long long*)red;
     double e = 0.0, w = 0.0;
-    long long ev = 0, wv = 0;
     if (ENERGY) {
       if (FIX) {
         e = esum - wsum - shsum;
@@ -1636,52 +1647,46 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
       } else if (FP64) {
         e = esum;
         w = wsum;
+      }
+    }
+    __syncthreads();  // the queues are done with
+    if (ENERGY) {
+      if (FP64 || FIX) {
+        e = warp_sum2(e, w);
+        if ((lane & 15) == 0) red[8 * warp + (lane >> 4)] = e;
       } else {
-        ev = ek.v;
-        wv = wk.v;
-        e = (double)ek.side;
-        w = (double)wk.side;
+        const long long v = warp_sum2(ek.v, wk.v);
+        if ((lane & 15) == 0) redl[8 * warp + 2 + (lane >> 4)] = v;
+        if (__any_sync(FULL, ek.side != 0.f || wk.side != 0.f)) e = warp_sum2((double)ek.side, (double)wk.side);
+        if ((lane & 15) == 0) red[8 * warp + (lane >> 4)] = e;
       }
     }
-    e = warp_sum(e);
-    w = warp_sum(w);
-    ev = warp_sum(ev);
-    wv = warp_sum(wv);
-    const long long c1 = warp_sum((long long)ncand), c2 = warp_sum((long long)nacc),
-                    c3 = warp_sum((long long)neval);
-    long long* redl = (long long*)red;
-    __syncthreads();
-    if (lane == 0) {
-      red[8 * warp] = e;
-      red[8 * warp + 1] = w;
-      redl[8 * warp + 2] = ev;
-      redl[8 * warp + 3] = wv;
-      redl[8 * warp + 4] = c1;
-      redl[8 * warp + 5] = c2;
-      redl[8 * warp + 6] = c3;
+    if (COUNT) {
+      const long long c1 = warp_sum((long long)ncand), c2 = warp_sum((long long)nacc), c3 = warp_sum((long long)neval);
+      if (lane == 0) {
+        redl[8 * warp + 4] = c1;
+        redl[8 * warp + 5] = c2;
+        redl[8 * warp + 6] = c3;
+      }
     }
     __syncthreads();
-    if (tid == 0) {
-      double se = 0, sw = 0;
-      long long sev = 0, swv = 0, s1 = 0, s2 = 0, s3 = 0;
-      for (int k = 0; k < nw; ++k) {
-        se += red[8 * k];
-        sw += red[8 * k + 1];
-        sev += redl[8 * k + 2];
-        swv += redl[8 * k + 3];
-        s1 += redl[8 * k + 4];
-        s2 += redl[8 * k + 5];
-        s3 += redl[8 * k + 6];
-      }
+    if (warp == 0) {
+      const int k = min(lane, nw - 1);
+      const bool on = lane < nw;
       if (ENERGY) {
-        A.tileE[tile] = (double)sev * 0x1.0p-32 + se;
-        A.tileW[tile] = (double)swv * 0x1.0p-32 + sw;
+        const double se = red[8 * k], sw = red[8 * k + 1];
+        double t = 0.0;
+        if (FP64 || FIX || __any_sync(FULL, se != 0.0 || sw != 0.0)) t = warp_sum2(on ? se : 0.0, on ? sw : 0.0);
+        if (!(FP64 || FIX))
+          t += (double)warp_sum2(on ? redl[8 * k + 2] : 0ll, on ? redl[8 * k + 3] : 0ll) * 0x1.0p-32;
+        if (lane == 0) A.tileE[tile] = t;
+        if (lane == 16) A.tileW[tile] = t;
       }
-      if (COUNT) {
-        A.tileC[3 * tile] = s1;
-        A.tileC[3 * tile + 1] = s2;
-        A.tileC[3 * tile + 2] = s3;
-      }
+      if (COUNT)
+        for (int c = 0; c < 3; ++c) {
+          const long long n = warp_sum(on ? redl[8 * k + 4 + c] : 0ll);
+          if (lane == 0) A.tileC[3 * tile + c] = n;
+        }
     }
   }
 }
