@@ -1112,6 +1112,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
     const unsigned short* perm = A.lperm + ltile;
     const unsigned short* cnts = A.lcnt + ltile;
     const int ng = (total + 31) >> 5;
+    constexpr int kBurst = MULTI ? 1 : 2;  // entries taken together (several types: no registers for two)
     bool bigl = false, perr = false;  // a large term left out; a pair-function error
     // The origin offset between rows l and l + d (d = -2..2 for a listed
     // pair) is fmaf(image difference, r, d bl) in the tables: d bl itself
@@ -1153,78 +1154,96 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         nxt = four(k0 + 4);
         const unsigned wv[2] = {cur.x, cur.y};
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const unsigned en = (q & 1) ? wv[q >> 1] >> 16 : wv[q >> 1] & 0xffffu;
-          const int m = MULTI ? en & 0x3fff : en;  // the entry: the staged atom, and its type above 14 bits
-          const float4 pj = pf[m];
-          // y, z of atom i in the frame of atom j's row: (the row origins'
-          // offset) - pi, rounded once
-          float yi, zi;
-          if constexpr (TAB) {  // (the table entry of rows l, l + d: l kDT + d + 2)
-            const int cm = code[EXAMD_IDX(min(m, total - 1), cap, st)];
-            yi = dyt[((ci >> 5) & 31) * (kDT - 1) + 2 + ((cm >> 5) & 31)].x - pi.y;
-            zi = dzt[(ci >> 10) * (kDT - 1) + 2 + (cm >> 10)].x - pi.z;
-          } else {  // d bl, exact: both rows' differences d in one bf16x2 subtraction
-            const unsigned wj = __float_as_uint(pj.w);
-            const __nv_bfloat162 dr = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&wj),
-                                              *reinterpret_cast<const __nv_bfloat162*>(&wi));
-            const unsigned du = *reinterpret_cast<const unsigned*>(&dr);
-            yi = fmaf(__uint_as_float(du << 16), blf, -pi.y);
-            zi = fmaf(__uint_as_float(du & 0xffff0000u), blf, -pi.z);
+        for (int q0 = 0; q0 < 4; q0 += kBurst) {
+          unsigned en[kBurst];
+          float4 dq[kBurst];
+          LJ32 P[kBurst];
+          bool rare = false;
+#pragma unroll
+          for (int b = 0; b < kBurst; ++b) {
+            const int q = q0 + b;
+            en[b] = (q & 1) ? wv[q >> 1] >> 16 : wv[q >> 1] & 0xffffu;
+            const int m = MULTI ? en[b] & 0x3fff : en[b];  // the entry: the staged atom, and its type above 14 bits
+            const float4 pj = pf[m];
+            // y, z of atom i in the frame of atom j's row: (the row origins'
+            // offset) - pi, rounded once
+            float yi, zi;
+            if constexpr (TAB) {  // (the table entry of rows l, l + d: l kDT + d + 2)
+              const int cm = code[EXAMD_IDX(min(m, total - 1), cap, st)];
+              yi = dyt[((ci >> 5) & 31) * (kDT - 1) + 2 + ((cm >> 5) & 31)].x - pi.y;
+              zi = dzt[(ci >> 10) * (kDT - 1) + 2 + (cm >> 10)].x - pi.z;
+            } else {  // d bl, exact: both rows' differences d in one bf16x2 subtraction
+              const unsigned wj = __float_as_uint(pj.w);
+              const __nv_bfloat162 dr = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&wj),
+                                                *reinterpret_cast<const __nv_bfloat162*>(&wi));
+              const unsigned du = *reinterpret_cast<const unsigned*>(&dr);
+              yi = fmaf(__uint_as_float(du << 16), blf, -pi.y);
+              zi = fmaf(__uint_as_float(du & 0xffff0000u), blf, -pi.z);
+            }
+            dq[b].x = pj.x - pi.x;
+            dq[b].y = pj.y + yi;
+            dq[b].z = pj.z + zi;
+            dq[b].w = fmaf(dq[b].x, dq[b].x, fmaf(dq[b].y, dq[b].y, dq[b].z * dq[b].z));
+            P[b] = MULTI ? ljs32[lrow + (en[b] >> 14)] : q32;
+            rare |= fabsf(dq[b].w - P[b].rc2) <= (MULTI ? kBorder * P[b].rc2 : band0) || dq[b].w < P[b].r2big;
           }
-          float4 dq;
-          dq.x = pj.x - pi.x;
-          dq.y = pj.y + yi;
-          dq.z = pj.z + zi;
-          dq.w = fmaf(dq.x, dq.x, fmaf(dq.y, dq.y, dq.z * dq.z));
-          const int tj = MULTI ? en >> 14 : 0;
-          const LJ32 P = MULTI ? ljs32[lrow + tj] : q32;
           if (MODE == kListBig) {
-            bool acc = dq.w <= P.rc2;
-            redo_pair(acc, dq, i | (ti << 14) | (m << 16) | (tj << 30));
-          } else {
-            // The LJ family's expression of pair_fn32 (the potential was
-            // checked per tile) for every entry, its result kept where the
-            // entry applies: some lane of the warp takes nearly every entry,
-            // so a branch would only add reconvergence, and without it the
-            // four entries' arithmetic interleaves.  The same expressions:
-            // the same bits as pair_fn32 where it applies.  The scale kFix is
-            // in m24 (a power of two).
-            const float m24 = MULTI ? P.m24eps : m24k0;
-            const float band = MULTI ? kBorder * P.rc2 : band0;
-            const float ri = rcp_approx(dq.w);
-            const float s2 = P.sig2 * ri;
-            const float s6 = s2 * s2 * s2;
-            const float dgs = m24 * s6 * fmaf(2.f, s6, -1.f) * ri;
-            // an entry applies within rc (and the potential's own range) unless its
-            // term is too large; the rest is rare: an r^2 at the border (the
-            // FP64 test), a large term (left to the redo pass), a pair-function
-            // error (r^2 < kR2Min32 <= r2big)
-            bool fix = dq.w <= P.rc2 && dq.w >= P.r2big && !(CUT && dq.w > P.rcut2);
-            bool app = fix;
-            if (fabsf(dq.w - P.rc2) <= band || dq.w < P.r2big) {
-              const bool acc = fabsf(dq.w - P.rc2) <= band ? inside64(i, m, ti, tj) : dq.w <= P.rc2;
-              perr |= acc && !(dq.w >= kR2Min32);
-              app = acc && dq.w >= kR2Min32 && !(CUT && dq.w > P.rcut2);
-              bigl |= app && dq.w < P.r2big;
-              fix = app && !(dq.w < P.r2big);
-            }
-            if (ENERGY && app) {
-              ek.add(P.c4eps * s6 * (s6 - 1.f) - P.eshift);
-              wk.add(-(dgs * kFixInv) * dq.w);
-            }
-            // atom m's terms; atom i's are the same with the other sign
-            const int jx = __float2int_rn(-(dgs * dq.x)), jy = __float2int_rn(-(dgs * dq.y)),
-                      jz = __float2int_rn(-(dgs * dq.z));
-            if (fix) {
-              atomicAdd(&fa[3 * m], jx);
-              atomicAdd(&fa[3 * m + 1], jy);
-              atomicAdd(&fa[3 * m + 2], jz);
-              sx -= jx;
-              sy -= jy;
-              sz -= jz;
-            }
+#pragma unroll
+            for (int b = 0; b < kBurst; ++b)
+              redo_pair(dq[b].w <= P[b].rc2, dq[b], i | (ti << 14) | (int)(en[b] << 16));
+            continue;
           }
+          // The LJ family's expression of pair_fn32 (the potential was checked
+          // per tile) for every entry, its result kept where the entry applies:
+          // some lane of the warp takes nearly every entry.  The same expressions:
+          // the same bits as pair_fn32 where it applies.  The scale kFix is in m24
+          // (a power of two).  An entry applies within rc (and the potential's own
+          // range).  What is rare -- an r^2 at the border (the FP64 test), a large
+          // term (left to the redo pass), a pair-function error (r^2 < kR2Min32
+          // <= r2big) -- is looked for in kBurst entries at once, and all of the
+          // warp's then go through the careful version: with a branch in every
+          // entry their arithmetic did not interleave.
+          auto apply = [&](auto careful) {
+#pragma unroll
+            for (int b = 0; b < kBurst; ++b) {
+              const int m = MULTI ? en[b] & 0x3fff : en[b];
+              const float r2 = dq[b].w;
+              const float m24 = MULTI ? P[b].m24eps : m24k0;
+              const float ri = rcp_approx(r2);
+              const float s2 = P[b].sig2 * ri;
+              const float s6 = s2 * s2 * s2;
+              const float dgs = m24 * s6 * fmaf(2.f, s6, -1.f) * ri;
+              bool fix = r2 <= P[b].rc2 && !(CUT && r2 > P[b].rcut2);
+              bool app = fix;
+              if constexpr (decltype(careful)::value) {
+                const bool edge64 = fabsf(r2 - P[b].rc2) <= (MULTI ? kBorder * P[b].rc2 : band0);
+                const bool acc = edge64 ? inside64(i, m, ti, MULTI ? en[b] >> 14 : 0) : r2 <= P[b].rc2;
+                perr |= acc && !(r2 >= kR2Min32);
+                app = acc && r2 >= kR2Min32 && !(CUT && r2 > P[b].rcut2);
+                bigl |= app && r2 < P[b].r2big;
+                fix = app && !(r2 < P[b].r2big);
+              }
+              if (ENERGY && app) {
+                ek.add(P[b].c4eps * s6 * (s6 - 1.f) - P[b].eshift);
+                wk.add(-(dgs * kFixInv) * r2);
+              }
+              // atom m's terms; atom i's are the same with the other sign
+              const int jx = __float2int_rn(-(dgs * dq[b].x)), jy = __float2int_rn(-(dgs * dq[b].y)),
+                        jz = __float2int_rn(-(dgs * dq[b].z));
+              if (fix) {
+                atomicAdd(&fa[3 * m], jx);
+                atomicAdd(&fa[3 * m + 1], jy);
+                atomicAdd(&fa[3 * m + 2], jz);
+                sx -= jx;
+                sy -= jy;
+                sz -= jz;
+              }
+            }
+          };
+          if (__any_sync(FULL, rare))
+            apply(std::true_type{});
+          else
+            apply(std::false_type{});
         }
       }
       };
