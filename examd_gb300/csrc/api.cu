@@ -1376,18 +1376,30 @@ StepArgs step_args(examd_ctx* ctx) {
   return s;
 }
 
-// The device's address of a page-locked host array, or nullptr for any other.
-const void* device_view(const void* p) {
-  if (!p) return nullptr;
+cudaPointerAttributes attributes(const void* p) {
   cudaPointerAttributes a{};
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();  // clear the sticky-free error of an unknown pointer
-    return nullptr;
+    a.type = cudaMemoryTypeUnregistered;
   }
-  return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
+  return a;
 }
 
-bool pinned(const void* p) { return !p || device_view(p); }
+// Whether the kernels can use the caller's array of n doubles in place: its
+// first and its last byte page-locked host memory at the same address on the
+// device (part of an array may be registered), and doubles on their boundary.
+bool in_place(const void* p, size_t n) {
+  if (!p || n == 0 || reinterpret_cast<uintptr_t>(p) % sizeof(double)) return false;
+  for (const char* q : {(const char*)p, (const char*)p + n * sizeof(double) - 1}) {
+    const cudaPointerAttributes a = attributes(q);
+    if (a.type != cudaMemoryTypeHost || a.devicePointer != q) return false;
+  }
+  return true;
+}
+
+bool pinned(const void* p, size_t n) { return !p || in_place(p, n); }
+
+bool on_device(const void* p) { return p && attributes(p).type == cudaMemoryTypeDevice; }
 
 // The pair path at the resident positions, then the forces to the caller.  A
 // page-locked array of the caller is read and written across the link by the
@@ -1405,7 +1417,7 @@ int enqueue_forces(examd_ctx* ctx, double* forces, double* epot, double* virial,
   const int64_t N = ctx->N;
   const int nch = io_chunks(N);
   cudaEvent_t* ev_acc = ctx->ev_io + 2 * kIoChunks;
-  double* const df = (double*)device_view(forces);  // the caller's array, written in place
+  double* const df = in_place(forces, 3 * (size_t)N) ? forces : nullptr;
   if (forces && accumulate && N > 0 && !df) {
     CK(cudaEventRecord(ctx->ev_io[3 * kIoChunks], st));  // stage is free once earlier work is done
     CK(cudaStreamWaitEvent(st2, ctx->ev_io[3 * kIoChunks], 0));
@@ -1418,7 +1430,8 @@ int enqueue_forces(examd_ctx* ctx, double* forces, double* epot, double* virial,
     }
   }
   // (the energies too, where the arrays allow)
-  double *const de = (double*)device_view(epot), *const dw = (double*)device_view(virial);
+  const size_t nb = (size_t)ctx->nboxes;
+  double *const de = in_place(epot, nb) ? epot : nullptr, *const dw = in_place(virial, nb) ? virial : nullptr;
   int rc = run_pair(ctx, energy, false, de, dw);
   if (rc) return rc;
   if (df && N > 0) {
@@ -1542,7 +1555,7 @@ int enqueue_forces_at(examd_ctx* ctx, const double* pos, double* forces, double*
     // host->device copy of chunk c + 1 (second stream) overlaps the gather and
     // binning count of chunk c
     CK(ensure_inv(ctx));
-    const double* const dp = (const double*)device_view(pos);
+    const double* const dp = in_place(pos, 3 * (size_t)N) ? pos : nullptr;
     auto gather = [&](const double* src, int64_t i0, int64_t i1) {
       if (ctx->list)
         return launch_gather_pos_list(i0, i1, src, ctx->d_boxes, ctx->p.strict_box, ctx->X[s][0], ctx->X[s][1],
@@ -1652,11 +1665,13 @@ int examd_gpu_forces_at(examd_ctx* ctx, const double* pos, double* forces, doubl
   if (!ctx->atoms_set) return EXAMD_ERR_STATE;
   cudaSetDevice(ctx->dev);
   CK(ensure_inv(ctx));  // outside any captured sequence
-  if (ctx->N > 0 && ctx->N <= kSmallIo) {
+  const size_t n3 = 3 * (size_t)ctx->N, nb = (size_t)ctx->nboxes;
+  if (ctx->N > 0 && ctx->N <= kSmallIo && !on_device(pos) && !on_device(forces) && !on_device(epot) &&
+      !on_device(virial)) {
     if (ctx->small_calls == 2) return forces_at_small(ctx, pos, forces, epot, virial, accumulate);
     ++ctx->small_calls;  // a context used for a call or two is not worth a capture
   }
-  if (ctx->N < kIoMinChunk || !pinned(pos) || !pinned(forces) || !pinned(epot) || !pinned(virial))
+  if (ctx->N < kIoMinChunk || !pinned(pos, n3) || !pinned(forces, n3) || !pinned(epot, nb) || !pinned(virial, nb))
     return finish_forces_at_eager(ctx, pos, forces, epot, virial, accumulate);
   // same pinned buffers as last time at this parity: replay the captured call
   return forces_at_graph(ctx, ctx->io_graph[ctx->cur], pos, forces, epot, virial, accumulate);
