@@ -1077,13 +1077,21 @@ int apply_capacity(examd_ctx* ctx, bool* grew = nullptr) {
   int want_r = std::max(((occ + occ / 4 + 64) + 7) & ~7, ctx->cap_redo);
   int want = ctx->pc.fp64 && !ctx->pc.fix ? want_r : ((occ + occ / 16 + 32) + 7) & ~7;
   if (want <= ctx->cap) return EXAMD_OK;
-  int bytes = pair_smem_bytes(ctx->pc, want, want_r, ctx->ne_max, ctx->ext_max);
-  if (bytes > ctx->smem_limit) {
-    // fall back to the exact need if the headroom does not fit
-    want = want_r = (occ + 7) & ~7;
+  int bytes = 0;
+  auto fits = [&] {
     bytes = pair_smem_bytes(ctx->pc, want, want_r, ctx->ne_max, ctx->ext_max);
-    if (bytes > ctx->smem_limit) return EXAMD_ERR_CELL_OVERFLOW;
+    return bytes <= ctx->smem_limit;
+  };
+  bool ok = fits();  // (the redo pass binds: the 12-warp CTAs' tables never do)
+  if (!ok) {  // the exact need if the headroom does not fit
+    want = want_r = (occ + 7) & ~7;
+    ok = fits();
   }
+  if (!ok && ctx->pc.fix) {  // the FP64 pass has smaller per-warp tables (about 110 atoms)
+    ctx->pc.fix = false;
+    ok = fits();
+  }
+  if (!ok) return EXAMD_ERR_CELL_OVERFLOW;
   ctx->cap = want;
   ctx->cap_redo = want_r;
   ctx->smem = bytes;

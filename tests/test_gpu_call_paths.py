@@ -174,3 +174,24 @@ def test_warps_give_the_same_forces(gpulib, precision, m):
             out.append((f, e[0]))
     for f, e in out[1:]:
         assert np.array_equal(f, out[0][0]) and e == pytest.approx(out[0][1], rel=TOL64)
+
+
+@pytest.mark.parametrize("atoms", [2500, 2700, 3180, 3290])
+def test_tiles_at_the_shared_memory_limit(gpulib, oracle, atoms):
+    """FP64 tiles of 4 cells (6^3 of the box's 8^3 staged) of about this many atoms: with the passes' headroom (to
+    2,617 atoms), without it, and beyond what the fixed-point pass's tables leave room for (3,216), where the FP64
+    body takes every tile (to 3,336)."""
+    rc, m = 5.0, 24
+    L = np.full(3, 8 * rc / 2)
+    g = (np.arange(m) + 0.5) * (L[0] / m)
+    pos = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3)
+    rng = np.random.default_rng(atoms)
+    n = int(atoms / (6 / 8) ** 3)
+    pos = pos[rng.permutation(len(pos))[:n]] + rng.uniform(-0.02, 0.02, (n, 3))
+    with gpulib.MidpointLJ(L, [n], precision="fp64", rc=rc, tile=(4, 4, 4)) as s:
+        s.set_atoms(pos)
+        f, e, _ = s.forces(energy=True)
+        assert 0 <= s.counters()["max_tile_atoms"] - atoms <= 50
+    ref = oracle.forces_typed(pos, L, rc, threads=0)
+    check(f, ref["forces"], "fp64")
+    assert e[0] == pytest.approx(ref["epot"], rel=TOL64)
