@@ -1307,7 +1307,7 @@ int init_lists(examd_ctx* ctx) {
 }
 
 int run_pair(examd_ctx* ctx, bool energy, bool count, double* boxE = nullptr, double* boxW = nullptr,
-             bool side = false);
+             bool side = false, bool sums = true);
 
 // Pair-list mode, between runs of steps: a tile with an atom whose list
 // outgrew its capacity since the last check, or with more staged atoms than
@@ -1336,8 +1336,9 @@ int update_lists(examd_ctx* ctx, bool cap_grew) {
 }
 
 // The pair pass; with energy the per-box sums to boxE, boxW (nullptr: the
-// context's), on the second stream for a step of a loop (side).
-int run_pair(examd_ctx* ctx, bool energy, bool count, double* boxE, double* boxW, bool side) {
+// context's), on the second stream for a step of a loop (side); sums = false
+// leaves them to the caller.
+int run_pair(examd_ctx* ctx, bool energy, bool count, double* boxE, double* boxW, bool side, bool sums) {
   PairConfig c = ctx->pc;
   c.energy = energy;
   c.count = count;
@@ -1347,16 +1348,16 @@ int run_pair(examd_ctx* ctx, bool energy, bool count, double* boxE, double* boxW
     ctx->side_pe = false;
   }
   CK(launch_pair(c, pair_args(ctx), ctx->ntiles, ctx->smem, ctx->st));
-  if (!energy) return EXAMD_OK;
-  cudaStream_t sums = side ? ctx->st2 : ctx->st;
+  if (!energy || !sums) return EXAMD_OK;
+  cudaStream_t to = side ? ctx->st2 : ctx->st;
   if (side) {
     CK(cudaEventRecord(ctx->ev_side[1], ctx->st));
-    CK(cudaStreamWaitEvent(sums, ctx->ev_side[1], 0));
+    CK(cudaStreamWaitEvent(to, ctx->ev_side[1], 0));
   }
   CK(launch_reduce_tiles(ctx->nboxes, ctx->d_tile0, ctx->maxc_tiles, ctx->tileE, ctx->tileW, ctx->partial,
-                         boxE ? boxE : ctx->boxE, boxW ? boxW : ctx->boxW, sums));
+                         boxE ? boxE : ctx->boxE, boxW ? boxW : ctx->boxW, to));
   if (side) {
-    CK(cudaEventRecord(ctx->ev_side[3], sums));
+    CK(cudaEventRecord(ctx->ev_side[3], to));
     ctx->side_pe = true;
   }
   return EXAMD_OK;
@@ -1440,18 +1441,35 @@ int enqueue_forces(examd_ctx* ctx, double* forces, double* epot, double* virial,
   // (the energies too, where the arrays allow)
   const size_t nb = (size_t)ctx->nboxes;
   double *const de = in_place(epot, nb) ? epot : nullptr, *const dw = in_place(virial, nb) ? virial : nullptr;
-  int rc = run_pair(ctx, energy, false, de, dw);
+  // with the forces written in place, the call's last kernel sums the energies
+  // of boxes of one chunk and passes on the status word
+  const bool tail_sums = df && N > 0 && energy && ctx->maxc_tiles == 1;
+  int rc = run_pair(ctx, energy, false, de, dw, false, !tail_sums);
   if (rc) return rc;
+  bool status_sent = false;
   if (df && N > 0) {
+    ForcesTail tail;
+    if (tail_sums) {
+      tail.nboxes = ctx->nboxes;
+      tail.tile0 = ctx->d_tile0;
+      tail.tileE = ctx->tileE;
+      tail.tileW = ctx->tileW;
+      tail.boxE = de ? de : ctx->boxE;
+      tail.boxW = dw ? dw : ctx->boxW;
+    }
+#ifndef EXAMD_CHECKED  // (there the kernel's own index checks write the word)
+    tail.host_status = ctx->h_status;
+    status_sent = true;
+#endif
     CK(ensure_inv(ctx));
-    CK(launch_forces_out(step_args(ctx), 0, N, ctx->inv, df, accumulate, st));
+    CK(launch_forces_out(step_args(ctx), 0, N, ctx->inv, df, accumulate, tail, st));
   } else if (forces && N > 0) {
     CK(ensure_inv(ctx));
     for (int c = 0; c < nch; ++c) {
       int64_t i0, i1;
       io_range(N, nch, c, i0, i1);
       if (accumulate) CK(cudaStreamWaitEvent(st, ev_acc[c], 0));
-      CK(launch_forces_out(step_args(ctx), i0, i1, ctx->inv, ctx->stage, accumulate, st));
+      CK(launch_forces_out(step_args(ctx), i0, i1, ctx->inv, ctx->stage, accumulate, ForcesTail{}, st));
       CK(cudaEventRecord(ctx->ev_io[kIoChunks + c], st));
       CK(cudaStreamWaitEvent(st2, ctx->ev_io[kIoChunks + c], 0));
       CK(cudaMemcpyAsync(forces + 3 * i0, ctx->stage + 3 * i0, 3 * (i1 - i0) * sizeof(double),
@@ -1464,7 +1482,7 @@ int enqueue_forces(examd_ctx* ctx, double* forces, double* epot, double* virial,
     CK(cudaEventRecord(ctx->ev_io[3 * kIoChunks], st2));
     CK(cudaStreamWaitEvent(st, ctx->ev_io[3 * kIoChunks], 0));
   }
-  CK(queue_status(ctx));
+  if (!status_sent) CK(queue_status(ctx));
   return EXAMD_OK;
 }
 

@@ -8,7 +8,7 @@
 // the order in which the counting pass drew their slots.  Neither form's
 // results depend on that order: the mixed form's force and energy sums are
 // exact fixed point and each pair's FP32 term is antisymmetric in its two
-// atoms, and the FP64 form's shared-memory atomics fix no order anyway.
+// atoms, and the FP64 form's first pass sums exact integers.
 // HBM-bound work.
 #include "common.cuh"
 #include "kernels.cuh"

@@ -1,9 +1,9 @@
 // common.cuh -- shared device-side definitions of the GB300 midpoint LJ path.
 //
 // Layout in HBM (all per-atom arrays in "sorted order": atoms grouped by cell,
-// cells in (box, z, y, x) order, atoms of a cell in ascending caller index,
-// i.e. the reference's block order and linked-list order,
-// SRC/exaMD_input_formats.f90:66-92):
+// cells in (box, z, y, x) order, the reference's block order,
+// SRC/exaMD_input_formats.f90:66-92; inside a cell the order of the counting
+// pass's slots):
 //   X[3][N], V[3][N]  FP64 positions / velocities (SoA), double-buffered
 //   meta[N]           box << 8 | type
 //   id[N]             caller index

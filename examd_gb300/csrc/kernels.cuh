@@ -152,7 +152,7 @@ struct PairConfig {
 };
 
 // Dynamic shared memory for the tile capacities: the larger of the first
-// pass's need at cap and, mixed form, the redo pass's at cap_redo.
+// pass's need at cap and, where there is one, the redo pass's at cap_redo.
 int pair_smem_bytes(const PairConfig& cfg, int cap, int cap_redo, int ne_max, int ext_max);
 cudaError_t pair_prepare(const PairConfig& cfg, int smem_bytes);  // opt-in smem attribute
 cudaError_t launch_pair(const PairConfig& cfg, const PairArgs& a, int ntiles, int smem_bytes, cudaStream_t st);
@@ -174,8 +174,17 @@ struct StepArgs {
 };
 
 // F = Fown + halo partials, in caller order, AoS doubles (out[3*id + a]); += if accumulate.
+// What the last kernel of a force call does besides (nullptr: not): the status
+// word to the host, and the boxes' energies where every box has one chunk of tiles.
+struct ForcesTail {
+  int nboxes = 0;  // > 0: sums of the boxes' tile energies and virials
+  const int* tile0 = nullptr;
+  const double *tileE = nullptr, *tileW = nullptr;
+  double *boxE = nullptr, *boxW = nullptr;
+  int* host_status = nullptr;
+};
 cudaError_t launch_forces_out(const StepArgs& s, int64_t i0, int64_t i1, const int* inv, double* out, int accumulate,
-                              cudaStream_t st);
+                              const ForcesTail& tail, cudaStream_t st);
 // Per-box sums of the per-tile energy/virial partials (FP64, fixed order).
 // Per-box sums in two fixed-order levels (chunks of 4096 entries, then the
 // box's chunks in order); partial holds nboxes * maxc doubles (tiles: twice).

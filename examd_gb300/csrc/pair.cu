@@ -19,11 +19,17 @@
 // of one step (at most 32) have their candidate pairs laid end to end and
 // tested 32 at a time, one per lane.  Accepted pairs are queued and their
 // forces computed in batches of 32, both atoms' sums updated (Newton's third
-// law).  The FP64 form builds items per (ext cell, row) instead: the block
-// of the cell's atoms against the row's owned j-cells, untrimmed, tested with
-// an FP32 prefilter on a widened cutoff; the queued pairs are computed in
-// FP64.  Its batches then hold pairs of many different i atoms, so their FP64
-// shared-memory atomics (the FP64 form's bound) rarely hit one address.
+// law).  The FP64 form's first pass (k_pair_fix) walks the same items, tested
+// with an FP32 prefilter on a widened cutoff, and computes the queued pairs in
+// fixed point (force_batch_fix).  Its FP64 body (the tiles that the fixed-point
+// pass lists, and systems it cannot hold) builds items per (ext cell, row): the
+// block of the cell's atoms against the row's owned j-cells, untrimmed; its
+// batches then hold pairs of many different i atoms, so their FP64
+// shared-memory atomics (compare-and-swap loops) rarely hit one address.
+//
+// What bounds the passes (1M liquid): the enumeration and the FP64 pass issue
+// (73-81 % of the slots; ALU pipe 50 %); the list pass issue and shared memory
+// (70 %; half of the wavefronts atomics); none of them DRAM (0.1-0.9 TB/s).
 //
 // Accumulation.  Mixed form: each per-atom force component is an exact 32-bit
 // fixed-point sum in shared memory (scale 2^17, native integer atomics), so
@@ -37,7 +43,8 @@
 // launch (k_pair_redo) recomputes the flagged tiles, sums their large terms
 // in FP32 and adds them to the outputs; thermal configurations flag no tile
 // and the launch returns at once (only the rare FP32 sums' order can vary
-// between runs).  FP64 form: FP64 shared-memory atomics.
+// between runs).  FP64 form: 64-bit integer sums in the first pass, FP64
+// shared-memory atomics in the FP64 body.
 //
 // Output: forces of the tile's home atoms go to Fown, those of halo copies to
 // the partial slot P[s] (s = bitmask of the axes on which the copy is a halo
@@ -852,7 +859,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   const unsigned lt = (1u << lane) - 1u;
   const unsigned le = FULL >> (31 - lane);
   auto r2l = EXAMD_ARR(unsigned char, smem + L.r2l + 64 * warp, FP64 ? 64 : 1, st);  // FP64 form: two rank -> lane tables of 32
-  // ---- accepted pairs go to the warp's queue (a ring of kQueue entries);
+  // ---- accepted pairs go to the warp's queue (a stack of kQueue entries);
   // their forces are computed in full batches of 32 ----
   // list build: an accepted pair (i, m) is entry k of atom i in the scratch
   // (i's entries side by side, lk per atom), k from the atom's counter (fa);

@@ -5,8 +5,9 @@
 // The reference has no integrator (one force evaluation, exaMD.f90:247-251);
 // the gather replaces its reverse force exchange, which adds received halo
 // forces into the owner's blocks (SRC/exaMD_comms.f90:330-376).  All of these
-// are HBM-bound; FP64 is used only where positions, velocities and the
-// reductions need it.
+// are bound by HBM and, the kick, by the FP64 pipe (nine operations an atom;
+// 46.6 us at 1M atoms on lists, 555 us at 16.8M); FP64 is used only where
+// positions, velocities and the reductions need it.
 #include <algorithm>
 #include <type_traits>
 
@@ -135,15 +136,54 @@ __device__ __forceinline__ void gather_force(const StepArgs& a, int64_t s, doubl
   }
 }
 
+// Entries [a0, a1) of v0 (and v1) summed by a block of 256 threads with a fixed
+// tree; thread 0's s0, s1 are the sums.
+template <int NV>
+__device__ __forceinline__ void block_sums(int64_t a0, int64_t a1, const double* __restrict__ v0,
+                                           const double* __restrict__ v1, double (*sh)[256], double& s0, double& s1) {
+  s0 = s1 = 0.0;
+  for (int64_t i = a0 + threadIdx.x; i < a1; i += 256) {
+    s0 += v0[i];
+    if (NV > 1) s1 += v1[i];
+  }
+  sh[0][threadIdx.x] = s0;
+  if (NV > 1) sh[NV - 1][threadIdx.x] = s1;
+  __syncthreads();
+  for (int o = 128; o > 0; o >>= 1) {
+    if (threadIdx.x < o) {
+      sh[0][threadIdx.x] += sh[0][threadIdx.x + o];
+      if (NV > 1) sh[NV - 1][threadIdx.x] += sh[NV - 1][threadIdx.x + o];
+    }
+    __syncthreads();
+  }
+  s0 = sh[0][0];
+  s1 = sh[NV - 1][0];
+}
+
 // Forces of the caller's atoms [i0, i1) in caller order (AoS): the atom's
-// partials gathered at its sorted slot inv[i]; written or added (acc).
+// partials gathered at its sorted slot inv[i]; written or added (acc).  The
+// blocks past the atoms' (tail.nboxes) sum a box's tile energies each, and the
+// status word goes to the host from here: as a launch and a copy of their own
+// they took 6 of the 50 us of a call of 1,000 atoms and 9 of the 310 of 276k.
 template <bool FP64>
 __global__ void __launch_bounds__(kIoThreads) k_forces_out(const StepArgs a, int64_t i0, int64_t i1,
                                                            const int* __restrict__ inv, double* __restrict__ out,
-                                                           int acc) {
+                                                           int acc, const ForcesTail tail) {
   __shared__ double sh[3 * kIoThreads];
   grid_trigger();
   grid_wait();
+  const int na = (int)gridDim.x - tail.nboxes;  // blocks of atoms
+  if ((int)blockIdx.x >= na) {
+    const int b = (int)blockIdx.x - na;
+    double e, w;
+    block_sums<2>(tail.tile0[b], tail.tile0[b + 1], tail.tileE, tail.tileW, (double(*)[256])sh, e, w);
+    if (threadIdx.x == 0) {
+      tail.boxE[b] = e;
+      tail.boxW[b] = w;
+    }
+    return;
+  }
+  if (tail.host_status && blockIdx.x == 0 && threadIdx.x == 0) *tail.host_status = *a.status;
   const int64_t b0 = i0 + blockIdx.x * (int64_t)kIoThreads, i = b0 + threadIdx.x;
   const int n = (int)min((int64_t)kIoThreads, i1 - b0);
   out += 3 * b0;
@@ -168,12 +208,12 @@ __global__ void __launch_bounds__(kIoThreads) k_forces_out(const StepArgs a, int
 }
 
 cudaError_t launch_forces_out(const StepArgs& s, int64_t i0, int64_t i1, const int* inv, double* out, int accumulate,
-                              cudaStream_t st) {
+                              const ForcesTail& tail, cudaStream_t st) {
   if (i1 <= i0) return cudaSuccess;
-  const unsigned g = (unsigned)((i1 - i0 + kIoThreads - 1) / kIoThreads);
+  const unsigned g = (unsigned)((i1 - i0 + kIoThreads - 1) / kIoThreads) + tail.nboxes;
   if (s.fp64)
-    return launch_chained(true, k_forces_out<true>, g, kIoThreads, st, s, i0, i1, inv, out, accumulate);
-  return launch_chained(true, k_forces_out<false>, g, kIoThreads, st, s, i0, i1, inv, out, accumulate);
+    return launch_chained(true, k_forces_out<true>, g, kIoThreads, st, s, i0, i1, inv, out, accumulate, tail);
+  return launch_chained(true, k_forces_out<false>, g, kIoThreads, st, s, i0, i1, inv, out, accumulate, tail);
 }
 
 // Per-box FP64 sums of per-tile partials: one block per box, fixed-order tree.
@@ -192,24 +232,11 @@ __global__ void k_chunk_sums(const Off* __restrict__ off, const double* __restri
   const int c = blockIdx.x, b = blockIdx.y;
   const int64_t a0 = (int64_t)off[b] + (int64_t)c * kRedChunk;
   const int64_t a1 = min((int64_t)off[b + 1], a0 + kRedChunk);
-  double s0 = 0.0, s1 = 0.0;
-  for (int64_t i = a0 + threadIdx.x; i < a1; i += blockDim.x) {
-    s0 += v0[i];
-    if (NV > 1) s1 += v1[i];
-  }
-  sh[0][threadIdx.x] = s0;
-  if (NV > 1) sh[NV - 1][threadIdx.x] = s1;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      sh[0][threadIdx.x] += sh[0][threadIdx.x + o];
-      if (NV > 1) sh[NV - 1][threadIdx.x] += sh[NV - 1][threadIdx.x + o];
-    }
-    __syncthreads();
-  }
+  double s0, s1;
+  block_sums<NV>(a0, a1, v0, v1, sh, s0, s1);
   if (threadIdx.x == 0) {
-    p0[(size_t)b * maxc + c] = sh[0][0];
-    if (NV > 1) p1[(size_t)b * maxc + c] = sh[NV - 1][0];
+    p0[(size_t)b * maxc + c] = s0;
+    if (NV > 1) p1[(size_t)b * maxc + c] = s1;
   }
 }
 
