@@ -123,8 +123,8 @@ class MidpointLJ:
     (ntypes, ntypes) tables; block_length defaults to max(rc)/2 as the
     reference (exaMD.f90:56).  potential: the pair function, "lj" (the
     reference's lennardjones_12), "lj_shifted" or "wca".  pair_tables: the
-    mixed form's per-warp tables, "auto" (compact where that fits more CTAs
-    on an SM), "wide" or "compact"; the forces are the same bit for bit.
+    per-warp tables, "auto", "wide" or "compact": they have one layout, so
+    the three are the same.
     tile_balance: 0 splits each axis into tiles by cell count, 1 by width (the
     wide last cell that absorbs the box's remainder counts as two).
     pair_skin: 0 (the reference's schedule: cells and candidate pairs at
@@ -207,7 +207,8 @@ class MidpointLJ:
     def forces_at(self, pos, out=None, accumulate=False, energy=False):
         """New positions (same atoms, caller order) and one force evaluation.
 
-        With pos and out in pinned memory (pinned_empty) the library replays the
+        With pos and out in pinned memory (pinned_empty) the kernels read and write
+        them in place, and the library replays the
         call as a captured CUDA graph from the second call with the same arrays;
         the energies then land in pinned arrays of this object and are copied."""
         p = pos if (isinstance(pos, np.ndarray) and pos.dtype == np.float64 and pos.flags.c_contiguous) \

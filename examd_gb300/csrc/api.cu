@@ -154,7 +154,7 @@ long long fixed_of(double x, int ue) {
 // The tables of the FP64 form's fixed-point pass (pair.cu, force_batch_fix), or
 // false where the parameters do not suit it and the FP64 body computes every
 // tile: type pairs whose force scales eps / sigma differ by more than 16 (the
-// sums have one unit, and the weakest pair's forces keep 2^-45 of its scale), a
+// sums have one unit, and the weakest pair's forces keep 2^-47 of its scale), a
 // cutoff inside the range of the forces too large for the sums, or lengths and
 // energies whose powers leave FP64's range.
 bool build_fix(const LJTable& lj, const examd_params& p, FixTable& fx) {
@@ -170,14 +170,17 @@ bool build_fix(const LJTable& lj, const examd_params& p, FixTable& fx) {
   if (std::ldexp(1.0, f0) < f0max) ++f0;
   fx.ue = std::ilogb(rmax) + 1 - 62;  // every separation within the cutoff is below 2^62 units
   fx.sf = kFixSumBits - f0;
-  const double fbig = std::ldexp(1.0, kFixTermBits + f0);
+  const double fbig = std::ldexp(1.0, kFixTermBits + f0), fmed = std::ldexp(1.0, kFixMedBits + f0);
   const int w = 2 * fx.ue + 64;  // r^2 = D 2^w
-  double r2big[EXAMD_MAX_TYPES * EXAMD_MAX_TYPES], gmax = 0.0;
+  double r2big[EXAMD_MAX_TYPES * EXAMD_MAX_TYPES], r2med[EXAMD_MAX_TYPES * EXAMD_MAX_TYPES];
+  double gmax = 0.0, gbig = 0.0;
   for (int k = 0; k < n2; ++k) {
     r2big[k] = std::max(r2_of_force(p.eps[k], p.sigma[k], fbig), 1.001e-12);  // coincident atoms (kR2Min64) as well
-    gmax = std::max(gmax, fbig / std::sqrt(r2big[k]));
+    r2med[k] = std::max(r2_of_force(p.eps[k], p.sigma[k], fmed), r2big[k]);
+    gmax = std::max(gmax, fmed / std::sqrt(r2med[k]));
+    gbig = std::max(gbig, fbig / std::sqrt(r2big[k]));
   }
-  if (!std::isnormal(gmax)) return false;
+  if (!std::isnormal(gmax) || !(std::ldexp(gbig, -kFixMedShift) < gmax)) return false;
   const int sg = 61 - std::ilogb(gmax);  // |dg| 2^sg < 2^62
   const int K = sg - fx.ue - fx.sf;
   if (K < 33 || K > 63) return false;
@@ -191,11 +194,12 @@ bool build_fix(const LJTable& lj, const examd_params& p, FixTable& fx) {
     q.s6 = (double)std::ldexp(s6, -3 * w);
     q.e4 = lj.p64[k].eps4;
     q.eshift = lj.p64[k].eshift;
-    const double lim = std::ldexp(lj.p64[k].rcut2, -w), big = std::ldexp(r2big[k], -w);
+    const double lim = std::ldexp(lj.p64[k].rcut2, -w), big = std::ldexp(r2big[k], -w), med = std::ldexp(r2med[k], -w);
     if (!std::isnormal(q.c6) || !std::isnormal(q.c12) || !std::isnormal(q.s6) || !(big >= 0x1p36) ||
-        !(lim >= 0x1p44) || !(lim < 0x1p61) || !(big < lim))
+        !(lim >= 0x1p44) || !(lim < 0x1p61) || !(med < lim))
       return false;
     q.limh = (int)((long long)lim >> 32);
+    q.medh = (int)((long long)med >> 32) + 1;
     q.bigh = (int)((long long)big >> 32) + 1;
     q.pre = lj.p32[k].rc2 * 1.0001f;
   }

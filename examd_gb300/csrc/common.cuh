@@ -119,11 +119,14 @@ struct LJ32 {
 // component of a kept term is below 2^28 in fixed point, so a component's
 // int32 sum needs more than 8 near-maximal terms of one sign to overflow.
 constexpr float kFixMaxForce = 2048.f;
-// FP64 form's fixed-point pass: the force sums' unit is 2^-49 of the power of
-// two F0 at or above the largest eps / sigma, the largest kept term 2^11 F0, so
-// that a sum overflows 64 bits only by more than 8 near-maximal terms of one sign
-// (as above; 2^-49 F0 is about 1e-17 of a liquid's rms force)
-constexpr int kFixSumBits = 49, kFixTermBits = 11;
+// FP64 form's fixed-point pass: the force sums' unit is 2^-51 of the power of
+// two F0 at or above the largest eps / sigma.  A term below 2^9 F0 (r > 0.83
+// sigma) may be added any number of times: a sum overflows 64 bits only by more
+// than 8 near-maximal ones of one sign (as above).  A term of 2^9 to 2^11 F0
+// takes up to four of those eight, so an atom may have one of them (a second one
+// sends the tile to the FP64 body); a term above 2^11 F0 always does.
+constexpr int kFixSumBits = 51, kFixMedBits = 9, kFixTermBits = 11;
+constexpr int kFixMedShift = 3;  // the larger terms' factor, taken that much coarser to fit its 63 bits
 struct LJ64 {
   double sig2, eps24, eps4, rc2;   // as user_func.f90:58-59 computes them
   double rcut2, eshift;
@@ -136,7 +139,8 @@ struct FixPair {
   double c6, c12;
   double e4, s6;    // energy: 4 eps, and sigma^6 in units of D^3
   double eshift;
-  int limh, bigh;   // high words of D at the range (rc or the potential's own) and at the largest kept force
+  int limh;         // high words of D at the range (rc or the potential's own),
+  int medh, bigh;   // at forces of 2^kFixMedBits and of 2^kFixTermBits F0
   float pre;        // FP32 prefilter of the candidates: rc^2 widened
 };
 

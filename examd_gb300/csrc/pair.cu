@@ -441,11 +441,11 @@ __device__ __forceinline__ void force_batch64(int cnt, const QK& qk, const PD& p
 // the FP64 body's own r^2 (in64), so that both accept the same pairs; a pair
 // whose force is too large for the sums' range flags the tile, and the FP64
 // body redoes it.
-template <bool MULTI, bool ENERGY, bool COUNT, class QK, class PX, class FA, class FACE, class IN64>
+template <bool MULTI, bool ENERGY, bool COUNT, class QK, class PX, class FA, class FACE, class IN64, class SECOND>
 __device__ __forceinline__ void force_batch_fix(int cnt, int q0, const QK& qk, const PX& px, FA& fa, int cap,
                                                 const PairArgs& A, const FixPair* ljx, double& s12, double& s6s,
                                                 double& shift, int& nacc, int* big_flag, bool edge, const FACE& face,
-                                                const IN64& in64) {
+                                                const IN64& in64, const SECOND& second) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   int i = -1, m = 0;
@@ -470,9 +470,11 @@ __device__ __forceinline__ void force_batch_fix(int cnt, int q0, const QK& qk, c
     const int Dh = (int)(D >> 32);
     app = Dh < P.limh;
     if (abs(Dh - P.limh) <= 1) app = in64(i, m, ti, tj);
-    if (app && Dh < P.bigh) {
-      *big_flag = 1;
-      app = false;
+    int up = 0;
+    if (app && Dh < P.medh) {  // rare
+      up = kFixMedShift;
+      app = Dh >= P.bigh;
+      if (!app || second(i, m)) *big_flag = 1;
     }
     if (app) {
       // D as a double: normalised so that its first bit is bit 62, 53 bits kept
@@ -496,11 +498,11 @@ __device__ __forceinline__ void force_batch_fix(int cnt, int q0, const QK& qk, c
         if (A.lj.pot != EXAMD_POT_LJ) shift += P.eshift;
       }
       if (COUNT) ++nacc;
-      // g as a 63-bit integer (|g| < 2^62), then G d / 2^(64 - ka), rounded
+      // g as a 63-bit integer (|g| < 2^62, a large one in units of 2^up), then G d / 2^(64 - ka), rounded
       const int gb = __double2hiint(g);
       const unsigned long long gm =
           ((((unsigned long long)(unsigned)((gb & 0xfffff) | 0x100000)) << 32) | (unsigned)__double2loint(g)) << 10;
-      const int gs = min(1085 - ((gb >> 20) & 0x7ff), 63);
+      const int gs = min(1085 + up - ((gb >> 20) & 0x7ff), 63);
       long long G = (long long)(gm >> gs);
       if (gb < 0) G = -G;
       const int gh = (int)((G + 0x80000000ll) >> 32), gl = (int)G;
@@ -519,6 +521,11 @@ __device__ __forceinline__ void force_batch_fix(int cnt, int q0, const QK& qk, c
       fx = term(hx, lx);
       fy = term(hy, ly);
       fz = term(hz, lz);
+      if (up) {
+        fx <<= up;
+        fy <<= up;
+        fz <<= up;
+      }
     }
   }
   // v to the 64-bit sum of component c of atom t: low word, carry, high word
@@ -880,7 +887,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   auto inside64 = [&](int a, int b, int ta, int tb) -> bool {
     auto gidx = [&](int t) {
       const int c = code[t];
-      const int e = (c & 31) + EX * (((c >> 5) & 31) + EY * (c >> 10));
+      const int e = (c & 31) + EX * (((c >> 5) & 31) + EY * ((c >> 10) & 31));
       return (int64_t)gfirst[e] + (t - (int)lstart[e]);
     };
     const int64_t ga = EXAMD_IDX(gidx(a), A.N, st), gb = EXAMD_IDX(gidx(b), A.N, st);
@@ -915,7 +922,17 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
     };
     round_axis(0, ci & 31, cm & 31, dx);
     round_axis(1, (ci >> 5) & 31, (cm >> 5) & 31, dy);
-    round_axis(2, ci >> 10, cm >> 10, dz);
+    round_axis(2, (ci >> 10) & 31, (cm >> 10) & 31, dz);
+  };
+  // kFixed: whether either atom already has a term above 2^kFixMedBits F0 (bit 15
+  // of its code), and marks both
+  auto second = [&](int i, int m) {
+    auto mark = [&](int t) {
+      const unsigned bit = 0x8000u << (16 * (t & 1));
+      return (atomicOr((unsigned*)(smem + L.code) + (t >> 1), bit) & bit) != 0u;
+    };
+    const bool a = mark(i), b = mark(m);
+    return a || b;
   };
   auto enqueue = [&](bool acc, const float4& dq, int key) {
     const unsigned bal = __ballot_sync(FULL, acc);
@@ -935,7 +952,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
                                             nacc, qn);
       else if (FIX)
         force_batch_fix<MULTI, ENERGY, COUNT>(32, qn, qk, px, fa, cap, A, ljx, esum, wsum, shsum, nacc, big_flag,
-                                              edge, face, inside64);
+                                              edge, face, inside64, second);
       else
         force_batch<MULTI, ENERGY, COUNT, MODE == kRedoFull>(32, qn, qd, fa, fr, cap, A, ljs32, ek, wk, nacc,
                                                              big_flag, inside64);
@@ -1288,7 +1305,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
       // per-atom quantities of lane l's atom c*32 + l
       const int ia = c * 32 + lane;
       const bool va = ia < total;
-      const int cia = code[va ? ia : 0];
+      const int cia = code[va ? ia : 0] & 0x7fff;  // (bit 15: see `second`)
       const int ax = cia & 31, ay = (cia >> 5) & 31, az = cia >> 10;
       const int acls = pos_class(ax - 1, tx) * 25 + pos_class(ay - 1, ty) * 5 + pos_class(az - 1, tz);
       const int aw = va ? (sown->nrow[acls] + kParts - 1 - part) / kParts : 0;
@@ -1476,7 +1493,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
                                           nacc, 0);
     else if (FIX)
       force_batch_fix<MULTI, ENERGY, COUNT>(qn, 0, qk, px, fa, cap, A, ljx, esum, wsum, shsum, nacc, big_flag,
-                                            edge, face, inside64);
+                                            edge, face, inside64, second);
     else
       force_batch<MULTI, ENERGY, COUNT, MODE == kRedoFull>(qn, 0, qd, fa, fr, cap, A, ljs32, ek, wk, nacc,
                                                            big_flag, inside64);
@@ -1614,7 +1631,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   // (4) write-back: home atoms -> Fown, halo copies -> P[slot]
   for (int t = tid; t < total; t += blockDim.x) {
     const int ci = code[t];
-    const int lx = ci & 31, ly = (ci >> 5) & 31, lz = ci >> 10;
+    const int lx = ci & 31, ly = (ci >> 5) & 31, lz = (ci >> 10) & 31;
     const int slot = ((lx == 0 || lx == EX - 1) ? 1 : 0) | ((ly == 0 || ly == EY - 1) ? 2 : 0) |
                      ((lz == 0 || lz == EZ - 1) ? 4 : 0);
     const int e = lx + EX * (ly + EY * lz);

@@ -63,9 +63,10 @@ extern "C" {
                                   candidate pairs and must be >= that range  */
 
 /* Precision forms. */
-#define EXAMD_FP64 0  /* FP64 end to end                                       */
-#define EXAMD_MIXED 1 /* FP32 pair forces on tile-frame offsets, Kahan-merged  */
-                      /* FP32 per-atom sums, FP64 integration/wrap/reductions  */
+#define EXAMD_FP64 0  /* FP64 accuracy end to end (the pair pass in exact      */
+                      /* fixed point where the system allows, else in FP64)    */
+#define EXAMD_MIXED 1 /* FP32 pair forces on tile-frame offsets, exact         */
+                      /* fixed-point sums, FP64 integration/wrap/reductions    */
 
 typedef struct examd_params {
   int precision;      /* EXAMD_FP64 or EXAMD_MIXED                            */
@@ -83,14 +84,15 @@ typedef struct examd_params {
    * absorbing the remainder (SRC/exaMD_utils.f90:179,
    * SRC/exaMD_module.f90:109-113). */
   double cell_edge;
-  int tile[3];        /* home cells per CTA tile per axis; 0 = default        */
+  int tile[3];        /* home cells per CTA tile per axis; 0 = default (4; in */
+                      /* the FP64 form 3 or 2 for systems of few tiles)       */
   int warps;          /* warps per CTA in the pair kernel; 0 = default        */
   int strict_box;     /* 1: positions outside [0,L) are an error (109);       */
                       /* 0: they are wrapped periodically                     */
   int device;         /* CUDA device ordinal                                  */
   int potential;      /* EXAMD_POT_*                                          */
-  int pair_tables;    /* mixed form's per-warp tables in the pair kernel:     */
-                      /* 0 = chosen by occupancy, 1 = wide, 2 = compact       */
+  int pair_tables;    /* 0, 1 or 2, all with the same effect (the per-warp    */
+                      /* tables have one layout)                              */
   int tile_balance;   /* split of an axis into tiles: 0 = by cell count;      */
                       /* 1 = by width, where the last cell (which absorbs the */
                       /* box's remainder) is >= 1.5 edges wide it counts as   */
@@ -155,8 +157,10 @@ int examd_gpu_set_atoms(examd_ctx *ctx, int64_t n, const double *pos,
 int examd_gpu_forces(examd_ctx *ctx, double *forces, double *epot,
                      double *virial, int accumulate);
 
-/* Same as examd_gpu_forces but with new positions given in the same call
- * (one host->device copy, the pair path, one device->host copy). */
+/* Same as examd_gpu_forces but with new positions given in the same call.
+ * Page-locked arrays are read and written in place by the kernels, others
+ * copied; calls of up to 16,384 atoms go through page-locked arrays of the
+ * context, from the third call on. */
 int examd_gpu_forces_at(examd_ctx *ctx, const double *pos, double *forces,
                         double *epot, double *virial, int accumulate);
 

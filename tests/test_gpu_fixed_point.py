@@ -105,6 +105,21 @@ def test_forces_beyond_the_sums(gpulib, oracle):
     against_oracle(gpulib, oracle, pos, L, rc=2.5)
 
 
+@pytest.mark.parametrize("neighbours", [1, 2, 4])
+def test_several_large_terms_on_one_atom(gpulib, oracle, neighbours):
+    """Atoms with 1, 2 or 4 neighbours at 0.745 to 0.83 sigma on one side, every term within the first pass's range
+    (|F| 500 to 2000); four of them add up to nearly what the sums hold (4096)."""
+    rng = np.random.default_rng(neighbours)
+    L = np.array([16.0, 20.0, 24.0])
+    c = np.stack(np.meshgrid(*[np.arange(1.0, b, 4.0) for b in L], indexing="ij"), -1).reshape(-1, 3)
+    t = np.radians(50.0)
+    parts = [c]
+    for k in range(neighbours):
+        u = np.array([np.cos(t), np.sin(t) * np.cos(k * np.pi / 2), np.sin(t) * np.sin(k * np.pi / 2)])
+        parts.append(c + rng.uniform(0.745, 0.83, (len(c), 1)) * u)
+    against_oracle(gpulib, oracle, np.concatenate(parts), L, rc=2.5)
+
+
 def test_first_pass_overflow(gpulib, oracle):
     """A density wave through forces_at packs tiles beyond the first pass's capacity (6 % + 32 atoms above the
     largest tile when the atoms were set), within the redo pass's (25 % + 64)."""
