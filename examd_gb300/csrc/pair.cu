@@ -139,8 +139,9 @@ __host__ __device__ inline int align16(int x) { return (x + 15) & ~15; }
 // queues, no ownership table: the queue region holds only the scan and
 // reduction scratch; kListBig's fr after everything).
 // ne_max, ext_max: the largest tile's ext cells and ext extent on one axis.
+// own: with a copy of the ownership table (see own_in_global).
 __host__ __device__ inline Layout make_layout(bool fp64, int cap, int ne_max, int ext_max, int nw, int mode,
-                                              bool multi) {
+                                              bool multi, bool own = true) {
   const bool from_list = mode == kList || mode == kListBig;
   Layout L;
   int o = 0;
@@ -155,7 +156,7 @@ __host__ __device__ inline Layout make_layout(bool fp64, int cap, int ne_max, in
   L.img = o;    o = align16(o + (fp64 || fix ? 3 * 32 : 0));  // periodic image per ext coordinate (FP64 form)
   L.cw = o;     o = align16(o + 16);  // unit counter, large-term flag, staged-atom total
   L.r2l = o;    o = align16(o + (fp64 ? 64 * nw : 0));  // rank -> lane tables (FP64 form)
-  L.lut = o;    o = align16(o + (from_list ? 0 : (int)sizeof(OwnLut)));
+  L.lut = o;    o = align16(o + (from_list || !own ? 0 : (int)sizeof(OwnLut)));
   // the LJ table per ordered type pair (several types): per-lane type indices
   // would serialise on the kernel-parameter bank, shared memory serves them at once
   L.ljt = o;    o = align16(o + (multi ? (fix ? (int)sizeof(FixPair) : (int)sizeof(LJ64)) * EXAMD_MAX_TYPES * EXAMD_MAX_TYPES : 0));
@@ -190,6 +191,17 @@ __host__ __device__ inline Layout make_layout(bool fp64, int cap, int ne_max, in
   return L;
 }
 
+// The FP64 form's first pass with one type, in grids of many waves, reads the
+// ownership table from global memory (its lines stay in L1) instead of a copy
+// of 3.4 KB in each CTA: a tile of 66 bytes an atom is near the size at which
+// an SM holds three CTAs instead of four (568 atoms at 8 warps with the copy, 616
+// without, at 4^3 cells; 1M liquid, 616: 885 -> 788 us a pass).  In few waves there is no
+// fourth CTA to gain and the copy is nearer (1,000 atoms 9.5 against 10 us); with
+// several types the registers allow three.
+__host__ __device__ constexpr bool own_in_global(bool fix, bool multi, int parts) {
+  return fix && !multi && parts == kUnitParts;
+}
+
 static int redo_smem_bytes(const PairConfig& cfg, int cap_redo, int ne_max, int ext_max) {
   if (cfg.fix) return make_layout(true, cap_redo, ne_max, ext_max, cfg.warps, kRedoFull, cfg.multi).bytes;
   const int b = std::max(make_layout(false, cap_redo, ne_max, ext_max, cfg.warps, kRedoBig, cfg.multi).bytes,
@@ -204,7 +216,9 @@ static bool uses_wide(const PairConfig& c) { return c.wide && !c.fp64 && !c.list
 // counters, which the enumeration gives) the list pass's.
 static int main_smem_bytes(const PairConfig& cfg, int cap, int ne_max, int ext_max) {
   const int mode = (cfg.list && !cfg.count && !cfg.fp64) ? kList : kMain;
-  if (cfg.fix) return make_layout(false, cap, ne_max, ext_max, cfg.warps, kFixed, cfg.multi).bytes;
+  if (cfg.fix)
+    return make_layout(false, cap, ne_max, ext_max, cfg.warps, kFixed, cfg.multi,
+                       !own_in_global(true, cfg.multi, cfg.fine && !cfg.count ? kFineParts : kUnitParts)).bytes;
   if (uses_wide(cfg)) return make_layout(false, cap, ne_max, ext_max, kWideWarps, kMain, cfg.multi).bytes;
   return make_layout(cfg.fp64, cap, ne_max, ext_max, cfg.warps, mode, cfg.multi).bytes;
 }
@@ -596,7 +610,8 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   if (kFromList && MODE == kList && A.lcount[tile] < 0) return;  // a fallback tile: the redo pass computes it
   constexpr bool FIX = MODE == kFixed;
   const int cap = (MODE == kMain || MODE == kListBuild || MODE == kList || FIX) ? A.cap : A.cap_redo;
-  const Layout L = make_layout(FP64, cap, A.ne_max, A.ext_max, nw, MODE, MULTI);
+  constexpr bool kOwnGlobal = own_in_global(FIX, MULTI, kParts);
+  const Layout L = make_layout(FP64, cap, A.ne_max, A.ext_max, nw, MODE, MULTI, !kOwnGlobal);
   // shared-memory arrays (index-checked in the checked build)
   int* const st = A.status;  // the index checks' status word (checked build)
   (void)st;
@@ -611,6 +626,8 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   double* red = (double*)(smem + L.queue);  // scan and reduction scratch, before and after the queues' use
   int* cw = (int*)(smem + L.cw);
   OwnLut* sown = (OwnLut*)(smem + L.lut);
+  auto own_nrow = [&](int c) -> int { return kOwnGlobal ? __ldg(&g_own.nrow[c]) : sown->nrow[c]; };
+  auto own_ent = [&](int c, int k) -> unsigned { return kOwnGlobal ? __ldg(&g_own.ent[c][k]) : sown->ent[c][k]; };
   LJ32* ljs32 = (LJ32*)(smem + L.ljt);
   LJ64* ljs64 = (LJ64*)(smem + L.ljt);
   FixPair* ljx = (FixPair*)(smem + L.ljt);
@@ -621,7 +638,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   {
     const uint4* src = reinterpret_cast<const uint4*>(&g_own);
     uint4* dst = reinterpret_cast<uint4*>(sown);
-    if (!kFromList)
+    if (!kFromList && !kOwnGlobal)
       for (int k = tid; k < (int)(sizeof(OwnLut) / 16); k += blockDim.x) dst[k] = src[k];
     if (MULTI)
       for (int k = tid; k < A.lj.nt * A.lj.nt; k += blockDim.x) {
@@ -1308,7 +1325,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
       const int cia = code[va ? ia : 0] & 0x7fff;  // (bit 15: see `second`)
       const int ax = cia & 31, ay = (cia >> 5) & 31, az = cia >> 10;
       const int acls = pos_class(ax - 1, tx) * 25 + pos_class(ay - 1, ty) * 5 + pos_class(az - 1, tz);
-      const int aw = va ? (sown->nrow[acls] + kParts - 1 - part) / kParts : 0;
+      const int aw = va ? (own_nrow(acls) + kParts - 1 - part) / kParts : 0;
       const float4 pa = pf[va ? ia : 0];
       // squared x-gaps to the cells dx = -2, -1, +1, +2 (ox has EX + 1 entries)
       const float gm2 = fmaxf(pa.x - ox[max(ax - 1, 0)], 0.f), gm1 = fmaxf(pa.x - ox[ax], 0.f);
@@ -1346,7 +1363,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         const int s_q = sq & 511, i = sq >> 9;
         const int cls = (cc >> 15) & 127;
         const int lx = cc & 31, ly = (cc >> 5) & 31, lz = (cc >> 10) & 31;
-        const unsigned ent = valid ? sown->ent[cls][kParts * (k - s_q) + part] : 0u;
+        const unsigned ent = valid ? own_ent(cls, kParts * (k - s_q) + part) : 0u;
         int mask = ent & 31;
         int lo1 = 0, n1 = 0, lo2 = 0, n2 = 0;
         float cy = 0.f, cz = 0.f;
@@ -1427,7 +1444,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
       const int ex = ee % EX, er = ee / EX, ey = er % EY, ez = er / EY;
       const int ai0 = lstart[ee], ana = ve ? lstart[ee + 1] - ai0 : 0;
       const int acls = pos_class(ex - 1, tx) * 25 + pos_class(ey - 1, ty) * 5 + pos_class(ez - 1, tz);
-      const int aw = ana > 0 ? (sown->nrow[acls] + kCellParts - 1 - part) / kCellParts : 0;
+      const int aw = ana > 0 ? (own_nrow(acls) + kCellParts - 1 - part) / kCellParts : 0;
       int incl = aw;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -1454,7 +1471,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         const int geo = __shfl_sync(FULL, ageo, ql);
         const int qpa = __shfl_sync(FULL, apa, ql);
         const int lx = geo & 31, ly = (geo >> 5) & 31, lz = (geo >> 10) & 31, cls = geo >> 15;
-        const unsigned ent = valid ? sown->ent[cls][kCellParts * (k - s_q) + part] : 0u;
+        const unsigned ent = valid ? own_ent(cls, kCellParts * (k - s_q) + part) : 0u;
         const int mask = ent & 31;
         int lo1 = 0, n1 = 0, lo2 = 0, n2 = 0;
         bool self = false;
