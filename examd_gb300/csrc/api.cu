@@ -228,7 +228,11 @@ int split_axis(int nb, double last_width, int tile_len, int balance, int* starts
 // SM, 2 where even 3^3 gives less than one.  (Pair pass at 4 / 3 / 2, us: 1,000
 // atoms in 27 / 64 / 125 tiles 24.7 / 19.9 / 16.5; 8,788 in 125 / 216 / 729
 // 47 / 33 / 33; 32,000 in 343 / 729 / 2197 59.5 / 52.8 / 64; 87,808 in 1000 / 2197
-// 97 / 108.)  The mixed form keeps 4: its FP32 x coordinates are the tile's.
+// 97 / 108.)  Also 3 where a tile of 4^3 is too large for three CTAs on an SM
+// (about 860 atoms with the headroom; expected from the mean density, the wide
+// last cell and three standard deviations): 1M liquid, 4^3 / 3^3: rc 3.0 1451 /
+// 1182, rc 3.5 2009 / 1797, rc 4.0 4664 / 2971; below it, rc 2.75 904 / 1058, rc 2.5
+// 781 / 969.  The mixed form keeps 4: its FP32 x coordinates are the tile's.
 int default_tile(const examd_params& p, int nboxes, const examd_box* boxes, double bl, int sms) {
   if (p.precision != EXAMD_FP64) return 4;
   auto tiles = [&](int t) {
@@ -240,7 +244,16 @@ int default_tile(const examd_params& p, int nboxes, const examd_box* boxes, doub
     }
     return n;
   };
-  return tiles(4) >= 4.0 * sms ? 4 : tiles(3) >= sms ? 3 : 2;
+  if (tiles(4) < 4.0 * sms) return tiles(3) >= sms ? 3 : 2;
+  for (int b = 0; b < nboxes; ++b) {
+    double atoms = (double)boxes[b].natoms;  // staged by the largest tile
+    for (int a = 0; a < 3; ++a) {
+      const double cells = boxes[b].L[a] / bl;
+      atoms *= std::min(1.0, (4 + 2 + (cells - std::floor(cells))) / cells);
+    }
+    if ((atoms + 3.0 * std::sqrt(atoms)) * 1.0625 + 32.0 > 860.0) return 3;
+  }
+  return 4;
 }
 
 }  // namespace

@@ -158,6 +158,22 @@ def test_fp64_default_tiles(gpulib, m):
         assert cg["accepted"] == c["accepted"] and cg["candidates"] == c["candidates"]
 
 
+@pytest.mark.parametrize("rc,tile", [(2.5, 4), (3.0, 3)])
+def test_fp64_default_tiles_by_their_atoms(gpulib, rc, tile):
+    """A box with tiles of 4 cells enough for the chip at either cutoff: at rc 3 they are too large for three CTAs."""
+    n = 4 * 30 ** 3
+    pos, L = crystal(gpulib, n)
+    out = []
+    for kw in ({}, dict(tile=(tile,) * 3), dict(tile=(7 - tile,) * 3)):
+        with gpulib.MidpointLJ(L, [n], precision="fp64", rc=rc, **kw) as s:
+            s.set_atoms(pos)
+            out.append((s.forces()[0], s.counters()))
+    assert out[0][1]["tiles"] == out[1][1]["tiles"] != out[2][1]["tiles"]
+    for f, c in out[1:]:
+        assert np.sqrt(((f - out[0][0]) ** 2).sum(1)).max() <= TOL64 * frms(out[0][0])
+        assert c["accepted"] == out[0][1]["accepted"]
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("m", [4, 14, 20, 24])
 def test_warps_give_the_same_forces(gpulib, precision, m):
