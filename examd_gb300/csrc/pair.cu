@@ -196,8 +196,9 @@ __host__ __device__ inline Layout make_layout(bool fp64, int cap, int ne_max, in
 // of 3.4 KB in each CTA: a tile of 66 bytes an atom is near the size at which
 // an SM holds three CTAs instead of four (568 atoms at 8 warps with the copy, 616
 // without, at 4^3 cells; 1M liquid, 616: 885 -> 788 us a pass).  In few waves there is no
-// fourth CTA to gain and the copy is nearer (1,000 atoms 9.5 against 10 us); with
-// several types the registers allow three.
+// fourth CTA to gain and the copy is nearer (1,000 atoms 9.5 against 10 us; a
+// 512-box ensemble, many waves at four CTAs either way, loses 1 %); with several
+// types the registers allow three.
 __host__ __device__ constexpr bool own_in_global(bool fix, bool multi, int parts) {
   return fix && !multi && parts == kUnitParts;
 }
