@@ -153,39 +153,43 @@ long long fixed_of(double x, int ue) {
 
 // The tables of the FP64 form's fixed-point pass (pair.cu, force_batch_fix), or
 // false where the parameters do not suit it and the FP64 body computes every
-// tile: type pairs whose force scales eps / sigma differ by more than 16 (the
-// sums have one unit, and the weakest pair's forces keep 2^-47 of its scale), a
-// cutoff inside the range of the forces too large for the sums, or lengths and
-// energies whose powers leave FP64's range.
+// tile: pairs whose force at their cutoff falls below 2^-11 of the largest force
+// scale eps / sigma (the sums' one unit would hold it to fewer bits than FP64
+// does), a cutoff inside the range of the forces too large for the sums, or
+// lengths and energies whose powers leave FP64's range.
 bool build_fix(const LJTable& lj, const examd_params& p, FixTable& fx) {
   const int n2 = lj.nt * lj.nt;
-  double rmax = 0.0, f0max = 0.0, f0min = INFINITY;
+  double rmax = 0.0, f0max = 0.0, fweak = INFINITY;  // fweak: the weakest pair's force at its cutoff (by its terms' size)
   for (int k = 0; k < n2; ++k) {
     rmax = std::max(rmax, p.rc[k]);
     f0max = std::max(f0max, p.eps[k] / p.sigma[k]);
-    f0min = std::min(f0min, p.eps[k] / p.sigma[k]);
+    const double s6 = std::pow(p.sigma[k] / p.rc[k], 6.0);
+    fweak = std::min(fweak, 24.0 * p.eps[k] * (s6 + 2.0 * s6 * s6) / p.rc[k]);
   }
-  if (!(f0min * 16.0 >= f0max) || !std::isnormal(f0max)) return false;
+  if (!std::isnormal(f0max)) return false;
   int f0 = std::ilogb(f0max);  // F0 = 2^f0
   if (std::ldexp(1.0, f0) < f0max) ++f0;
   fx.ue = std::ilogb(rmax) + 1 - 62;  // every separation within the cutoff is below 2^62 units
-  fx.sf = kFixSumBits - f0;
-  const double fbig = std::ldexp(1.0, kFixTermBits + f0), fmed = std::ldexp(1.0, kFixMedBits + f0);
+  const FixUnit* unit = nullptr;
+  for (const FixUnit& u : kFixUnits)
+    if (!unit && fweak >= std::ldexp(1.0, f0 - u.weak)) unit = &u;
+  if (!unit) return false;
+  fx.sf = unit->bits - f0;
+  fx.coarse = unit->coarse;
+  fx.atoms = unit->atoms;
+  const double fbig = std::ldexp(1.0, kFixTermBits + f0);
   const int w = 2 * fx.ue + 64;  // r^2 = D 2^w
-  double r2big[EXAMD_MAX_TYPES * EXAMD_MAX_TYPES], r2med[EXAMD_MAX_TYPES * EXAMD_MAX_TYPES];
-  double gmax = 0.0, gbig = 0.0;
+  double r2big[EXAMD_MAX_TYPES * EXAMD_MAX_TYPES];
+  double gmax = 0.0;
   for (int k = 0; k < n2; ++k) {
     r2big[k] = std::max(r2_of_force(p.eps[k], p.sigma[k], fbig), 1.001e-12);  // coincident atoms (kR2Min64) as well
-    r2med[k] = std::max(r2_of_force(p.eps[k], p.sigma[k], fmed), r2big[k]);
-    gmax = std::max(gmax, fmed / std::sqrt(r2med[k]));
-    gbig = std::max(gbig, fbig / std::sqrt(r2big[k]));
+    gmax = std::max(gmax, fbig / std::sqrt(r2big[k]));
   }
-  if (!std::isnormal(gmax) || !(std::ldexp(gbig, -kFixMedShift) < gmax)) return false;
+  if (!std::isnormal(gmax)) return false;
   const int sg = 61 - std::ilogb(gmax);  // |dg| 2^sg < 2^62
-  const int K = sg - fx.ue - fx.sf;
-  if (K < 33 || K > 63) return false;
-  fx.ka = 64 - K;
-  fx.kb = K - 32;
+  fx.k0 = sg - fx.ue - fx.sf;
+  // (the coarse word is formed from the product's top word: a step is at least 2^4 of its units)
+  if (fx.k0 + fx.coarse - 96 < 4 || fx.k0 > 63) return false;
   for (int k = 0; k < n2; ++k) {
     FixPair& q = fx.p[k];
     const long double s2 = (long double)lj.p64[k].sig2, s6 = s2 * s2 * s2, e = (long double)p.eps[k];
@@ -194,12 +198,11 @@ bool build_fix(const LJTable& lj, const examd_params& p, FixTable& fx) {
     q.s6 = (double)std::ldexp(s6, -3 * w);
     q.e4 = lj.p64[k].eps4;
     q.eshift = lj.p64[k].eshift;
-    const double lim = std::ldexp(lj.p64[k].rcut2, -w), big = std::ldexp(r2big[k], -w), med = std::ldexp(r2med[k], -w);
+    const double lim = std::ldexp(lj.p64[k].rcut2, -w), big = std::ldexp(r2big[k], -w);
     if (!std::isnormal(q.c6) || !std::isnormal(q.c12) || !std::isnormal(q.s6) || !(big >= 0x1p36) ||
-        !(lim >= 0x1p44) || !(lim < 0x1p61) || !(med < lim))
+        !(lim >= 0x1p44) || !(lim < 0x1p61) || !(big < lim))
       return false;
     q.limh = (int)((long long)lim >> 32);
-    q.medh = (int)((long long)med >> 32) + 1;
     q.bigh = (int)((long long)big >> 32) + 1;
     q.pre = lj.p32[k].rc2 * 1.0001f;
   }
@@ -226,13 +229,13 @@ int split_axis(int nb, double last_width, int tile_len, int balance, int* starts
 // The FP64 form, whose tiles take longer and whose results do not depend on
 // them, takes smaller ones where 4^3 would leave SMs idle: 3 below four tiles an
 // SM, 2 where even 3^3 gives less than one.  (Pair pass at 4 / 3 / 2, us: 1,000
-// atoms in 27 / 64 / 125 tiles 24.7 / 19.9 / 16.5; 8,788 in 125 / 216 / 729
-// 47 / 33 / 33; 32,000 in 343 / 729 / 2197 59.5 / 52.8 / 64; 87,808 in 1000 / 2197
-// 97 / 108.)  Also 3 where a tile of 4^3 is too large for three CTAs on an SM
-// (about 860 atoms with the headroom; expected from the mean density, the wide
-// last cell and three standard deviations): 1M liquid, 4^3 / 3^3: rc 3.0 1451 /
-// 1182, rc 3.5 2009 / 1797, rc 4.0 4664 / 2971; below it, rc 2.75 904 / 1058, rc 2.5
-// 781 / 969.  The mixed form keeps 4: its FP32 x coordinates are the tile's.
+// atoms in 8 / 27 / 64 tiles 44.8 / 27.1 / 17.1; 8,788 in 125 / 216 / 512
+// 46 / 35 / 31; 32,000 in 343 / 729 / 2197 63 / 47 / 56; 87,808 in 1000 / 2197
+// 100 / 98.)  Also 3 where a tile of 4^3 is too large for three CTAs on an SM
+// (about 820 atoms with the headroom; expected from the mean density, the wide
+// last cell and three standard deviations): 1M liquid, 4^3 / 3^3: rc 3.0 1561 /
+// 1309, 500k at rc 3.0 764 / 639; below it, rc 2.75 1000 / 1151, rc 2.5 844 / 1027.
+// The mixed form keeps 4: its FP32 x coordinates are the tile's.
 int default_tile(const examd_params& p, int nboxes, const examd_box* boxes, double bl, int sms) {
   if (p.precision != EXAMD_FP64) return 4;
   auto tiles = [&](int t) {
@@ -251,7 +254,7 @@ int default_tile(const examd_params& p, int nboxes, const examd_box* boxes, doub
       const double cells = boxes[b].L[a] / bl;
       atoms *= std::min(1.0, (4 + 2 + (cells - std::floor(cells))) / cells);
     }
-    if ((atoms + 3.0 * std::sqrt(atoms)) * 1.0625 + 32.0 > 860.0) return 3;
+    if ((atoms + 3.0 * std::sqrt(atoms)) * 1.0625 + 32.0 > 820.0) return 3;
   }
   return 4;
 }
@@ -290,7 +293,7 @@ struct examd_ctx {
   LJTable lj{};
   FixTable fx{};
   PairConfig pc;
-  int cap = 0, smem = 0, smem_limit = 0;
+  int cap = 0, smem = 0, smem_limit = 0, sm_smem = 0;
   int cap_redo = 0;     // staged-atom capacity of the redo pass
   int dev = 0;
   cudaStream_t st = nullptr;
@@ -599,6 +602,7 @@ int examd_gpu_create(const examd_params* params, int nboxes, const examd_box* bo
   ctx->bl = bl;
   ctx->dev = p.device;
   ctx->smem_limit = (int)prop.sharedMemPerBlockOptin;
+  ctx->sm_smem = (int)prop.sharedMemPerMultiprocessor;
   cudaSetDevice(ctx->dev);
 
   // pair-kernel configuration
@@ -1093,13 +1097,20 @@ int apply_capacity(examd_ctx* ctx, bool* grew = nullptr) {
   const int occ = ctx->h_status[1];
   int want_r = std::max(((occ + occ / 4 + 64) + 7) & ~7, ctx->cap_redo);
   int want = ctx->pc.fp64 && !ctx->pc.fix ? want_r : ((occ + occ / 16 + 32) + 7) & ~7;
+  // The fixed-point pass (78 bytes an atom) with half the headroom where the whole of it costs a CTA per SM (1M
+  // liquid 949 -> 844 us a pass, 500k at rc 3.0 719 -> 639)
+  if (ctx->pc.fix) {
+    const int least = ((occ + occ / 32 + 16) + 7) & ~7;
+    const int n = pair_ctas(ctx->pc, least, ctx->ne_max, ctx->ext_max, ctx->sm_smem);
+    while (want > least && pair_ctas(ctx->pc, want, ctx->ne_max, ctx->ext_max, ctx->sm_smem) < n) want -= 8;
+  }
   if (want <= ctx->cap) return EXAMD_OK;
   int bytes = 0;
   auto fits = [&] {
     bytes = pair_smem_bytes(ctx->pc, want, want_r, ctx->ne_max, ctx->ext_max);
-    return bytes <= ctx->smem_limit;
+    return bytes <= ctx->smem_limit && (!ctx->pc.fix || want <= ctx->fx.atoms);
   };
-  bool ok = fits();  // (the redo pass binds: the 12-warp CTAs' tables never do)
+  bool ok = fits();  // (the redo pass binds, or the fixed-point pass: the 12-warp CTAs' tables never do)
   if (!ok) {  // the exact need if the headroom does not fit
     want = want_r = (occ + 7) & ~7;
     ok = fits();

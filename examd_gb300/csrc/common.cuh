@@ -119,14 +119,22 @@ struct LJ32 {
 // component of a kept term is below 2^28 in fixed point, so a component's
 // int32 sum needs more than 8 near-maximal terms of one sign to overflow.
 constexpr float kFixMaxForce = 2048.f;
-// FP64 form's fixed-point pass: the force sums' unit is 2^-51 of the power of
-// two F0 at or above the largest eps / sigma.  A term below 2^9 F0 (r > 0.83
-// sigma) may be added any number of times: a sum overflows 64 bits only by more
-// than 8 near-maximal ones of one sign (as above).  A term of 2^9 to 2^11 F0
-// takes up to four of those eight, so an atom may have one of them (a second one
-// sends the tile to the FP64 body); a term above 2^11 F0 always does.
-constexpr int kFixSumBits = 51, kFixMedBits = 9, kFixTermBits = 11;
-constexpr int kFixMedShift = 3;  // the larger terms' factor, taken that much coarser to fit its 63 bits
+// FP64 form's fixed-point pass.  Terms below 2^kFixTermBits F0 (r > 0.74 sigma) are
+// kept, F0 the power of two at or above the largest eps / sigma; a larger one
+// sends the tile to the FP64 body.  A component's sum is held modulo 2^64 in two
+// words and once more in a third, in coarse steps, which says which multiple of
+// 2^64 it is: the third word's rounding (0.6 of a step per term at most) leaves the
+// sum known to 2^63, and its 31 bits hold every term of a tile's most atoms, so
+// that no number of terms on one atom can overflow a sum.  The unit is as fine as
+// the weakest pair needs to keep FP64's relative accuracy, alone at its cutoff:
+// unit bits below F0, the weakest force (bits below F0) that it serves, the step's
+// bits above the unit, most atoms.
+struct FixUnit {
+  int bits, weak, coarse, atoms;
+};
+constexpr int kFixTermBits = 11;
+constexpr FixUnit kFixUnits[2] = {{60, 9, 52, 3400},   // one type: rc <= 3.8 sigma
+                                  {62, 11, 53, 1700}}; // 4.6 sigma
 struct LJ64 {
   double sig2, eps24, eps4, rc2;   // as user_func.f90:58-59 computes them
   double rcut2, eshift;
@@ -139,14 +147,14 @@ struct FixPair {
   double c6, c12;
   double e4, s6;    // energy: 4 eps, and sigma^6 in units of D^3
   double eshift;
-  int limh;         // high words of D at the range (rc or the potential's own),
-  int medh, bigh;   // at forces of 2^kFixMedBits and of 2^kFixTermBits F0
+  int limh, bigh;   // high words of D at the range (rc or the potential's own) and at forces of 2^tb F0
   float pre;        // FP32 prefilter of the candidates: rc^2 widened
 };
 
 struct FixTable {
   int ue;           // the positions' unit is 2^ue
-  int ka, kb;       // a force term's 128-bit product is taken at bit 64 - ka = 32 + kb
+  int k0;           // a term's 128-bit product is taken at bit k0 where the factor is largest
+  int coarse, atoms;  // of FixUnit
   int sf;           // the force sums' unit is 2^-sf
   FixPair p[EXAMD_MAX_TYPES * EXAMD_MAX_TYPES];
 };

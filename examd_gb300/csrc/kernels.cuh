@@ -154,6 +154,8 @@ struct PairConfig {
 // Dynamic shared memory for the tile capacities: the larger of the first
 // pass's need at cap and, where there is one, the redo pass's at cap_redo.
 int pair_smem_bytes(const PairConfig& cfg, int cap, int cap_redo, int ne_max, int ext_max);
+// CTAs of the fixed-point pass that an SM's sm_smem bytes of shared memory and its registers hold.
+int pair_ctas(const PairConfig& cfg, int cap, int ne_max, int ext_max, int sm_smem);
 cudaError_t pair_prepare(const PairConfig& cfg, int smem_bytes);  // opt-in smem attribute
 cudaError_t launch_pair(const PairConfig& cfg, const PairArgs& a, int ntiles, int smem_bytes, cudaStream_t st);
 // Pair-list mode: build the per-tile lists (gated by a.gate).

@@ -43,8 +43,9 @@
 // launch (k_pair_redo) recomputes the flagged tiles, sums their large terms
 // in FP32 and adds them to the outputs; thermal configurations flag no tile
 // and the launch returns at once (only the rare FP32 sums' order can vary
-// between runs).  FP64 form: 64-bit integer sums in the first pass, FP64
-// shared-memory atomics in the FP64 body.
+// between runs).  FP64 form: integer sums that no number of terms overflows in
+// the first pass (common.cuh, FixUnit), FP64 shared-memory atomics in the FP64
+// body.
 //
 // Output: forces of the tile's home atoms go to Fown, those of halo copies to
 // the partial slot P[s] (s = bitmask of the axes on which the copy is a halo
@@ -108,6 +109,7 @@ constexpr int kRedoBlocks = 152;       // grid of the redo pass (1 per SM)
 constexpr int kMain = 0, kRedoBig = 1, kRedoFull = 2, kListBuild = 3, kList = 4, kListBig = 5, kFixed = 6;
 constexpr int kFullBit = 1 << 30;      // redo-list entry: tile | kFullBit for an overflowed tile
 constexpr int kSeg = 4;                // lanes per segment of the i-side force sums
+constexpr int kSegFix = 2;             // the same, kFixed (a shuffle of nine words per doubling)
 constexpr int kMaxListK = 1024;        // pair-list mode: most list entries of one atom
 // Mixed form: a pair whose FP32 r^2 lies within this fraction of rc^2 (a few
 // times the FP32 separation's rounding) is accepted or not on its FP64 r^2,
@@ -126,8 +128,11 @@ struct Layout {
 
 // Per-warp tables after the accepted-pair queues.  Mixed form and kFixed: one
 // step's items by rank (pt, float4) and the work unit's atoms by rank (bt, two
-// float4).  FP64 form: one step's items by lane (float4).
+// float4; kFixed: one, the positions are read again from the staged atoms, which
+// makes room for the coarse words of 340 atoms).  FP64 form: one step's items by
+// lane (float4).
 constexpr int kWarpTab = 32 * 16 + 32 * 32;
+constexpr int kWarpTabFix = 32 * 16 + 32 * 16;
 constexpr int kWarpTabFp64 = 32 * 16;
 
 __host__ __device__ inline int align16(int x) { return (x + 15) & ~15; }
@@ -161,11 +166,12 @@ __host__ __device__ inline Layout make_layout(bool fp64, int cap, int ne_max, in
   // would serialise on the kernel-parameter bank, shared memory serves them at once
   L.ljt = o;    o = align16(o + (multi ? (fix ? (int)sizeof(FixPair) : (int)sizeof(LJ64)) * EXAMD_MAX_TYPES * EXAMD_MAX_TYPES : 0));
   const int qbytes = (fp64 ? 4 * kQueue + kWarpTabFp64
-                           : (from_list ? 64 : (mode == kListBuild ? 0 : fix ? 4 : 16) * kQueue + kWarpTab)) * nw;
+                           : (from_list ? 64 : fix ? 4 * kQueue + kWarpTabFix : (mode == kListBuild ? 0 : 16) * kQueue + kWarpTab)) *
+                     nw;
   L.queue = o;  o = align16(o + qbytes);
   L.pf = o;     o = align16(o + 16 * (from_list ? cap + 1 : cap));  // list passes: + the padding atom
   if (fp64 || fix) {
-    L.fa = o;   o = align16(o + 3 * 8 * cap);  // FP64 force sums (kFixed: low words, then high words)
+    L.fa = o;   o = align16(o + 3 * (fix ? 12 : 8) * cap);  // FP64 force sums (kFixed: low, high and coarse words)
     L.px = o;   o = align16(o + 3 * 8 * cap);  // FP64 (kFixed: fixed-point) positions
   } else {
     L.fa = o;   o = align16(o + (mode == kListBuild ? 1 : 3) * 4 * cap);  // fixed-point force sums, x y z per atom (build: counts)
@@ -193,9 +199,9 @@ __host__ __device__ inline Layout make_layout(bool fp64, int cap, int ne_max, in
 
 // The FP64 form's first pass with one type, in grids of many waves, reads the
 // ownership table from global memory (its lines stay in L1) instead of a copy
-// of 3.4 KB in each CTA: a tile of 66 bytes an atom is near the size at which
-// an SM holds three CTAs instead of four (568 atoms at 8 warps with the copy, 616
-// without, at 4^3 cells; 1M liquid, 616: 885 -> 788 us a pass).  In few waves there is no
+// of 3.4 KB in each CTA: a tile of 78 bytes an atom is near the size at which
+// an SM holds three CTAs instead of four (528 atoms at 8 warps with the copy, 572
+// without, at 4^3 cells; 1M liquid, 951 -> 846 us a pass; 256k 249 -> 220).  In few waves there is no
 // fourth CTA to gain and the copy is nearer (1,000 atoms 9.5 against 10 us; a
 // 512-box ensemble, many waves at four CTAs either way, loses 1 %); with several
 // types the registers allow three.
@@ -236,6 +242,12 @@ int pair_smem_bytes(const PairConfig& cfg, int cap, int cap_redo, int ne_max, in
   if (cfg.list) b = std::max(b, std::max(main_smem_bytes(cfg, cap, ne_max, ext_max),
                                          build_smem_bytes(cfg, cap, ne_max, ext_max)));
   return b;
+}
+
+int pair_ctas(const PairConfig& cfg, int cap, int ne_max, int ext_max, int sm_smem) {
+  constexpr int kReserved = 1024;  // of every CTA, by the system
+  const int regs = 32 * cfg.warps * (cfg.multi ? 80 : 64);
+  return std::min(sm_smem / (main_smem_bytes(cfg, cap, ne_max, ext_max) + kReserved), 65536 / regs);
 }
 
 // Exact sum of FP32 terms in 64-bit fixed point (2^-32 resolution): the total
@@ -442,13 +454,17 @@ __device__ __forceinline__ void force_batch64(int cnt, const QK& qk, const PD& p
 // - D becomes a double (one rounding), y = 1/D from an FP32 estimate (relative
 //   error e of 2^-22) by one step of Householder's third-order iteration,
 //   y (1 + e + e^2), error e^3: three operations;
-// - the LJ force per unit distance is y^4 (c6 - c12 y^3), five operations;
-//   as an integer it multiplies the separation in 32-bit pieces, rounded at
-//   bit 2^-sf of the sum's unit;
-// - the sums are 64-bit integers in shared memory (low word with carry into
-//   the high word): exact, in any order, with native 32-bit atomics.
-// Every step keeps at least FP64's bits, and the forces do not depend on the
-// order.  Where the reference itself rounds coarsely, its rounding is kept: a
+// - the LJ force per unit distance is y^4 (c6 - c12 y^3), five operations; its
+//   53 bits, as an integer, multiply the separation in 32-bit pieces, and the
+//   product is taken at the bit that the factor's exponent gives, rounded at the
+//   sums' unit 2^-sf (common.cuh, FixUnit);
+// - the sums are integers in shared memory with native 32-bit atomics: two words
+//   modulo 2^64 (the low one with carry into the high one) and a coarse one:
+//   exact, in any order, whatever the number of terms.
+// An isolated pair's force is then off by less than the FP64 body's, RMS (1e-16:
+// r 0.9-1.1 sigma 9.1 against 11.5; 2.0-2.5 2.9 / 3.6; at rc 3.8 3.5 / 3.6; a pair of
+// a sixteenth of the strongest eps 3.1 / 3.6), and the forces do not depend on
+// the order.  Where the reference itself rounds coarsely, its rounding is kept: a
 // pair across the periodic face is first subtracted at box scale (x_j - x_i,
 // rounded to 53 bits of about L, then L added exactly), which moves its
 // separation by up to ulp(L) / 2; `face` gives that rounded separation.
@@ -456,15 +472,16 @@ __device__ __forceinline__ void force_batch64(int cnt, const QK& qk, const PD& p
 // the FP64 body's own r^2 (in64), so that both accept the same pairs; a pair
 // whose force is too large for the sums' range flags the tile, and the FP64
 // body redoes it.
-template <bool MULTI, bool ENERGY, bool COUNT, class QK, class PX, class FA, class FACE, class IN64, class SECOND>
+template <bool MULTI, bool ENERGY, bool COUNT, class QK, class PX, class FA, class FACE, class IN64>
 __device__ __forceinline__ void force_batch_fix(int cnt, int q0, const QK& qk, const PX& px, FA& fa, int cap,
                                                 const PairArgs& A, const FixPair* ljx, double& s12, double& s6s,
                                                 double& shift, int& nacc, int* big_flag, bool edge, const FACE& face,
-                                                const IN64& in64, const SECOND& second) {
+                                                const IN64& in64) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   int i = -1, m = 0;
-  long long fx = 0, fy = 0, fz = 0;  // the force on i, in units of 2^-sf
+  long long fx = 0, fy = 0, fz = 0;  // the force on i, in units of 2^-sf modulo 2^64,
+  int cx = 0, cy = 0, cz = 0;        // and in coarse steps
   bool app = false;
   if (lane < cnt) {
     const unsigned key = (unsigned)qk[q0 + lane];
@@ -485,11 +502,9 @@ __device__ __forceinline__ void force_batch_fix(int cnt, int q0, const QK& qk, c
     const int Dh = (int)(D >> 32);
     app = Dh < P.limh;
     if (abs(Dh - P.limh) <= 1) app = in64(i, m, ti, tj);
-    int up = 0;
-    if (app && Dh < P.medh) {  // rare
-      up = kFixMedShift;
-      app = Dh >= P.bigh;
-      if (!app || second(i, m)) *big_flag = 1;
+    if (app && Dh < P.bigh) {
+      app = false;
+      *big_flag = 1;
     }
     if (app) {
       // D as a double: normalised so that its first bit is bit 62, 53 bits kept
@@ -513,18 +528,22 @@ __device__ __forceinline__ void force_batch_fix(int cnt, int q0, const QK& qk, c
         if (A.lj.pot != EXAMD_POT_LJ) shift += P.eshift;
       }
       if (COUNT) ++nacc;
-      // g as a 63-bit integer (|g| < 2^62, a large one in units of 2^up), then G d / 2^(64 - ka), rounded
+      // g = G 2^(e - 1084) with its 53 bits at the top of 62 (|g| < 2^62), then G d / 2^K, rounded; where
+      // K would pass 63, G gives up its last bits (the first nine are zeros)
       const int gb = __double2hiint(g);
       const unsigned long long gm =
-          ((((unsigned long long)(unsigned)((gb & 0xfffff) | 0x100000)) << 32) | (unsigned)__double2loint(g)) << 10;
-      const int gs = min(1085 + up - ((gb >> 20) & 0x7ff), 63);
-      long long G = (long long)(gm >> gs);
+          ((((unsigned long long)(unsigned)((gb & 0xfffff) | 0x100000)) << 32) | (unsigned)__double2loint(g)) << 9;
+      const int Kg = A.fx.k0 + 1084 - ((gb >> 20) & 0x7ff), K = min(Kg, 63);
+      long long G = (long long)(gm >> min(Kg - K, 63));
       if (gb < 0) G = -G;
       const int gh = (int)((G + 0x80000000ll) >> 32), gl = (int)G;
-      const int ka = A.fx.ka, kb = A.fx.kb;
+      const int ka = 64 - K, kb = K - 32;
       const int half = 1 << (kb - 1);
-      auto term = [&](int h, int l) {
+      // (the coarse part from the product's top 32 bits, a step of which is 2^kc, 16 or more)
+      const int kc = K + A.fx.coarse - 96, halfc = 1 << (kc - 1);
+      auto term = [&](int h, int l, int& c) {
         const long long hi = (long long)gh * h;
+        c = ((int)(hi >> 32) + halfc) >> kc;
         const long long mid = (long long)gh * l + ((long long)gl * h + ((long long)__mulhi(gl, l) + half));
         const unsigned h0 = (unsigned)hi, h1 = (unsigned)((unsigned long long)hi >> 32);
         const unsigned m0 = (unsigned)mid, m1 = (unsigned)((unsigned long long)mid >> 32);
@@ -533,46 +552,46 @@ __device__ __forceinline__ void force_batch_fix(int cnt, int q0, const QK& qk, c
             ((unsigned long long)(unsigned)((int)m1 >> kb) << 32) | __funnelshift_r(m0, m1, kb);
         return (long long)(a + b);
       };
-      fx = term(hx, lx);
-      fy = term(hy, ly);
-      fz = term(hz, lz);
-      if (up) {
-        fx <<= up;
-        fy <<= up;
-        fz <<= up;
-      }
+      fx = term(hx, lx, cx);
+      fy = term(hy, ly, cy);
+      fz = term(hz, lz, cz);
     }
   }
-  // v to the 64-bit sum of component c of atom t: low word, carry, high word
-  auto add = [&](int t, int c, long long v) {
+  // v and its coarse part vc to the sum of component c of atom t: low word, carry, high word; coarse word
+  auto add = [&](int t, int c, long long v, int vc) {
     const unsigned lo = (unsigned)v;
     const unsigned old = atomicAdd((unsigned*)&fa[c * cap + t], lo);
+    atomicAdd(&fa[(6 + c) * cap + t], vc);
     atomicAdd(&fa[(3 + c) * cap + t], (int)(v >> 32) + (old + lo < lo ? 1 : 0));
   };
   if (app) {
-    add(m, 0, -fx);
-    add(m, 1, -fy);
-    add(m, 2, -fz);
+    add(m, 0, -fx, -cx);
+    add(m, 1, -fy, -cy);
+    add(m, 2, -fz, -cz);
   }
-  // i side: runs of equal i in segments of kSeg lanes, as in pair_force32
+  // i side: runs of equal i in segments of kSegFix lanes, as in pair_force32
   const int ip = __shfl_up_sync(FULL, i, 1);
   const unsigned hb = __ballot_sync(FULL, lane == 0 || ip != i);
-  const int dist = (lane - (31 - __clz(hb & (FULL >> (31 - lane))))) & (kSeg - 1);
+  const int dist = (lane - (31 - __clz(hb & (FULL >> (31 - lane))))) & (kSegFix - 1);
 #pragma unroll
-  for (int o = 1; o < kSeg; o <<= 1) {
+  for (int o = 1; o < kSegFix; o <<= 1) {
     const long long yx = __shfl_up_sync(FULL, fx, o), yy = __shfl_up_sync(FULL, fy, o),
                     yz = __shfl_up_sync(FULL, fz, o);
+    const int zx = __shfl_up_sync(FULL, cx, o), zy = __shfl_up_sync(FULL, cy, o), zz = __shfl_up_sync(FULL, cz, o);
     if (o <= dist) {
       fx += yx;
       fy += yy;
       fz += yz;
+      cx += zx;
+      cy += zy;
+      cz += zz;
     }
   }
-  const bool tail = lane == 31 || dist == kSeg - 1 || ((hb >> (lane + 1)) & 1u);
-  if (i >= 0 && tail && (fx | fy | fz) != 0) {
-    add(i, 0, fx);
-    add(i, 1, fy);
-    add(i, 2, fz);
+  const bool tail = lane == 31 || dist == kSegFix - 1 || ((hb >> (lane + 1)) & 1u);
+  if (i >= 0 && tail) {
+    add(i, 0, fx, cx);
+    add(i, 1, fy, cy);
+    add(i, 2, fz, cz);
   }
 }
 
@@ -789,7 +808,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   // time.  (One thread per ext cell, the cell's atoms one after the other, waited
   // for a read per atom: a third of the lanes idle and 188 us of the FP64 form's
   // 950 us on a 1M-atom liquid went into staging and write-back.)
-  auto fa = EXAMD_ARR(int, smem + L.fa, (MODE == kListBuild ? 1 : FIX ? 6 : 3) * cap, st);
+  auto fa = EXAMD_ARR(int, smem + L.fa, (MODE == kListBuild ? 1 : FIX ? 9 : 3) * cap, st);
   auto fr = EXAMD_ARR(float, smem + L.fr, 3 * cap, st);  // redo pass: FP32 sums of the large terms
   auto fd = EXAMD_ARR(double, smem + L.fa, 3 * cap, st);
   auto pd = EXAMD_ARR(double, smem + L.px, 3 * cap, st);
@@ -840,7 +859,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
           px[cap + t] = to_fixed(xx[k][1], A.fx.ue) + (unsigned long long)(img[32 + ly] * B.Lq[1]);
           px[2 * cap + t] = to_fixed(xx[k][2], A.fx.ue) + (unsigned long long)(img[64 + lz] * B.Lq[2]);
 #pragma unroll
-          for (int c = 0; c < 6; ++c) fa[c * cap + t] = 0;
+          for (int c = 0; c < 9; ++c) fa[c * cap + t] = 0;
         }
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -876,10 +895,10 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   auto qk = EXAMD_ARR(int, (int*)(smem + L.queue) + warp * kQueue, kQueue, st);
   // per-warp tables: one step's items (pt) and, but for the FP64 form, the
   // work unit's atoms (bt)
-  unsigned char* wtab = smem + L.queue + kQe * kQueue * nw + warp * (FP64 ? kWarpTabFp64 : kWarpTab);
+  unsigned char* wtab = smem + L.queue + kQe * kQueue * nw + warp * (FP64 ? kWarpTabFp64 : FIX ? kWarpTabFix : kWarpTab);
   auto pt = EXAMD_ARR(float4, wtab, 32, st);
   auto btA = EXAMD_ARR(float4, wtab + 32 * 16, 32, st);
-  auto btB = EXAMD_ARR(float4, wtab + 32 * 32, 32, st);
+  auto btB = EXAMD_ARR(float4, wtab + (FIX ? 32 * 16 : 32 * 32), 32, st);
   int qn = 0;  // queued pairs
   const unsigned lt = (1u << lane) - 1u;
   const unsigned le = FULL >> (31 - lane);
@@ -942,16 +961,6 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
     round_axis(1, (ci >> 5) & 31, (cm >> 5) & 31, dy);
     round_axis(2, (ci >> 10) & 31, (cm >> 10) & 31, dz);
   };
-  // kFixed: whether either atom already has a term above 2^kFixMedBits F0 (bit 15
-  // of its code), and marks both
-  auto second = [&](int i, int m) {
-    auto mark = [&](int t) {
-      const unsigned bit = 0x8000u << (16 * (t & 1));
-      return (atomicOr((unsigned*)(smem + L.code) + (t >> 1), bit) & bit) != 0u;
-    };
-    const bool a = mark(i), b = mark(m);
-    return a || b;
-  };
   auto enqueue = [&](bool acc, const float4& dq, int key) {
     const unsigned bal = __ballot_sync(FULL, acc);
     if (acc) {
@@ -970,7 +979,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
                                             nacc, qn);
       else if (FIX)
         force_batch_fix<MULTI, ENERGY, COUNT>(32, qn, qk, px, fa, cap, A, ljx, esum, wsum, shsum, nacc, big_flag,
-                                              edge, face, inside64, second);
+                                              edge, face, inside64);
       else
         force_batch<MULTI, ENERGY, COUNT, MODE == kRedoFull>(32, qn, qd, fa, fr, cap, A, ljs32, ek, wk, nacc,
                                                              big_flag, inside64);
@@ -1323,7 +1332,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
       // per-atom quantities of lane l's atom c*32 + l
       const int ia = c * 32 + lane;
       const bool va = ia < total;
-      const int cia = code[va ? ia : 0] & 0x7fff;  // (bit 15: see `second`)
+      const int cia = code[va ? ia : 0];
       const int ax = cia & 31, ay = (cia >> 5) & 31, az = cia >> 10;
       const int acls = pos_class(ax - 1, tx) * 25 + pos_class(ay - 1, ty) * 5 + pos_class(az - 1, tz);
       const int aw = va ? (own_nrow(acls) + kParts - 1 - part) / kParts : 0;
@@ -1346,8 +1355,9 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         // the gaps as FP16 rounded toward zero: they prune no more than they may
         const __half2 hm = __halves2half2(__float2half_rz(am2), __float2half_rz(am1));
         const __half2 hp = __halves2half2(__float2half_rz(ap1), __float2half_rz(ap2));
-        btA[rk] = make_float4(pa.x, pa.y, pa.z, *reinterpret_cast<const float*>(&hm));
-        btB[rk] = make_float4(*reinterpret_cast<const float*>(&hp), __int_as_float(wa), __int_as_float(wc), 0.f);
+        if (!FIX) btA[rk] = make_float4(pa.x, pa.y, pa.z, 0.f);
+        btB[rk] = make_float4(*reinterpret_cast<const float*>(&hp), __int_as_float(wa), __int_as_float(wc),
+                              *reinterpret_cast<const float*>(&hm));
       }
       __syncwarp();
       int qb = 0;  // working atoms that start before K
@@ -1359,9 +1369,10 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         qb += __popc(M);
         const int k = K + lane;
         const bool valid = k < W;
-        const float4 b0v = btA[qr], b1v = btB[qr];
+        const float4 b1v = btB[qr];
         const int sq = __float_as_int(b1v.y), cc = __float_as_int(b1v.z);
         const int s_q = sq & 511, i = sq >> 9;
+        const float4 b0v = FIX ? pf[i] : btA[qr];
         const int cls = (cc >> 15) & 127;
         const int lx = cc & 31, ly = (cc >> 5) & 31, lz = (cc >> 10) & 31;
         const unsigned ent = valid ? own_ent(cls, kParts * (k - s_q) + part) : 0u;
@@ -1392,7 +1403,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
           if (tr < 0.f) mask = 0;
           // the x-gaps beyond tr, compared as FP16 (tr rounded up, so that no cell is pruned wrongly)
           const __half2 tr2 = __half2half2(__float2half_ru(tr));
-          const unsigned pm = (__hgt2_mask(*reinterpret_cast<const __half2*>(&b0v.w), tr2) & 0x00020001u) |
+          const unsigned pm = (__hgt2_mask(*reinterpret_cast<const __half2*>(&b1v.w), tr2) & 0x00020001u) |
                               (__hgt2_mask(*reinterpret_cast<const __half2*>(&b1v.x), tr2) & 0x00100008u);
           mask &= ~(pm | (pm >> 16));
           if (mask) {
@@ -1511,7 +1522,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
                                           nacc, 0);
     else if (FIX)
       force_batch_fix<MULTI, ENERGY, COUNT>(qn, 0, qk, px, fa, cap, A, ljx, esum, wsum, shsum, nacc, big_flag,
-                                            edge, face, inside64, second);
+                                            edge, face, inside64);
     else
       force_batch<MULTI, ENERGY, COUNT, MODE == kRedoFull>(qn, 0, qd, fa, fr, cap, A, ljs32, ek, wk, nacc,
                                                            big_flag, inside64);
@@ -1659,10 +1670,15 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         double f;
-        if (FIX) {  // the integer sum, times 2^-sf
-          const long long v = ((long long)fa[(3 + c) * cap + t] << 32) | (unsigned)fa[c * cap + t];
-          const double d = __ll2double_rn(v);
-          f = v ? __hiloint2double(__double2hiint(d) - (A.fx.sf << 20), __double2loint(d)) : 0.0;
+        if (FIX) {
+          // the sum, times 2^-sf: C 2^coarse + r, C the coarse word and r the rest of the 64 bits, a signed
+          // number; as h 2^32 + l with |h| < 2^53, so that one rounding is left
+          const int C = fa[(6 + c) * cap + t], sh = A.fx.coarse - 32;
+          const int rh = (int)((unsigned)fa[(3 + c) * cap + t] - ((unsigned)C << sh));
+          const long long h = ((long long)C << sh) + rh;
+          const unsigned l = (unsigned)fa[c * cap + t];
+          const double d = fma((double)h, 0x1p32, (double)l);
+          f = (h | l) ? __hiloint2double(__double2hiint(d) - (A.fx.sf << 20), __double2loint(d)) : 0.0;
         } else {
           f = fd[c * cap + t];
         }

@@ -1,0 +1,127 @@
+"""The range and the resolution of the FP64 form's fixed-point pass.
+
+- Any number of terms on one atom: many small neighbours on one side of a large
+  atom, and a cluster whose own pairs another tile computes.
+- Weak pairs keep FP64's relative accuracy: isolated pairs near the cutoff, at
+  cutoffs of 2.5 to 8 sigma, of the weakest type pair beside a strong one, and
+  contact pairs far inside the largest cutoff.  The bound is that of the FP64
+  body's own expression, in units of u = 2^-53: each separation is rounded once
+  (1 u), r^2 5 u, 1 / r^2 6 u, sigma^2 / r^2 8 u, its cube 26 u, squared 53 u, the
+  difference, eps, 1 / r^2 and the separation 12 u more: 65 u of the repulsive
+  and 38 u of the attractive term.
+"""
+import numpy as np
+import pytest
+
+pytestmark = [pytest.mark.gpu]
+
+TOL64 = 1e-12
+U = 2.0 ** -53
+
+
+def lj_exact(pos, pairs, eps, sigma):
+    """Forces of the listed pairs from the exact difference of their coordinates (no periodic images), in extended
+    precision, and the bound of the FP64 expression's error."""
+    q = np.longdouble
+    d = pos.astype(q)[pairs[:, 1]] - pos.astype(q)[pairs[:, 0]]
+    r2 = (d * d).sum(1)
+    s6 = (q(sigma) * q(sigma) / r2) ** 3
+    dg = -24 * q(eps) * (2 * s6 * s6 - s6) / r2
+    size = 24 * q(eps) / np.sqrt(r2) * (2 * s6 * s6 * 65 + s6 * 38) * U
+    return dg[:, None] * d, size
+
+
+def directions(k, rng):
+    u = rng.normal(size=(k, 3))
+    return u / np.sqrt((u * u).sum(1))[:, None]
+
+
+@pytest.mark.parametrize("sigma_b,count,angle", [(0.2, 27, 60.0), (0.45, 15, 78.0), (0.45, 9, 60.0)])
+def test_many_small_neighbours_on_one_side(gpulib, oracle, sigma_b, count, angle):
+    """Atoms of type 0 with `count` atoms of type 1 on a cap of 0.826 sigma around each, every term below 2^9 but
+    their sum twice 4096 or so; the small ones beyond their own potential's minimum from each other."""
+    L = np.array([18.0, 24.0, 30.0])
+    c = np.stack(np.meshgrid(*[np.arange(3.0, b, 6.0) for b in L], indexing="ij"), -1).reshape(-1, 3)
+    # spiral points on the cap, evenly spread
+    k = np.arange(count) + 0.5
+    z = 1.0 - (1.0 - np.cos(np.radians(angle))) * k / count
+    phi = np.pi * (1.0 + 5.0 ** 0.5) * k
+    u = np.stack([z, np.sqrt(1 - z * z) * np.cos(phi), np.sqrt(1 - z * z) * np.sin(phi)], 1)
+    parts, types = [c], [np.zeros(len(c), dtype=np.int32)]
+    for v in 0.826 * u:
+        parts.append(c + v)
+        types.append(np.ones(len(c), dtype=np.int32))
+    pos, types = np.concatenate(parts), np.concatenate(types)
+    lj = dict(ntypes=2, eps=[[1.0, 1.0], [1.0, sigma_b]], sigma=[[1.0, 1.0], [1.0, sigma_b]],
+              rc=[[2.5, 2.5], [2.5, 2.5 * sigma_b]])
+    ref = oracle.forces_typed(pos, L, lj["rc"], types=types, threads=0, block_length=1.25,
+                              **{k: lj[k] for k in ("eps", "sigma", "ntypes")})
+    with gpulib.MidpointLJ(L, [len(pos)], precision="fp64", **lj) as s:
+        s.set_atoms(pos, types)
+        f, e, _ = s.forces(energy=True)
+    fr = ref["forces"]
+    assert np.abs(fr[:len(c), 0]).min() > (4096 if count > 9 else 2000)
+    assert np.sqrt(((f - fr) ** 2).sum(1)).max() <= TOL64 * np.sqrt((fr * fr).sum(1).mean())
+    assert e[0] == pytest.approx(ref["epot"], rel=TOL64)
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("side", [-1.0, 1.0])
+def test_cluster_in_the_next_tile(gpulib, axis, side):
+    """16 atoms within 0.01 of each other, 0.84 sigma from a single atom across each tile face of the axis: the tile
+    of the cluster's own pairs may not be the one that sums the single atom's."""
+    L = np.full(3, 30.0)
+    rng = np.random.default_rng(1)
+    singles, clusters = [], []
+    for t in (2, 3, 4):  # tiles of t cells of 1.25 on every axis
+        for k in range(1, int(24 / t)):
+            x = np.full(3, 5.0)
+            x[(axis + 1) % 3] += 2.6 * (k % 8)
+            x[(axis + 2) % 3] += 2.6 * (k // 8) + 7.8 * (t - 2)
+            x[axis] = 1.25 * t * k - side * 0.42
+            y = x.copy()
+            y[axis] += side * 0.84
+            if all(np.abs(x - z).max() > 4.5 for z in singles):
+                singles.append(x)
+                clusters.append(y + rng.uniform(-0.005, 0.005, (16, 3)))
+    pos = np.concatenate([np.array(singles)] + clusters)
+    n = len(singles)
+    assert n >= 3
+    for tile in (2, 3, 4):
+        with gpulib.MidpointLJ(L, [len(pos)], precision="fp64", tile=tile) as s:
+            s.set_atoms(pos)
+            f = s.forces()[0]
+        for i in range(n):
+            k = n + 16 * i + np.arange(16)
+            F, size = lj_exact(pos, np.stack([np.full(16, i), k], 1), 1.0, 1.0)
+            # the exact terms' sum, their own error and that of 16 FP64 additions
+            assert np.abs(f[i] - F.sum(0)).max() <= float(size.sum()) + 16 * U * float(np.abs(F).sum())
+
+
+@pytest.mark.parametrize("rc", [2.5, 3.0, 3.8, 4.0, 5.0, 6.0, 8.0])
+@pytest.mark.parametrize("what", ["cutoff", "middle", "contact", "weak"])
+def test_isolated_pairs(gpulib, rc, what):
+    """weak: the type pair of a sixteenth of the strongest one's eps."""
+    m = 7
+    spacing = 2.2 * rc
+    L = np.full(3, m * spacing)
+    rng = np.random.default_rng(int(10 * rc))
+    c = (np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3) + 0.5) * spacing
+    lo, hi = {"cutoff": (0.95 * rc, 0.999 * rc), "middle": (1.5, 2.4), "contact": (0.9, 1.05),
+              "weak": (0.8 * rc, 0.999 * rc)}[what]
+    half = 0.5 * rng.uniform(lo, hi, len(c))[:, None] * directions(len(c), rng)
+    pos = np.concatenate([c - half, c + half])
+    pairs = np.stack([np.arange(len(c)), np.arange(len(c)) + len(c)], 1)
+    if what == "weak":
+        lj, types, eps = dict(ntypes=2, eps=[[1.0, 0.25], [0.25, 0.0625]], rc=rc), np.ones(len(pos), dtype=np.int32), 0.0625
+    else:
+        lj, types, eps = dict(rc=rc), None, 1.0
+    F, size = lj_exact(pos, pairs, eps, 1.0)
+    with gpulib.MidpointLJ(L, [len(pos)], precision="fp64", **lj) as s:
+        s.set_atoms(pos, types)
+        f = s.forces()[0]
+        assert s.counters()["accepted"] == len(c)
+    n = len(c)
+    for sign, g in ((1, f[:n]), (-1, f[n:])):
+        err = np.sqrt(((sign * g - F) ** 2).sum(1)).astype(np.float64)
+        assert (err <= size.astype(np.float64)).all(), float((err / size).max())
