@@ -155,8 +155,11 @@ long long fixed_of(double x, int ue) {
 // false where the parameters do not suit it and the FP64 body computes every
 // tile: pairs whose force at their cutoff falls below 2^-11 of the largest force
 // scale eps / sigma (the sums' one unit would hold it to fewer bits than FP64
-// does), a cutoff inside the range of the forces too large for the sums, or
-// lengths and energies whose powers leave FP64's range.
+// does), pairs so small beside the longest cutoff (sigma below about a sixth of
+// it), whose square is below 2^62 units, that their r^2 has less than FP64's bits
+// (RMS error of contact pairs at sigmas 1 : 8 was 8.6e-15 where FP64 has 1.1e-15), a
+// cutoff inside the range of the forces too large for the sums, or lengths and
+// energies whose powers leave FP64's range.
 bool build_fix(const LJTable& lj, const examd_params& p, FixTable& fx) {
   const int n2 = lj.nt * lj.nt;
   double rmax = 0.0, f0max = 0.0, fweak = INFINITY;  // fweak: the weakest pair's force at its cutoff (by its terms' size)
@@ -199,8 +202,8 @@ bool build_fix(const LJTable& lj, const examd_params& p, FixTable& fx) {
     q.e4 = lj.p64[k].eps4;
     q.eshift = lj.p64[k].eshift;
     const double lim = std::ldexp(lj.p64[k].rcut2, -w), big = std::ldexp(r2big[k], -w);
-    if (!std::isnormal(q.c6) || !std::isnormal(q.c12) || !std::isnormal(q.s6) || !(big >= 0x1p36) ||
-        !(lim >= 0x1p44) || !(lim < 0x1p61) || !(big < lim))
+    if (!std::isnormal(q.c6) || !std::isnormal(q.c12) || !std::isnormal(q.s6) || !(big >= 0x1.8p52) ||
+        !(lim < 0x1p61) || !(big < lim))
       return false;
     q.limh = (int)((long long)lim >> 32);
     q.bigh = (int)((long long)big >> 32) + 1;

@@ -447,10 +447,11 @@ __device__ __forceinline__ void force_batch64(int cnt, const QK& qk, const PD& p
 // add on the same pipe.  With the reference's operations and six such atomics
 // a pair cost 35 FP64 operations and more, and the pass was bound by that
 // pipe (79 % busy, issue 17 %).  Here the pair keeps eight:
-// - positions are integers in units of 2^ue (L < 2^62 of them modulo 2^64,
-//   rc < 2^62), so the separation is exact, and D = r^2 / 2^64 to one unit in
-//   2^57 or better by 32-bit multiplies (the lowest product, below one unit
-//   of D, is left out);
+// - positions are integers in units of 2^ue (modulo 2^64, rc < 2^62), so the
+//   separation is exact, and D = r^2 / 2^64 to less than one unit by 32-bit
+//   multiplies (of the lowest product, below one unit, only the mean is taken):
+//   2^55 units or more at r > 0.74 sigma and rc = 2.5 sigma, 3 2^51 at least
+//   (build_fix);
 // - D becomes a double (one rounding), y = 1/D from an FP32 estimate (relative
 //   error e of 2^-22) by one step of Householder's third-order iteration,
 //   y (1 + e + e^2), error e^3: three operations;
@@ -493,12 +494,13 @@ __device__ __forceinline__ void force_batch_fix(int cnt, int q0, const QK& qk, c
     long long dy = (long long)(px[cap + m] - px[cap + i]);
     long long dz = (long long)(px[2 * cap + m] - px[2 * cap + i]);
     if (edge) face(i, m, dx, dy, dz);  // the tile holds periodic copies
-    // d = h 2^32 + l with signed l: r^2 / 2^64 = sum h^2 + 2^-31 sum h l + (sum l^2 / 2^64, below one)
+    // d = h 2^32 + l with signed l: r^2 / 2^64 = sum h^2 + 2^-31 sum h l + sum l^2 / 2^64, the second term rounded and
+    // the third (below one) at its mean, a quarter: 3 / 4 before the shift rounds down
     const int hx = (int)((dx + 0x80000000ll) >> 32), lx = (int)dx;
     const int hy = (int)((dy + 0x80000000ll) >> 32), ly = (int)dy;
     const int hz = (int)((dz + 0x80000000ll) >> 32), lz = (int)dz;
     const long long D = (long long)hx * hx + (long long)hy * hy + (long long)hz * hz +
-                        (((long long)hx * lx + (long long)hy * ly + (long long)hz * lz) >> 31);
+                        ((0x60000000ll + (long long)hx * lx + (long long)hy * ly + (long long)hz * lz) >> 31);
     const int Dh = (int)(D >> 32);
     app = Dh < P.limh;
     if (abs(Dh - P.limh) <= 1) app = in64(i, m, ti, tj);
