@@ -494,13 +494,14 @@ __device__ __forceinline__ void force_batch_fix(int cnt, int q0, const QK& qk, c
     long long dy = (long long)(px[cap + m] - px[cap + i]);
     long long dz = (long long)(px[2 * cap + m] - px[2 * cap + i]);
     if (edge) face(i, m, dx, dy, dz);  // the tile holds periodic copies
-    // d = h 2^32 + l with signed l: r^2 / 2^64 = sum h^2 + 2^-31 sum h l + sum l^2 / 2^64, the second term rounded and
-    // the third (below one) at its mean, a quarter: 3 / 4 before the shift rounds down
+    // d = h 2^32 + l with signed l: r^2 / 2^64 = sum h^2 + 2^-31 sum h l + sum l^2 / 2^64, the third term (below one)
+    // at its mean, a quarter.  The shift rounds down, by half a unit on average, which the conversion to a double,
+    // halves up, makes good
     const int hx = (int)((dx + 0x80000000ll) >> 32), lx = (int)dx;
     const int hy = (int)((dy + 0x80000000ll) >> 32), ly = (int)dy;
     const int hz = (int)((dz + 0x80000000ll) >> 32), lz = (int)dz;
     const long long D = (long long)hx * hx + (long long)hy * hy + (long long)hz * hz +
-                        ((0x60000000ll + (long long)hx * lx + (long long)hy * ly + (long long)hz * lz) >> 31);
+                        ((0x20000000ll + (long long)hx * lx + (long long)hy * ly + (long long)hz * lz) >> 31);
     const int Dh = (int)(D >> 32);
     app = Dh < P.limh;
     if (abs(Dh - P.limh) <= 1) app = in64(i, m, ti, tj);

@@ -164,3 +164,44 @@ def test_small_pairs_beside_a_long_cutoff(gpulib, ratio):
         return float(np.sqrt((((g - F) ** 2).sum(1) / size ** 2).mean()))
 
     assert rms(f[:n]) <= 1.2 * rms(f64) and rms(-f[n:]) <= 1.2 * rms(f64)
+
+
+@pytest.mark.parametrize("potential,m,rho,jitter,rc", [("wca", 16, 1.05, 0.0001, 2.5), ("wca", 16, 1.0, 0.02, 2.5),
+                                                      ("lj_shifted", 12, 0.95, 0.03, 1.6), ("lj", 14, 0.8442, 0.09, 2.5)])
+def test_energy_and_virial_to_fp64(gpulib, potential, m, rho, jitter, rc):
+    """Energies near a potential's end and sums over many pairs: the RMS error over eight configurations is the pairs'
+    own in FP64 (independent, as the FP64 expression has them) and the rounding of the last few sums, 0.41 u."""
+    from scipy.spatial import cKDTree
+    q = np.longdouble
+    a = (4.0 / rho) ** (1.0 / 3.0)
+    L = np.full(3, m * a)
+    basis = np.array([[0, 0, 0], [0.5, 0.5, 0], [0.5, 0, 0.5], [0, 0.5, 0.5]])
+    g = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 1, 3)
+    shift = {"lj": q(0), "wca": q(-1), "lj_shifted": 4 * (1 / q(rc) ** 12 - 1 / q(rc) ** 6)}[potential]
+    rel, allow = [], 0.0
+    for seed in range(8):
+        rng = np.random.default_rng(seed)
+        x = ((g + basis).reshape(-1, 3) + 0.25 + jitter * rng.uniform(-1, 1, (4 * m ** 3, 3))) * a % L
+        p = cKDTree(x, boxsize=L).query_pairs(rc, output_type="ndarray")
+        d = x[p[:, 1]] - x[p[:, 0]]
+        d -= np.rint(d / L) * L
+        r2 = (d.astype(q) ** 2).sum(1)
+        use = r2 <= min(rc * rc, 2.0 ** (1 / 3) if potential == "wca" else np.inf)
+        d, r2 = d[use], r2[use]
+        s6 = 1 / r2 ** 3
+        e, w = 4 * (s6 * s6 - s6) - shift, 24 * (2 * s6 * s6 - s6)
+        i2 = 1.0 / (d * d).sum(1)
+        t6 = i2 * i2 * i2
+        own = [np.asarray(4.0 * (t6 * t6 - t6) - float(shift) - e, dtype=np.float64),
+               np.asarray(24.0 * (2.0 * t6 * t6 - t6) - w, dtype=np.float64)]
+        with gpulib.MidpointLJ(L, [len(x)], precision="fp64", rc=rc, potential=potential) as s:
+            s.set_atoms(x)
+            _, ep, vir = s.forces(energy=True)
+        exact = [e.sum(), w.sum()]
+        rel.append([float((q(v[0]) - z) / abs(z)) for v, z in zip((ep, vir), exact)])
+        allow = max(allow, *(np.sqrt(len(d)) * o.std() / abs(float(z)) for o, z in zip(own, exact)))
+    rms = np.sqrt(np.mean(np.square(rel), axis=0))
+    # (1 u: the last sums' 0.41 u with room for eight samples; lj_shifted: its shift is a double, whose own rounding
+    # is in every pair)
+    tol = U + 2 * allow + (U * len(d) * abs(float(shift)) / abs(float(exact[0])) if potential == "lj_shifted" else 0.0)
+    assert (rms <= tol).all(), (rms / U, tol / U)
