@@ -160,7 +160,7 @@ long long fixed_of(double x, int ue) {
 // (RMS error of contact pairs at sigmas 1 : 8 was 8.6e-15 where FP64 has 1.1e-15), a
 // cutoff inside the range of the forces too large for the sums, or lengths and
 // energies whose powers leave FP64's range.
-bool build_fix(const LJTable& lj, const examd_params& p, FixTable& fx) {
+bool build_fix(const LJTable& lj, const examd_params& p, double bl, FixTable& fx) {
   const int n2 = lj.nt * lj.nt;
   double rmax = 0.0, f0max = 0.0, fweak = INFINITY;  // fweak: the weakest pair's force at its cutoff (by its terms' size)
   for (int k = 0; k < n2; ++k) {
@@ -207,7 +207,10 @@ bool build_fix(const LJTable& lj, const examd_params& p, FixTable& fx) {
       return false;
     q.limh = (int)((long long)lim >> 32);
     q.bigh = (int)((long long)big >> 32) + 1;
-    q.pre = lj.p32[k].rc2 * 1.0001f;
+    // The prefilter's cutoff covers the FP32 separations' rounding: relative to it, and absolute, to the cell edge (x
+    // from the tile's centre, up to 11 edges away, y and z from the atoms' own rows: 80 2^-24 edges in all)
+    const double wide = p.rc[k] + 5e-6 * bl;
+    q.pre = std::max(lj.p32[k].rc2 * 1.0001f, (float)(wide * wide * 1.000001));
   }
   return true;
 }
@@ -691,8 +694,8 @@ int examd_gpu_create(const examd_params* params, int nboxes, const examd_box* bo
     lj.minv[a] = 1.0 / m;
   }
 
-  // (the prefilter's margin covers the FP32 coordinates for edges up to 8 rc)
-  ctx->pc.fix = ctx->pc.fp64 && bl <= 8.0 * rcmax && build_fix(lj, p, ctx->fx);
+  // (in larger cells the prefilter would pass too many candidates)
+  ctx->pc.fix = ctx->pc.fp64 && bl <= 8.0 * rcmax && build_fix(lj, p, bl, ctx->fx);
 
   // Tiles of a batch: the tile edge T is the densest box's.  A box with fewer
   // atoms per cell gets tiles up to 2 cells longer per axis, as long as its

@@ -205,3 +205,39 @@ def test_energy_and_virial_to_fp64(gpulib, potential, m, rho, jitter, rc):
     # is in every pair)
     tol = U + 2 * allow + (U * len(d) * abs(float(shift)) / abs(float(exact[0])) if potential == "lj_shifted" else 0.0)
     assert (rms <= tol).all(), (rms / U, tol / U)
+
+
+@pytest.mark.parametrize("sigma,rc", [(0.42, 0.32), (0.04, 0.1)])
+def test_short_cutoff_in_large_cells(gpulib, oracle, sigma, rc):
+    """A type pair whose cutoff is a sixtieth of the cell edge or less, in tiles of 14 cells: pairs just inside it, on
+    both sides of the face where the tile's FP32 coordinates are largest, are the oracle's, each of them."""
+    rng = np.random.default_rng(8)
+    cross = 0.5 * (1.0 + sigma)
+    lj = dict(ntypes=2, eps=[[1.0, cross], [cross, sigma]], sigma=[[1.0, cross], [cross, sigma]],
+              rc=[[2.5, 2.5 * cross], [2.5 * cross, rc]])
+    n, nbox = 250, 24
+    boxes, parts = [], []
+    for _ in range(nbox):
+        L = 14 * 19.9 + rng.uniform(0.0, 4.0, 3)
+        c = np.stack([np.zeros(n), rng.permutation(n) * (L[1] / n), (np.arange(n) + 0.5) * (L[2] / n)], 1)
+        u = np.stack([np.ones(n), rng.uniform(-0.02, 0.02, n), rng.uniform(-0.02, 0.02, n)], 1)
+        u /= np.sqrt((u * u).sum(1))[:, None]
+        r = rc * (1.0 - 10.0 ** rng.uniform(-9, -7, n))[:, None]
+        s = rng.uniform(0.1, 0.9, n)[:, None]
+        p = np.concatenate([c - s * r * u, c + (1 - s) * r * u]) % L
+        parts.append(p)
+        boxes.append(L)
+    pos, boxes = np.concatenate(parts), np.array(boxes)
+    with gpulib.MidpointLJ(boxes, [2 * n] * nbox, precision="fp64", block_length=19.9, tile=(14, 14, 14), **lj) as sysm:
+        sysm.set_atoms(pos, np.ones(len(pos), dtype=np.int32))
+        f = sysm.forces()[0]
+        accepted = sysm.counters()["accepted"]
+    want = 0
+    for b in range(nbox):
+        k = slice(2 * n * b, 2 * n * (b + 1))
+        ref = oracle.forces_typed(pos[k], boxes[b], lj["rc"], types=np.ones(2 * n, dtype=np.int32), threads=0,
+                                  block_length=19.900390625, **{x: lj[x] for x in ("eps", "sigma", "ntypes")})
+        want += ref["counts"].accepted
+        fr = ref["forces"]
+        assert np.sqrt(((f[k] - fr) ** 2).sum(1)).max() <= TOL64 * np.sqrt((fr * fr).sum(1).mean())
+    assert want > 0.98 * n * nbox and accepted == want
