@@ -191,6 +191,8 @@ bool build_fix(const LJTable& lj, const examd_params& p, double bl, FixTable& fx
   if (!std::isnormal(gmax)) return false;
   const int sg = 61 - std::ilogb(gmax);  // |dg| 2^sg < 2^62
   fx.k0 = sg - fx.ue - fx.sf;
+  fx.wunit = std::ldexp(1.0, w - sg);
+  if (!std::isnormal(fx.wunit)) return false;
   // (the coarse word is formed from the product's top word: a step is at least 2^4 of its units)
   if (fx.k0 + fx.coarse - 96 < 4 || fx.k0 > 63) return false;
   for (int k = 0; k < n2; ++k) {

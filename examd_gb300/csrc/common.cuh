@@ -156,6 +156,7 @@ struct FixTable {
   int k0;           // a term's 128-bit product is taken at bit k0 where the factor is largest
   int coarse, atoms;  // of FixUnit
   int sf;           // the force sums' unit is 2^-sf
+  double wunit;     // of the virial's sum
   FixPair p[EXAMD_MAX_TYPES * EXAMD_MAX_TYPES];
 };
 

@@ -475,8 +475,8 @@ __device__ __forceinline__ void force_batch64(int cnt, const QK& qk, const PD& p
 // body redoes it.
 template <bool MULTI, bool ENERGY, bool COUNT, class QK, class PX, class FA, class FACE, class IN64>
 __device__ __forceinline__ void force_batch_fix(int cnt, int q0, const QK& qk, const PX& px, FA& fa, int cap,
-                                                const PairArgs& A, const FixPair* ljx, double& s12, double& s6s,
-                                                double& shift, int& nacc, int* big_flag, bool edge, const FACE& face,
+                                                const PairArgs& A, const FixPair* ljx, double& esum, double& wsum,
+                                                int& nacc, int* big_flag, bool edge, const FACE& face,
                                                 const IN64& in64) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -525,10 +525,12 @@ __device__ __forceinline__ void force_batch_fix(int cnt, int q0, const QK& qk, c
       const double y3 = y2 * y;
       const double g = (y2 * y2) * fma(-P.c12, y3, P.c6);
       if (ENERGY) {
-        const double q6 = P.s6 * y3, e6 = P.e4 * q6;
-        s12 = fma(e6, q6, s12);
-        s6s += e6;
-        if (A.lj.pot != EXAMD_POT_LJ) shift += P.eshift;
+        // differences per pair, as the FP64 body forms them (sums of the terms apart cancel at the end), in four
+        // operations: 4 eps (s^6 - 1) s^6, and -g r^2 in the tables' units
+        const double q6 = P.s6 * y3;
+        esum = fma(fma(P.e4, q6, -P.e4), q6, esum);
+        if (A.lj.pot != EXAMD_POT_LJ) esum -= P.eshift;
+        wsum = fma(-g, Dd, wsum);
       }
       if (COUNT) ++nacc;
       // g = G 2^(e - 1084) with its 53 bits at the top of 62 (|g| < 2^62), then G d / 2^K, rounded; where
@@ -886,8 +888,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
 
   const LJ32 q32 = A.lj.p32[0];
   const float rcpre = A.lj.rc2max * 1.0001f + 1e-4f;  // FP32 prefilter of the FP64 form
-  double esum = 0.0, wsum = 0.0;  // FP64 form (kFixed: the sums of 4 eps s^12 and 4 eps s^6)
-  double shsum = 0.0;             // kFixed: the sum of the energy shifts
+  double esum = 0.0, wsum = 0.0;  // FP64 form
   FixSum ek, wk;                  // mixed form: exact fixed-point sums of FP32 terms
   int ncand = 0, neval = 0, nacc = 0;
   // per-warp queue of accepted pairs (mixed form: the separation and the key
@@ -981,7 +982,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         force_batch64<MULTI, ENERGY, COUNT>(32, qk, pd, code, img, B.L, fd, cap, A.lj, ljs64, esum, wsum, A.status,
                                             nacc, qn);
       else if (FIX)
-        force_batch_fix<MULTI, ENERGY, COUNT>(32, qn, qk, px, fa, cap, A, ljx, esum, wsum, shsum, nacc, big_flag,
+        force_batch_fix<MULTI, ENERGY, COUNT>(32, qn, qk, px, fa, cap, A, ljx, esum, wsum, nacc, big_flag,
                                               edge, face, inside64);
       else
         force_batch<MULTI, ENERGY, COUNT, MODE == kRedoFull>(32, qn, qd, fa, fr, cap, A, ljs32, ek, wk, nacc,
@@ -1524,7 +1525,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
       force_batch64<MULTI, ENERGY, COUNT>(qn, qk, pd, code, img, B.L, fd, cap, A.lj, ljs64, esum, wsum, A.status,
                                           nacc, 0);
     else if (FIX)
-      force_batch_fix<MULTI, ENERGY, COUNT>(qn, 0, qk, px, fa, cap, A, ljx, esum, wsum, shsum, nacc, big_flag,
+      force_batch_fix<MULTI, ENERGY, COUNT>(qn, 0, qk, px, fa, cap, A, ljx, esum, wsum, nacc, big_flag,
                                             edge, face, inside64);
     else
       force_batch<MULTI, ENERGY, COUNT, MODE == kRedoFull>(qn, 0, qd, fa, fr, cap, A, ljs32, ek, wk, nacc,
@@ -1721,12 +1722,9 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
     long long* redl = (long long*)red;
     double e = 0.0, w = 0.0;
     if (ENERGY) {
-      if (FIX) {
-        e = esum - wsum - shsum;
-        w = 12.0 * esum - 6.0 * wsum;
-      } else if (FP64) {
+      if (FP64 || FIX) {
         e = esum;
-        w = wsum;
+        w = FIX ? wsum * A.fx.wunit : wsum;
       }
     }
     __syncthreads();  // the queues are done with
