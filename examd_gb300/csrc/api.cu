@@ -301,6 +301,7 @@ struct examd_ctx {
   LJTable lj{};
   FixTable fx{};
   PairConfig pc;
+  bool fix = false;     // the system has a fixed-point pass (pc.fix: the present capacities leave room for it)
   int cap = 0, smem = 0, smem_limit = 0, sm_smem = 0;
   int cap_redo = 0;     // staged-atom capacity of the redo pass
   int dev = 0;
@@ -697,7 +698,7 @@ int examd_gpu_create(const examd_params* params, int nboxes, const examd_box* bo
   }
 
   // (in larger cells the prefilter would pass too many candidates)
-  ctx->pc.fix = ctx->pc.fp64 && bl <= 8.0 * rcmax && build_fix(lj, p, bl, ctx->fx);
+  ctx->fix = ctx->pc.fix = ctx->pc.fp64 && bl <= 8.0 * rcmax && build_fix(lj, p, bl, ctx->fx);
 
   // Tiles of a batch: the tile edge T is the densest box's.  A box with fewer
   // atoms per cell gets tiles up to 2 cells longer per axis, as long as its
@@ -1103,45 +1104,63 @@ int queue_occupancy(examd_ctx* ctx) {
 int apply_capacity(examd_ctx* ctx, bool* grew = nullptr) {
   if (grew) *grew = false;
   const int occ = ctx->h_status[1];
-  int want_r = std::max(((occ + occ / 4 + 64) + 7) & ~7, ctx->cap_redo);
-  int want = ctx->pc.fp64 && !ctx->pc.fix ? want_r : ((occ + occ / 16 + 32) + 7) & ~7;
-  // The fixed-point pass (78 bytes an atom) with half the headroom where the whole of it costs a CTA per SM (1M
-  // liquid 949 -> 844 us a pass, 500k at rc 3.0 719 -> 639)
-  if (ctx->pc.fix) {
-    const int least = ((occ + occ / 32 + 16) + 7) & ~7;
-    const int n = pair_ctas(ctx->pc, least, ctx->ne_max, ctx->ext_max, ctx->sm_smem);
-    while (want > least && pair_ctas(ctx->pc, want, ctx->ne_max, ctx->ext_max, ctx->sm_smem) < n) want -= 8;
-  }
-  if (want <= ctx->cap) return EXAMD_OK;
-  int bytes = 0;
+  PairConfig pc = ctx->pc;  // (the context changes only once a choice fits)
+  int cap = 0, redo = 0, bytes = 0;
   auto fits = [&] {
-    bytes = pair_smem_bytes(ctx->pc, want, want_r, ctx->ne_max, ctx->ext_max);
-    return bytes <= ctx->smem_limit && (!ctx->pc.fix || want <= ctx->fx.atoms);
+    bytes = pair_smem_bytes(pc, cap, redo, ctx->ne_max, ctx->ext_max);
+    return bytes <= ctx->smem_limit && (!pc.fix || cap <= ctx->fx.atoms);
   };
-  bool ok = fits();  // (the redo pass binds, or the fixed-point pass: the 12-warp CTAs' tables never do)
-  if (!ok) {  // the exact need if the headroom does not fit
-    want = want_r = (occ + 7) & ~7;
-    ok = fits();
+  auto up8 = [](int n) { return (n + 7) & ~7; };
+  auto headroom = [&] {  // not below what the same pass has now
+    redo = std::max(up8(occ + occ / 4 + 64), pc.fix == ctx->pc.fix ? ctx->cap_redo : 0);
+    cap = pc.fp64 && !pc.fix ? redo : up8(occ + occ / 16 + 32);
+    // The fixed-point pass (78 bytes an atom) with half the headroom where the whole of it costs a CTA per SM (1M
+    // liquid 949 -> 844 us a pass, 500k at rc 3.0 719 -> 639)
+    if (pc.fix) {
+      const int least = up8(occ + occ / 32 + 16);
+      const int n = pair_ctas(pc, least, ctx->ne_max, ctx->ext_max, ctx->sm_smem);
+      while (cap > least && pair_ctas(pc, cap, ctx->ne_max, ctx->ext_max, ctx->sm_smem) < n) cap -= 8;
+    }
+    return fits();
+  };
+  auto exact = [&] {
+    cap = redo = up8(occ);
+    return fits();
+  };
+  // (the redo pass binds, or the fixed-point pass: the 12-warp CTAs' tables never do)
+  pc.fix = ctx->fix;
+  bool ok = headroom();
+  if (pc.fix == ctx->pc.fix) {
+    if (cap <= ctx->cap) return EXAMD_OK;
+    ok = ok || exact();
   }
-  if (!ok && ctx->pc.fix) {  // the FP64 pass has smaller per-warp tables (about 110 atoms)
-    ctx->pc.fix = false;
-    ok = fits();
+  if (!ok && pc.fix) {
+    // The FP64 body has smaller tables; it takes every tile as long as the fixed-point pass does not fit the largest
+    // with its headroom
+    pc.fix = false;
+    ok = headroom();
+    if (!ctx->pc.fix && cap <= ctx->cap) return EXAMD_OK;
+    ok = ok || exact();
   }
   if (!ok) return EXAMD_ERR_CELL_OVERFLOW;
-  ctx->cap = want;
-  ctx->cap_redo = want_r;
-  ctx->smem = bytes;
-  if (grew) *grew = true;
+  if (pc.fix == ctx->pc.fix && cap == ctx->cap && redo == ctx->cap_redo) return EXAMD_OK;
   // all variants used by this context (the attribute is the kernel's, shared
   // with every other context of the process: the device's limit, so that none
   // takes away what another needs)
-  PairConfig c = ctx->pc;
   for (int e = 0; e < 2; ++e)
     for (int n = 0; n < 2; ++n) {
-      c.energy = e;
-      c.count = n;
-      CK(pair_prepare(c, ctx->smem_limit));
+      pc.energy = e;
+      pc.count = n;
+      CK(pair_prepare(pc, ctx->smem_limit));
     }
+  ctx->pc.fix = pc.fix;
+  ctx->cap = cap;
+  ctx->cap_redo = redo;
+  ctx->smem = bytes;
+  if (ctx->gexec) cudaGraphExecDestroy(ctx->gexec);
+  ctx->gexec = nullptr;
+  drop_io_graphs(ctx);
+  if (grew) *grew = true;
   return EXAMD_OK;
 }
 

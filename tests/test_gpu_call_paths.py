@@ -211,3 +211,42 @@ def test_tiles_at_the_shared_memory_limit(gpulib, oracle, atoms):
     ref = oracle.forces_typed(pos, L, rc, threads=0)
     check(f, ref["forces"], "fp64")
     assert e[0] == pytest.approx(ref["epot"], rel=TOL64)
+
+
+def packed(gpulib, n, size, L, seed):
+    """n atoms at random in a cube of `size` in the box's corner."""
+    return np.ascontiguousarray(np.random.default_rng(seed).uniform(0.0, size, (n, 3)) % L)
+
+
+@pytest.mark.parametrize("n,size", [(8000, 3.0), (3300, 3.7), (2900, 3.7)])
+@pytest.mark.parametrize("before", [False, True])
+def test_fixed_point_pass_after_a_crowded_tile(gpulib, n, size, before):
+    """Atoms that no pass has room for in one tile (refused), or only the FP64 body; the next configuration is computed
+    as by a context that never saw them, bit for bit (the fixed-point pass: FP64 sums would differ from run to run)."""
+    L = np.full(3, 32.0)
+    m = int(np.ceil(n ** (1 / 3)))
+    g = (np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n] + 0.5) * (32.0 / m)
+    good = g + np.random.default_rng(1).uniform(-0.1, 0.1, g.shape)
+    bad = packed(gpulib, n, size, L, 2)
+    with gpulib.MidpointLJ(L, [n], precision="fp64", tile=(3, 3, 3)) as s:
+        s.set_atoms(good)
+        want = [s.forces()[0], s.forces_at(good)[0], s.forces(energy=True)[0]]
+        state = s.run(8, 0.001, graph_chunk=4) and s.state()
+    with gpulib.MidpointLJ(L, [n], precision="fp64", tile=(3, 3, 3)) as s:
+        if before:
+            s.set_atoms(good)
+            s.run(8, 0.001, graph_chunk=4)
+        if n == 8000:
+            for _ in range(2):
+                with pytest.raises(gpulib.ExamdError):
+                    s.set_atoms(bad)
+        else:
+            s.set_atoms(bad)
+            s.forces()
+        s.set_atoms(good)
+        got = [s.forces()[0], s.forces_at(good)[0], s.forces(energy=True)[0]]
+        for a, b in zip(got, want):
+            assert np.array_equal(a, b)
+        s.run(8, 0.001, graph_chunk=4)
+        for a, b in zip(s.state(), state):
+            assert np.array_equal(a, b)
