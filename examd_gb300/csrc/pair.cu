@@ -22,7 +22,7 @@
 // law).  The FP64 form's first pass (k_pair_fix) walks the same items, tested
 // with an FP32 prefilter on a widened cutoff, and computes the queued pairs in
 // fixed point (force_batch_fix).  Its FP64 body (the tiles that the fixed-point
-// pass lists, and systems it cannot hold) builds items per (ext cell, row): the
+// pass cannot take, and systems it cannot hold) builds items per (ext cell, row): the
 // block of the cell's atoms against the row's owned j-cells, untrimmed; its
 // batches then hold pairs of many different i atoms, so their FP64
 // shared-memory atomics (compare-and-swap loops) rarely hit one address.
@@ -105,7 +105,8 @@ constexpr int kRedoBlocks = 152;       // grid of the redo pass (1 per SM)
 // writing the tile's pairs instead of their forces), the forces from the
 // list, and the redo of a listed tile's large terms.
 // kFixed: the FP64 form's first pass in fixed point (enumerated as the mixed
-// form's first pass; its listed tiles are redone by the FP64 form's own body).
+// form's first pass; tiles with terms too large are computed by the FP64 form's
+// own body in the same CTA, tiles over its capacity by the redo pass).
 constexpr int kMain = 0, kRedoBig = 1, kRedoFull = 2, kListBuild = 3, kList = 4, kListBig = 5, kFixed = 6;
 constexpr int kFullBit = 1 << 30;      // redo-list entry: tile | kFullBit for an overflowed tile
 constexpr int kSeg = 4;                // lanes per segment of the i-side force sums
@@ -223,9 +224,10 @@ static bool uses_wide(const PairConfig& c) { return c.wide && !c.fp64 && !c.list
 // counters, which the enumeration gives) the list pass's.
 static int main_smem_bytes(const PairConfig& cfg, int cap, int ne_max, int ext_max) {
   const int mode = (cfg.list && !cfg.count && !cfg.fp64) ? kList : kMain;
-  if (cfg.fix)
-    return make_layout(false, cap, ne_max, ext_max, cfg.warps, kFixed, cfg.multi,
-                       !own_in_global(true, cfg.multi, cfg.fine && !cfg.count ? kFineParts : kUnitParts)).bytes;
+  if (cfg.fix)  // (and the FP64 body in the same CTA)
+    return std::max(make_layout(true, cap, ne_max, ext_max, cfg.warps, kMain, cfg.multi).bytes,
+                    make_layout(false, cap, ne_max, ext_max, cfg.warps, kFixed, cfg.multi,
+                                !own_in_global(true, cfg.multi, cfg.fine && !cfg.count ? kFineParts : kUnitParts)).bytes);
   if (uses_wide(cfg)) return make_layout(false, cap, ne_max, ext_max, kWideWarps, kMain, cfg.multi).bytes;
   return make_layout(cfg.fp64, cap, ne_max, ext_max, cfg.warps, mode, cfg.multi).bytes;
 }
@@ -617,9 +619,10 @@ __device__ __forceinline__ void force_batch_fix(int cnt, int q0, const QK& qk, c
 //   expressions as the first pass (the same bits when the atoms are where
 //   the list was built), outputs, energy and the large-term flag as there;
 // - kListBig: kRedoBig from the list.
+// kFixed: returns true, nothing written, for a tile with a term too large.
 // CUT (list pass): the potential's own range rcut2 is tested (WCA; infinite otherwise).
 template <bool FP64, bool MULTI, bool ENERGY, bool COUNT, int MODE, bool CUT = true, int kParts = kUnitParts>
-__device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
+__device__ __forceinline__ bool pair_tile(const PairArgs& A, const int tile) {
   extern __shared__ __align__(16) unsigned char smem[];
   const unsigned FULL = 0xffffffffu;
   // ownership table, type table and axis tables come first: they are fixed for the context
@@ -632,7 +635,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   const int NE = EX * EY * EZ;
   constexpr bool kFromList = MODE == kList || MODE == kListBig;
   if (MODE == kMain || MODE == kFixed) grid_trigger();
-  if (kFromList && MODE == kList && A.lcount[tile] < 0) return;  // a fallback tile: the redo pass computes it
+  if (kFromList && MODE == kList && A.lcount[tile] < 0) return false;  // a fallback tile: the redo pass computes it
   constexpr bool FIX = MODE == kFixed;
   const int cap = (MODE == kMain || MODE == kListBuild || MODE == kList || FIX) ? A.cap : A.cap_redo;
   constexpr bool kOwnGlobal = own_in_global(FIX, MULTI, kParts);
@@ -777,22 +780,22 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   const int total = cw[2];
   if (kFromList && A.lcount[tile] != total) {  // the lists of another binning: not computed from
     if (tid == 0) atomicOr(A.status, ST_BOUNDS);
-    return;
+    return false;
   }
   if (kFromList && !(A.lj.pot == EXAMD_POT_LJ || A.lj.pot == EXAMD_POT_LJ_SHIFTED || A.lj.pot == EXAMD_POT_WCA)) {
     if (tid == 0) atomicOr(A.status, ST_PAIRFN);  // a potential the list passes do not evaluate
-    return;
+    return false;
   }
   if (MODE == kListBuild && (total > cap || total > A.lslots)) {  // no list: the redo pass enumerates it every step
     if (tid == 0) {
       A.lcount[tile] = -1;
       A.fb[atomicAdd(&A.lw[LW_FBN], 1)] = tile;
     }
-    return;
+    return false;
   }
   if ((FIX || (!FP64 && MODE == kMain)) && total > cap) {  // the redo pass computes it at its capacity
     if (tid == 0) A.redo[atomicAdd(A.redo_n, 1)] = tile | kFullBit;
-    return;
+    return false;
   }
   if (total > cap) {
     if (tid == 0) {
@@ -807,7 +810,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         A.tileC[3 * tile + 2] = 0;
       }
     }
-    return;
+    return false;
   }
   // (3) stage atoms, one thread per atom, kStage atoms' reads in flight at a
   // time.  (One thread per ext cell, the cell's atoms one after the other, waited
@@ -1329,7 +1332,8 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
     const float prune2 = MODE == kListBuild ? A.lj.prune2_list : A.lj.prune2;
     while (true) {
       int u = 0;
-      if (lane == 0) u = atomicAdd(ucnt, 1);
+      // (kFixed: a tile with a term too large is the FP64 body's, and not finished here)
+      if (lane == 0) u = FIX && *(volatile int*)big_flag ? nunits : atomicAdd(ucnt, 1);
       u = __shfl_sync(FULL, u, 0);
       if (u >= nunits) break;
       const int c = u / kParts, part = u - c * kParts;
@@ -1533,9 +1537,9 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
   }
   __syncthreads();
   // a large term was left out: list the tile for the redo pass
-  // (kFixed: the FP64 body computes it in full)
-  if (!FP64 && (MODE == kMain || MODE == kList || FIX) && tid == 0 && *big_flag)
-    A.redo[atomicAdd(A.redo_n, 1)] = FIX ? tile | kFullBit : tile;
+  // (kFixed: the same CTA computes it in full by the FP64 body)
+  if (!FP64 && (MODE == kMain || MODE == kList) && tid == 0 && *big_flag) A.redo[atomicAdd(A.redo_n, 1)] = tile;
+  if (FIX && *big_flag) return true;
   if (MODE == kListBuild) {
     // The atoms in the order of their entry counts, most first (a counting
     // sort), and the entries moved from the scratch into that order; a tile
@@ -1658,7 +1662,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         A.lcount[tile] = total;
       }
     }
-    return;
+    return false;
   }
 
   // (4) write-back: home atoms -> Fown, halo copies -> P[slot]
@@ -1767,6 +1771,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs& A, const int tile) {
         }
     }
   }
+  return false;
 }
 
 template <bool FP64, bool MULTI, bool ENERGY, bool COUNT>
@@ -1782,11 +1787,18 @@ __global__ void __launch_bounds__(32 * kWideWarps, 3) k_pair_wide(const PairArgs
   pair_tile<false, MULTI, ENERGY, false, kMain, true, kFineParts>(A, A.order[blockIdx.x]);
 }
 
-// FP64 form: the first pass in fixed point, and the FP64 body for the tiles that
-// it listed (normally none).
+// FP64 form: the first pass in fixed point; a tile with a term too large for it by
+// the FP64 body, in the same CTA: all of them in a system with overlapping atoms
+// (131,072 atoms at random, density 0.5, no least distance: 376 us a pass, 352 by
+// the FP64 body alone; 942 where such tiles were finished here first and then
+// listed for k_pair_redo64, one CTA an SM).
 template <bool MULTI, bool ENERGY, bool COUNT, int PARTS>
 __global__ void __launch_bounds__(256, MULTI ? 3 : 4) k_pair_fix(const PairArgs A) {
-  pair_tile<false, MULTI, ENERGY, COUNT, kFixed, true, PARTS>(A, A.order[blockIdx.x]);
+  const int tile = A.order[blockIdx.x];
+  if (pair_tile<false, MULTI, ENERGY, COUNT, kFixed, true, PARTS>(A, tile)) {
+    __syncthreads();
+    pair_tile<true, MULTI, ENERGY, COUNT, kMain>(A, tile);
+  }
 }
 
 // Pair-list mode: the forces of every tile from its list (fallback tiles
@@ -1835,6 +1847,7 @@ __global__ void __launch_bounds__(256, 3) k_pair_redo(const PairArgs A) {
   }
 }
 
+// FP64 form: the tiles over the first pass's capacity.
 template <bool MULTI, bool ENERGY, bool COUNT>
 __global__ void __launch_bounds__(256, 3) k_pair_redo64(const PairArgs A) {
   grid_trigger();

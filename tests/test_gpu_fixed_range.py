@@ -241,3 +241,35 @@ def test_short_cutoff_in_large_cells(gpulib, oracle, sigma, rc):
         fr = ref["forces"]
         assert np.sqrt(((f[k] - fr) ** 2).sum(1)).max() <= TOL64 * np.sqrt((fr * fr).sum(1).mean())
     assert want > 0.98 * n * nbox and accepted == want
+
+
+@pytest.mark.parametrize("tile", [2, 4])
+@pytest.mark.parametrize("apart", [0.0, 0.5, 0.74])
+def test_overlapping_atoms(gpulib, oracle, tile, apart):
+    """Atoms at random, no nearer than `apart`: every tile, most or a few are the FP64 body's, in grids above and below
+    its blocks.  Energies, counters and forces as the oracle's, each to the accuracy of its own atom's terms."""
+    n = 12000
+    L = np.full(3, (n / 0.6) ** (1.0 / 3.0))
+    pos = gpulib.gen_random(n, L, apart, 13) if apart else np.random.default_rng(13).uniform(0.0, 1.0, (n, 3)) * L
+    ref = oracle.forces_typed(pos, L, 2.5, threads=0)
+    with gpulib.MidpointLJ(L, [n], precision="fp64", tile=(tile,) * 3) as s:
+        s.set_atoms(pos)
+        for _ in range(2):
+            f, e, w = s.forces(energy=True)
+        plain = s.forces()[0]
+        cnt = s.counters()
+    # an atom's largest term bounds its force's error: 60 terms' roundings and the separations', amplified 14 times;
+    # a difference across the box's face is rounded at the box's scale, 2^-49, up to 14 times that over r
+    from scipy.spatial import cKDTree
+    p = cKDTree(pos, boxsize=L).query_pairs(2.5, output_type="ndarray")
+    d = pos[p[:, 1]] - pos[p[:, 0]]
+    d -= np.rint(d / L) * L
+    r = np.sqrt((d * d).sum(1))
+    t = 24.0 * (2.0 * r ** -13 + r ** -7) * (60 * 14 * 2.0 ** -53 + 14 * 2.0 ** -48 / r)
+    size = np.zeros(n)
+    np.add.at(size, p[:, 0], t)
+    np.add.at(size, p[:, 1], t)
+    for g in (f, plain):
+        assert (np.abs(g - ref["forces"]).max(1) <= size).all()
+    assert e[0] == pytest.approx(ref["epot"], rel=TOL64) and w[0] == pytest.approx(ref["virial"], rel=TOL64)
+    assert cnt["candidates"] == ref["counts"].candidates and cnt["accepted"] == ref["counts"].accepted
