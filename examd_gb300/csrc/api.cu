@@ -278,7 +278,13 @@ int examd_tile_split(int nb, double last_width, int tile_len, int tile_balance, 
 }
 
 constexpr int kIoChunks = 4;            // host <-> device transfers of the force call, in chunks
-constexpr int kEagerSlots = 32;         // energies of eager steps kept on the device before one copy
+// Energies of eager steps kept on the device before one copy: this many steps of
+// them, or as many as fit in kEagerBytes per array (one at least).
+constexpr int kEagerSlots = 32;
+constexpr size_t kEagerBytes = (size_t)4 << 20;
+int eager_slots(int nboxes) {
+  return (int)std::min<size_t>(kEagerSlots, std::max<size_t>(1, kEagerBytes / (sizeof(double) * (size_t)nboxes)));
+}
 // Force calls at new positions of at most this many atoms go through the
 // context's own page-locked arrays (two host copies of up to 393 KB) from the
 // third call on, so that they replay one captured graph whatever the caller's
@@ -1829,17 +1835,24 @@ int ensure_ebuf(examd_ctx* ctx, int steps, bool host) {
   if (host && cudaHostAlloc((void**)&ctx->h_e, 2 * (size_t)(steps + 1) * ctx->nboxes * sizeof(double),
                             cudaHostAllocDefault) != cudaSuccess) {
     ctx->h_e = nullptr;
+    cudaGetLastError();  // reported here, not by the next launch
     return EXAMD_ERR_NOMEM;
   }
   if (steps <= ctx->ebuf_steps) return EXAMD_OK;
-  if (ctx->boxE) cudaFree(ctx->boxE);
-  if (ctx->boxW) cudaFree(ctx->boxW);
-  if (ctx->boxKE) cudaFree(ctx->boxKE);
-  ctx->boxE = ctx->boxW = ctx->boxKE = nullptr;
   size_t n = (size_t)(steps + 1) * ctx->nboxes;
   int rc;
-  if ((rc = dalloc(ctx, &ctx->boxE, n)) || (rc = dalloc(ctx, &ctx->boxW, n)) || (rc = dalloc(ctx, &ctx->boxKE, n)))
+  double *e = nullptr, *w = nullptr, *ke = nullptr;  // (the old ones stay if there is no room)
+  if ((rc = dalloc(ctx, &e, n)) || (rc = dalloc(ctx, &w, n)) || (rc = dalloc(ctx, &ke, n))) {
+    cudaGetLastError();
+    for (double* q : {e, w, ke})
+      if (q) cudaFree(q);
     return rc;
+  }
+  for (double* q : {ctx->boxE, ctx->boxW, ctx->boxKE})
+    if (q) cudaFree(q);
+  ctx->boxE = e;
+  ctx->boxW = w;
+  ctx->boxKE = ke;
   ctx->ebuf_steps = steps;
   // every captured graph that names the old energy buffers is stale: the step
   // loop's and the force call's (whose energy variant writes and reads boxE,
@@ -1907,8 +1920,8 @@ int examd_gpu_run(examd_ctx* ctx, int nsteps, double dt, int graph_chunk, double
   const int nb = ctx->nboxes;
   const bool wantE = energies != nullptr;
   int chunk = graph_chunk > 0 ? (graph_chunk + 1) / 2 * 2 : 0;
-  // eager steps' energies wait on the device too, up to kEagerSlots of them
-  const int slots = std::max(chunk, wantE ? kEagerSlots : 1) + 1;
+  // eager steps' energies wait on the device too
+  const int eager = eager_slots(nb), slots = std::max(chunk, wantE ? eager : 1) + 1;
   int rc = ensure_ebuf(ctx, slots, wantE);
   if (rc) return rc;
   if (!ctx->forces_valid) {
@@ -1983,7 +1996,7 @@ int examd_gpu_run(examd_ctx* ctx, int nsteps, double dt, int graph_chunk, double
       if (rc) return rc;
       if (ctx->list && (rc = update_lists(ctx, grew))) return rc;
     } else {
-      if (wantE && held == kEagerSlots && (rc = fetch())) return rc;
+      if (wantE && held >= eager && (rc = fetch())) return rc;
       if (held == 0) first = done;
       rc = step_once(ctx, dt, dt, slot(ctx->boxKE), slot(ctx->boxE), slot(ctx->boxW));
       if (rc) return rc;
@@ -2023,7 +2036,7 @@ int examd_gpu_prepare_run(examd_ctx* ctx, double dt, int graph_chunk, int energi
   if (!ctx->atoms_set) return EXAMD_ERR_STATE;
   cudaSetDevice(ctx->dev);
   const int chunk = graph_chunk > 0 ? (graph_chunk + 1) / 2 * 2 : 0;
-  int rc = ensure_ebuf(ctx, std::max(chunk, energies ? kEagerSlots : 1) + 1, energies != 0);
+  int rc = ensure_ebuf(ctx, std::max(chunk, energies ? eager_slots(ctx->nboxes) : 1) + 1, energies != 0);
   if (rc) return rc;
   if (!ctx->forces_valid) {
     rc = run_pair(ctx, false, false);

@@ -250,3 +250,25 @@ def test_fixed_point_pass_after_a_crowded_tile(gpulib, n, size, before):
         s.run(8, 0.001, graph_chunk=4)
         for a, b in zip(s.state(), state):
             assert np.array_equal(a, b)
+
+
+def test_energies_of_many_boxes(gpulib):
+    """An eager run with energies keeps a few MB of them (4 per array and three steps' more), however many boxes, and
+    gives the energies of a run in graphs."""
+    torch = pytest.importorskip("torch")
+    n = 65535  # (the most whose energies are summed)
+    rng = np.random.default_rng(1)
+    with gpulib.MidpointLJ(np.full((n, 3), 6.25), np.ones(n, dtype=np.int64), precision="mixed") as s:
+        pos, vel = rng.uniform(0.0, 6.25, (n, 3)), rng.normal(size=(n, 3))
+        s.set_atoms(pos, vel=vel)
+        s.run(2, 0.001)
+        free = torch.cuda.mem_get_info()[0]
+        a = s.run(7, 0.001, energies=True)
+        # three arrays of 4 MB and three steps of 0.5 MB, each in 2 MB blocks
+        assert free - torch.cuda.mem_get_info()[0] <= 3 * (4 + 3 * 0.53 + 2) * 2 ** 20
+        s.set_atoms(pos, vel=vel)
+        s.run(2, 0.001)
+        b = s.run(7, 0.001, graph_chunk=2, energies=True)
+    for k in ("ekin", "epot"):
+        assert np.array_equal(a[k], b[k])
+    assert np.allclose(a["ekin"], 0.5 * (vel ** 2).sum(1), rtol=1e-12) and not a["epot"].any()
