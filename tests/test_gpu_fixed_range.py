@@ -273,3 +273,34 @@ def test_overlapping_atoms(gpulib, oracle, tile, apart):
         assert (np.abs(g - ref["forces"]).max(1) <= size).all()
     assert e[0] == pytest.approx(ref["epot"], rel=TOL64) and w[0] == pytest.approx(ref["virial"], rel=TOL64)
     assert cnt["candidates"] == ref["counts"].candidates and cnt["accepted"] == ref["counts"].accepted
+
+
+@pytest.mark.parametrize("sigma", [500.0, 1.0, 1e-4])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_pruning_at_the_ends_of_fp16(gpulib, oracle, precision, sigma):
+    """The enumeration prunes cells on FP16 gaps: lengths whose squares are beyond FP16's largest number and below its
+    smallest, atoms on and next to the cells' faces.  The same pairs as the oracle, which prunes nothing."""
+    rng = np.random.default_rng(4)
+    L = np.array([11.3, 12.5, 13.7]) * sigma
+    h = 1.25 * sigma
+    unit = 2.0 ** (np.floor(np.log2(h)) - 13)
+    edge = float(np.ceil(h / unit) * unit)
+    pos = gpulib.gen_random(1200, L / sigma, 0.85, 6) * sigma
+    k = rng.integers(0, 1200, 500)
+    a = rng.integers(0, 3, 500)
+    pos[k, a] = np.floor(pos[k, a] / edge) * edge + rng.choice([0.0, 1e-9, -1e-9, 1e-6, -1e-6], 500) * sigma
+    pos %= L
+    from scipy.spatial import cKDTree
+    close = cKDTree(pos, boxsize=L).query_pairs(0.8 * sigma, output_type="ndarray")
+    keep = np.ones(len(pos), dtype=bool)
+    keep[close[:, 1]] = False
+    pos = np.ascontiguousarray(pos[keep])
+    lj = dict(eps=sigma, sigma=sigma)  # forces of about 1
+    ref = oracle.forces_typed(pos, L, 2.5 * sigma, threads=0, block_length=edge, **lj)
+    with gpulib.MidpointLJ(L, [len(pos)], precision=precision, rc=2.5 * sigma, **lj) as s:
+        s.set_atoms(pos)
+        f = s.forces()[0]
+        cnt = s.counters()
+    assert cnt["candidates"] == ref["counts"].candidates and cnt["accepted"] == ref["counts"].accepted
+    d, fr = np.sqrt(((f - ref["forces"]) ** 2).sum(1)), np.sqrt((ref["forces"] ** 2).sum(1).mean())
+    assert d.max() <= TOL64 * fr if precision == "fp64" else np.sqrt((d * d).mean()) <= 1e-5 * fr
