@@ -1113,6 +1113,7 @@ int apply_capacity(examd_ctx* ctx, bool* grew = nullptr) {
   PairConfig pc = ctx->pc;  // (the context changes only once a choice fits)
   int cap = 0, redo = 0, bytes = 0;
   auto fits = [&] {
+    pc.own_global = pair_own_global(pc, cap, ctx->ne_max, ctx->ext_max, ctx->sm_smem);
     bytes = pair_smem_bytes(pc, cap, redo, ctx->ne_max, ctx->ext_max);
     return bytes <= ctx->smem_limit && (!pc.fix || cap <= ctx->fx.atoms);
   };
@@ -1123,6 +1124,7 @@ int apply_capacity(examd_ctx* ctx, bool* grew = nullptr) {
     // The fixed-point pass (78 bytes an atom) with half the headroom where the whole of it costs a CTA per SM (1M
     // liquid 949 -> 844 us a pass, 500k at rc 3.0 719 -> 639)
     if (pc.fix) {
+      pc.own_global = !pc.multi;
       const int least = up8(occ + occ / 32 + 16);
       const int n = pair_ctas(pc, least, ctx->ne_max, ctx->ext_max, ctx->sm_smem);
       while (cap > least && pair_ctas(pc, cap, ctx->ne_max, ctx->ext_max, ctx->sm_smem) < n) cap -= 8;
@@ -1160,6 +1162,7 @@ int apply_capacity(examd_ctx* ctx, bool* grew = nullptr) {
       CK(pair_prepare(pc, ctx->smem_limit));
     }
   ctx->pc.fix = pc.fix;
+  ctx->pc.own_global = pc.own_global;
   ctx->cap = cap;
   ctx->cap_redo = redo;
   ctx->smem = bytes;

@@ -5,10 +5,12 @@
 // per-block linked lists built once by exaMD_particles_generate /
 // exaMD_read_particles (SRC/exaMD_input_formats.f90:66-92, 169-192).  Cells
 // come in the reference's (z, y, x) block order; inside a cell the atoms keep
-// the order in which the counting pass drew their slots.  Neither form's
-// results depend on that order: the mixed form's force and energy sums are
-// exact fixed point and each pair's FP32 term is antisymmetric in its two
-// atoms, and the FP64 form's first pass sums exact integers.
+// the order in which the counting pass drew their slots.  The forces do not
+// depend on that order: the mixed form's force and energy sums are exact fixed
+// point and each pair's FP32 term is antisymmetric in its two atoms, and the
+// FP64 form's first pass sums exact integers.  The FP64 form's energies and
+// virials, and the forces of tiles computed by its FP64 body, are FP64 sums whose
+// last bits do depend on it; so do the rare large terms of the mixed form.
 // HBM-bound work.
 #include "common.cuh"
 #include "kernels.cuh"

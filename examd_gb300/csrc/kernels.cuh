@@ -146,6 +146,7 @@ struct PairConfig {
   bool list = false;    // mixed form: pair-list mode (forces from the per-tile lists)
   bool cut = true;      // list pass: the potential's own range is finite (WCA) and tested
   bool fine = false;    // FP64 form: finer work units (grids of few waves)
+  bool own_global = false;  // fixed-point pass: the ownership table in global memory
   bool chain = false;   // the pair and redo passes as chained launches
   bool wide = false;    // mixed form without lists: the enumeration with 12 warps per CTA
   int warps = 8;
@@ -156,6 +157,8 @@ struct PairConfig {
 int pair_smem_bytes(const PairConfig& cfg, int cap, int cap_redo, int ne_max, int ext_max);
 // CTAs of the fixed-point pass that an SM's sm_smem bytes of shared memory and its registers hold.
 int pair_ctas(const PairConfig& cfg, int cap, int ne_max, int ext_max, int sm_smem);
+// Whether it holds more of them with the ownership table in global memory.
+bool pair_own_global(PairConfig cfg, int cap, int ne_max, int ext_max, int sm_smem);
 cudaError_t pair_prepare(const PairConfig& cfg, int smem_bytes);  // opt-in smem attribute
 cudaError_t launch_pair(const PairConfig& cfg, const PairArgs& a, int ntiles, int smem_bytes, cudaStream_t st);
 // Pair-list mode: build the per-tile lists (gated by a.gate).

@@ -145,7 +145,7 @@ __host__ __device__ inline int align16(int x) { return (x + 15) & ~15; }
 // queues, no ownership table: the queue region holds only the scan and
 // reduction scratch; kListBig's fr after everything).
 // ne_max, ext_max: the largest tile's ext cells and ext extent on one axis.
-// own: with a copy of the ownership table (see own_in_global).
+// own: with a copy of the ownership table (see pair_own_global).
 __host__ __device__ inline Layout make_layout(bool fp64, int cap, int ne_max, int ext_max, int nw, int mode,
                                               bool multi, bool own = true) {
   const bool from_list = mode == kList || mode == kListBig;
@@ -198,18 +198,6 @@ __host__ __device__ inline Layout make_layout(bool fp64, int cap, int ne_max, in
   return L;
 }
 
-// The FP64 form's first pass with one type, in grids of many waves, reads the
-// ownership table from global memory (its lines stay in L1) instead of a copy
-// of 3.4 KB in each CTA: a tile of 78 bytes an atom is near the size at which
-// an SM holds three CTAs instead of four (528 atoms at 8 warps with the copy, 572
-// without, at 4^3 cells; 1M liquid, 951 -> 846 us a pass; 256k 249 -> 220).  In few waves there is no
-// fourth CTA to gain and the copy is nearer (1,000 atoms 9.5 against 10 us; a
-// 512-box ensemble, many waves at four CTAs either way, loses 1 %); with several
-// types the registers allow three.
-__host__ __device__ constexpr bool own_in_global(bool fix, bool multi, int parts) {
-  return fix && !multi && parts == kUnitParts;
-}
-
 static int redo_smem_bytes(const PairConfig& cfg, int cap_redo, int ne_max, int ext_max) {
   if (cfg.fix) return make_layout(true, cap_redo, ne_max, ext_max, cfg.warps, kRedoFull, cfg.multi).bytes;
   const int b = std::max(make_layout(false, cap_redo, ne_max, ext_max, cfg.warps, kRedoBig, cfg.multi).bytes,
@@ -226,8 +214,7 @@ static int main_smem_bytes(const PairConfig& cfg, int cap, int ne_max, int ext_m
   const int mode = (cfg.list && !cfg.count && !cfg.fp64) ? kList : kMain;
   if (cfg.fix)  // (and the FP64 body in the same CTA)
     return std::max(make_layout(true, cap, ne_max, ext_max, cfg.warps, kMain, cfg.multi).bytes,
-                    make_layout(false, cap, ne_max, ext_max, cfg.warps, kFixed, cfg.multi,
-                                !own_in_global(true, cfg.multi, cfg.fine && !cfg.count ? kFineParts : kUnitParts)).bytes);
+                    make_layout(false, cap, ne_max, ext_max, cfg.warps, kFixed, cfg.multi, !cfg.own_global).bytes);
   if (uses_wide(cfg)) return make_layout(false, cap, ne_max, ext_max, kWideWarps, kMain, cfg.multi).bytes;
   return make_layout(cfg.fp64, cap, ne_max, ext_max, cfg.warps, mode, cfg.multi).bytes;
 }
@@ -250,6 +237,21 @@ int pair_ctas(const PairConfig& cfg, int cap, int ne_max, int ext_max, int sm_sm
   constexpr int kReserved = 1024;  // of every CTA, by the system
   const int regs = 32 * cfg.warps * (cfg.multi ? 80 : 64);
   return std::min(sm_smem / (main_smem_bytes(cfg, cap, ne_max, ext_max) + kReserved), 65536 / regs);
+}
+
+// The FP64 form's first pass with one type reads the ownership table from global
+// memory (its lines stay in L1) where a copy of 3.4 KB in each CTA would cost one
+// of the SM's CTAs: at 78 bytes an atom an SM holds four of 528 atoms with the
+// copy and of 572 without (8 warps, 4^3 cells; 1M liquid, 568: 951 -> 846 us a
+// pass; 87,808 atoms, 536: 100 -> 92).  Elsewhere the copy is nearer (1,000 atoms 9.5
+// against 10 us, a 512-box ensemble 1 %); with several types the registers allow
+// three either way.
+bool pair_own_global(PairConfig cfg, int cap, int ne_max, int ext_max, int sm_smem) {
+  if (!cfg.fix || cfg.multi) return false;
+  cfg.own_global = false;
+  const int n = pair_ctas(cfg, cap, ne_max, ext_max, sm_smem);
+  cfg.own_global = true;
+  return pair_ctas(cfg, cap, ne_max, ext_max, sm_smem) > n;
 }
 
 // Exact sum of FP32 terms in 64-bit fixed point (2^-32 resolution): the total
@@ -621,7 +623,9 @@ __device__ __forceinline__ void force_batch_fix(int cnt, int q0, const QK& qk, c
 // - kListBig: kRedoBig from the list.
 // kFixed: returns true, nothing written, for a tile with a term too large.
 // CUT (list pass): the potential's own range rcut2 is tested (WCA; infinite otherwise).
-template <bool FP64, bool MULTI, bool ENERGY, bool COUNT, int MODE, bool CUT = true, int kParts = kUnitParts>
+// kOwnGlobal: the ownership table in global memory.
+template <bool FP64, bool MULTI, bool ENERGY, bool COUNT, int MODE, bool CUT = true, int kParts = kUnitParts,
+          bool kOwnGlobal = false>
 __device__ __forceinline__ bool pair_tile(const PairArgs& A, const int tile) {
   extern __shared__ __align__(16) unsigned char smem[];
   const unsigned FULL = 0xffffffffu;
@@ -638,7 +642,6 @@ __device__ __forceinline__ bool pair_tile(const PairArgs& A, const int tile) {
   if (kFromList && MODE == kList && A.lcount[tile] < 0) return false;  // a fallback tile: the redo pass computes it
   constexpr bool FIX = MODE == kFixed;
   const int cap = (MODE == kMain || MODE == kListBuild || MODE == kList || FIX) ? A.cap : A.cap_redo;
-  constexpr bool kOwnGlobal = own_in_global(FIX, MULTI, kParts);
   const Layout L = make_layout(FP64, cap, A.ne_max, A.ext_max, nw, MODE, MULTI, !kOwnGlobal);
   // shared-memory arrays (index-checked in the checked build)
   int* const st = A.status;  // the index checks' status word (checked build)
@@ -1792,10 +1795,10 @@ __global__ void __launch_bounds__(32 * kWideWarps, 3) k_pair_wide(const PairArgs
 // (131,072 atoms at random, density 0.5, no least distance: 376 us a pass, 352 by
 // the FP64 body alone; 942 where such tiles were finished here first and then
 // listed for k_pair_redo64, one CTA an SM).
-template <bool MULTI, bool ENERGY, bool COUNT, int PARTS>
+template <bool MULTI, bool ENERGY, bool COUNT, int PARTS, bool OWNG>
 __global__ void __launch_bounds__(256, MULTI ? 3 : 4) k_pair_fix(const PairArgs A) {
   const int tile = A.order[blockIdx.x];
-  if (pair_tile<false, MULTI, ENERGY, COUNT, kFixed, true, PARTS>(A, tile)) {
+  if (pair_tile<false, MULTI, ENERGY, COUNT, kFixed, true, PARTS, OWNG>(A, tile)) {
     __syncthreads();
     pair_tile<true, MULTI, ENERGY, COUNT, kMain>(A, tile);
   }
@@ -1882,12 +1885,14 @@ static void* pick_enum(const PairConfig& c) {
 // enumeration counts) the list pass.
 static bool uses_list(const PairConfig& c) { return c.list && !c.fp64 && !c.count; }
 
-template <bool MULTI>
+template <bool MULTI, bool OWNG>
 static void* pick_fix(const PairConfig& c) {
   constexpr int P = kUnitParts, F = kFineParts;
-  if (c.count) return c.energy ? (void*)&k_pair_fix<MULTI, true, true, P> : (void*)&k_pair_fix<MULTI, false, true, P>;
-  if (c.fine) return c.energy ? (void*)&k_pair_fix<MULTI, true, false, F> : (void*)&k_pair_fix<MULTI, false, false, F>;
-  return c.energy ? (void*)&k_pair_fix<MULTI, true, false, P> : (void*)&k_pair_fix<MULTI, false, false, P>;
+  if (c.count)
+    return c.energy ? (void*)&k_pair_fix<MULTI, true, true, P, OWNG> : (void*)&k_pair_fix<MULTI, false, true, P, OWNG>;
+  if (c.fine)
+    return c.energy ? (void*)&k_pair_fix<MULTI, true, false, F, OWNG> : (void*)&k_pair_fix<MULTI, false, false, F, OWNG>;
+  return c.energy ? (void*)&k_pair_fix<MULTI, true, false, P, OWNG> : (void*)&k_pair_fix<MULTI, false, false, P, OWNG>;
 }
 
 template <bool MULTI>
@@ -1901,7 +1906,7 @@ static void* pick(const PairConfig& c) {
     if (c.multi) return c.energy ? (void*)&k_pair_wide<true, true> : (void*)&k_pair_wide<true, false>;
     return c.energy ? (void*)&k_pair_wide<false, true> : (void*)&k_pair_wide<false, false>;
   }
-  if (c.fix) return c.multi ? pick_fix<true>(c) : pick_fix<false>(c);
+  if (c.fix) return c.multi ? pick_fix<true, false>(c) : c.own_global ? pick_fix<false, true>(c) : pick_fix<false, false>(c);
   if (uses_list(c)) {
     if (c.cut) {
       if (c.multi) return c.energy ? (void*)&k_pair_list<true, true, true> : (void*)&k_pair_list<true, false, true>;
