@@ -310,6 +310,7 @@ struct examd_ctx {
   bool fix = false;     // the system has a fixed-point pass (pc.fix: the present capacities leave room for it)
   int cap = 0, smem = 0, smem_limit = 0, sm_smem = 0;
   int cap_redo = 0;     // staged-atom capacity of the redo pass
+  bool whole_headroom = false;  // never half of it (see keep_headroom)
   int dev = 0;
   cudaStream_t st = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr, e3 = nullptr;
@@ -1123,7 +1124,7 @@ int apply_capacity(examd_ctx* ctx, bool* grew = nullptr) {
     cap = pc.fp64 && !pc.fix ? redo : up8(occ + occ / 16 + 32);
     // The fixed-point pass (78 bytes an atom) with half the headroom where the whole of it costs a CTA per SM (1M
     // liquid 949 -> 844 us a pass, 500k at rc 3.0 719 -> 639)
-    if (pc.fix) {
+    if (pc.fix && !ctx->whole_headroom) {
       pc.own_global = !pc.multi;
       const int least = up8(occ + occ / 32 + 16);
       const int n = pair_ctas(pc, least, ctx->ne_max, ctx->ext_max, ctx->sm_smem);
@@ -1567,6 +1568,13 @@ int forces_common(examd_ctx* ctx, double* forces, double* epot, double* virial, 
 }  // namespace
 
 extern "C" {
+
+// For the autotuner's trials on one configuration: a shape that keeps its CTAs per
+// SM only with half the headroom loses one as soon as the atoms move on (the 16.8M
+// mixture, tuned on its lattice, took tiles of 6x4x4 that way, whose 800 atoms
+// later left two CTAs an SM: 8.2e8 atom-steps/s in FP64, 9.8e8 in the 5x4x4 that
+// the trials now pick).
+__attribute__((visibility("hidden"))) void examd_keep_headroom(examd_ctx* ctx) { ctx->whole_headroom = true; }
 
 int examd_gpu_set_atoms(examd_ctx* ctx, int64_t n, const double* pos, const int* type, const double* vel) {
   if (!ctx || (n > 0 && !pos) || n != ctx->N) return EXAMD_ERR_ARG;

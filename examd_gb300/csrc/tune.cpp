@@ -39,6 +39,8 @@
 
 #include "../../include/examd_gb300.h"
 
+extern "C" __attribute__((visibility("hidden"))) void examd_keep_headroom(examd_ctx* ctx);  // api.cu
+
 namespace {
 
 constexpr int kReps = 3;
@@ -149,6 +151,7 @@ extern "C" int examd_autotune(const examd_params* params, int nboxes, const exam
   auto time_one = [&](const examd_params& p, double* t) {
     examd_ctx* ctx = nullptr;
     int rc = examd_gpu_create(&p, nboxes, boxes, &ctx);
+    if (rc == EXAMD_OK) examd_keep_headroom(ctx);
     if (rc == EXAMD_OK) rc = examd_gpu_set_atoms(ctx, n, pos, type, nullptr);
     if (rc == EXAMD_OK) rc = examd_gpu_time_forces(ctx, kReps, nullptr, t);
     if (rc == EXAMD_OK && p.pair_skin > 0.0) {  // the score: a step's share of a rebuild too
