@@ -28,7 +28,7 @@
 // shared-memory atomics (compare-and-swap loops) rarely hit one address.
 //
 // What bounds the passes (1M liquid): the enumeration and the FP64 pass issue
-// (73-81 % of the slots; ALU pipe 50 %); the list pass issue and shared memory
+// (71-81 % of the slots; ALU pipe 50 %); the list pass issue and shared memory
 // (70 %; half of the wavefronts atomics); none of them DRAM (0.1-0.9 TB/s).
 //
 // Accumulation.  Mixed form: each per-atom force component is an exact 32-bit
@@ -467,7 +467,7 @@ __device__ __forceinline__ void force_batch64(int cnt, const QK& qk, const PD& p
 //   modulo 2^64 (the low one with carry into the high one) and a coarse one:
 //   exact, in any order, whatever the number of terms.
 // An isolated pair's force is then off by less than the FP64 body's, RMS (1e-16:
-// r 0.9-1.1 sigma 9.1 against 11.5; 2.0-2.5 2.9 / 3.6; at rc 3.8 3.5 / 3.6; a pair of
+// r 0.9-1.1 sigma 9.0 against 11.5; 2.0-2.5 2.9 / 3.6; at rc 4.6 3.4 / 3.7; a pair of
 // a sixteenth of the strongest eps 3.1 / 3.6), and the forces do not depend on
 // the order.  Where the reference itself rounds coarsely, its rounding is kept: a
 // pair across the periodic face is first subtracted at box scale (x_j - x_i,
@@ -476,7 +476,7 @@ __device__ __forceinline__ void force_batch64(int cnt, const QK& qk, const PD& p
 // A pair within a unit of D's high word (a few 1e-9) of its range is decided on
 // the FP64 body's own r^2 (in64), so that both accept the same pairs; a pair
 // whose force is too large for the sums' range flags the tile, and the FP64
-// body redoes it.
+// body computes it.
 template <bool MULTI, bool ENERGY, bool COUNT, class QK, class PX, class FA, class FACE, class IN64>
 __device__ __forceinline__ void force_batch_fix(int cnt, int q0, const QK& qk, const PX& px, FA& fa, int cap,
                                                 const PairArgs& A, const FixPair* ljx, double& esum, double& wsum,

@@ -85,7 +85,8 @@ typedef struct examd_params {
    * SRC/exaMD_module.f90:109-113). */
   double cell_edge;
   int tile[3];        /* home cells per CTA tile per axis; 0 = default (4; in */
-                      /* the FP64 form 3 or 2 for systems of few tiles)       */
+                      /* the FP64 form 3 or 2 for systems of few tiles, and 3 */
+                      /* for long cutoffs)                                    */
   int warps;          /* warps per CTA in the pair kernel; 0 = default        */
   int strict_box;     /* 1: positions outside [0,L) are an error (109);       */
                       /* 0: they are wrapped periodically                     */
