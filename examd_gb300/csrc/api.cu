@@ -153,7 +153,7 @@ long long fixed_of(double x, int ue) {
 
 // The tables of the FP64 form's fixed-point pass (pair.cu, force_batch_fix), or
 // false where the parameters do not suit it and the FP64 body computes every
-// tile: pairs whose force at their cutoff falls below 2^-11 of the largest force
+// tile: pairs whose force at their cutoff falls below 2^-13 of the largest force
 // scale eps / sigma (the sums' one unit would hold it to fewer bits than FP64
 // does), pairs so small beside the longest cutoff (sigma below about a sixth of
 // it), whose square is below 2^62 units, that their r^2 has less than FP64's bits
@@ -180,7 +180,7 @@ bool build_fix(const LJTable& lj, const examd_params& p, double bl, FixTable& fx
   fx.sf = unit->bits - f0;
   fx.coarse = unit->coarse;
   fx.atoms = unit->atoms;
-  const double fbig = std::ldexp(1.0, kFixTermBits + f0);
+  const double fbig = std::ldexp(1.0, unit->term + f0);
   const int w = 2 * fx.ue + 64;  // r^2 = D 2^w
   double r2big[EXAMD_MAX_TYPES * EXAMD_MAX_TYPES];
   double gmax = 0.0;
@@ -242,7 +242,10 @@ int split_axis(int nb, double last_width, int tile_len, int balance, int* starts
 // 100 / 98.)  Also 3 where a tile of 4^3 is too large for three CTAs on an SM
 // (about 820 atoms with the headroom; expected from the mean density, the wide
 // last cell and three standard deviations): 1M liquid, 4^3 / 3^3: rc 3.0 1561 /
-// 1309, 500k at rc 3.0 764 / 639; below it, rc 2.75 1000 / 1151, rc 2.5 844 / 1027.
+// 1309, 500k at rc 3.0 764 / 639; below it, rc 2.75 1000 / 1151, rc 2.5 844 / 1027;
+// and 2 where one of 3^3 would have more atoms than the fixed-point pass takes at
+// such cutoffs (1M at rc 5, 3^3 / 2^3: 59.3
+// ms by the FP64 body / 10.7).
 // The mixed form keeps 4: its FP32 x coordinates are the tile's.
 int default_tile(const examd_params& p, int nboxes, const examd_box* boxes, double bl, int sms) {
   if (p.precision != EXAMD_FP64) return 4;
@@ -255,16 +258,19 @@ int default_tile(const examd_params& p, int nboxes, const examd_box* boxes, doub
     }
     return n;
   };
-  if (tiles(4) < 4.0 * sms) return tiles(3) >= sms ? 3 : 2;
-  for (int b = 0; b < nboxes; ++b) {
-    double atoms = (double)boxes[b].natoms;  // staged by the largest tile
-    for (int a = 0; a < 3; ++a) {
-      const double cells = boxes[b].L[a] / bl;
-      atoms *= std::min(1.0, (4 + 2 + (cells - std::floor(cells))) / cells);
+  double most[2] = {0.0, 0.0};  // staged by the largest tile of 3^3 and of 4^3 cells
+  for (int b = 0; b < nboxes; ++b)
+    for (int t = 3; t <= 4; ++t) {
+      double atoms = (double)boxes[b].natoms;
+      for (int a = 0; a < 3; ++a) {
+        const double cells = boxes[b].L[a] / bl;
+        atoms *= std::min(1.0, (t + 2 + (cells - std::floor(cells))) / cells);
+      }
+      most[t - 3] = std::max(most[t - 3], (atoms + 3.0 * std::sqrt(atoms)) * 1.0625 + 32.0);
     }
-    if ((atoms + 3.0 * std::sqrt(atoms)) * 1.0625 + 32.0 > 820.0) return 3;
-  }
-  return 4;
+  int t = most[1] <= 820.0 ? 4 : 3;
+  if (tiles(4) < 4.0 * sms) t = tiles(3) >= sms ? 3 : 2;
+  return t == 3 && most[0] > kFixUnits[2].atoms ? 2 : t;
 }
 
 }  // namespace

@@ -119,22 +119,23 @@ struct LJ32 {
 // component of a kept term is below 2^28 in fixed point, so a component's
 // int32 sum needs more than 8 near-maximal terms of one sign to overflow.
 constexpr float kFixMaxForce = 2048.f;
-// FP64 form's fixed-point pass.  Terms below 2^kFixTermBits F0 (r > 0.74 sigma) are
-// kept, F0 the power of two at or above the largest eps / sigma; a larger one
-// sends the tile to the FP64 body.  A component's sum is held modulo 2^64 in two
+// FP64 form's fixed-point pass.  Terms below 2^term F0 (r > 0.74 sigma at 11 bits,
+// 0.82 at 9) are kept, F0 the power of two at or above the largest eps / sigma; a
+// larger one sends the tile to the FP64 body.  A component's sum is held modulo 2^64 in two
 // words and once more in a third, in coarse steps, which says which multiple of
 // 2^64 it is: the third word's rounding (0.6 of a step per term at most) leaves the
 // sum known to 2^63, and its 31 bits hold every term of a tile's most atoms, so
 // that no number of terms on one atom can overflow a sum.  The unit is as fine as
 // the weakest pair needs to keep FP64's relative accuracy, alone at its cutoff:
-// unit bits below F0, the weakest force (bits below F0) that it serves, the step's
-// bits above the unit, most atoms.
+// unit bits below F0, terms' bits above it, the weakest force (bits below F0) that
+// it serves, the step's bits above the unit, most atoms (0.6 2^coarse atoms < 2^63
+// and 2^(term + bits) atoms < 2^(31 + coarse)).
 struct FixUnit {
-  int bits, weak, coarse, atoms;
+  int bits, term, weak, coarse, atoms;
 };
-constexpr int kFixTermBits = 11;
-constexpr FixUnit kFixUnits[2] = {{60, 9, 52, 3400},   // one type: rc <= 3.8 sigma
-                                  {62, 11, 53, 1700}}; // 4.6 sigma
+constexpr FixUnit kFixUnits[3] = {{60, 11, 9, 52, 3400},   // one type: rc <= 3.8 sigma
+                                  {62, 11, 11, 53, 1700},  // 4.6 sigma
+                                  {64, 9, 13, 53, 1700}};  // 5.7 sigma
 struct LJ64 {
   double sig2, eps24, eps4, rc2;   // as user_func.f90:58-59 computes them
   double rcut2, eshift;
@@ -147,7 +148,7 @@ struct FixPair {
   double c6, c12;
   double e4, s6;    // energy: 4 eps, and sigma^6 in units of D^3
   double eshift;
-  int limh, bigh;   // high words of D at the range (rc or the potential's own) and at forces of 2^tb F0
+  int limh, bigh;   // high words of D at the range (rc or the potential's own) and at forces of 2^term F0
   float pre;        // FP32 prefilter of the candidates: rc^2 widened
 };
 
